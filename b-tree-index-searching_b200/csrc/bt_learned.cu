@@ -35,6 +35,7 @@
 #include <atomic>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "bt_search.cuh"
@@ -64,10 +65,9 @@ void free_learned(LearnedState *s) {
 
 namespace {
 
-constexpr uint64_t kPlaChunk = 1ull << 14;  // keys per segmentation thread
-constexpr int kHullCap = 32;                 // points per convex hull
+constexpr uint64_t kPlaChunk = 1ull << 14;  // keys per segmentation warp
+constexpr int kHullCap = 32;                 // points per convex hull (one per lane)
 constexpr int kPlaThreads = 64;              // segmentation threads per CTA
-constexpr int kPlaHullStride = 2 * kHullCap + 1;  // hull points per thread in shared memory
 constexpr size_t kStageBudget = 160 * 1024;  // shared memory for the staged keys
 constexpr int kMaxWalk = 8;                  // extra units read before the full descent
 // Search CTA shapes (one CTA per SM: the staged keys), bt_learned_set_shape:
@@ -158,13 +158,6 @@ struct PlaPt {
     int64_t y;   // rank - segment's first rank, +/- eps
 };
 
-// > 0 when b lies above the directed line o -> a (x increasing); exact.
-__device__ __forceinline__ __int128 pla_cross(const PlaPt &o, const PlaPt &a, const PlaPt &b) {
-    const __int128 ax = (__int128)a.x - (__int128)o.x, bx = (__int128)b.x - (__int128)o.x;
-    const __int128 ay = (__int128)a.y - (__int128)o.y, by = (__int128)b.y - (__int128)o.y;
-    return ax * by - ay * bx;
-}
-
 // Slope of the line through a and b and its value at x = 0, in double with
 // explicit rounding (no contraction); flat for two points of one key.
 __device__ __forceinline__ double pla_line_at0(const PlaPt &a, const PlaPt &b, double *slope) {
@@ -178,8 +171,33 @@ __device__ __forceinline__ double pla_line_at0(const PlaPt &a, const PlaPt &b, d
     return __dsub_rn(__ll2double_rn(a.y), __dmul_rn(sl, __ull2double_rn(a.x)));
 }
 
+// Number types of one chunk's segmentation.  Narrow: the chunk's keys span
+// less than 2^31 and eps is at most kPlaNarrowEps, so key offsets, rank
+// offsets +/- eps and their differences fit 32 bits and a cross product's two
+// terms stay below 2^62 each.  Wide: any keys and any eps, 128-bit products.
+constexpr uint32_t kPlaNarrowEps = 1u << 29;
+struct PlaNarrow {
+    using X = uint32_t;   // key - the chunk's first key
+    using Y = int32_t;    // rank in the chunk, +/- eps
+    using W = long long;  // cross products
+};
+struct PlaWide {
+    using X = unsigned long long;
+    using Y = long long;
+    using W = __int128;
+};
+
+// Cross product of the vectors (ax, ay) and (bx, by), ax, bx >= 0: > 0 when
+// b points above a.  Exact (see the number types).
+template <typename T>
+__device__ __forceinline__ typename T::W pla_cross(typename T::X ax, typename T::Y ay,
+                                                   typename T::X bx, typename T::Y by) {
+    using W = typename T::W;
+    return (W)ax * (W)by - (W)ay * (W)bx;
+}
+
 // Error-bounded segmentation of the points (key[i], i) of one chunk of
-// kPlaChunk keys, one thread per chunk: greedy maximal segments, each with a
+// kPlaChunk keys, one warp per chunk: greedy maximal segments, each with a
 // line within eps of all its points (the optimal streaming fit of O'Rourke,
 // CACM 1981, as in the PGM-index, Ferragina & Vinciguerra, VLDB 2020).  An
 // open segment keeps the upper convex hull of its lower points (x, y - eps),
@@ -190,84 +208,198 @@ __device__ __forceinline__ double pla_line_at0(const PlaPt &a, const PlaPt &b, d
 // COUNT: counts[c] = segments of chunk c.  Otherwise writes segment k of
 // chunk c at offsets[c] + k: first rank and the mean of M and N as
 // rank - first = icpt + slope * (key - first key).
-template <typename K, typename V, bool COUNT>
-__global__ void pla_kernel(const unsigned char *__restrict__ leaves, uint64_t n, uint32_t eps,
-                           uint64_t nchunks, uint64_t *__restrict__ counts,
-                           const uint64_t *__restrict__ offsets, uint32_t *__restrict__ starts,
-                           double *__restrict__ slopes, double *__restrict__ icpts) {
-    const uint64_t c = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (c >= nchunks) return;
-    // the two hulls of this thread in shared memory (kPlaHullStride points
-    // apart per thread: the padding spreads the threads over the banks)
-    extern __shared__ PlaPt pla_sh[];
-    PlaPt *lh = pla_sh + (size_t)threadIdx.x * kPlaHullStride;
-    PlaPt *uh = lh + kHullCap;
-    const int64_t e = (int64_t)eps;
-    const uint64_t end = min(n, (c + 1) * kPlaChunk);
-    uint64_t nseg = 0, out = COUNT ? 0 : offsets[c];
-    uint64_t i = c * kPlaChunk;
-    while (i < end) {
-        const uint64_t s = i;
-        const uint64_t x0 = (uint64_t)leaf_key<K, V>(leaves, s);
-        int nl = 1, nu = 1;
-        lh[0] = {0, -e};
-        uh[0] = {0, e};
-        PlaPt Ma = lh[0], Mb = uh[0], Na = uh[0], Nb = lh[0];
-        uint64_t j = s + 1;
-        if (j < end) {
-            const PlaPt L = {(uint64_t)leaf_key<K, V>(leaves, j) - x0, 1 - e};
-            const PlaPt U = {L.x, 1 + e};
-            Mb = U;
-            Nb = L;
-            lh[nl++] = L;
-            uh[nu++] = U;
-            for (j = s + 2; j < end; j++) {
-                const int64_t y = (int64_t)(j - s);
-                const uint64_t x = (uint64_t)leaf_key<K, V>(leaves, j) - x0;
-                const PlaPt L2 = {x, y - e}, U2 = {x, y + e};
-                if (pla_cross(Ma, Mb, L2) > 0 || pla_cross(Na, Nb, U2) < 0) break;
-                int nl2 = nl, nu2 = nu;
-                while (nl2 >= 2 && pla_cross(lh[nl2 - 2], lh[nl2 - 1], L2) >= 0) nl2--;
-                while (nu2 >= 2 && pla_cross(uh[nu2 - 2], uh[nu2 - 1], U2) <= 0) nu2--;
-                if (nl2 >= kHullCap || nu2 >= kHullCap) break;
-                if (pla_cross(Ma, Mb, U2) < 0) {  // M now pivots on U2
-                    int b = 0;
-                    for (int k = 1; k < nl; k++)
-                        if (pla_cross(lh[b], U2, lh[k]) > 0) b = k;
-                    Ma = lh[b];
-                    Mb = U2;
+//
+// The fit is a chain of 2^14 dependent points per chunk, bound by its
+// instructions and their latency (the keys are read once, coalesced, a batch
+// ahead).  What one point needs is spread over the warp:
+//  * point k of either hull is in lane k (kHullCap = 32), with the edge from
+//    point k - 1.  A new point pops a hull's tail: every lane tests its own
+//    edge, a ballot shows the last edge that stays.  The edge into the new
+//    point's slot starts at the point before it: the lane's own old one when
+//    points were popped, else the point pushed last.
+//  * a batch of 32 points is tested against M and N by its 32 lanes at once;
+//    the ballots hold until M or N moves.
+//  * M (N) pivots on the hull point of least (largest) slope to the new
+//    point: along a convex chain the steps that improve it come first, so
+//    one ballot of the edges counts them.
+// The two hulls are those of the points themselves: moving all y by eps
+// changes no cross product.  One thread per chunk, its hulls in shared
+// memory and 128-bit products, took 80 ms per pass at 2^26 keys and 110 at
+// 2^28 (lanes of a warp in different loops).
+template <typename K, typename V, bool COUNT, typename T>
+__device__ __forceinline__ void pla_chunk(const unsigned char *__restrict__ leaves, uint64_t base,
+                                          uint32_t m, uint64_t key0, uint32_t eps, uint64_t c,
+                                          uint64_t *__restrict__ counts,
+                                          const uint64_t *__restrict__ offsets,
+                                          uint32_t *__restrict__ starts,
+                                          double *__restrict__ slopes, double *__restrict__ icpts) {
+    using X = typename T::X;
+    using Y = typename T::Y;
+    const int lane = threadIdx.x & 31;
+    const Y e = (Y)eps;
+    uint64_t out = COUNT ? 0 : offsets[c];
+    uint32_t nseg = 0;
+    // hull point `lane` and the edge into it from point lane - 1
+    X lx = 0, lex = 0, ux = 0, uex = 0;
+    Y ly = 0, ley = 0, uy = 0, uey = 0;
+    int nl = 0, nu = 0;              // hull sizes
+    X mx = 0, mdx = 0, nx = 0, ndx = 0;  // Ma, Mb - Ma, Na, Nb - Na
+    Y my = 0, mdy = 0, ny = 0, ndy = 0;
+    uint32_t s = 0;                  // the open segment's first point
+    X sx = 0, qx = 0;                // its key offset; that of the point pushed last
+    uint32_t in_seg = 0;             // points of the open segment
+    auto close = [&](uint32_t j) {   // the open segment ends before point j
+        if constexpr (!COUNT) {
+            if (lane == 0) {
+                double sl = 0.0, ic = 0.0;
+                if (in_seg >= 2) {
+                    const PlaPt Ma = {(uint64_t)(mx - sx), (int64_t)my - (int64_t)s};
+                    const PlaPt Mb = {(uint64_t)(mx + mdx - sx), (int64_t)(my + mdy) - (int64_t)s};
+                    const PlaPt Na = {(uint64_t)(nx - sx), (int64_t)ny - (int64_t)s};
+                    const PlaPt Nb = {(uint64_t)(nx + ndx - sx), (int64_t)(ny + ndy) - (int64_t)s};
+                    double sm, sn;
+                    const double m0 = pla_line_at0(Ma, Mb, &sm);
+                    const double n0 = pla_line_at0(Na, Nb, &sn);
+                    sl = __dmul_rn(__dadd_rn(sm, sn), 0.5);
+                    ic = __dmul_rn(__dadd_rn(m0, n0), 0.5);
                 }
-                if (pla_cross(Na, Nb, L2) > 0) {  // N now pivots on L2
-                    int b = 0;
-                    for (int k = 1; k < nu; k++)
-                        if (pla_cross(uh[b], L2, uh[k]) < 0) b = k;
-                    Na = uh[b];
-                    Nb = L2;
-                }
-                lh[nl2] = L2;
-                nl = nl2 + 1;
-                uh[nu2] = U2;
-                nu = nu2 + 1;
+                starts[out] = (uint32_t)(base + s);
+                slopes[out] = sl;
+                icpts[out] = ic;
             }
-        }
-        if (!COUNT) {
-            double sl = 0.0, ic = 0.0;
-            if (j - s >= 2) {
-                double sm, sn;
-                const double m0 = pla_line_at0(Ma, Mb, &sm);
-                const double n0 = pla_line_at0(Na, Nb, &sn);
-                sl = __dmul_rn(__dadd_rn(sm, sn), 0.5);
-                ic = __dmul_rn(__dadd_rn(m0, n0), 0.5);
-            }
-            starts[out] = (uint32_t)s;
-            slopes[out] = sl;
-            icpts[out] = ic;
             out++;
         }
         nseg++;
-        i = j;
+        s = j;
+        in_seg = 0;
+    };
+    auto key_of = [&](uint32_t i) -> X {
+        return i < m ? (X)((uint64_t)leaf_key<K, V>(leaves, base + i) - key0) : (X)0;
+    };
+    X xn = key_of(lane);
+    for (uint32_t b0 = 0; b0 < m; b0 += 32) {
+        const X x = xn;
+        xn = key_of(b0 + 32 + lane);  // the next batch's keys arrive behind this one
+        const Y yi = (Y)(b0 + lane);
+        const int cnt = (int)min(32u, m - b0);
+        unsigned inf = 0, um = 0, un = 0;  // infeasible; moves M; moves N
+        bool stale = true;
+        int p = 0;
+        while (p < cnt) {
+            const X px = __shfl_sync(0xffffffffu, x, p);
+            const uint32_t j = b0 + (uint32_t)p;
+            const Y pj = (Y)j;
+            if (in_seg < 2) {  // the first two points of a segment
+                if (in_seg == 0) {
+                    sx = px;
+                    if (lane == 0) {
+                        lx = ux = px;
+                        ly = uy = pj;
+                    }
+                    nl = nu = 1;
+                } else {
+                    if (lane == 1) {
+                        lx = ux = px;
+                        ly = uy = pj;
+                        lex = uex = px - sx;
+                        ley = uey = 1;
+                    }
+                    nl = nu = 2;
+                    mx = nx = sx;
+                    mdx = ndx = px - sx;
+                    my = (Y)s - e;
+                    mdy = 1 + 2 * e;
+                    ny = (Y)s + e;
+                    ndy = 1 - 2 * e;
+                    stale = true;
+                }
+                in_seg++;
+                qx = px;
+                p++;
+                continue;
+            }
+            if (stale) {  // this batch's points against M and N
+                const bool v = lane >= p;
+                const X bm = x - mx, bn = x - nx;
+                const Y ym = yi - my, yn = yi - ny;
+                inf = __ballot_sync(0xffffffffu, v && (pla_cross<T>(mdx, mdy, bm, ym - e) > 0 ||
+                                                       pla_cross<T>(ndx, ndy, bn, yn + e) < 0));
+                um = __ballot_sync(0xffffffffu, v && pla_cross<T>(mdx, mdy, bm, ym + e) < 0);
+                un = __ballot_sync(0xffffffffu, v && pla_cross<T>(ndx, ndy, bn, yn - e) > 0);
+                stale = false;
+            }
+            // the hull edges that stay: those the new point does not pop
+            const bool sl = pla_cross<T>(lex, ley, px - lx + lex, pj - ly + ley) < 0;
+            const bool su = pla_cross<T>(uex, uey, px - ux + uex, pj - uy + uey) > 0;
+            const unsigned kl = __ballot_sync(0xffffffffu, sl && lane >= 1 && lane < nl);
+            const unsigned ku = __ballot_sync(0xffffffffu, su && lane >= 1 && lane < nu);
+            const int nl2 = kl ? 32 - __clz((int)kl) : 1;
+            const int nu2 = ku ? 32 - __clz((int)ku) : 1;
+            if (((inf >> p) & 1u) || nl2 >= kHullCap || nu2 >= kHullCap) {
+                close(j);
+                continue;  // point j opens the next segment
+            }
+            if (((um | un) >> p) & 1u) {
+                if ((um >> p) & 1u) {  // M pivots on (px, j + e)
+                    const bool up = pla_cross<T>(px - lx + lex, pj - ly + ley + 2 * e, lex, ley) > 0;
+                    const unsigned t = __ballot_sync(0xffffffffu, up && lane >= 1 && lane < nl) >> 1;
+                    const int b = __ffs((int)~t) - 1;  // leading improving edges
+                    mx = __shfl_sync(0xffffffffu, lx, b);
+                    my = __shfl_sync(0xffffffffu, ly, b) - e;
+                    mdx = px - mx;
+                    mdy = pj + e - my;
+                }
+                if ((un >> p) & 1u) {  // N pivots on (px, j - e)
+                    const bool dn = pla_cross<T>(px - ux + uex, pj - uy + uey - 2 * e, uex, uey) < 0;
+                    const unsigned t = __ballot_sync(0xffffffffu, dn && lane >= 1 && lane < nu) >> 1;
+                    const int b = __ffs((int)~t) - 1;
+                    nx = __shfl_sync(0xffffffffu, ux, b);
+                    ny = __shfl_sync(0xffffffffu, uy, b) + e;
+                    ndx = px - nx;
+                    ndy = pj - e - ny;
+                }
+                stale = true;
+            }
+            if (lane == nl2) {  // push: the edge starts at hull point nl2 - 1
+                lex = nl2 == nl ? px - qx : px - lx + lex;
+                ley = nl2 == nl ? (Y)1 : pj - ly + ley;
+                lx = px;
+                ly = pj;
+            }
+            if (lane == nu2) {
+                uex = nu2 == nu ? px - qx : px - ux + uex;
+                uey = nu2 == nu ? (Y)1 : pj - uy + uey;
+                ux = px;
+                uy = pj;
+            }
+            nl = nl2 + 1;
+            nu = nu2 + 1;
+            in_seg++;
+            qx = px;
+            p++;
+        }
     }
-    if (COUNT) counts[c] = nseg;
+    close(m);
+    if (COUNT && lane == 0) counts[c] = nseg;
+}
+
+// The chunks of one kind (WIDE or narrow); the other kind's warps return, so
+// that each kernel keeps only its own registers.
+template <typename K, typename V, bool COUNT, bool WIDE>
+__global__ void __launch_bounds__(kPlaThreads)
+pla_kernel(const unsigned char *__restrict__ leaves, uint64_t n, uint32_t eps, uint64_t nchunks,
+           uint64_t *__restrict__ counts, const uint64_t *__restrict__ offsets,
+           uint32_t *__restrict__ starts, double *__restrict__ slopes, double *__restrict__ icpts) {
+    const uint64_t c = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+    if (c >= nchunks) return;
+    const uint64_t base = c * kPlaChunk;
+    const uint32_t m = (uint32_t)min(kPlaChunk, n - base);
+    const uint64_t key0 = (uint64_t)leaf_key<K, V>(leaves, base);
+    const uint64_t span = (uint64_t)leaf_key<K, V>(leaves, base + m - 1) - key0;
+    const bool wide = span >= (1ull << 31) || eps > kPlaNarrowEps;
+    if (wide != WIDE) return;
+    pla_chunk<K, V, COUNT, std::conditional_t<WIDE, PlaWide, PlaNarrow>>(
+        leaves, base, m, key0, eps, c, counts, offsets, starts, slopes, icpts);
 }
 
 // Segment lines from the segmentation (one thread per line): first keys,
@@ -1075,16 +1207,14 @@ bt_status train_impl(bt_tree *t, const bt_learned_config &cfg, cudaStream_t s,
     BT_CUDA(cudaMalloc(&boff.p, nchunks * sizeof(uint64_t)));
     BT_CUDA(cudaMalloc(&btot.p, sizeof(uint64_t)));
     uint64_t *cnt = (uint64_t *)bcnt.p, *off = (uint64_t *)boff.p, *tot = (uint64_t *)btot.p;
-    const unsigned pg = (unsigned)((nchunks + kPlaThreads - 1) / kPlaThreads);
-    const size_t pla_smem = (size_t)kPlaThreads * kPlaHullStride * sizeof(PlaPt);
-    BT_CUDA(cudaFuncSetAttribute(pla_kernel<K, V, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)pla_smem));
-    BT_CUDA(cudaFuncSetAttribute(pla_kernel<K, V, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)pla_smem));
+    const unsigned pg = (unsigned)((nchunks * 32 + kPlaThreads - 1) / kPlaThreads);
     auto count_at = [&](uint32_t eps, uint64_t *total) -> bt_status {
         count_launch();
-        pla_kernel<K, V, true><<<pg, kPlaThreads, pla_smem, s>>>(leaves, n, eps, nchunks, cnt, nullptr, nullptr,
-                                                 nullptr, nullptr);
+        pla_kernel<K, V, true, false><<<pg, kPlaThreads, 0, s>>>(leaves, n, eps, nchunks, cnt, nullptr,
+                                                                 nullptr, nullptr, nullptr);
+        count_launch();
+        pla_kernel<K, V, true, true><<<pg, kPlaThreads, 0, s>>>(leaves, n, eps, nchunks, cnt, nullptr,
+                                                                nullptr, nullptr, nullptr);
         BT_CUDA(cudaGetLastError());
         bt_status r = launch_scan_u64(cnt, off, nchunks, tot, s);
         if (r != BT_OK) return r;
@@ -1154,8 +1284,11 @@ bt_status train_impl(bt_tree *t, const bt_learned_config &cfg, cudaStream_t s,
     BT_CUDA(cudaMalloc(&bsl.p, nseg * sizeof(double)));
     BT_CUDA(cudaMalloc(&bic.p, nseg * sizeof(double)));
     count_launch();
-    pla_kernel<K, V, false><<<pg, kPlaThreads, pla_smem, s>>>(leaves, n, eps, nchunks, nullptr, off,
-                                              (uint32_t *)bst.p, (double *)bsl.p, (double *)bic.p);
+    pla_kernel<K, V, false, false><<<pg, kPlaThreads, 0, s>>>(
+        leaves, n, eps, nchunks, nullptr, off, (uint32_t *)bst.p, (double *)bsl.p, (double *)bic.p);
+    count_launch();
+    pla_kernel<K, V, false, true><<<pg, kPlaThreads, 0, s>>>(
+        leaves, n, eps, nchunks, nullptr, off, (uint32_t *)bst.p, (double *)bsl.p, (double *)bic.p);
     BT_CUDA(cudaGetLastError());
 
     // ---- segment lines and their exact bounds
