@@ -173,11 +173,12 @@ __device__ __forceinline__ double pla_line_at0(const PlaPt &a, const PlaPt &b, d
 
 // Number types of one chunk's segmentation.  Narrow: the chunk's keys span
 // less than 2^31 and eps is at most kPlaNarrowEps, so key offsets, rank
-// offsets +/- eps and their differences fit 32 bits and a cross product's two
-// terms stay below 2^62 each.  Wide: any keys and any eps, 128-bit products.
+// offsets +/- 2 eps and their differences fit 32 bits and a cross product's
+// two terms stay below 2^62 each.  Wide: any keys and any eps, 128-bit
+// products.
 constexpr uint32_t kPlaNarrowEps = 1u << 29;
 struct PlaNarrow {
-    using X = uint32_t;   // key - the chunk's first key
+    using X = int32_t;    // key - the chunk's first key
     using Y = int32_t;    // rank in the chunk, +/- eps
     using W = long long;  // cross products
 };
@@ -210,22 +211,31 @@ __device__ __forceinline__ typename T::W pla_cross(typename T::X ax, typename T:
 // rank - first = icpt + slope * (key - first key).
 //
 // The fit is a chain of 2^14 dependent points per chunk, bound by its
-// instructions and their latency (the keys are read once, coalesced, a batch
-// ahead).  What one point needs is spread over the warp:
-//  * point k of either hull is in lane k (kHullCap = 32), with the edge from
-//    point k - 1.  A new point pops a hull's tail: every lane tests its own
-//    edge, a ballot shows the last edge that stays.  The edge into the new
-//    point's slot starts at the point before it: the lane's own old one when
-//    points were popped, else the point pushed last.
-//  * a batch of 32 points is tested against M and N by its 32 lanes at once;
-//    the ballots hold until M or N moves.
-//  * M (N) pivots on the hull point of least (largest) slope to the new
-//    point: along a convex chain the steps that improve it come first, so
-//    one ballot of the edges counts them.
-// The two hulls are those of the points themselves: moving all y by eps
-// changes no cross product.  One thread per chunk, its hulls in shared
-// memory and 128-bit products, took 80 ms per pass at 2^26 keys and 110 at
-// 2^28 (lanes of a warp in different loops).
+// instructions (and, with few chunks, their latency); the keys are read
+// once, coalesced, a batch ahead.  What one point needs is spread over the
+// warp.  Mirrored in y, the lower hull and N become an upper hull and an M,
+// so lanes 0-15 work on y and lanes 16-31 on -y with the same instructions:
+//  * hull point h of a half is in its lane h (points 16-31 in a second set
+//    of registers, touched only while a hull is that long), with the edge
+//    from point h - 1.  A new point pops a hull's tail: every lane tests its
+//    own edge, a ballot shows the last edge that stays.  The edge into the
+//    new point's slot starts at the point before it: the lane's own old one
+//    when points were popped, else the point pushed last.  The hulls are
+//    those of the points themselves: moving all y by eps changes no cross
+//    product of edges.
+//  * one cross product c of M with the point decides both of its tests: the
+//    lower point is above M when c > eps * mdx, and the upper point moves M
+//    when c < -eps * mdx.
+//  * M pivots on the hull point of least slope to the new point; along a
+//    convex chain the steps that improve it come first, so one ballot of the
+//    edges counts them, and the hull test's cross product already holds what
+//    that needs.
+// M or N moves at every third (eps 181) to second (eps 45) point of
+// lognormal keys, so testing 32 points ahead against them does not pay.
+// Per pass at 2^26 keys, eps ~45: one thread per chunk with its hulls in
+// shared memory and 128-bit products 80 ms (the lanes of a warp in different
+// loops); a warp per chunk with a lane per point of both hulls and batches
+// of 32 points tested ahead 12.6 ms; this form 9.6 ms.
 template <typename K, typename V, bool COUNT, typename T>
 __device__ __forceinline__ void pla_chunk(const unsigned char *__restrict__ leaves, uint64_t base,
                                           uint32_t m, uint64_t key0, uint32_t eps, uint64_t c,
@@ -235,21 +245,29 @@ __device__ __forceinline__ void pla_chunk(const unsigned char *__restrict__ leav
                                           double *__restrict__ slopes, double *__restrict__ icpts) {
     using X = typename T::X;
     using Y = typename T::Y;
+    using W = typename T::W;
+    constexpr int HH = kHullCap / 2;
     const int lane = threadIdx.x & 31;
+    const int half = lane & HH, h = lane & (HH - 1);
+    const Y sg = half ? -1 : 1;
     const Y e = (Y)eps;
     uint64_t out = COUNT ? 0 : offsets[c];
     uint32_t nseg = 0;
-    // hull point `lane` and the edge into it from point lane - 1
-    X lx = 0, lex = 0, ux = 0, uex = 0;
-    Y ly = 0, ley = 0, uy = 0, uey = 0;
-    int nl = 0, nu = 0;              // hull sizes
-    X mx = 0, mdx = 0, nx = 0, ndx = 0;  // Ma, Mb - Ma, Na, Nb - Na
-    Y my = 0, mdy = 0, ny = 0, ndy = 0;
-    uint32_t s = 0;                  // the open segment's first point
-    X sx = 0, qx = 0;                // its key offset; that of the point pushed last
-    uint32_t in_seg = 0;             // points of the open segment
-    auto close = [&](uint32_t j) {   // the open segment ends before point j
+    X hx = 0, ex = 0, hx2 = 0, ex2 = 0;  // hull points h and HH + h, edges into them
+    Y hy = 0, ey = 0, hy2 = 0, ey2 = 0;
+    int n = 0;                           // this half's hull size
+    X mx = 0, mdx = 0;                   // Ma, Mb - Ma (of the half)
+    Y my = 0, mdy = 0;
+    W me = 0;                            // eps * mdx
+    uint32_t s = 0;                      // the open segment's first point
+    uint32_t in_seg = 0;                 // its points
+    X sx = 0, qx = 0;                    // its key offset; that of the point pushed last
+    bool ext = false;                    // a hull reaches the second register set
+    auto half_of = [&](unsigned b) { return (b >> half) & ((1u << HH) - 1u); };
+    auto close = [&](uint32_t j) {       // the open segment ends before point j
         if constexpr (!COUNT) {
+            const X nx = __shfl_sync(0xffffffffu, mx, HH), ndx = __shfl_sync(0xffffffffu, mdx, HH);
+            const Y ny = -__shfl_sync(0xffffffffu, my, HH), ndy = -__shfl_sync(0xffffffffu, mdy, HH);
             if (lane == 0) {
                 double sl = 0.0, ic = 0.0;
                 if (in_seg >= 2) {
@@ -272,6 +290,7 @@ __device__ __forceinline__ void pla_chunk(const unsigned char *__restrict__ leav
         nseg++;
         s = j;
         in_seg = 0;
+        ext = false;
     };
     auto key_of = [&](uint32_t i) -> X {
         return i < m ? (X)((uint64_t)leaf_key<K, V>(leaves, base + i) - key0) : (X)0;
@@ -280,102 +299,96 @@ __device__ __forceinline__ void pla_chunk(const unsigned char *__restrict__ leav
     for (uint32_t b0 = 0; b0 < m; b0 += 32) {
         const X x = xn;
         xn = key_of(b0 + 32 + lane);  // the next batch's keys arrive behind this one
-        const Y yi = (Y)(b0 + lane);
         const int cnt = (int)min(32u, m - b0);
-        unsigned inf = 0, um = 0, un = 0;  // infeasible; moves M; moves N
-        bool stale = true;
         int p = 0;
+        X px = __shfl_sync(0xffffffffu, x, 0);
         while (p < cnt) {
-            const X px = __shfl_sync(0xffffffffu, x, p);
+            const X pnext = __shfl_sync(0xffffffffu, x, (p + 1) & 31);
             const uint32_t j = b0 + (uint32_t)p;
-            const Y pj = (Y)j;
+            const Y py = half ? -(Y)j : (Y)j;
             if (in_seg < 2) {  // the first two points of a segment
+                if (h == (int)in_seg) {
+                    hx = px;
+                    hy = py;
+                    ex = px - sx;
+                    ey = sg;
+                }
                 if (in_seg == 0) {
                     sx = px;
-                    if (lane == 0) {
-                        lx = ux = px;
-                        ly = uy = pj;
-                    }
-                    nl = nu = 1;
                 } else {
-                    if (lane == 1) {
-                        lx = ux = px;
-                        ly = uy = pj;
-                        lex = uex = px - sx;
-                        ley = uey = 1;
-                    }
-                    nl = nu = 2;
-                    mx = nx = sx;
-                    mdx = ndx = px - sx;
-                    my = (Y)s - e;
-                    mdy = 1 + 2 * e;
-                    ny = (Y)s + e;
-                    ndy = 1 - 2 * e;
-                    stale = true;
+                    mx = sx;
+                    my = (half ? -(Y)s : (Y)s) - e;
+                    mdx = px - sx;
+                    mdy = sg + 2 * e;
+                    me = (W)mdx * (W)e;
                 }
                 in_seg++;
+                n = (int)in_seg;
                 qx = px;
+                px = pnext;
                 p++;
                 continue;
             }
-            if (stale) {  // this batch's points against M and N
-                const bool v = lane >= p;
-                const X bm = x - mx, bn = x - nx;
-                const Y ym = yi - my, yn = yi - ny;
-                inf = __ballot_sync(0xffffffffu, v && (pla_cross<T>(mdx, mdy, bm, ym - e) > 0 ||
-                                                       pla_cross<T>(ndx, ndy, bn, yn + e) < 0));
-                um = __ballot_sync(0xffffffffu, v && pla_cross<T>(mdx, mdy, bm, ym + e) < 0);
-                un = __ballot_sync(0xffffffffu, v && pla_cross<T>(ndx, ndy, bn, yn - e) > 0);
-                stale = false;
+            const W lc = pla_cross<T>(mdx, mdy, px - mx, py - my);
+            const bool inf = __any_sync(0xffffffffu, lc > me);
+            const bool mv = lc < -me;
+            const X bx = px - hx;
+            const Y by = py - hy;
+            // edge x (point - edge start) = edge x (point - edge end)
+            const W hc = pla_cross<T>(ex, ey, bx, by);
+            unsigned keep = half_of(__ballot_sync(0xffffffffu, hc < 0 && h >= 1 && h < n));
+            W hc2 = 0;
+            if (ext) {
+                hc2 = pla_cross<T>(ex2, ey2, px - hx2, py - hy2);
+                keep |= half_of(__ballot_sync(0xffffffffu, hc2 < 0 && HH + h < n)) << HH;
             }
-            // the hull edges that stay: those the new point does not pop
-            const bool sl = pla_cross<T>(lex, ley, px - lx + lex, pj - ly + ley) < 0;
-            const bool su = pla_cross<T>(uex, uey, px - ux + uex, pj - uy + uey) > 0;
-            const unsigned kl = __ballot_sync(0xffffffffu, sl && lane >= 1 && lane < nl);
-            const unsigned ku = __ballot_sync(0xffffffffu, su && lane >= 1 && lane < nu);
-            const int nl2 = kl ? 32 - __clz((int)kl) : 1;
-            const int nu2 = ku ? 32 - __clz((int)ku) : 1;
-            if (((inf >> p) & 1u) || nl2 >= kHullCap || nu2 >= kHullCap) {
+            const int n2 = keep ? 32 - __clz((int)keep) : 1;
+            const bool over = ext && __any_sync(0xffffffffu, n2 >= kHullCap);
+            if (inf || over) {
                 close(j);
                 continue;  // point j opens the next segment
             }
-            if (((um | un) >> p) & 1u) {
-                if ((um >> p) & 1u) {  // M pivots on (px, j + e)
-                    const bool up = pla_cross<T>(px - lx + lex, pj - ly + ley + 2 * e, lex, ley) > 0;
-                    const unsigned t = __ballot_sync(0xffffffffu, up && lane >= 1 && lane < nl) >> 1;
-                    const int b = __ffs((int)~t) - 1;  // leading improving edges
-                    mx = __shfl_sync(0xffffffffu, lx, b);
-                    my = __shfl_sync(0xffffffffu, ly, b) - e;
+            if (__any_sync(0xffffffffu, mv)) {  // M pivots on the point's upper point
+                unsigned t = half_of(__ballot_sync(0xffffffffu,
+                                                   hc + (W)ex * (W)(2 * e) < 0 && h >= 1 && h < n));
+                if (ext)
+                    t |= half_of(__ballot_sync(0xffffffffu,
+                                               hc2 + (W)ex2 * (W)(2 * e) < 0 && HH + h < n)) << HH;
+                const int b = __ffs((int)~(t >> 1)) - 1;  // leading improving edges
+                X ax = __shfl_sync(0xffffffffu, hx, half + (b & (HH - 1)));
+                Y ay = __shfl_sync(0xffffffffu, hy, half + (b & (HH - 1)));
+                if (ext) {
+                    const X a2 = __shfl_sync(0xffffffffu, hx2, half + (b & (HH - 1)));
+                    const Y y2 = __shfl_sync(0xffffffffu, hy2, half + (b & (HH - 1)));
+                    ax = b >= HH ? a2 : ax;
+                    ay = b >= HH ? y2 : ay;
+                }
+                if (mv) {
+                    mx = ax;
+                    my = ay - e;
                     mdx = px - mx;
-                    mdy = pj + e - my;
+                    mdy = py + e - my;
+                    me = (W)mdx * (W)e;
                 }
-                if ((un >> p) & 1u) {  // N pivots on (px, j - e)
-                    const bool dn = pla_cross<T>(px - ux + uex, pj - uy + uey - 2 * e, uex, uey) < 0;
-                    const unsigned t = __ballot_sync(0xffffffffu, dn && lane >= 1 && lane < nu) >> 1;
-                    const int b = __ffs((int)~t) - 1;
-                    nx = __shfl_sync(0xffffffffu, ux, b);
-                    ny = __shfl_sync(0xffffffffu, uy, b) + e;
-                    ndx = px - nx;
-                    ndy = pj - e - ny;
-                }
-                stale = true;
             }
-            if (lane == nl2) {  // push: the edge starts at hull point nl2 - 1
-                lex = nl2 == nl ? px - qx : px - lx + lex;
-                ley = nl2 == nl ? (Y)1 : pj - ly + ley;
-                lx = px;
-                ly = pj;
+            if (h == n2) {  // push: the edge starts at hull point n2 - 1
+                ex = n2 == n ? px - qx : bx + ex;
+                ey = n2 == n ? sg : by + ey;
+                hx = px;
+                hy = py;
             }
-            if (lane == nu2) {
-                uex = nu2 == nu ? px - qx : px - ux + uex;
-                uey = nu2 == nu ? (Y)1 : pj - uy + uey;
-                ux = px;
-                uy = pj;
+            if (ext && HH + h == n2) {
+                ex2 = n2 == n ? px - qx : px - hx2 + ex2;
+                ey2 = n2 == n ? sg : py - hy2 + ey2;
+                hx2 = px;
+                hy2 = py;
             }
-            nl = nl2 + 1;
-            nu = nu2 + 1;
+            n = n2 + 1;
+            // the next point may go to slot HH: its registers join in
+            ext = __any_sync(0xffffffffu, n >= HH);
             in_seg++;
             qx = px;
+            px = pnext;
             p++;
         }
     }
