@@ -23,6 +23,7 @@
 // atomicAdd scatter is not, grouping.cu:451-452).
 #include <algorithm>
 #include <atomic>
+#include <type_traits>
 #include <vector>
 
 #include "bt_internal.cuh"
@@ -30,12 +31,6 @@
 
 namespace bt {
 namespace {
-
-constexpr int kPT = 512;             // partition threads per CTA
-constexpr int kPWarps = kPT / 32;    // 16
-constexpr int kIPL = 8;              // items per lane
-constexpr int kPTile = kPT * kIPL;   // 4096 items per tile
-constexpr int kPerWarp = 32 * kIPL;  // 256 items per warp sub-tile
 
 struct GroupKeyParams {
     int kind;   // PartitionKind
@@ -65,378 +60,432 @@ __device__ __forceinline__ uint32_t group_key(K a, K b, const GroupKeyParams &p)
     return spread16((uint32_t)x) | (spread16((uint32_t)y) << 1);
 }
 
-// Digit histogram of one tile: per-warp shared-memory histograms (atomics
-// only collide inside a warp), summed per digit at the end.
-template <typename K, bool HAS_B>
-__global__ void __launch_bounds__(kPT)
-part_hist_kernel(const K *__restrict__ a, const K *__restrict__ b, uint64_t n, GroupKeyParams gp,
-                 int pass, uint32_t *__restrict__ counts, uint64_t ntiles) {
-    __shared__ uint32_t h[kPWarps][256];
-    for (int i = threadIdx.x; i < kPWarps * 256; i += kPT) (&h[0][0])[i] = 0;
-    __syncthreads();
-    const int w = threadIdx.x >> 5;
-    const uint64_t t0 = (uint64_t)blockIdx.x * kPTile;
-    K av[kIPL], bv[kIPL];
-#pragma unroll
-    for (int j = 0; j < kIPL; j++) {
-        const uint64_t i = t0 + (uint64_t)j * kPT + threadIdx.x;
-        av[j] = i < n ? a[i] : (K)0;
-        bv[j] = (HAS_B && i < n) ? b[i] : (K)0;
-    }
-#pragma unroll
-    for (int j = 0; j < kIPL; j++) {
-        const uint64_t i = t0 + (uint64_t)j * kPT + threadIdx.x;
-        if (i < n) atomicAdd(&h[w][(group_key<K>(av[j], bv[j], gp) >> (8 * pass)) & 0xFFu], 1u);
-    }
-    __syncthreads();
-    for (int d = threadIdx.x; d < 256; d += kPT) {
-        uint32_t c = 0;
-#pragma unroll
-        for (int ww = 0; ww < kPWarps; ww++) c += h[ww][d];
-        counts[(uint64_t)d * ntiles + blockIdx.x] = c;
-    }
-}
-
-// Exclusive scan of 256 values held one per thread by threads 0..255.
-__device__ __forceinline__ uint32_t block_exscan256(uint32_t v, uint32_t *warp_tot) {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    uint32_t x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-    }
-    if (lane == 31) warp_tot[w] = x;
-    __syncwarp();
-    return x - v;  // exclusive within the warp; caller adds the warp prefix
-}
-
-template <typename K, bool HAS_B>
-__global__ void __launch_bounds__(kPT, 3)
-part_scatter_kernel(const K *__restrict__ a, const K *__restrict__ b,
-                    const uint32_t *__restrict__ perm_in, uint64_t n, GroupKeyParams gp, int pass,
-                    const uint32_t *__restrict__ base, uint64_t ntiles, K *__restrict__ oa,
-                    K *__restrict__ ob, uint32_t *__restrict__ operm) {
-    __shared__ uint32_t cnt[kPWarps][256];
-    __shared__ uint32_t tile_start[256];
-    __shared__ uint32_t tile_base[256];  // global start of each digit's run of this tile
-    __shared__ uint32_t digit_tot[256];  // items of each digit in this tile
-    __shared__ uint32_t warp_tot[8];
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    K *sa = reinterpret_cast<K *>(smem_raw);
-    K *sb = sa + kPTile;
-    uint32_t *sp = reinterpret_cast<uint32_t *>(sb + (HAS_B ? kPTile : 0));
-    uint8_t *sd = reinterpret_cast<uint8_t *>(sp + kPTile);
-
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (int i = threadIdx.x; i < kPWarps * 256; i += kPT) (&cnt[0][0])[i] = 0;
-    if (threadIdx.x < 256) tile_base[threadIdx.x] = base[(uint64_t)threadIdx.x * ntiles + blockIdx.x];
-    __syncthreads();
-
-    const uint64_t t0 = (uint64_t)blockIdx.x * kPTile;
-    K av[kIPL], bv[kIPL];
-    uint32_t pv[kIPL], dg[kIPL], rk[kIPL];
-#pragma unroll
-    for (int j = 0; j < kIPL; j++) {
-        const uint64_t i = t0 + (uint64_t)w * kPerWarp + (uint64_t)j * 32 + lane;
-        dg[j] = 0xFFFFFFFFu;
-        av[j] = 0;
-        bv[j] = 0;
-        pv[j] = 0;
-        if (i < n) {
-            av[j] = a[i];
-            if (HAS_B) bv[j] = b[i];
-            pv[j] = perm_in ? perm_in[i] : (uint32_t)i;
-            dg[j] = (group_key<K>(av[j], bv[j], gp) >> (8 * pass)) & 0xFFu;
-        }
-    }
-    // Stable rank of every item among the same-digit items of this warp's
-    // sub-tile (item order = j-major, then lane).  The peer masks do not
-    // depend on the counters: take them all first.
-    const unsigned lt = (1u << lane) - 1u;
-    unsigned mm[kIPL];
-#pragma unroll
-    for (int j = 0; j < kIPL; j++) mm[j] = __match_any_sync(0xffffffffu, dg[j]);
-    // Rows in order: each row's leader of a digit adds the row's count to the
-    // warp's counter and hands the old value to its peers (the next row's
-    // atomic comes after this row's shuffle, so the order is the item order).
-#pragma unroll
-    for (int j = 0; j < kIPL; j++) {
-        const unsigned m = mm[j];
-        const int leader = __ffs(m) - 1;
-        uint32_t c = 0;
-        if (dg[j] != 0xFFFFFFFFu && lane == leader) c = atomicAdd(&cnt[w][dg[j]], (uint32_t)__popc(m));
-        c = __shfl_sync(0xffffffffu, c, leader);
-        rk[j] = c + __popc(m & lt);
-    }
-    __syncthreads();
-    // Per digit: exclusive prefix over the 16 warps, and the tile total.
-    // Warp ww handles digits 16 ww .. 16 ww + 15, half a lane-row each of
-    // the warps 0-7 and 8-15.
-    {
-        const int d = 16 * w + (lane & 15);
-        const int h = lane >> 4;
-        uint32_t v[kPWarps / 2], run = 0;
-#pragma unroll
-        for (int k = 0; k < kPWarps / 2; k++) v[k] = cnt[(kPWarps / 2) * h + k][d];
-        uint32_t half_tot = 0;
-#pragma unroll
-        for (int k = 0; k < kPWarps / 2; k++) half_tot += v[k];
-        const uint32_t other = __shfl_xor_sync(0xffffffffu, half_tot, 16);
-        run = h ? other : 0u;
-#pragma unroll
-        for (int k = 0; k < kPWarps / 2; k++) {
-            cnt[(kPWarps / 2) * h + k][d] = run;
-            run += v[k];
-        }
-        if (h == 0) digit_tot[d] = half_tot + other;
-    }
-    __syncthreads();
-    uint32_t tot = threadIdx.x < 256 ? digit_tot[threadIdx.x] : 0u;
-    uint32_t ex = 0;
-    if (threadIdx.x < 256) ex = block_exscan256(tot, warp_tot);
-    __syncthreads();
-    if (threadIdx.x < 256) {
-        uint32_t wp = 0;
-        for (int ww = 0; ww < (threadIdx.x >> 5); ww++) wp += warp_tot[ww];
-        tile_start[threadIdx.x] = ex + wp;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int j = 0; j < kIPL; j++) {
-        if (dg[j] != 0xFFFFFFFFu) {
-            const uint32_t lp = tile_start[dg[j]] + cnt[w][dg[j]] + rk[j];
-            sa[lp] = av[j];
-            if (HAS_B) sb[lp] = bv[j];
-            sp[lp] = pv[j];
-            sd[lp] = (uint8_t)dg[j];
-        }
-    }
-    __syncthreads();
-    const uint32_t tn = (uint32_t)min((uint64_t)kPTile, n - t0);
-    for (uint32_t lp = threadIdx.x; lp < tn; lp += kPT) {
-        const uint32_t d = sd[lp];
-        const uint64_t g = (uint64_t)tile_base[d] + (lp - tile_start[d]);
-        oa[g] = sa[lp];
-        if (HAS_B) ob[g] = sb[lp];
-        operm[g] = sp[lp];
-    }
-}
-
-// ------------------------------------------- single-pass partition ----
+// ------------------------------------------------------------ partition ----
 //
-// The kernels above take three launches per pass (tile histograms, a global
-// scan of the tile x digit table, the scatter), read the keys twice per pass
-// and load each tile's 256 digit bases from a table laid out digit-major
-// (256 scattered reads per tile).  The path below makes one read of the keys
-// for the global digit counts of every pass, then one scatter launch per
-// pass: tiles are taken in launch order from a counter, and each tile learns
-// where its digits start from the tiles before it by decoupled look-back
-// (Merrill & Garland, "Single-pass parallel prefix scan with decoupled
-// look-back", 2016; used per digit in the onesweep radix sort of Adinets &
-// Merrill, 2022): it publishes its digit counts, then walks back over its
-// predecessors' published values until it meets an inclusive prefix.
+// One stable partition by an 8-bit digit.  The batch is cut into tiles, and
+// runs of consecutive tiles into one chunk per resident CTA:
+//   part_count_kernel    counts the digits chunk by chunk (and how many of
+//                        the chunk's come before each of its tiles);
+//   part_prefix_kernel   turns the chunk counts into exclusive prefixes over
+//                        the chunks, and the digit totals (small tables are
+//                        summed by the next kernel itself);
+//   part_scatter_kernel  ranks a tile's items, orders them in shared memory
+//                        and writes them out digit by digit.  The tiles in
+//                        flight are consecutive ones, so what they write for
+//                        a digit is one stretch.
+// The keys are read twice, but no tile waits for another: a single pass with
+// decoupled look-back (Merrill & Garland 2016) walked back over most of the
+// hundreds of tiles in flight.  u32 pairs, 2^26: 1.09 ms a pass with the
+// look-back, 0.45 ms here (count 0.065, scatter 0.37; 1.3 GB, 0.2 ms at the
+// copy rate).  What bounds the scatter: 72 warp instructions a row of 32
+// items, 42 of them on the half-rate integer pipe, and 22 shared-memory
+// wavefronts, at 47% issue (32 warps per SM between barriers).  Smaller tiles
+// with three CTAs per SM: 0.47 ms; 256-thread CTAs: 0.51 and more.
+constexpr int kPT = 512;             // partition threads per CTA
+constexpr int kPWarps = kPT / 32;
+constexpr int kPartCtas = 2;         // CTAs per SM
+constexpr int kPartMaxChunks = 512;
+constexpr uint64_t kPartMinTile = 1024;  // items a CTA takes at least
+constexpr int kPartDirect = 64;      // tables of up to so many rows are summed by the scatter
 
-constexpr int kMaxPasses = 8;
-constexpr unsigned long long kStAgg = 1ull << 62;   // tile aggregate published
-constexpr unsigned long long kStInc = 2ull << 62;   // inclusive prefix published
-constexpr unsigned long long kStVal = (1ull << 62) - 1;
-constexpr uint32_t kLookbackSpins = 1u << 22;       // polls of one predecessor before giving up
-
-// Look-backs that gave up (a predecessor never published: impossible while
-// tiles are taken in order, as they are here); read by
-// bt_partition_lookback_timeouts.
-__device__ unsigned int g_lookback_timeouts = 0;
-
-__device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long long *p) {
-    unsigned long long v;
-    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return v;
+// Items per thread of a tile, as many as two CTAs per SM have registers (64 a
+// thread) and shared memory for: a tile's stretch of a digit gets longer.
+// Whole sorts at 2^26, items per thread 8 / 12 / 16: u32 pairs 1.93 / 1.80 /
+// 1.78 ms, u64 pairs 5.8 / 7.2 / 7.3 ms.
+template <int ITEM_BYTES>
+__host__ __device__ constexpr int part_ipt() {
+    return ITEM_BYTES <= 8 ? 16 : ITEM_BYTES <= 12 ? 12 : 8;
 }
 
-__device__ __forceinline__ void st_release_u64(unsigned long long *p, unsigned long long v) {
-    asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+// Source and destination of one pass.  b only for two-key items; p_in may be
+// null (the item's index is its payload).
+template <typename K, typename P>
+struct PassIO {
+    const K *a_in, *b_in;
+    const P *p_in;
+    K *a_out, *b_out;
+    P *p_out;
+};
+
+// The sort's buffers.  `vary` has a bit set where some key differs from the
+// first one: a pass whose digit has no such bit would change nothing and is
+// skipped (pass 0, which fills vary in, never is), so which buffers a pass
+// uses depends on how many are skipped.
+template <typename K, typename P>
+struct SortIO {
+    const K *in;
+    const P *p_in;
+    K *tk[2], *out;
+    P *tp[2], *p_out;
+    unsigned long long *vary;
+    int passes;
+};
+
+// True when pass p runs; io receives its buffers (the count of pass 0, which
+// is still filling vary in, only uses the source).
+template <typename K, typename P>
+__device__ __forceinline__ bool sort_pass(const SortIO<K, P> &s, int p, PassIO<K, P> &io) {
+    const unsigned long long v = *s.vary | 0xFFull;
+    if (((v >> (8 * p)) & 0xFFull) == 0) return false;
+    int before = 0, after = 0;
+    for (int k = 0; k < s.passes; k++) {
+        const bool runs = ((v >> (8 * k)) & 0xFFull) != 0;
+        before += k < p && runs;
+        after += k > p && runs;
+    }
+    io.a_in = before == 0 ? s.in : s.tk[(before - 1) & 1];
+    io.p_in = before == 0 ? s.p_in : s.tp[(before - 1) & 1];
+    io.a_out = after == 0 ? s.out : s.tk[before & 1];
+    io.p_out = after == 0 ? s.p_out : s.tp[before & 1];
+    io.b_in = nullptr;
+    io.b_out = nullptr;
+    return true;
 }
 
 // Digit of pass p of an item: byte p of its group key (of the key itself for
 // the radix sort).
 template <typename K>
 __device__ __forceinline__ uint32_t pass_digit(K a, K b, const GroupKeyParams &gp, int p) {
-    if (gp.kind == kPartRadix) return (uint32_t)(((uint64_t)a >> (8 * p)) & 0xFFu);
+    if (gp.kind == kPartRadix) return (uint32_t)(a >> (8 * p)) & 0xFFu;
     return (group_key<K>(a, b, gp) >> (8 * p)) & 0xFFu;
 }
 
-// hist[p * 256 + d] += items whose pass-p digit is d, for every pass, in one
-// read of the items (the digits do not depend on the order the passes leave).
-template <typename K, bool HAS_B>
+// How a batch is cut: tiles of `tile` items, `per` consecutive tiles to a
+// chunk.
+struct PartCut {
+    uint64_t n;
+    uint32_t tile, per, ntiles, nchunks;
+};
+
+// Row c of chunk_tab: the digits of chunk c.  Row t of tile_tab (when a chunk
+// has several tiles): those of the chunk's tiles before tile t.  Counters per
+// warp in shared memory (atomics only collide inside a warp).
+template <typename K, typename P, bool HAS_B, bool SORT, typename IO>
 __global__ void __launch_bounds__(kPT)
-part_hist_all_kernel(const K *__restrict__ a, const K *__restrict__ b, uint64_t n,
-                     GroupKeyParams gp, int passes, uint32_t *__restrict__ hist) {
-    constexpr int C = 4;  // copies, so that one hot digit is not one hot counter
-    __shared__ uint32_t h[C][kMaxPasses * 256];
-    for (int i = threadIdx.x; i < C * kMaxPasses * 256; i += kPT) (&h[0][0])[i] = 0;
-    __syncthreads();
-    uint32_t *hc = h[(threadIdx.x >> 5) & (C - 1)];
-    for (uint64_t i = blockIdx.x * (uint64_t)kPT + threadIdx.x; i < n; i += (uint64_t)gridDim.x * kPT) {
-        const K av = a[i];
-        const K bv = HAS_B ? b[i] : (K)0;
-        for (int p = 0; p < passes; p++) atomicAdd(&hc[p * 256 + pass_digit<K>(av, bv, gp, p)], 1u);
+part_count_kernel(const __grid_constant__ IO io_in, const __grid_constant__ PartCut cut,
+                  GroupKeyParams gp, int pass, uint32_t *__restrict__ chunk_tab,
+                  uint32_t *__restrict__ tile_tab) {
+    __shared__ uint32_t h[kPWarps][256];
+    __shared__ unsigned long long s_vary;
+    PassIO<K, P> io;
+    if constexpr (SORT) {
+        if (!sort_pass<K, P>(io_in, pass, io)) return;
+    } else {
+        io = io_in;
     }
-    __syncthreads();
-    for (int i = threadIdx.x; i < passes * 256; i += kPT) {
-        uint32_t c = 0;
+    const K *__restrict__ a = io.a_in;
+    const K *__restrict__ b = io.b_in;
+    for (int i = threadIdx.x; i < kPWarps * 256; i += kPT) (&h[0][0])[i] = 0;
+    if (threadIdx.x == 0) s_vary = 0;
+    uint32_t *hw = h[threadIdx.x >> 5];
+    K diff = 0;
+    const K first = SORT && pass == 0 ? a[0] : (K)0;
+    uint32_t run = 0;  // digit threadIdx.x in the chunk so far
+    const uint32_t t0 = blockIdx.x * cut.per, t1 = min(cut.ntiles, t0 + cut.per);
+    for (uint32_t t = t0; t < t1; t++) {
+        __syncthreads();
+        const uint64_t c0 = (uint64_t)t * cut.tile, c1 = min(cut.n, c0 + cut.tile);
+        constexpr int U = 8;  // loads in flight per thread
+        uint64_t i = c0 + threadIdx.x;
+        for (; i + (U - 1) * kPT < c1; i += U * kPT) {
+            K av[U], bv[U];
 #pragma unroll
-        for (int k = 0; k < C; k++) c += h[k][i];
-        if (c) atomicAdd(&hist[i], c);
+            for (int j = 0; j < U; j++) {
+                av[j] = a[i + j * kPT];
+                bv[j] = HAS_B ? b[i + j * kPT] : (K)0;
+            }
+#pragma unroll
+            for (int j = 0; j < U; j++) {
+                atomicAdd(&hw[pass_digit<K>(av[j], bv[j], gp, pass)], 1u);
+                if (SORT) diff |= av[j] ^ first;
+            }
+        }
+        for (; i < c1; i += kPT) {
+            const K av = a[i];
+            atomicAdd(&hw[pass_digit<K>(av, HAS_B ? b[i] : (K)0, gp, pass)], 1u);
+            if (SORT) diff |= av ^ first;
+        }
+        if (tile_tab && threadIdx.x < 256) tile_tab[t * 256u + threadIdx.x] = run;
+        __syncthreads();
+        if (threadIdx.x < 256) {
+#pragma unroll
+            for (int w = 0; w < kPWarps; w++) {
+                run += h[w][threadIdx.x];
+                h[w][threadIdx.x] = 0;
+            }
+        }
+    }
+    if (threadIdx.x < 256) chunk_tab[blockIdx.x * 256u + threadIdx.x] = run;
+    if constexpr (SORT) {
+        if (pass == 0) {
+            if (diff) atomicOr(&s_vary, (unsigned long long)diff);
+            __syncthreads();
+            if (threadIdx.x == 0 && s_vary) atomicOr(io_in.vary, s_vary);
+        }
     }
 }
 
-// One pass of the stable partition: the tile taken from *tile_ctr (in launch
-// order) is ranked exactly as in part_scatter_kernel, its digit bases come
-// from the global digit starts (exclusive scan of hist) plus the look-back
-// over the tiles before it, and it is written out through shared memory.
-template <typename K, bool HAS_B>
-__global__ void __launch_bounds__(kPT, 3)
-part_onesweep_kernel(const K *__restrict__ a, const K *__restrict__ b,
-                     const uint32_t *__restrict__ perm_in, uint64_t n, GroupKeyParams gp, int pass,
-                     const uint32_t *__restrict__ hist, unsigned int *__restrict__ tile_ctr,
-                     unsigned long long *__restrict__ status, K *__restrict__ oa,
-                     K *__restrict__ ob, uint32_t *__restrict__ operm) {
-    __shared__ uint32_t cnt[kPWarps][256];
-    __shared__ uint32_t tile_start[256];
-    __shared__ uint32_t tile_base[256];
-    __shared__ uint32_t digit_tot[256];
-    __shared__ uint32_t warp_tot[8];
-    __shared__ uint32_t s_tile;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    K *sa = reinterpret_cast<K *>(smem_raw);
-    K *sb = sa + kPTile;
-    uint32_t *sp = reinterpret_cast<uint32_t *>(sb + (HAS_B ? kPTile : 0));
-    uint8_t *sd = reinterpret_cast<uint8_t *>(sp + kPTile);
+// Column d of the table (one warp per digit) -> exclusive prefix over the
+// rows; its sum goes to row `rows`.  A lane takes consecutive rows, all its
+// loads in flight.
+__global__ void __launch_bounds__(256)
+part_prefix_kernel(uint32_t *__restrict__ table, int rows) {
+    constexpr int R = kPartMaxChunks / 32;
+    const int d = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    const int per = (rows + 31) / 32;
+    uint32_t v[R], sum = 0;
+#pragma unroll
+    for (int k = 0; k < R; k++) {
+        const int r = lane * per + k;
+        v[k] = k < per && r < rows ? table[r * 256 + d] : 0u;
+        sum += v[k];
+    }
+    uint32_t x = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    uint32_t run = x - sum;
+#pragma unroll
+    for (int k = 0; k < R; k++) {
+        const int r = lane * per + k;
+        if (k < per && r < rows) table[r * 256 + d] = run;
+        run += v[k];
+    }
+    if (lane == 31) table[rows * 256 + d] = x;
+}
 
+// Exclusive scan of the values of threads 0-255; warp_tot is 8 words.  Every
+// thread of the CTA calls it (one barrier; another one has to pass before
+// the next call).
+__device__ __forceinline__ uint32_t block_exscan256(uint32_t v, uint32_t *warp_tot) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (int i = threadIdx.x; i < kPWarps * 256; i += kPT) (&cnt[0][0])[i] = 0;
-    if (threadIdx.x == 0) s_tile = atomicAdd(tile_ctr, 1u);
-    // global start of every digit: exclusive scan of this pass's counts
-    uint32_t gstart = 0;
-    if (threadIdx.x < 256) gstart = block_exscan256(hist[pass * 256 + threadIdx.x], warp_tot);
-    __syncthreads();
-    if (threadIdx.x < 256) {
-        uint32_t wp = 0;
-        for (int ww = 0; ww < (threadIdx.x >> 5); ww++) wp += warp_tot[ww];
-        gstart += wp;
-    }
-    const uint64_t tile = s_tile;
-    const uint64_t t0 = tile * kPTile;
-    K av[kIPL], bv[kIPL];
-    uint32_t pv[kIPL], dg[kIPL], rk[kIPL];
+    uint32_t x = v;
+    if (w < 8) {
 #pragma unroll
-    for (int j = 0; j < kIPL; j++) {
-        const uint64_t i = t0 + (uint64_t)w * kPerWarp + (uint64_t)j * 32 + lane;
-        dg[j] = 0xFFFFFFFFu;
-        av[j] = 0;
-        bv[j] = 0;
-        pv[j] = 0;
-        if (i < n) {
-            av[j] = a[i];
-            if (HAS_B) bv[j] = b[i];
-            pv[j] = perm_in ? perm_in[i] : (uint32_t)i;
-            dg[j] = pass_digit<K>(av[j], bv[j], gp, pass);
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
         }
-    }
-    const unsigned lt = (1u << lane) - 1u;
-    unsigned mm[kIPL];
-#pragma unroll
-    for (int j = 0; j < kIPL; j++) mm[j] = __match_any_sync(0xffffffffu, dg[j]);
-#pragma unroll
-    for (int j = 0; j < kIPL; j++) {
-        const unsigned m = mm[j];
-        const int leader = __ffs(m) - 1;
-        uint32_t c = 0;
-        if (dg[j] != 0xFFFFFFFFu && lane == leader) c = atomicAdd(&cnt[w][dg[j]], (uint32_t)__popc(m));
-        c = __shfl_sync(0xffffffffu, c, leader);
-        rk[j] = c + __popc(m & lt);
+        if (lane == 31) warp_tot[w] = x;
     }
     __syncthreads();
+    uint32_t wp = 0;
+    if (w < 8) {
+#pragma unroll
+        for (int k = 0; k < 8; k++) wp += k < w ? warp_tot[k] : 0u;
+    }
+    return x - v + wp;
+}
+
+template <typename K, typename P, bool HAS_B>
+struct PartSmem {
+    static constexpr int IPT = part_ipt<(int)(sizeof(K) * (HAS_B ? 2 : 1) + sizeof(P))>();
+    static constexpr int T = kPT * IPT;  // items per tile
+    // key and payload of one width go through shared memory as one record
+    static constexpr bool REC = !HAS_B && sizeof(K) == sizeof(P);
+    struct alignas(sizeof(K) * 2) Rec {
+        K a;
+        P p;
+    };
+    static constexpr size_t bytes = kPWarps * 256 * sizeof(uint32_t) + 256 * sizeof(uint32_t) +
+                                    (size_t)T * (sizeof(K) * (HAS_B ? 2 : 1) + sizeof(P));
+};
+
+// The lanes whose 8-bit digit equals this lane's, among those with `valid`
+// (0 for the others): one vote per bit, four instructions each (the compiler's
+// own form of the same took six).  The whole sort of 2^26 u32 pairs: 3.05 ms
+// with __match_any_sync, whose time grows with the number of distinct digits,
+// 2.0 with the votes left to the compiler, 1.95 with a shared-memory word per
+// digit that lanes set their bit in (conflicts), 1.82 with these.
+template <bool ALL>
+__device__ __forceinline__ unsigned same_digit(uint32_t d, bool valid) {
+    unsigned m = ALL ? 0xffffffffu : __ballot_sync(0xffffffffu, valid);
+#pragma unroll
+    for (int b = 0; b < 8; b++) {
+        asm("{\n\t.reg .pred p;\n\t.reg .b32 t, v;\n\t"
+            "and.b32 t, %1, %2;\n\t"
+            "setp.ne.u32 p, t, 0;\n\t"
+            "vote.sync.ballot.b32 v, p, 0xffffffff;\n\t"
+            "@!p not.b32 v, v;\n\t"
+            "and.b32 %0, %0, v;\n\t}"
+            : "+r"(m)
+            : "r"(d), "r"(1u << b));
+    }
+    return m;
+}
+
+template <typename K, typename P, bool HAS_B, bool SORT, typename IO>
+__global__ void __launch_bounds__(kPT, kPartCtas)
+part_scatter_kernel(const __grid_constant__ IO io_in, const __grid_constant__ PartCut cut,
+                    GroupKeyParams gp, int pass, const uint32_t *__restrict__ chunk_tab,
+                    const uint32_t *__restrict__ tile_tab) {
+    using PS = PartSmem<K, P, HAS_B>;
+    constexpr int IPT = PS::IPT;
+    constexpr uint32_t T = PS::T;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ uint32_t warp_tot[8];
+    uint32_t(*cnt)[256] = reinterpret_cast<uint32_t(*)[256]>(smem_raw);
+    uint32_t *gbase = reinterpret_cast<uint32_t *>(cnt + kPWarps);
+    // the ordered tile: a record per item, or an array per field
+    using Rec = typename PS::Rec;
+    Rec *sr = reinterpret_cast<Rec *>(gbase + 256);
+    K *sa = reinterpret_cast<K *>(gbase + 256);
+    K *sb = sa + (HAS_B ? T : 0);
+    P *sp = reinterpret_cast<P *>(sb + T);
+    PassIO<K, P> io;
+    if constexpr (SORT) {
+        if (!sort_pass<K, P>(io_in, pass, io)) return;
+    } else {
+        io = io_in;
+    }
+    const K *__restrict__ a = io.a_in;
+    const K *__restrict__ b = io.b_in;
+    const P *__restrict__ pin = io.p_in;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const uint32_t rows = cut.nchunks;
+
+    // where the batch's items of digit `threadIdx.x` start (for a small table
+    // also where this CTA's one tile puts its own)
+    uint32_t first = 0;
     {
-        const int d = 16 * w + (lane & 15);
-        const int h = lane >> 4;
-        uint32_t v[kPWarps / 2];
-#pragma unroll
-        for (int k = 0; k < kPWarps / 2; k++) v[k] = cnt[(kPWarps / 2) * h + k][d];
-        uint32_t half_tot = 0;
-#pragma unroll
-        for (int k = 0; k < kPWarps / 2; k++) half_tot += v[k];
-        const uint32_t other = __shfl_xor_sync(0xffffffffu, half_tot, 16);
-        uint32_t run = h ? other : 0u;
-#pragma unroll
-        for (int k = 0; k < kPWarps / 2; k++) {
-            cnt[(kPWarps / 2) * h + k][d] = run;
-            run += v[k];
-        }
-        if (h == 0) digit_tot[d] = half_tot + other;
-    }
-    __syncthreads();
-    // publish this tile's counts, then sum the predecessors' (look-back)
-    if (threadIdx.x < 256) {
-        const int d = threadIdx.x;
-        const uint32_t agg = digit_tot[d];
-        unsigned long long *mine = status + tile * 256 + d;
-        unsigned long long prefix = 0;
-        if (tile == 0) {
-            st_release_u64(mine, kStInc | agg);
-        } else {
-            st_release_u64(mine, kStAgg | agg);
-            uint64_t tp = tile - 1;
-            uint32_t spins = 0;
-            for (;;) {
-                const unsigned long long v = ld_acquire_u64(status + tp * 256 + d);
-                const unsigned long long f = v & ~kStVal;
-                if (f == 0) {
-                    if (++spins > kLookbackSpins) {  // never in a correct launch; bounded anyway
-                        atomicAdd(&g_lookback_timeouts, 1u);
-                        break;
-                    }
-                    __nanosleep(32);
-                    continue;
+        uint32_t tot = 0, pre = 0;
+        if (threadIdx.x < 256) {
+            if (rows > kPartDirect) {
+                tot = chunk_tab[rows * 256u + threadIdx.x];
+            } else {
+#pragma unroll 8
+                for (uint32_t r = 0; r < rows; r++) {
+                    const uint32_t v = chunk_tab[r * 256u + threadIdx.x];
+                    pre += r < blockIdx.x ? v : 0u;
+                    tot += v;
                 }
-                spins = 0;
-                prefix += v & kStVal;
-                if (f == kStInc || tp == 0) break;
-                tp--;
             }
-            st_release_u64(mine, kStInc | (prefix + agg));
         }
-        tile_base[d] = gstart + (uint32_t)prefix;
+        first = block_exscan256(tot, warp_tot) + pre;
     }
-    uint32_t tot = threadIdx.x < 256 ? digit_tot[threadIdx.x] : 0u;
-    uint32_t ex = 0;
-    if (threadIdx.x < 256) ex = block_exscan256(tot, warp_tot + 0);
-    __syncthreads();
-    if (threadIdx.x < 256) {
-        uint32_t wp = 0;
-        for (int ww = 0; ww < (threadIdx.x >> 5); ww++) wp += warp_tot[ww];
-        tile_start[threadIdx.x] = ex + wp;
-    }
-    __syncthreads();
+    uint32_t *cw = cnt[w];
+    K av[IPT], bv[HAS_B ? IPT : 1];
+    uint32_t rpw = 0;  // rows of 32 items per warp: IPT, or fewer in a short tile
+    auto tile_items = [&](uint32_t t) {
+        return (uint32_t)min((uint64_t)cut.tile, cut.n - (uint64_t)t * cut.tile);
+    };
+    auto load_keys = [&](uint32_t t) {
+        const uint64_t t0 = (uint64_t)t * cut.tile;
+        const uint32_t tn = tile_items(t);
+        rpw = tn == T ? (uint32_t)IPT : (tn + kPT - 1) / kPT;
 #pragma unroll
-    for (int j = 0; j < kIPL; j++) {
-        if (dg[j] != 0xFFFFFFFFu) {
-            const uint32_t lp = tile_start[dg[j]] + cnt[w][dg[j]] + rk[j];
-            sa[lp] = av[j];
-            if (HAS_B) sb[lp] = bv[j];
-            sp[lp] = pv[j];
-            sd[lp] = (uint8_t)dg[j];
+        for (int j = 0; j < IPT; j++) {
+            const uint32_t i = (w * rpw + j) * 32 + lane;
+            const bool v = tn == T || (j < (int)rpw && i < tn);
+            av[j] = v ? a[t0 + i] : (K)0;
+            if (HAS_B) bv[j] = v ? b[t0 + i] : (K)0;
         }
-    }
-    __syncthreads();
-    const uint32_t tn = t0 < n ? (uint32_t)min((uint64_t)kPTile, n - t0) : 0u;
-    for (uint32_t lp = threadIdx.x; lp < tn; lp += kPT) {
-        const uint32_t d = sd[lp];
-        const uint64_t g = (uint64_t)tile_base[d] + (lp - tile_start[d]);
-        oa[g] = sa[lp];
-        if (HAS_B) ob[g] = sb[lp];
-        operm[g] = sp[lp];
+    };
+    const unsigned lt = (1u << lane) - 1u;
+    // One tile: FULL has every item (no bounds to check).
+    auto tile = [&](auto full_tag, uint32_t t, uint32_t tn) {
+        constexpr bool FULL = decltype(full_tag)::value;
+        const uint64_t t0 = (uint64_t)t * cut.tile;
+        const uint32_t r0 = w * (FULL ? (uint32_t)IPT : rpw) * 32 + lane;  // the lane's first item
+        auto live = [&](int j) { return FULL || (j < (int)rpw && r0 + j * 32 < tn); };
+#pragma unroll
+        for (int k = 0; k < 2; k++) reinterpret_cast<uint4 *>(cw)[k * 32 + lane] = make_uint4(0, 0, 0, 0);
+        __syncwarp();
+        // Stable rank of every item among the same-digit items of its warp
+        // (item order = row, then lane).
+        uint32_t rk[IPT];
+#pragma unroll
+        for (int j = 0; j < IPT; j++) {
+            const bool v = live(j);
+            const uint32_t d = pass_digit<K>(av[j], HAS_B ? bv[j] : (K)0, gp, pass);
+            const unsigned m = same_digit<FULL>(d, v);
+            const uint32_t c = v ? cw[d] : 0u;
+            const uint32_t below = __popc(m & lt);
+            __syncwarp();
+            if (v && below == 0) cw[d] = c + __popc(m);
+            __syncwarp();
+            rk[j] = c + below;
+        }
+        // the payload arrives while the digits are scanned
+        P pv[IPT];
+#pragma unroll
+        for (int j = 0; j < IPT; j++) {
+            const uint64_t i = t0 + r0 + j * 32;
+            pv[j] = pin ? (live(j) ? pin[i] : (P)0) : (P)i;
+        }
+        uint32_t run = first;  // where the tile's first item of digit `threadIdx.x` goes
+        if (threadIdx.x < 256) {
+            if (rows > kPartDirect) run += chunk_tab[(t / cut.per) * 256u + threadIdx.x];
+            if (tile_tab) run += tile_tab[t * 256u + threadIdx.x];
+        }
+        __syncthreads();
+        // per digit: the tile's total, then every warp's first slot
+        uint32_t tot = 0;
+        if (threadIdx.x < 256) {
+#pragma unroll
+            for (int k = 0; k < kPWarps; k++) tot += cnt[k][threadIdx.x];
+        }
+        const uint32_t start = block_exscan256(tot, warp_tot);
+        if (threadIdx.x < 256) {
+            uint32_t x = start;
+#pragma unroll
+            for (int k = 0; k < kPWarps; k++) {
+                const uint32_t c = cnt[k][threadIdx.x];
+                cnt[k][threadIdx.x] = x;
+                x += c;
+            }
+            gbase[threadIdx.x] = run - start;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < IPT; j++) {
+            if (live(j)) {
+                const uint32_t d = pass_digit<K>(av[j], HAS_B ? bv[j] : (K)0, gp, pass);
+                const uint32_t lp = cw[d] + rk[j];
+                if constexpr (PS::REC) {
+                    sr[lp] = Rec{av[j], pv[j]};
+                } else {
+                    sa[lp] = av[j];
+                    if (HAS_B) sb[lp] = bv[j];
+                    sp[lp] = pv[j];
+                }
+            }
+        }
+        __syncthreads();
+        if (t + gridDim.x < cut.ntiles) load_keys(t + gridDim.x);  // these arrive behind the writes
+        auto put = [&](uint32_t lp) {
+            K ka, kb = 0;
+            P kp;
+            if constexpr (PS::REC) {
+                const Rec r = sr[lp];
+                ka = r.a;
+                kp = r.p;
+            } else {
+                ka = sa[lp];
+                if (HAS_B) kb = sb[lp];
+                kp = sp[lp];
+            }
+            const uint32_t g = gbase[pass_digit<K>(ka, kb, gp, pass)] + lp;
+            io.a_out[g] = ka;
+            if (HAS_B) io.b_out[g] = kb;
+            io.p_out[g] = kp;
+        };
+        if constexpr (FULL) {
+#pragma unroll
+            for (int j = 0; j < IPT; j++) put(j * kPT + threadIdx.x);
+        } else {
+            for (uint32_t lp = threadIdx.x; lp < tn; lp += kPT) put(lp);
+        }
+        // no barrier here: the next tile writes gbase and the ordered items
+        // only after its first one
+    };
+    if (blockIdx.x < cut.ntiles) load_keys(blockIdx.x);
+    for (uint32_t t = blockIdx.x; t < cut.ntiles; t += gridDim.x) {
+        const uint32_t tn = tile_items(t);
+        if (tn == T) tile(std::true_type{}, t, T);
+        else tile(std::false_type{}, t, tn);
     }
 }
 
@@ -562,231 +611,140 @@ bt_status scan_impl(const T *d_in, T *d_out, uint64_t n, T *d_total, cudaStream_
 
 // -------------------------------------------------------- partition host --
 
-// Dynamic shared memory of part_scatter_kernel<K, HAS_B> and its one-time
-// raise above the 48 KB default (per device and instantiation; function
-// attributes are per device, and the server's worker and user threads may
-// partition at once).
-template <typename K, bool HAS_B>
-constexpr size_t scatter_smem() {
-    return (size_t)kPTile * (sizeof(K) * (HAS_B ? 2 : 1) + sizeof(uint32_t) + 1);
-}
-
-template <typename K, bool HAS_B>
+// One-time raise of a scatter instantiation's dynamic shared memory above the
+// 48 KB default (function attributes are per device; the server's worker and
+// user threads may partition at once).
+template <typename K, typename P, bool HAS_B, bool SORT, typename IO>
 bt_status scatter_smem_attr() {
     static std::atomic<bool> done[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && done[dev].load(std::memory_order_acquire)) return BT_OK;
-    BT_CUDA(cudaFuncSetAttribute(part_scatter_kernel<K, HAS_B>,
+    BT_CUDA(cudaFuncSetAttribute(part_scatter_kernel<K, P, HAS_B, SORT, IO>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)scatter_smem<K, HAS_B>()));
+                                 (int)PartSmem<K, P, HAS_B>::bytes));
     if (dev >= 0 && dev < 64) done[dev].store(true, std::memory_order_release);
     return BT_OK;
 }
 
-template <typename K, bool HAS_B>
-bt_status onesweep_smem_attr() {
-    static std::atomic<bool> done[64] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev >= 0 && dev < 64 && done[dev].load(std::memory_order_acquire)) return BT_OK;
-    BT_CUDA(cudaFuncSetAttribute(part_onesweep_kernel<K, HAS_B>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)scatter_smem<K, HAS_B>()));
-    if (dev >= 0 && dev < 64) done[dev].store(true, std::memory_order_release);
-    return BT_OK;
+// The tables of a pass: a row per chunk and the totals, then a row per tile
+// when chunks have several.
+size_t part_table_bytes(uint64_t n, uint32_t tile_cap) {
+    const uint64_t ntiles = (n + tile_cap - 1) / tile_cap;
+    return (size_t)(kPartMaxChunks + 1 + ntiles) * 256 * sizeof(uint32_t);
 }
 
-// Workspace of the single-pass partition: digit counts of every pass, one
-// tile counter per pass, the look-back status of one pass.
-struct SweepWs {
-    uint32_t *hist;
-    unsigned int *ctr;
-    unsigned long long *status;
-    static size_t bytes(uint64_t ntiles) {
-        return kMaxPasses * 256 * sizeof(uint32_t) + 256 + ntiles * 256 * sizeof(unsigned long long);
-    }
-    void carve(unsigned char *p) {
-        hist = reinterpret_cast<uint32_t *>(p);
-        ctr = reinterpret_cast<unsigned int *>(p + kMaxPasses * 256 * sizeof(uint32_t));
-        status = reinterpret_cast<unsigned long long *>(p + kMaxPasses * 256 * sizeof(uint32_t) + 256);
-    }
-};
-
-// Stable partition of n items by `passes` digits: pass p reads (ia, ib, ip)
-// and writes (oa[p], ob[p], op[p]); the histogram of every pass comes from
-// one read of the input.
-template <typename K, bool HAS_B>
-bt_status sweep_passes(const K *a, const K *b, uint64_t n, GroupKeyParams gp, int passes,
-                       K *const *oa, K *const *ob, uint32_t *const *op, SweepWs ws,
-                       cudaStream_t s) {
-    const uint64_t ntiles = (n + kPTile - 1) / kPTile;
-    BT_CUDA(cudaMemsetAsync(ws.hist, 0, kMaxPasses * 256 * sizeof(uint32_t) + 256, s));
-    bt_status st = onesweep_smem_attr<K, HAS_B>();
+template <typename K, typename P, bool HAS_B, bool SORT, typename IO>
+bt_status part_pass(const IO &io, uint64_t n, GroupKeyParams gp, int pass, uint32_t *table,
+                    cudaStream_t s) {
+    bt_status st = scatter_smem_attr<K, P, HAS_B, SORT, IO>();
     if (st != BT_OK) return st;
+    // two CTAs per SM; a batch that does not fill them with whole tiles gets
+    // smaller ones, in whole rows of a warp
+    const uint64_t ctas = std::min<uint64_t>(kPartMaxChunks, (uint64_t)kPartCtas * (uint64_t)sm_count());
+    constexpr uint64_t T = PartSmem<K, P, HAS_B>::T;
+    PartCut cut;
+    cut.n = n;
+    cut.tile = (uint32_t)std::min<uint64_t>(
+        T, std::max<uint64_t>(kPartMinTile, ((n + ctas - 1) / ctas + 31) / 32 * 32));
+    cut.ntiles = (uint32_t)((n + cut.tile - 1) / cut.tile);
+    cut.per = (uint32_t)((cut.ntiles + ctas - 1) / ctas);
+    cut.nchunks = (cut.ntiles + cut.per - 1) / cut.per;
+    uint32_t *tile_tab = cut.per > 1 ? table + (kPartMaxChunks + 1) * 256 : nullptr;
     count_launch();
-    part_hist_all_kernel<K, HAS_B>
-        <<<(unsigned)std::min<uint64_t>(ntiles, (uint64_t)sm_count() * 4), kPT, 0, s>>>(
-            a, b, n, gp, passes, ws.hist);
-    const K *ia = a, *ib = b;
-    const uint32_t *ip = nullptr;
-    for (int p = 0; p < passes; p++) {
-        BT_CUDA(cudaMemsetAsync(ws.status, 0, ntiles * 256 * sizeof(unsigned long long), s));
+    part_count_kernel<K, P, HAS_B, SORT, IO><<<cut.nchunks, kPT, 0, s>>>(io, cut, gp, pass, table, tile_tab);
+    if (cut.nchunks > kPartDirect) {
         count_launch();
-        part_onesweep_kernel<K, HAS_B><<<(unsigned)ntiles, kPT, scatter_smem<K, HAS_B>(), s>>>(
-            ia, ib, ip, n, gp, p, ws.hist, ws.ctr + p, ws.status, oa[p], HAS_B ? ob[p] : nullptr,
-            op[p]);
-        BT_CUDA(cudaGetLastError());
-        ia = oa[p];
-        ib = HAS_B ? ob[p] : nullptr;
-        ip = op[p];
+        part_prefix_kernel<<<32, 256, 0, s>>>(table, (int)cut.nchunks);
     }
+    count_launch();
+    part_scatter_kernel<K, P, HAS_B, SORT, IO>
+        <<<(unsigned)std::min<uint64_t>(cut.ntiles, ctas), kPT, PartSmem<K, P, HAS_B>::bytes, s>>>(
+            io, cut, gp, pass, table, tile_tab);
+    BT_CUDA(cudaGetLastError());
     return BT_OK;
 }
+
+size_t align256(size_t x) { return (x + 255) / 256 * 256; }
 
 template <typename K, bool HAS_B>
 bt_status partition_impl(const bt_tree *t, int kind, const K *d_a, const K *d_b, uint64_t nq,
                          K *out_a, K *out_b, uint32_t *out_perm, cudaStream_t s) {
     GroupKeyParams gp;
     gp.kind = kind;
-    const int kb = bitlen64(t->max_key);
-    int dbits;
-    if (kind == kPartPoint) {
-        dbits = kPointGroupBits;
-        gp.cbits = dbits;
-    } else {
-        dbits = kRangeGroupBits * 2;  // two coordinates
-        gp.cbits = kRangeGroupBits;
-    }
-    gp.shift = std::max(0, kb - gp.cbits);
-    const int passes = (dbits + 7) / 8;
-    const uint64_t ntiles = (nq + kPTile - 1) / kPTile;
-    if (ntiles * 256 >= (1ull << 32)) return fail(BT_ERR_INVALID_ARGUMENT, "batch too large");
-
-    // One workspace: digit counts, scan scratch and, for two passes, one
-    // intermediate copy of the payload.  (The look-back path of
-    // sweep_passes was measured slower here -- one or two passes, 2^24
-    // queries: 0.325 ms against 0.239 -- so grouping keeps tile histograms,
-    // one scan and the scatter; the device sort, with four or eight passes
-    // served by one histogram read, uses sweep_passes.)
-    const uint64_t ncounts = ntiles * 256;
-    const uint64_t scan_we = scan_ws_elems(ncounts);
-    const size_t pp_bytes = passes > 1 ? nq * (sizeof(K) * (HAS_B ? 2 : 1) + sizeof(uint32_t)) + 512 : 0;
-    const size_t cbytes = ((ncounts + scan_we) * sizeof(uint32_t) + 255) / 256 * 256;
-    unsigned char *ws = nullptr;
-    bt_status st = ws_alloc((void **)&ws, cbytes + pp_bytes, s);
+    gp.cbits = kind == kPartPoint ? kPointGroupBits : kRangeGroupBits;  // per coordinate
+    gp.shift = std::max(0, bitlen64(t->max_key) - gp.cbits);
+    const int passes = ((kind == kPartPoint ? 1 : 2) * gp.cbits + 7) / 8;
+    if (passes > 2) return fail(BT_ERR_INTERNAL, "partition supports at most two passes");
+    // the table and, for two passes, one intermediate copy of the items
+    const size_t ab = align256(nq * sizeof(K)), pb = align256(nq * sizeof(uint32_t));
+    WsGuard ws(s);
+    const size_t tb = align256(part_table_bytes(nq, PartSmem<K, uint32_t, HAS_B>::T));
+    bt_status st = ws.alloc(tb + (passes > 1 ? ab * (HAS_B ? 2 : 1) + pb : 0));
     if (st != BT_OK) return st;
-    uint32_t *counts = reinterpret_cast<uint32_t *>(ws);
-    uint32_t *scan_ws = counts + ncounts;
-    K *oa[2] = {out_a, out_a}, *ob[2] = {out_b, out_b};
-    uint32_t *op[2] = {out_perm, out_perm};
-    if (passes > 1) {  // pass 0 into the intermediate copy, pass 1 into the caller's arrays
-        unsigned char *pp = ws + cbytes;
-        oa[0] = reinterpret_cast<K *>(pp);
-        pp += (nq * sizeof(K) + 255) / 256 * 256;
-        if (HAS_B) {
-            ob[0] = reinterpret_cast<K *>(pp);
-            pp += (nq * sizeof(K) + 255) / 256 * 256;
-        }
-        op[0] = reinterpret_cast<uint32_t *>(pp);
+    unsigned char *p = ws.as<unsigned char>();
+    uint32_t *table = reinterpret_cast<uint32_t *>(p);
+    using IO = PassIO<K, uint32_t>;
+    IO io{d_a, d_b, nullptr, out_a, out_b, out_perm};
+    if (passes > 1) {
+        p += tb;
+        IO mid = io;
+        mid.a_out = reinterpret_cast<K *>(p);
+        mid.b_out = HAS_B ? reinterpret_cast<K *>(p + ab) : nullptr;
+        mid.p_out = reinterpret_cast<uint32_t *>(p + ab * (HAS_B ? 2 : 1));
+        st = part_pass<K, uint32_t, HAS_B, false, IO>(mid, nq, gp, 0, table, s);
+        if (st != BT_OK) return st;
+        io.a_in = mid.a_out;
+        io.b_in = mid.b_out;
+        io.p_in = mid.p_out;
     }
-    if (passes > 2) st = fail(BT_ERR_INTERNAL, "partition supports at most two passes");
-    if (st == BT_OK) st = scatter_smem_attr<K, HAS_B>();
-    const K *ia = d_a, *ib = d_b;
-    const uint32_t *ip = nullptr;
-    for (int p = 0; p < passes && st == BT_OK; p++) {
-        count_launch();
-        part_hist_kernel<K, HAS_B><<<(unsigned)ntiles, kPT, 0, s>>>(ia, ib, nq, gp, p, counts, ntiles);
-        st = scan_run<uint32_t>(counts, counts, ncounts, nullptr, scan_ws, s);
-        if (st != BT_OK) break;
-        count_launch();
-        part_scatter_kernel<K, HAS_B><<<(unsigned)ntiles, kPT, scatter_smem<K, HAS_B>(), s>>>(
-            ia, ib, ip, nq, gp, p, counts, ntiles, oa[p], ob[p], op[p]);
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) st = cuda_fail(e, "partition kernels");
-        ia = oa[p];
-        ib = ob[p];
-        ip = op[p];
-    }
-    ws_free(ws, s);
-    return st;
+    return part_pass<K, uint32_t, HAS_B, false, IO>(io, nq, gp, passes - 1, table, s);
 }
 
-template <typename V>
-__global__ void gather_kernel(const V *__restrict__ in, const uint32_t *__restrict__ idx, uint64_t n,
-                              V *__restrict__ out) {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
-         i += (uint64_t)gridDim.x * blockDim.x)
-        out[i] = in[idx[i]];
-}
-
-// LSD radix sort of keys carrying the input index: pass p partitions by
-// byte p of the key (stable), so after the last pass the keys are sorted and
-// equal keys keep their input order; then values are gathered by index.
-template <typename K, typename V>
-bt_status sort_pairs_impl(const K *d_keys, const V *d_vals, uint64_t n, K *out_keys, V *out_vals,
-                          cudaStream_t s) {
-    const int passes = (int)sizeof(K);
-    const uint64_t ntiles = (n + kPTile - 1) / kPTile;
-    const size_t sweep_bytes = (SweepWs::bytes(ntiles) + 255) / 256 * 256;
-    const size_t kbytes = (n * sizeof(K) + 255) / 256 * 256;
-    const size_t pbytes = (n * sizeof(uint32_t) + 255) / 256 * 256;
-    unsigned char *ws = nullptr;
-    bt_status st = ws_alloc((void **)&ws, sweep_bytes + 2 * (kbytes + pbytes), s);
+// LSD radix sort of n keys carrying a payload (p_in, or the item's index when
+// p_in is null): pass p partitions by byte p of the key (stable), so after
+// the last pass the keys are sorted and equal keys keep their input order.
+// The values travel with their keys: carrying the index and gathering the
+// values at the end cost 1.18 ms of random reads at 2^26 u32 pairs, more
+// than all passes' extra bytes.
+template <typename K, typename P>
+bt_status radix_sort(const K *d_keys, const P *p_in, uint64_t n, int passes, K *out_keys, P *out_p,
+                     cudaStream_t s) {
+    const size_t kb = align256(n * sizeof(K)), pb = align256(n * sizeof(P));
+    const size_t tb = align256(part_table_bytes(n, PartSmem<K, P, false>::T));
+    WsGuard ws(s);
+    bt_status st = ws.alloc(256 + tb + 2 * (kb + pb));
     if (st != BT_OK) return st;
-    SweepWs sw;
-    sw.carve(ws);
-    unsigned char *pp = ws + sweep_bytes;
-    K *tk[2] = {reinterpret_cast<K *>(pp), reinterpret_cast<K *>(pp + kbytes + pbytes)};
-    uint32_t *tp[2] = {reinterpret_cast<uint32_t *>(pp + kbytes),
-                       reinterpret_cast<uint32_t *>(pp + 2 * kbytes + pbytes)};
-    K *ok[kMaxPasses];
-    uint32_t *op[kMaxPasses];
-    for (int p = 0; p < passes; p++) {
-        ok[p] = p == passes - 1 ? out_keys : tk[p & 1];
-        op[p] = tp[p & 1];
+    unsigned char *w = ws.as<unsigned char>();
+    using IO = SortIO<K, P>;
+    IO io;
+    io.in = d_keys;
+    io.p_in = p_in;
+    io.out = out_keys;
+    io.p_out = out_p;
+    io.vary = reinterpret_cast<unsigned long long *>(w);
+    io.passes = passes;
+    uint32_t *table = reinterpret_cast<uint32_t *>(w + 256);
+    for (int i = 0; i < 2; i++) {
+        io.tk[i] = reinterpret_cast<K *>(w + 256 + tb + i * (kb + pb));
+        io.tp[i] = reinterpret_cast<P *>(w + 256 + tb + i * (kb + pb) + kb);
     }
-    GroupKeyParams gp;
-    gp.kind = kPartRadix;
-    gp.cbits = 8;
-    gp.shift = 0;
-    st = sweep_passes<K, false>(d_keys, nullptr, n, gp, passes, ok, nullptr, op, sw, s);
-    if (st == BT_OK) {
-        count_launch();
-        gather_kernel<V><<<(unsigned)std::min<uint64_t>((n + 255) / 256, (uint64_t)sm_count() * 16), 256, 0, s>>>(
-            d_vals, op[passes - 1], n, out_vals);
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) st = cuda_fail(e, "value gather");
-    }
-    ws_free(ws, s);
+    BT_CUDA(cudaMemsetAsync(io.vary, 0, sizeof(*io.vary), s));
+    GroupKeyParams gp{kPartRadix, 0, 8};
+    for (int p = 0; p < passes && st == BT_OK; p++)
+        st = part_pass<K, P, false, true, IO>(io, n, gp, p, table, s);
     return st;
 }
 
 bt_status order_u16_impl(const uint32_t *d_keys, uint64_t n, uint32_t *d_perm, cudaStream_t s) {
-    const uint64_t ntiles = (n + kPTile - 1) / kPTile;
-    const size_t sweep_bytes = (SweepWs::bytes(ntiles) + 255) / 256 * 256;
-    const size_t b = (n * sizeof(uint32_t) + 255) / 256 * 256;
-    unsigned char *ws = nullptr;
-    bt_status st = ws_alloc((void **)&ws, sweep_bytes + 3 * b, s);
+    WsGuard ws(s);  // the sorted keys, which nobody reads
+    bt_status st = ws.alloc(n * sizeof(uint32_t));
     if (st != BT_OK) return st;
-    SweepWs sw;
-    sw.carve(ws);
-    uint32_t *k0 = reinterpret_cast<uint32_t *>(ws + sweep_bytes);
-    uint32_t *k1 = reinterpret_cast<uint32_t *>(ws + sweep_bytes + b);
-    uint32_t *p0 = reinterpret_cast<uint32_t *>(ws + sweep_bytes + 2 * b);
-    uint32_t *ok[2] = {k0, k1};
-    uint32_t *op[2] = {p0, d_perm};
-    GroupKeyParams gp;
-    gp.kind = kPartRadix;
-    gp.cbits = 8;
-    gp.shift = 0;
-    st = sweep_passes<uint32_t, false>(d_keys, nullptr, n, gp, 2, ok, nullptr, op, sw, s);
-    ws_free(ws, s);
-    return st;
+    return radix_sort<uint32_t, uint32_t>(d_keys, nullptr, n, 2, ws.as<uint32_t>(), d_perm, s);
 }
 
 // Single-pass point partition into caller-provided memory (no allocation):
-// counts and scan scratch come from `ws` (partition_ws_bytes bytes).
+// the table comes from `ws` (partition_point_ws_bytes bytes).
 template <typename K>
 bt_status partition_point_prealloc(const bt_tree *t, const K *d_q, uint64_t nq, K *out_q,
                                    uint32_t *out_perm, unsigned char *ws, cudaStream_t s) {
@@ -794,23 +752,9 @@ bt_status partition_point_prealloc(const bt_tree *t, const K *d_q, uint64_t nq, 
     gp.kind = kPartPoint;
     gp.cbits = kPointGroupBits;
     gp.shift = std::max(0, bitlen64(t->max_key) - gp.cbits);
-    const uint64_t ntiles = (nq + kPTile - 1) / kPTile;
-    const uint64_t ncounts = ntiles * 256;
-    uint32_t *counts = reinterpret_cast<uint32_t *>(ws);
-    uint32_t *scan_ws = counts + ncounts;
-    const size_t smem = scatter_smem<K, false>();
-    auto scat = part_scatter_kernel<K, false>;
-    bt_status sa = scatter_smem_attr<K, false>();
-    if (sa != BT_OK) return sa;
-    count_launch();
-    part_hist_kernel<K, false><<<(unsigned)ntiles, kPT, 0, s>>>(d_q, nullptr, nq, gp, 0, counts, ntiles);
-    bt_status st = scan_run<uint32_t>(counts, counts, ncounts, nullptr, scan_ws, s);
-    if (st != BT_OK) return st;
-    count_launch();
-    scat<<<(unsigned)ntiles, kPT, smem, s>>>(d_q, nullptr, nullptr, nq, gp, 0, counts, ntiles, out_q,
-                                             nullptr, out_perm);
-    BT_CUDA(cudaGetLastError());
-    return BT_OK;
+    using IO = PassIO<K, uint32_t>;
+    return part_pass<K, uint32_t, false, false, IO>(IO{d_q, nullptr, nullptr, out_q, nullptr, out_perm},
+                                                    nq, gp, 0, reinterpret_cast<uint32_t *>(ws), s);
 }
 
 // --------------------------------------------------------- range fill ----
@@ -983,14 +927,14 @@ bt_status launch_sort_pairs(int key_bytes, int value_bytes, const void *d_keys, 
     if (n >= (1ull << 32)) return fail(BT_ERR_INVALID_ARGUMENT, "sort needs fewer than 2^32 pairs");
     if (key_bytes == 4)
         return value_bytes == 4
-                   ? sort_pairs_impl<uint32_t, uint32_t>((const uint32_t *)d_keys, (const uint32_t *)d_vals, n,
+                   ? radix_sort<uint32_t, uint32_t>((const uint32_t *)d_keys, (const uint32_t *)d_vals, n, 4,
                                                          (uint32_t *)out_keys, (uint32_t *)out_vals, s)
-                   : sort_pairs_impl<uint32_t, uint64_t>((const uint32_t *)d_keys, (const uint64_t *)d_vals, n,
+                   : radix_sort<uint32_t, uint64_t>((const uint32_t *)d_keys, (const uint64_t *)d_vals, n, 4,
                                                          (uint32_t *)out_keys, (uint64_t *)out_vals, s);
     return value_bytes == 4
-               ? sort_pairs_impl<uint64_t, uint32_t>((const uint64_t *)d_keys, (const uint32_t *)d_vals, n,
+               ? radix_sort<uint64_t, uint32_t>((const uint64_t *)d_keys, (const uint32_t *)d_vals, n, 8,
                                                      (uint64_t *)out_keys, (uint32_t *)out_vals, s)
-               : sort_pairs_impl<uint64_t, uint64_t>((const uint64_t *)d_keys, (const uint64_t *)d_vals, n,
+               : radix_sort<uint64_t, uint64_t>((const uint64_t *)d_keys, (const uint64_t *)d_vals, n, 8,
                                                      (uint64_t *)out_keys, (uint64_t *)out_vals, s);
 }
 
@@ -1001,8 +945,8 @@ bt_status launch_order_u16(const uint32_t *d_keys, uint64_t n, uint32_t *d_perm,
 }
 
 size_t partition_point_ws_bytes(uint64_t nq) {
-    const uint64_t ncounts = ((nq + kPTile - 1) / kPTile) * 256;
-    return (ncounts + scan_ws_elems(ncounts)) * sizeof(uint32_t);
+    return std::max(part_table_bytes(nq, PartSmem<uint32_t, uint32_t, false>::T),
+                    part_table_bytes(nq, PartSmem<uint64_t, uint32_t, false>::T));
 }
 
 bt_status launch_partition_point_prealloc(const bt_tree *t, const void *d_q, uint64_t nq,
@@ -1125,10 +1069,7 @@ bt_status launch_segment_sort(const bt_tree *t, const uint64_t *d_counts, const 
 
 extern "C" {
 
-uint64_t bt_partition_lookback_timeouts(void) {
-    unsigned int v = 0;
-    if (cudaMemcpyFromSymbol(&v, bt::g_lookback_timeouts, sizeof(v)) != cudaSuccess) return ~0ull;
-    return v;
-}
+// No partition pass waits on another CTA.
+uint64_t bt_partition_lookback_timeouts(void) { return 0; }
 
 }  // extern "C"
