@@ -74,6 +74,19 @@ __global__ void pad_kernel(K *__restrict__ dst, uint64_t from, uint64_t to) {
         dst[j] = key_max<K>();
 }
 
+// How evenly the keys fill the buckets of a large point batch.
+bt_status measure_buckets(bt_tree *t, cudaStream_t s) {
+    WsGuard g(s);
+    bt_status st = g.alloc(sizeof(uint32_t));
+    if (st != BT_OK) return st;
+    BT_CUDA(cudaMemsetAsync(g.p, 0, sizeof(uint32_t), s));
+    st = launch_bucket_blocks(t, g.as<uint32_t>(), s);
+    if (st != BT_OK) return st;
+    BT_CUDA(cudaMemcpyAsync(&t->bucket_blocks, g.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    BT_CUDA(cudaStreamSynchronize(s));
+    return BT_OK;
+}
+
 unsigned grid_for(uint64_t n, int block) {
     uint64_t g = (n + block - 1) / block;
     uint64_t cap = (uint64_t)sm_count() * 16;
@@ -169,7 +182,7 @@ bt_status build_impl(bt_tree *t, const void *d_keys, const void *d_vals, cudaStr
     dt.smem_entries = (uint32_t)t->lvl_entries[sl];
     // whole 128-byte bank rows, so the swizzle stays inside the staged region
     dt.smem_bytes = (uint32_t)(((t->lvl_entries[sl] * sizeof(K)) + 127) / 128 * 128);
-    return BT_OK;
+    return measure_buckets(t, s);
 }
 
 template <typename K>
@@ -411,7 +424,6 @@ bt_status bt_save(const bt_tree *t, const char *path) {
 
 bt_status bt_load(const char *path, void *stream, bt_tree **out) {
     using namespace bt;
-    (void)stream;
     if (!path || !out) return fail(BT_ERR_INVALID_ARGUMENT, "path or out is NULL");
     *out = nullptr;
     int dev = 0;
@@ -467,6 +479,13 @@ bt_status bt_load(const char *path, void *stream, bt_tree **out) {
     dt.smem_level = h.smem_level;
     dt.smem_entries = h.smem_entries;
     dt.smem_bytes = h.smem_bytes;
+    if (t->n) {
+        st = measure_buckets(t, (cudaStream_t)stream);
+        if (st != BT_OK) {
+            free_tree(t);
+            return st;
+        }
+    }
     *out = t;
     return BT_OK;
 }

@@ -140,6 +140,7 @@ struct bt_tree {
     uint64_t lvl_entries[bt::kMaxLevels];
     uint64_t min_key, max_key;
     int values_sorted;
+    uint32_t bucket_blocks;  // leaf blocks of the fullest bucket (0: not measured)
     int search_cfg;  // index into the search kernels' (lanes, rounds) table
     bt::DevTree dev;
     bt::LearnedState *learned;  // trained learned index, or null
@@ -248,6 +249,59 @@ bt_status launch_learned_search(const bt_tree *t, const void *d_q, uint64_t nq, 
                                 uint8_t *d_found, cudaStream_t s);
 // Zeroes those counters (stream-ordered).
 bt_status reset_learned_stats(const bt_tree *t, cudaStream_t s);
+
+// Buckets of a point batch: equal stretches of the tree's key range
+// [min, max], numbered by the key's offset from the smallest key shifted
+// right; keys outside the range go to the end buckets.
+constexpr int kMaxBuckets = 2048;
+struct BucketMap {
+    uint64_t min;
+    int shift;
+    uint32_t last;  // the highest bucket
+    template <typename K>
+    __device__ __forceinline__ uint32_t of(K k) const {
+        const K d = k > (K)min ? k - (K)min : (K)0;
+        const K b = d >> shift;
+        return b < (K)last ? (uint32_t)b : last;
+    }
+    __device__ __forceinline__ uint64_t first_key(uint32_t b) const {
+        return b == 0 ? 0ull : min + ((uint64_t)b << shift);
+    }
+};
+// Most queries of one work item of the bucket search.
+constexpr uint32_t kBucketSlice = 16384;
+// What the passes of the bucket order leave for the search.
+struct BucketPlan {
+    uint32_t *scratch;  // 2 * kMaxBuckets words
+    uint32_t *first;    // leaf block where bucket b's keys start, b = 0 .. last + 1
+    uint4 *items;       // work items: bucket, first slot, slots
+    uint32_t *n_items;  // at most kMaxBuckets + nq / kBucketSlice
+};
+// d_q ordered by bucket into out_q (query i in slot pos[i]).
+bt_status launch_buckets(const bt_tree *t, const BucketMap &map, const void *d_q, uint64_t nq,
+                         void *out_q, uint32_t *pos, const BucketPlan &bp, cudaStream_t s);
+// d_out[i] = res[pos[i]], and the found flags when d_found is not null.
+bt_status launch_bucket_gather(int val_bytes, const void *res, const uint8_t *rfound,
+                               const uint32_t *pos, uint64_t nq, void *d_out, uint8_t *d_found,
+                               cudaStream_t s);
+// The tree's map: as many buckets as kMaxBuckets allows.
+inline BucketMap bucket_map(uint64_t min_key, uint64_t max_key) {
+    const int span = bitlen64(max_key - min_key);
+    BucketMap m;
+    m.min = min_key;
+    m.shift = span > 11 ? span - 11 : 0;
+    m.last = (uint32_t)((max_key - min_key) >> m.shift);
+    return m;
+}
+static_assert(kMaxBuckets == 1 << 11, "bucket_map takes 11 bits");
+// Measures t->bucket_blocks into *d_blocks (zeroed by the caller); the
+// tree's arrays, sizes and key ends are set.
+bt_status launch_bucket_blocks(const bt_tree *t, uint32_t *d_blocks, cudaStream_t s);
+// Whether a point batch is searched by buckets, and that search (workspace
+// from the pool; BT_ERR_OUT_OF_MEMORY when it cannot be had).
+bool bucket_search_pays(const bt_tree *t, uint64_t nq, cudaStream_t s);
+bt_status launch_bucket_search(const bt_tree *t, const void *d_q, uint64_t nq, void *d_out,
+                               cudaStream_t s, uint8_t *d_found);
 
 // Partition kinds for launch_partition.
 enum PartitionKind { kPartPoint = 0, kPart2D = 1, kPartZ = 2, kPartRadix = 3 };

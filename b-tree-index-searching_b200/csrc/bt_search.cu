@@ -56,7 +56,7 @@ constexpr int kWarps = kThreads / 32;
 __host__ __device__ inline size_t scratch_offset(const DevTree &t) { return ((size_t)t.smem_bytes + 15) / 16 * 16; }
 
 template <typename K, typename V, int G, int R, bool PERM>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, 2)
 point_kernel(const __grid_constant__ DevTree t, const K *__restrict__ q,
              const uint32_t *__restrict__ perm, uint64_t nq, V *__restrict__ out,
              uint8_t *__restrict__ found) {
@@ -246,6 +246,241 @@ point_window_kernel(const __grid_constant__ DevTree t, const K *__restrict__ q,
                 },
                 [&](int s) -> uint8_t * { return found ? found + pv[s] : nullptr; });
         }
+    }
+}
+
+// ---- point search of a batch ordered by bucket (launch_buckets) ------------
+//
+// A CTA takes one work item: up to kBucketSlice queries of one bucket, whose
+// leaf blocks lie between first[bucket] and first[bucket + 1].  It stages that
+// window of the deepest separator level that fits in its shared memory, 64-bit
+// separators as 32-bit offsets where their span allows it, so that one binary
+// search there takes a query past every level above -- for most trees straight
+// to its leaf block.  Leaf blocks are then read
+//   4-byte keys: by a thread per query, four queries at a time: one 32-byte
+//     load of the block's keys, then the matching value;
+//   8-byte keys: by a lane pair per query, two queries at a time: one lane the
+//     key sector, one the value sector, as one request.
+// A quarter of the instructions of the lane-quad form of point_kernel (19 a
+// query, which bound this kernel to 0.37 ms at 2^26 u32 keys and 2^24
+// queries): 0.178 ms with a thread per query, 0.21 with pairs.  With u64 keys
+// (2^28, 2^24 queries) the leaf reads' DRAM access rate bounds it: pairs
+// 0.56 ms, thread per query 0.60.
+
+
+// Staged window slot of sorted element p: a padding word after every 32 and
+// every 1,024 elements keeps a binary search's probes in different banks
+// (two instructions, where swz takes four; the window is not a power of two).
+__device__ __forceinline__ uint32_t win_slot(uint32_t p) { return p + (p >> 5) + (p >> 10); }
+constexpr uint64_t kBktMinQueries = 1ull << 22;
+constexpr size_t kBktWinBytes = 200 * 1024;
+constexpr size_t kBktWinMin = 16 * 1024;  // room for some level of any tree
+constexpr size_t win_words(size_t n) { return n + n / 32 + n / 1024 + 2; }
+
+// First element of the n staged ones at or above q, n if none, for U queries
+// in step.
+template <typename W, int U>
+__device__ __forceinline__ void win_bound(const W *__restrict__ s, uint32_t n, const W (&q)[U],
+                                          uint32_t (&pos)[U]) {
+#pragma unroll
+    for (int u = 0; u < U; u++) pos[u] = 0;
+    while (n > 1) {
+        const uint32_t half = n >> 1;
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const uint32_t p = pos[u] + half;
+            pos[u] = s[win_slot(p)] < q[u] ? p : pos[u];
+        }
+        n -= half;
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) pos[u] += s[win_slot(pos[u])] < q[u] ? 1u : 0u;
+}
+
+// 32 bytes of a leaf block by one thread.  Not evict-first: a block's value
+// sector, which comes with its key sector, is read a moment later (evicted
+// before that, 2^24 u64 queries took 1.19 ms instead of 0.84).
+__device__ __forceinline__ void load_sector(const void *p, uint32_t (&w)[8]) {
+    asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]),
+                   "=r"(w[7])
+                 : "l"(p));
+}
+
+// The first of a key sector's S keys equal to q, -1 if none (unused slots
+// hold all-ones keys, which a query above the largest key may equal).
+template <typename K, int S>
+__device__ __forceinline__ int first_match(const uint32_t (&w)[8], K q, K tmax) {
+    int at = -1;
+#pragma unroll
+    for (int k = S - 1; k >= 0; k--)
+        if (key_at<K>(w, k) == q) at = k;
+    return q <= tmax ? at : -1;
+}
+
+// The qn queries of an item by their staged window: node = w0 + position in
+// the window of level wlvl, then the levels below it (lane quads, one line
+// per query and level), then the leaf block.
+template <typename K, typename V, typename W, int T>
+__device__ __forceinline__ void bucket_item(const DevTree &t, const W *s_win, uint32_t w0, uint32_t wm,
+                                            int wlvl, K base, const K *__restrict__ q, uint32_t qn,
+                                            V *__restrict__ out, uint8_t *__restrict__ found) {
+    using LG = LeafGeom<K, V>;
+    constexpr bool PAIR = sizeof(K) == 8;
+    constexpr int U = PAIR ? 2 : 4;  // queries per thread at a time
+    const int lane = threadIdx.x & 31;
+    const K tmax = (K)t.max_key;
+    const unsigned char *leaves = static_cast<const unsigned char *>(t.leaves);
+    for (uint32_t i0 = threadIdx.x & ~31u; i0 < qn; i0 += T * U) {
+        K qv[U];
+        W qw[U];
+        uint32_t node[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const uint32_t i = i0 + u * T + lane;
+            qv[u] = i < qn ? q[i] : (K)0;
+            const K c = qv[u] < tmax ? qv[u] : tmax;
+            if constexpr (sizeof(W) < sizeof(K)) {
+                const K d = c > base ? c - base : (K)0;
+                qw[u] = d < (K)0xFFFFFFFFu ? (W)d : (W)0xFFFFFFFFu;
+            } else {
+                qw[u] = c;
+            }
+        }
+        win_bound<W, U>(s_win, wm, qw, node);
+#pragma unroll
+        for (int u = 0; u < U; u++) node[u] = w0 + (node[u] < wm ? node[u] : wm - 1u);
+        if (wlvl + 1 < t.nlevels) {  // uniform: the window is not the bottom level
+            constexpr int G = 4, NG = 32 / G;
+            const int grp = lane / G, gl = lane % G;
+#pragma unroll 1
+            for (int u = 0; u < U; u++) {
+                K qe[G];
+                bool up[G];
+                uint32_t nd[G];
+#pragma unroll
+                for (int s = 0; s < G; s++) {
+                    K x = 0;
+                    uint32_t y = 0;
+#pragma unroll
+                    for (int z = 0; z < U; z++)
+                        if (z == u) {
+                            x = qv[z];
+                            y = node[z];
+                        }
+                    qe[s] = __shfl_sync(0xffffffffu, x, s * NG + grp);
+                    nd[s] = __shfl_sync(0xffffffffu, y, s * NG + grp);
+                    qe[s] = qe[s] < tmax ? qe[s] : tmax;
+                    up[s] = false;
+                }
+                walk_from<K, G, G>(t, wlvl + 1, qe, up, nd, grp, gl);
+                uint32_t r = 0;
+#pragma unroll
+                for (int s = 0; s < G; s++) {
+                    const uint32_t y = __shfl_sync(0xffffffffu, nd[s], (lane % NG) * G);
+                    r = lane / NG == s ? y : r;
+                }
+#pragma unroll
+                for (int z = 0; z < U; z++) node[z] = z == u ? r : node[z];
+            }
+        }
+        if constexpr (PAIR) {
+            static_assert(sizeof(K) == 4 || LG::BS == 2 * kSectorBytes, "values in the second sector");
+            uint32_t w[U][2][8];
+            K qk[U][2];
+#pragma unroll
+            for (int u = 0; u < U; u++)
+#pragma unroll
+                for (int h = 0; h < 2; h++) {  // lanes 2k, 2k + 1: query 16 h + k of the 32
+                    const int k = h * 16 + (lane >> 1);
+                    const uint32_t nd = __shfl_sync(0xffffffffu, node[u], k);
+                    qk[u][h] = __shfl_sync(0xffffffffu, qv[u], k);
+                    load_sector(leaves + (size_t)nd * LG::BS + (lane & 1) * kSectorBytes, w[u][h]);
+                }
+#pragma unroll
+            for (int u = 0; u < U; u++)
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    int at = first_match<K, LG::S>(w[u][h], qk[u][h], tmax);
+                    at = __shfl_sync(0xffffffffu, at, lane & ~1);  // the key lane's
+                    V v = key_max<V>();
+#pragma unroll
+                    for (int k = 0; k < LG::S; k++)
+                        if (at == k) v = key_at<V>(w[u][h], k);
+                    const uint32_t i = i0 + u * T + h * 16 + (lane >> 1);
+                    if ((lane & 1) && i < qn) {
+                        out[i] = v;
+                        if (found) found[i] = at >= 0 ? 1 : 0;
+                    }
+                }
+        } else {
+            uint32_t w[U][8];
+#pragma unroll
+            for (int u = 0; u < U; u++) load_sector(leaves + (size_t)node[u] * LG::BS, w[u]);
+            int at[U];
+            V v[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                at[u] = first_match<K, LG::S>(w[u], qv[u], tmax);
+                v[u] = at[u] >= 0 ? __ldg(reinterpret_cast<const V *>(leaves + (size_t)node[u] * LG::BS +
+                                                                     kSectorBytes) + at[u])
+                                  : key_max<V>();
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const uint32_t i = i0 + u * T + lane;
+                if (i < qn) {
+                    out[i] = v[u];
+                    if (found) found[i] = at[u] >= 0 ? 1 : 0;
+                }
+            }
+        }
+    }
+}
+
+template <typename K, typename V, int T>
+__global__ void __launch_bounds__(T, 1024 / T)
+bucket_search_kernel(const __grid_constant__ DevTree t, const uint32_t *__restrict__ first,
+                     const uint4 *__restrict__ items, const uint32_t *__restrict__ n_items,
+                     uint32_t win_bytes, const K *__restrict__ q, V *__restrict__ out,
+                     uint8_t *__restrict__ found) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    constexpr int F = kLineBytes / (int)sizeof(K);
+    constexpr int LOGF = F == 32 ? 5 : 4;
+    if (blockIdx.x >= *n_items) return;
+    const uint4 it = items[blockIdx.x];
+    const uint32_t blo = first[it.x], bhi = first[it.x + 1];
+    const K *seps = static_cast<const K *>(t.seps);
+    // the deepest level whose window fits; not more than 32 entries staged
+    // per query (a line of the level per query)
+    int wlvl = t.nlevels - 1, sh = 0;
+    uint32_t w0, wm;
+    const K *src;
+    bool narrow;
+    for (;;) {
+        w0 = blo >> sh;
+        wm = (bhi >> sh) - w0 + 1u;
+        src = seps + t.lvl_off[wlvl] + w0;
+        narrow = sizeof(K) == 4 || (uint64_t)src[wm - 1] - (uint64_t)src[0] < 0xFFFFFFFFull;
+        if (wlvl == 0 || (win_words(wm) * (narrow ? 4 : 8) <= win_bytes && wm / 32 <= it.z)) break;
+        wlvl--;
+        sh += LOGF;
+    }
+    const K base = sizeof(K) == 8 && narrow ? src[0] : (K)0;
+    if (narrow) {
+        uint32_t *s_win = reinterpret_cast<uint32_t *>(smem_raw);
+#pragma unroll 8
+        for (uint32_t i = threadIdx.x; i < wm; i += T) s_win[win_slot(i)] = (uint32_t)(src[i] - base);
+        __syncthreads();
+        bucket_item<K, V, uint32_t, T>(t, s_win, w0, wm, wlvl, base, q + it.y, it.z, out + it.y,
+                                       found ? found + it.y : nullptr);
+    } else if constexpr (sizeof(K) == 8) {
+        uint64_t *s_win = reinterpret_cast<uint64_t *>(smem_raw);
+#pragma unroll 8
+        for (uint32_t i = threadIdx.x; i < wm; i += T) s_win[win_slot(i)] = (uint64_t)src[i];
+        __syncthreads();
+        bucket_item<K, V, uint64_t, T>(t, s_win, w0, wm, wlvl, base, q + it.y, it.z, out + it.y,
+                                       found ? found + it.y : nullptr);
     }
 }
 
@@ -486,6 +721,33 @@ bt_status window_launch(const bt_tree *t, const void *d_q, const uint32_t *d_per
     return BT_OK;
 }
 
+template <typename K, typename V, int T>
+bt_status bucket_launch(const bt_tree *t, const BucketPlan &bp, uint64_t max_items, size_t smem,
+                        const void *d_q, void *d_out, uint8_t *d_found, cudaStream_t s) {
+    auto fn = bucket_search_kernel<K, V, T>;
+    bt_status st = set_smem(fn, smem);
+    if (st != BT_OK) return st;
+    count_launch();
+    fn<<<(unsigned)max_items, T, smem, s>>>(t->dev, bp.first, bp.items, bp.n_items, (uint32_t)smem,
+                                            (const K *)d_q, (V *)d_out, d_found);
+    BT_CUDA(cudaGetLastError());
+    return BT_OK;
+}
+
+template <typename K, typename V>
+bt_status bucket_cfg(const bt_tree *t, const BucketMap &map, const BucketPlan &bp, uint64_t max_items,
+                     const void *d_q, void *d_out, uint8_t *d_found, cudaStream_t s) {
+    // the fullest bucket's window of the deepest level that fits, in 32-bit
+    // entries (the kernel goes a level up where its own does not)
+    constexpr int LOGF = sizeof(K) == 4 ? 5 : 4;
+    size_t m = t->bucket_blocks;
+    while (win_words(m) * sizeof(uint32_t) > kBktWinBytes) m = (m >> LOGF) + 2;
+    const size_t smem = std::max<size_t>(win_words(m) * sizeof(uint32_t), kBktWinMin);
+    // two CTAs per SM where two windows fit
+    if (smem <= kBktWinBytes / 2) return bucket_launch<K, V, 512>(t, bp, max_items, smem, d_q, d_out, d_found, s);
+    return bucket_launch<K, V, 1024>(t, bp, max_items, smem, d_q, d_out, d_found, s);
+}
+
 template <typename K, typename V, bool PERM>
 bt_status point_cfg(const bt_tree *t, const void *d_q, const uint32_t *d_perm, uint64_t nq,
                     void *d_out, uint8_t *d_found, cudaStream_t s) {
@@ -575,6 +837,62 @@ bt_status launch_point_search(const bt_tree *t, const void *d_q, const uint32_t 
     }
     return d_perm ? point_types<true>(t, d_q, d_perm, nq, d_out, d_found, s)
                   : point_types<false>(t, d_q, d_perm, nq, d_out, d_found, s);
+}
+
+// Both ways timed at 2^14 to 2^28 keys, u32 and u64, 2^17 to 2^24 queries (us,
+// direct / by buckets):
+//                 2^21 queries   2^22          2^24
+//   u32, 2^14      52 / 68       97 / 91      381 / 247
+//   u32, 2^26      86 / 108     160 / 152     607 / 374
+//   u64, 2^18      81 / 97      155 / 141     604 / 423
+//   u64, 2^26     148 / 149     275 / 204    1056 / 544
+//   u64, 2^28     187 / 268     352 / 361    1305 / 808
+// The passes of the order cost some 70 us at 2^21 queries, and every query
+// pays for its share of the staged separators: eight per query (2^23 queries
+// at 2^28 u64 keys: 674 / 515) are still worth it.  Trees whose keys crowd
+// into few of the equal stretches (a bucket of over four times the average)
+// keep the direct search: their windows lie levels above the leaves.  So does
+// a stream under capture, whose graph then holds no allocation.
+bool bucket_search_pays(const bt_tree *t, uint64_t nq, cudaStream_t s) {
+    if (t->n == 0 || nq >= (1ull << 32)) return false;
+    if (nq < kBktMinQueries || nq < t->n_sectors / 8) return false;
+    const uint64_t buckets = bucket_map(t->min_key, t->max_key).last + 1;
+    if (t->bucket_blocks == 0 || t->bucket_blocks > 4 * (t->n_sectors / buckets) + 64) return false;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone) return true;
+    cudaGetLastError();
+    return false;
+}
+
+bt_status launch_bucket_search(const bt_tree *t, const void *d_q, uint64_t nq, void *d_out,
+                               cudaStream_t s, uint8_t *d_found) {
+    const BucketMap map = bucket_map(t->min_key, t->max_key);
+    auto up256 = [](size_t x) { return (x + 255) / 256 * 256; };
+    const size_t kb = up256(nq * t->key_bytes), pb = up256(nq * sizeof(uint32_t));
+    const size_t vb = up256(nq * t->val_bytes), fb = d_found ? up256(nq) : 0;
+    const uint64_t max_items = map.last + 1 + nq / kBucketSlice;
+    WsGuard ws(s);
+    bt_status st = ws.alloc(kb + pb + vb + fb + max_items * sizeof(uint4) +
+                            (3 * kMaxBuckets + 64) * sizeof(uint32_t));
+    if (st != BT_OK) return st;
+    unsigned char *q = ws.as<unsigned char>(), *res = q + kb + pb;
+    uint32_t *pos = reinterpret_cast<uint32_t *>(q + kb);
+    uint8_t *rf = d_found ? res + vb : nullptr;
+    BucketPlan bp;
+    bp.items = reinterpret_cast<uint4 *>(res + vb + fb);
+    bp.scratch = reinterpret_cast<uint32_t *>(bp.items + max_items);
+    bp.first = bp.scratch + 2 * kMaxBuckets;
+    bp.n_items = bp.first + kMaxBuckets + 1;
+    st = launch_buckets(t, map, d_q, nq, q, pos, bp, s);
+    if (st != BT_OK) return st;
+    if (t->key_bytes == 4)
+        st = t->val_bytes == 4 ? bucket_cfg<uint32_t, uint32_t>(t, map, bp, max_items, q, res, rf, s)
+                               : bucket_cfg<uint32_t, uint64_t>(t, map, bp, max_items, q, res, rf, s);
+    else
+        st = t->val_bytes == 4 ? bucket_cfg<uint64_t, uint32_t>(t, map, bp, max_items, q, res, rf, s)
+                               : bucket_cfg<uint64_t, uint64_t>(t, map, bp, max_items, q, res, rf, s);
+    if (st != BT_OK) return st;
+    return launch_bucket_gather(t->val_bytes, res, rf, pos, nq, d_out, d_found, s);
 }
 
 bt_status launch_bounds(const bt_tree *t, const void *d_lo, const void *d_hi,
