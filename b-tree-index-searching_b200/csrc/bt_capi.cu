@@ -60,7 +60,7 @@ bt_status point_device(const bt_tree *t, int mode, const void *d_q, uint64_t nq,
         if (st != BT_ERR_OUT_OF_MEMORY) return st;
         cudaGetLastError();  // no room for the ordered copy: the direct search
     }
-    if (mode == BT_POINT_BASIC || t->n == 0)
+    if (mode == BT_POINT_BASIC || t->n == 0 || (mode == BT_POINT_GROUPED && nq < kBktMinQueries))
         return launch_point_search(t, d_q, nullptr, nq, d_out, s, d_found);
     if (mode == BT_POINT_LEARNED) return launch_learned_search(t, d_q, nq, d_out, d_found, s);
     void *gq = nullptr;
@@ -76,7 +76,12 @@ bt_status point_device(const bt_tree *t, int mode, const void *d_q, uint64_t nq,
 
 bt_status count_device(const bt_tree *t, int mode, const void *d_lo, const void *d_hi, uint64_t nq,
                        uint64_t *d_counts, uint64_t *d_lb, cudaStream_t s) {
-    if (mode == BT_RANGE_BASIC || t->n == 0)
+    if (bucket_bounds_pay(t, nq, s)) {  // whatever the mode: results do not depend on it
+        const bt_status st = launch_bucket_bounds(t, d_lo, d_hi, nq, d_counts, d_lb, s);
+        if (st != BT_ERR_OUT_OF_MEMORY) return st;
+        cudaGetLastError();
+    }
+    if (mode == BT_RANGE_BASIC || t->n == 0 || nq < kOrderMinRanges)
         return launch_bounds(t, d_lo, d_hi, nullptr, nq, d_counts, d_lb, s);
     const int kind = mode == BT_RANGE_GROUPED_2D ? kPart2D : kPartZ;
     void *ga = nullptr, *gb = nullptr;

@@ -519,9 +519,23 @@ struct BucketSmem {
     static constexpr size_t bytes = (size_t)T * sizeof(K) + 2 * kMaxBuckets * sizeof(uint32_t);
 };
 
+// Query i of a batch.  A range batch is two batches of lower bounds, lo[i]
+// and then hi[i] + 1 (the bound of an hi at the largest value is not used).
 template <typename K>
+struct PointBatch {
+    const K *q;
+    __device__ __forceinline__ K get(uint64_t i) const { return q[i]; }
+};
+template <typename K>
+struct RangeBatch {
+    const K *lo, *hi;
+    uint64_t nr;
+    __device__ __forceinline__ K get(uint64_t i) const { return i < nr ? lo[i] : (K)(hi[i - nr] + 1); }
+};
+
+template <typename K, typename B>
 __global__ void __launch_bounds__(kBT)
-bucket_count_kernel(const K *__restrict__ q, uint64_t n, const __grid_constant__ BucketMap map,
+bucket_count_kernel(const __grid_constant__ B q, uint64_t n, const __grid_constant__ BucketMap map,
                     uint32_t *__restrict__ total) {
     constexpr int C = kMaxBuckets <= 2048 ? 4 : kMaxBuckets <= 4096 ? 2 : 1;  // copies
     __shared__ uint32_t h[C][kMaxBuckets];
@@ -534,7 +548,7 @@ bucket_count_kernel(const K *__restrict__ q, uint64_t n, const __grid_constant__
     for (uint64_t i0 = (uint64_t)blockIdx.x * kBT * U + threadIdx.x; i0 < n; i0 += step) {
         K v[U];
 #pragma unroll
-        for (int j = 0; j < U; j++) v[j] = i0 + j * kBT < n ? q[i0 + j * kBT] : (K)0;
+        for (int j = 0; j < U; j++) v[j] = i0 + j * kBT < n ? q.get(i0 + j * kBT) : (K)0;
 #pragma unroll
         for (int j = 0; j < U; j++)
             if (i0 + j * kBT < n) atomicAdd(&hw[map.of(v[j])], 1u);
@@ -632,9 +646,9 @@ bucket_blocks_kernel(const __grid_constant__ DevTree t, const __grid_constant__ 
     if (lane == 0) atomicMax(blocks, m);
 }
 
-template <typename K>
+template <typename K, typename B>
 __global__ void __launch_bounds__(kBT, 2)
-bucket_scatter_kernel(const K *__restrict__ q, uint64_t n, const __grid_constant__ BucketMap map,
+bucket_scatter_kernel(const __grid_constant__ B q, uint64_t n, const __grid_constant__ BucketMap map,
                       uint32_t *__restrict__ cursor, K *__restrict__ oq, uint32_t *__restrict__ pos) {
     using BS = BucketSmem<K>;
     constexpr int IPT = BS::IPT;
@@ -655,7 +669,7 @@ bucket_scatter_kernel(const K *__restrict__ q, uint64_t n, const __grid_constant
 #pragma unroll
         for (int j = 0; j < IPT; j++) {
             const uint32_t i = j * kBT + threadIdx.x;
-            v[j] = i < tn ? q[t0 + i] : (K)0;
+            v[j] = i < tn ? q.get(t0 + i) : (K)0;
         }
         for (uint32_t i = threadIdx.x; i < kMaxBuckets; i += kBT) cnt[i] = 0;
         __syncthreads();
@@ -742,6 +756,42 @@ bucket_gather_kernel(const V *__restrict__ res, const uint8_t *__restrict__ rfou
 #pragma unroll
         for (int j = 0; j < U; j++)
             if (i0 + j * 512 < n) found[i0 + j * 512] = f[j];
+    }
+}
+
+// counts[i] = keys in [lo[i], hi[i]] from the two bounds' ranks, and the
+// lower bounds when lb is not null.
+template <typename K>
+__global__ void __launch_bounds__(512)
+range_gather_kernel(const uint32_t *__restrict__ rank, const uint32_t *__restrict__ pos,
+                    const K *__restrict__ lo, const K *__restrict__ hi, uint64_t nr, K tmax, uint64_t n,
+                    uint64_t *__restrict__ counts, uint64_t *__restrict__ lb) {
+    constexpr int U = 4;
+    const uint64_t i0 = (uint64_t)blockIdx.x * (512 * U) + threadIdx.x;
+    K a[U], b[U];
+    uint32_t pa[U], pb[U];
+#pragma unroll
+    for (int j = 0; j < U; j++) {
+        const uint64_t i = i0 + j * 512 < nr ? i0 + j * 512 : 0;
+        a[j] = lo[i];
+        b[j] = hi[i];
+        pa[j] = pos[i];
+        pb[j] = pos[nr + i];
+    }
+    uint64_t ra[U], rb[U];
+#pragma unroll
+    for (int j = 0; j < U; j++) {
+        ra[j] = rank[pa[j]];
+        rb[j] = rank[pb[j]];
+    }
+#pragma unroll
+    for (int j = 0; j < U; j++) {
+        if (a[j] > tmax) ra[j] = n;
+        if (b[j] >= tmax) rb[j] = n;
+        if (i0 + j * 512 < nr) {
+            counts[i0 + j * 512] = a[j] <= b[j] && rb[j] > ra[j] ? rb[j] - ra[j] : 0;
+            if (lb) lb[i0 + j * 512] = ra[j];
+        }
     }
 }
 
@@ -1222,14 +1272,14 @@ bt_status launch_scan_u64(const uint64_t *d_in, uint64_t *d_out, uint64_t n, uin
 }
 
 namespace {
-template <typename K>
-bt_status bucket_impl(const bt_tree *t, const BucketMap &map, const K *d_q, uint64_t nq, K *out_q,
+template <typename K, typename B>
+bt_status bucket_impl(const bt_tree *t, const BucketMap &map, const B &q, uint64_t nq, K *out_q,
                       uint32_t *pos, const BucketPlan &bp, cudaStream_t s) {
     static std::atomic<bool> done[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64 || !done[dev].load(std::memory_order_acquire)) {
-        BT_CUDA(cudaFuncSetAttribute(bucket_scatter_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        BT_CUDA(cudaFuncSetAttribute(bucket_scatter_kernel<K, B>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)BucketSmem<K>::bytes));
         if (dev >= 0 && dev < 64) done[dev].store(true, std::memory_order_release);
     }
@@ -1237,26 +1287,51 @@ bt_status bucket_impl(const bt_tree *t, const BucketMap &map, const K *d_q, uint
     BT_CUDA(cudaMemsetAsync(total, 0, kMaxBuckets * sizeof(uint32_t), s));
     const uint64_t sms = (uint64_t)sm_count();
     count_launch();
-    bucket_count_kernel<K><<<(unsigned)std::min<uint64_t>((nq + kBT * 8 - 1) / (kBT * 8), sms * 4), kBT, 0, s>>>(
-        d_q, nq, map, total);
+    bucket_count_kernel<K, B><<<(unsigned)std::min<uint64_t>((nq + kBT * 8 - 1) / (kBT * 8), sms * 4), kBT, 0, s>>>(
+        q, nq, map, total);
     count_launch();
-    bucket_start_kernel<K><<<1 + ((map.last + 2) * 8 + 1023) / 1024, 1024, 0, s>>>(t->dev, map, total, cursor, bp.first,
-                                                                                bp.items, bp.n_items);
+    bucket_start_kernel<K><<<1 + ((map.last + 2) * 8 + 1023) / 1024, 1024, 0, s>>>(
+        t->dev, map, total, cursor, bp.first, bp.items, bp.n_items);
     count_launch();
     constexpr uint64_t T = BucketSmem<K>::T;
-    bucket_scatter_kernel<K><<<(unsigned)std::min<uint64_t>((nq + T - 1) / T, sms * 2), kBT,
-                               BucketSmem<K>::bytes, s>>>(d_q, nq, map, cursor, out_q, pos);
+    bucket_scatter_kernel<K, B><<<(unsigned)std::min<uint64_t>((nq + T - 1) / T, sms * 2), kBT,
+                                  BucketSmem<K>::bytes, s>>>(q, nq, map, cursor, out_q, pos);
     BT_CUDA(cudaGetLastError());
     return BT_OK;
 }
+
+template <typename K>
+bt_status bucket_k(const bt_tree *t, const BucketMap &map, const void *d_q, const void *d_hi,
+                   uint64_t nq, void *out_q, uint32_t *pos, const BucketPlan &bp, cudaStream_t s) {
+    if (!d_hi)
+        return bucket_impl<K>(t, map, PointBatch<K>{(const K *)d_q}, nq, (K *)out_q, pos, bp, s);
+    return bucket_impl<K>(t, map, RangeBatch<K>{(const K *)d_q, (const K *)d_hi, nq}, 2 * nq,
+                          (K *)out_q, pos, bp, s);
+}
 }  // namespace
 
-bt_status launch_buckets(const bt_tree *t, const BucketMap &map, const void *d_q, uint64_t nq,
-                         void *out_q, uint32_t *pos, const BucketPlan &bp, cudaStream_t s) {
-    return t->key_bytes == 4 ? bucket_impl<uint32_t>(t, map, (const uint32_t *)d_q, nq,
-                                                     (uint32_t *)out_q, pos, bp, s)
-                             : bucket_impl<uint64_t>(t, map, (const uint64_t *)d_q, nq,
-                                                     (uint64_t *)out_q, pos, bp, s);
+bt_status launch_buckets(const bt_tree *t, const BucketMap &map, const void *d_q, const void *d_hi,
+                         uint64_t nq, void *out_q, uint32_t *pos, const BucketPlan &bp,
+                         cudaStream_t s) {
+    return t->key_bytes == 4 ? bucket_k<uint32_t>(t, map, d_q, d_hi, nq, out_q, pos, bp, s)
+                             : bucket_k<uint64_t>(t, map, d_q, d_hi, nq, out_q, pos, bp, s);
+}
+
+bt_status launch_range_gather(const bt_tree *t, const uint32_t *rank, const uint32_t *pos,
+                              const void *d_lo, const void *d_hi, uint64_t nr, uint64_t *d_counts,
+                              uint64_t *d_lb, cudaStream_t s) {
+    const unsigned grid = (unsigned)((nr + 2047) / 2048);
+    count_launch();
+    if (t->key_bytes == 4)
+        range_gather_kernel<uint32_t><<<grid, 512, 0, s>>>(rank, pos, (const uint32_t *)d_lo,
+                                                           (const uint32_t *)d_hi, nr,
+                                                           (uint32_t)t->max_key, t->n, d_counts, d_lb);
+    else
+        range_gather_kernel<uint64_t><<<grid, 512, 0, s>>>(rank, pos, (const uint64_t *)d_lo,
+                                                           (const uint64_t *)d_hi, nr, t->max_key,
+                                                           t->n, d_counts, d_lb);
+    BT_CUDA(cudaGetLastError());
+    return BT_OK;
 }
 
 bt_status launch_bucket_blocks(const bt_tree *t, uint32_t *d_blocks, cudaStream_t s) {

@@ -277,9 +277,15 @@ struct BucketPlan {
     uint4 *items;       // work items: bucket, first slot, slots
     uint32_t *n_items;  // at most kMaxBuckets + nq / kBucketSlice
 };
-// d_q ordered by bucket into out_q (query i in slot pos[i]).
-bt_status launch_buckets(const bt_tree *t, const BucketMap &map, const void *d_q, uint64_t nq,
-                         void *out_q, uint32_t *pos, const BucketPlan &bp, cudaStream_t s);
+// d_q ordered by bucket into out_q (query i in slot pos[i]).  With d_hi, the
+// 2 nq bounds of the ranges [d_q[i], d_hi[i]]: d_q[i], then d_hi[i] + 1.
+bt_status launch_buckets(const bt_tree *t, const BucketMap &map, const void *d_q, const void *d_hi,
+                         uint64_t nq, void *out_q, uint32_t *pos, const BucketPlan &bp,
+                         cudaStream_t s);
+// Counts (and lower bounds) of the ranges from the bounds' ranks.
+bt_status launch_range_gather(const bt_tree *t, const uint32_t *rank, const uint32_t *pos,
+                              const void *d_lo, const void *d_hi, uint64_t nr, uint64_t *d_counts,
+                              uint64_t *d_lb, cudaStream_t s);
 // d_out[i] = res[pos[i]], and the found flags when d_found is not null.
 bt_status launch_bucket_gather(int val_bytes, const void *res, const uint8_t *rfound,
                                const uint32_t *pos, uint64_t nq, void *d_out, uint8_t *d_found,
@@ -297,9 +303,18 @@ static_assert(kMaxBuckets == 1 << 11, "bucket_map takes 11 bits");
 // Measures t->bucket_blocks into *d_blocks (zeroed by the caller); the
 // tree's arrays, sizes and key ends are set.
 bt_status launch_bucket_blocks(const bt_tree *t, uint32_t *d_blocks, cudaStream_t s);
+// Least batches that are put into any order before the search; below them
+// the order costs more than it gives, whatever the mode asks for (2^20 point
+// queries, u32 keys, 2^20 / 2^26: 36 / 47 us directly, 65 / 77 grouped first;
+// 2^19 ranges 50 / 66 us directly, 108 / 127 grouped first).
+constexpr uint64_t kBktMinQueries = 1ull << 22;
+constexpr uint64_t kOrderMinRanges = 1ull << 20;
 // Whether a point batch is searched by buckets, and that search (workspace
 // from the pool; BT_ERR_OUT_OF_MEMORY when it cannot be had).
 bool bucket_search_pays(const bt_tree *t, uint64_t nq, cudaStream_t s);
+bool bucket_bounds_pay(const bt_tree *t, uint64_t nr, cudaStream_t s);
+bt_status launch_bucket_bounds(const bt_tree *t, const void *d_lo, const void *d_hi, uint64_t nr,
+                               uint64_t *d_counts, uint64_t *d_lb, cudaStream_t s);
 bt_status launch_bucket_search(const bt_tree *t, const void *d_q, uint64_t nq, void *d_out,
                                cudaStream_t s, uint8_t *d_found);
 

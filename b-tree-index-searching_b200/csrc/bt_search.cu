@@ -18,6 +18,7 @@
 // spread over the group's lanes, so a hit costs one HBM round trip.
 #include <map>
 #include <mutex>
+#include <type_traits>
 
 #include "bt_search.cuh"
 
@@ -272,7 +273,6 @@ point_window_kernel(const __grid_constant__ DevTree t, const K *__restrict__ q,
 // every 1,024 elements keeps a binary search's probes in different banks
 // (two instructions, where swz takes four; the window is not a power of two).
 __device__ __forceinline__ uint32_t win_slot(uint32_t p) { return p + (p >> 5) + (p >> 10); }
-constexpr uint64_t kBktMinQueries = 1ull << 22;
 constexpr size_t kBktWinBytes = 200 * 1024;
 constexpr size_t kBktWinMin = 16 * 1024;  // room for some level of any tree
 constexpr size_t win_words(size_t n) { return n + n / 32 + n / 1024 + 2; }
@@ -318,15 +318,20 @@ __device__ __forceinline__ int first_match(const uint32_t (&w)[8], K q, K tmax) 
     return q <= tmax ? at : -1;
 }
 
+// What a bucket search writes: values, or (BOUND) ranks of lower bounds.
+template <typename V, bool BOUND>
+using BktOut = std::conditional_t<BOUND, uint32_t, V>;
+
 // The qn queries of an item by their staged window: node = w0 + position in
 // the window of level wlvl, then the levels below it (lane quads, one line
 // per query and level), then the leaf block.
-template <typename K, typename V, typename W, int T>
+template <typename K, typename V, typename W, int T, bool BOUND>
 __device__ __forceinline__ void bucket_item(const DevTree &t, const W *s_win, uint32_t w0, uint32_t wm,
                                             int wlvl, K base, const K *__restrict__ q, uint32_t qn,
-                                            V *__restrict__ out, uint8_t *__restrict__ found) {
+                                            BktOut<V, BOUND> *__restrict__ out,
+                                            uint8_t *__restrict__ found) {
     using LG = LeafGeom<K, V>;
-    constexpr bool PAIR = sizeof(K) == 8;
+    constexpr bool PAIR = sizeof(K) == 8 && !BOUND;
     constexpr int U = PAIR ? 2 : 4;  // queries per thread at a time
     const int lane = threadIdx.x & 31;
     const K tmax = (K)t.max_key;
@@ -384,7 +389,17 @@ __device__ __forceinline__ void bucket_item(const DevTree &t, const W *s_win, ui
                 for (int z = 0; z < U; z++) node[z] = z == u ? r : node[z];
             }
         }
-        if constexpr (PAIR) {
+        if constexpr (BOUND) {  // position of the first key at or above the query
+            uint32_t w[U][8];
+#pragma unroll
+            for (int u = 0; u < U; u++) load_sector(leaves + (size_t)node[u] * LG::BS, w[u]);
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const K c = qv[u] < tmax ? qv[u] : tmax;
+                const uint32_t i = i0 + u * T + lane;
+                if (i < qn) out[i] = node[u] * (uint32_t)LG::S + count_below<K, LG::S>(w[u], c, false);
+            }
+        } else if constexpr (PAIR) {
             static_assert(sizeof(K) == 4 || LG::BS == 2 * kSectorBytes, "values in the second sector");
             uint32_t w[U][2][8];
             K qk[U][2];
@@ -438,11 +453,11 @@ __device__ __forceinline__ void bucket_item(const DevTree &t, const W *s_win, ui
     }
 }
 
-template <typename K, typename V, int T>
+template <typename K, typename V, int T, bool BOUND>
 __global__ void __launch_bounds__(T, 1024 / T)
 bucket_search_kernel(const __grid_constant__ DevTree t, const uint32_t *__restrict__ first,
                      const uint4 *__restrict__ items, const uint32_t *__restrict__ n_items,
-                     uint32_t win_bytes, const K *__restrict__ q, V *__restrict__ out,
+                     uint32_t win_bytes, const K *__restrict__ q, BktOut<V, BOUND> *__restrict__ out,
                      uint8_t *__restrict__ found) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int F = kLineBytes / (int)sizeof(K);
@@ -472,14 +487,14 @@ bucket_search_kernel(const __grid_constant__ DevTree t, const uint32_t *__restri
 #pragma unroll 8
         for (uint32_t i = threadIdx.x; i < wm; i += T) s_win[win_slot(i)] = (uint32_t)(src[i] - base);
         __syncthreads();
-        bucket_item<K, V, uint32_t, T>(t, s_win, w0, wm, wlvl, base, q + it.y, it.z, out + it.y,
+        bucket_item<K, V, uint32_t, T, BOUND>(t, s_win, w0, wm, wlvl, base, q + it.y, it.z, out + it.y,
                                        found ? found + it.y : nullptr);
     } else if constexpr (sizeof(K) == 8) {
         uint64_t *s_win = reinterpret_cast<uint64_t *>(smem_raw);
 #pragma unroll 8
         for (uint32_t i = threadIdx.x; i < wm; i += T) s_win[win_slot(i)] = (uint64_t)src[i];
         __syncthreads();
-        bucket_item<K, V, uint64_t, T>(t, s_win, w0, wm, wlvl, base, q + it.y, it.z, out + it.y,
+        bucket_item<K, V, uint64_t, T, BOUND>(t, s_win, w0, wm, wlvl, base, q + it.y, it.z, out + it.y,
                                        found ? found + it.y : nullptr);
     }
 }
@@ -721,21 +736,21 @@ bt_status window_launch(const bt_tree *t, const void *d_q, const uint32_t *d_per
     return BT_OK;
 }
 
-template <typename K, typename V, int T>
+template <typename K, typename V, int T, bool BOUND>
 bt_status bucket_launch(const bt_tree *t, const BucketPlan &bp, uint64_t max_items, size_t smem,
                         const void *d_q, void *d_out, uint8_t *d_found, cudaStream_t s) {
-    auto fn = bucket_search_kernel<K, V, T>;
+    auto fn = bucket_search_kernel<K, V, T, BOUND>;
     bt_status st = set_smem(fn, smem);
     if (st != BT_OK) return st;
     count_launch();
     fn<<<(unsigned)max_items, T, smem, s>>>(t->dev, bp.first, bp.items, bp.n_items, (uint32_t)smem,
-                                            (const K *)d_q, (V *)d_out, d_found);
+                                            (const K *)d_q, (BktOut<V, BOUND> *)d_out, d_found);
     BT_CUDA(cudaGetLastError());
     return BT_OK;
 }
 
-template <typename K, typename V>
-bt_status bucket_cfg(const bt_tree *t, const BucketMap &map, const BucketPlan &bp, uint64_t max_items,
+template <typename K, typename V, bool BOUND>
+bt_status bucket_cfg(const bt_tree *t, const BucketPlan &bp, uint64_t max_items,
                      const void *d_q, void *d_out, uint8_t *d_found, cudaStream_t s) {
     // the fullest bucket's window of the deepest level that fits, in 32-bit
     // entries (the kernel goes a level up where its own does not)
@@ -744,8 +759,8 @@ bt_status bucket_cfg(const bt_tree *t, const BucketMap &map, const BucketPlan &b
     while (win_words(m) * sizeof(uint32_t) > kBktWinBytes) m = (m >> LOGF) + 2;
     const size_t smem = std::max<size_t>(win_words(m) * sizeof(uint32_t), kBktWinMin);
     // two CTAs per SM where two windows fit
-    if (smem <= kBktWinBytes / 2) return bucket_launch<K, V, 512>(t, bp, max_items, smem, d_q, d_out, d_found, s);
-    return bucket_launch<K, V, 1024>(t, bp, max_items, smem, d_q, d_out, d_found, s);
+    if (smem <= kBktWinBytes / 2) return bucket_launch<K, V, 512, BOUND>(t, bp, max_items, smem, d_q, d_out, d_found, s);
+    return bucket_launch<K, V, 1024, BOUND>(t, bp, max_items, smem, d_q, d_out, d_found, s);
 }
 
 template <typename K, typename V, bool PERM>
@@ -853,9 +868,8 @@ bt_status launch_point_search(const bt_tree *t, const void *d_q, const uint32_t 
 // into few of the equal stretches (a bucket of over four times the average)
 // keep the direct search: their windows lie levels above the leaves.  So does
 // a stream under capture, whose graph then holds no allocation.
-bool bucket_search_pays(const bt_tree *t, uint64_t nq, cudaStream_t s) {
-    if (t->n == 0 || nq >= (1ull << 32)) return false;
-    if (nq < kBktMinQueries || nq < t->n_sectors / 8) return false;
+static bool buckets_suit(const bt_tree *t, uint64_t nq, cudaStream_t s) {
+    if (t->n == 0 || nq >= (1ull << 32) || nq < t->n_sectors / 8) return false;
     const uint64_t buckets = bucket_map(t->min_key, t->max_key).last + 1;
     if (t->bucket_blocks == 0 || t->bucket_blocks > 4 * (t->n_sectors / buckets) + 64) return false;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -864,35 +878,86 @@ bool bucket_search_pays(const bt_tree *t, uint64_t nq, cudaStream_t s) {
     return false;
 }
 
+bool bucket_search_pays(const bt_tree *t, uint64_t nq, cudaStream_t s) {
+    return nq >= kBktMinQueries && buckets_suit(t, nq, s);
+}
+
+// Range bounds, direct / by buckets (us; the buckets take both bounds of a
+// range as queries of their own, so its width does not matter):
+//                          2^19 ranges   2^20        2^22
+//   u32, 2^20 keys          50 / 65      83 / 77    312 / 184
+//   u32, 2^26              66 / 90     113 / 109    409 / 227
+//   u32, 2^26, 100,000 keys wide
+//                           76 / 90     133 / 110    477 / 229
+//   u64, 2^26              105 / 109    176 / 142    654 / 331
+bool bucket_bounds_pay(const bt_tree *t, uint64_t nr, cudaStream_t s) {
+    return nr >= kOrderMinRanges && nr < (1ull << 31) && t->n < (1ull << 32) && buckets_suit(t, 2 * nr, s);
+}
+
+namespace {
+// Workspace of a bucket search: the ordered queries, every query's slot, the
+// results by slot (and their found flags), the plan.
+struct BucketWs {
+    WsGuard ws;
+    unsigned char *q = nullptr, *res = nullptr;
+    uint32_t *pos = nullptr;
+    uint8_t *found = nullptr;
+    uint64_t max_items = 0;
+    BucketPlan bp;
+    explicit BucketWs(cudaStream_t s) : ws(s) {}
+    bt_status alloc(uint64_t nq, uint32_t buckets, size_t key_bytes, size_t res_bytes, bool flags) {
+        auto up256 = [](size_t x) { return (x + 255) / 256 * 256; };
+        const size_t kb = up256(nq * key_bytes), pb = up256(nq * sizeof(uint32_t));
+        const size_t rb = up256(nq * res_bytes), fb = flags ? up256(nq) : 0;
+        max_items = buckets + nq / kBucketSlice;
+        const bt_status st = ws.alloc(kb + pb + rb + fb + max_items * sizeof(uint4) +
+                                      (3 * kMaxBuckets + 64) * sizeof(uint32_t));
+        if (st != BT_OK) return st;
+        q = ws.as<unsigned char>();
+        pos = reinterpret_cast<uint32_t *>(q + kb);
+        res = q + kb + pb;
+        found = flags ? res + rb : nullptr;
+        bp.items = reinterpret_cast<uint4 *>(res + rb + fb);
+        bp.scratch = reinterpret_cast<uint32_t *>(bp.items + max_items);
+        bp.first = bp.scratch + 2 * kMaxBuckets;
+        bp.n_items = bp.first + kMaxBuckets + 1;
+        return BT_OK;
+    }
+};
+
+template <bool BOUND>
+bt_status bucket_types(const bt_tree *t, const BucketWs &w, cudaStream_t s) {
+    if (t->key_bytes == 4)
+        return t->val_bytes == 4
+                   ? bucket_cfg<uint32_t, uint32_t, BOUND>(t, w.bp, w.max_items, w.q, w.res, w.found, s)
+                   : bucket_cfg<uint32_t, uint64_t, BOUND>(t, w.bp, w.max_items, w.q, w.res, w.found, s);
+    return t->val_bytes == 4
+               ? bucket_cfg<uint64_t, uint32_t, BOUND>(t, w.bp, w.max_items, w.q, w.res, w.found, s)
+               : bucket_cfg<uint64_t, uint64_t, BOUND>(t, w.bp, w.max_items, w.q, w.res, w.found, s);
+}
+}  // namespace
+
 bt_status launch_bucket_search(const bt_tree *t, const void *d_q, uint64_t nq, void *d_out,
                                cudaStream_t s, uint8_t *d_found) {
     const BucketMap map = bucket_map(t->min_key, t->max_key);
-    auto up256 = [](size_t x) { return (x + 255) / 256 * 256; };
-    const size_t kb = up256(nq * t->key_bytes), pb = up256(nq * sizeof(uint32_t));
-    const size_t vb = up256(nq * t->val_bytes), fb = d_found ? up256(nq) : 0;
-    const uint64_t max_items = map.last + 1 + nq / kBucketSlice;
-    WsGuard ws(s);
-    bt_status st = ws.alloc(kb + pb + vb + fb + max_items * sizeof(uint4) +
-                            (3 * kMaxBuckets + 64) * sizeof(uint32_t));
+    BucketWs w(s);
+    bt_status st = w.alloc(nq, map.last + 1, t->key_bytes, t->val_bytes, d_found != nullptr);
+    if (st == BT_OK) st = launch_buckets(t, map, d_q, nullptr, nq, w.q, w.pos, w.bp, s);
+    if (st == BT_OK) st = bucket_types<false>(t, w, s);
     if (st != BT_OK) return st;
-    unsigned char *q = ws.as<unsigned char>(), *res = q + kb + pb;
-    uint32_t *pos = reinterpret_cast<uint32_t *>(q + kb);
-    uint8_t *rf = d_found ? res + vb : nullptr;
-    BucketPlan bp;
-    bp.items = reinterpret_cast<uint4 *>(res + vb + fb);
-    bp.scratch = reinterpret_cast<uint32_t *>(bp.items + max_items);
-    bp.first = bp.scratch + 2 * kMaxBuckets;
-    bp.n_items = bp.first + kMaxBuckets + 1;
-    st = launch_buckets(t, map, d_q, nq, q, pos, bp, s);
+    return launch_bucket_gather(t->val_bytes, w.res, w.found, w.pos, nq, d_out, d_found, s);
+}
+
+bt_status launch_bucket_bounds(const bt_tree *t, const void *d_lo, const void *d_hi, uint64_t nr,
+                               uint64_t *d_counts, uint64_t *d_lb, cudaStream_t s) {
+    const BucketMap map = bucket_map(t->min_key, t->max_key);
+    BucketWs w(s);
+    bt_status st = w.alloc(2 * nr, map.last + 1, t->key_bytes, sizeof(uint32_t), false);
+    if (st == BT_OK) st = launch_buckets(t, map, d_lo, d_hi, nr, w.q, w.pos, w.bp, s);
+    if (st == BT_OK) st = bucket_types<true>(t, w, s);
     if (st != BT_OK) return st;
-    if (t->key_bytes == 4)
-        st = t->val_bytes == 4 ? bucket_cfg<uint32_t, uint32_t>(t, map, bp, max_items, q, res, rf, s)
-                               : bucket_cfg<uint32_t, uint64_t>(t, map, bp, max_items, q, res, rf, s);
-    else
-        st = t->val_bytes == 4 ? bucket_cfg<uint64_t, uint32_t>(t, map, bp, max_items, q, res, rf, s)
-                               : bucket_cfg<uint64_t, uint64_t>(t, map, bp, max_items, q, res, rf, s);
-    if (st != BT_OK) return st;
-    return launch_bucket_gather(t->val_bytes, res, rf, pos, nq, d_out, d_found, s);
+    return launch_range_gather(t, reinterpret_cast<const uint32_t *>(w.res), w.pos, d_lo, d_hi, nr,
+                               d_counts, d_lb, s);
 }
 
 bt_status launch_bounds(const bt_tree *t, const void *d_lo, const void *d_hi,

@@ -98,3 +98,37 @@ def test_capture_takes_the_direct_search(bt, cuda):
         gr.replay()
         torch.cuda.synchronize()
         assert torch.equal(out.view(torch.int32), exp.view(torch.int32))
+
+
+@pytest.mark.parametrize("kt,vt", [(np.uint32, np.uint32), (np.uint64, np.uint64)])
+@pytest.mark.parametrize("kind", ["uniform", "high", "narrow", "crowded", "equal", "one", "three"])
+@pytest.mark.parametrize("width", ["near", "far"])
+def test_large_range_batches_equal_the_oracle(bt, orc, cuda, kt, vt, kind, width):
+    """2^20 ranges and a few more (both bounds by buckets): narrow and wide
+    ones, inverted ones, ends at the smallest and largest value."""
+    import torch
+    n = (1 << 20) + 77
+    g = np.random.default_rng(len(kind))
+    keys = _keys(kind, kt, g)
+    top = int(np.iinfo(kt).max)
+    lo = _batch("mixed", keys, kt, n, g)
+    if width == "near":
+        hi = np.minimum(lo, kt(top - 300)) + g.integers(0, 300, size=n).astype(kt)
+    else:
+        hi = _batch("mixed", keys, kt, n, g)
+    lo[:4], hi[:4] = [0, 0, top, top], [0, top, top, 0]
+    dlo, dhi = torch.from_numpy(lo).to(cuda), torch.from_numpy(hi).to(cuda)
+    exp = orc.range_count(keys, lo, hi)
+    with bt.Tree.build(torch.from_numpy(keys).to(cuda),
+                       torch.arange(len(keys), device=cuda).to(
+                           torch.int32 if vt == np.uint32 else torch.int64)) as t:
+        for mode in ("basic", "2d", "zorder"):
+            assert np.array_equal(t.range_count(dlo, dhi, mode=mode).cpu().numpy(), exp), mode
+        if width == "near" and exp.sum() < 1 << 27:
+            c, o, ids = t.range_search(dlo, dhi)
+            c, o, ids = c.cpu().numpy(), o.cpu().numpy(), ids.cpu().numpy()
+            assert np.array_equal(c, exp)
+            assert np.array_equal(o, np.cumsum(exp) - exp)
+            first = np.searchsorted(keys, lo)  # values are ranks: each segment counts up
+            assert np.array_equal(ids, (np.repeat(first - o.astype(np.int64), exp.astype(np.int64))
+                                        + np.arange(len(ids))).astype(vt))
