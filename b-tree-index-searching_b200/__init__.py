@@ -108,6 +108,10 @@ _PROTOS = {
     "bt_group_queries": (_I, [_P, _P, _U64, _P, _P, _P]),
     "bt_range_count": (_I, [_P, _I, _P, _P, _U64, _P, _P]),
     "bt_range_search": (_I, [_P, _I, _P, _P, _U64, _P, _P, _P, _U64, ctypes.POINTER(_U64), _P]),
+    "bt_range_search_alloc": (_I, [_P, _I, _P, _P, _U64, _P, _P, _P, ctypes.py_object,
+                                   ctypes.POINTER(_U64), _P]),
+    "bt_rect_search_alloc": (_I, [_P, _I, _P, _P, _P, _P, _U64, _P, _P, _P, ctypes.py_object,
+                                  ctypes.POINTER(_U64), _P]),
     "bt_range_count_host": (_I, [_P, _I, _P, _P, _U64, _P, _P]),
     "bt_point_search_grouped_batch": (_I, [_P, _P, _P, _U64, _P, _P]),
     "bt_kernel_launches": (ctypes.c_uint64, []),
@@ -189,6 +193,35 @@ def _is_cuda(x):
 def _torch_dtype(nbytes):
     import torch
     return {4: torch.uint32, 8: torch.uint64}[nbytes]
+
+
+class _IdBuffer:
+    """The ID tensor of one search, made when the library asks for it."""
+
+    def __init__(self, value_bytes, device):
+        self.dtype, self.device = _torch_dtype(value_bytes), device
+        self.ids, self.error = None, None
+
+    def done(self, status, where):
+        """The tensor (empty when there were no hits)."""
+        if self.error is not None:
+            raise self.error
+        _check(status, where)
+        if self.ids is None:
+            import torch
+            self.ids = torch.empty(0, dtype=self.dtype, device=self.device)
+        return self.ids
+
+
+@ctypes.CFUNCTYPE(ctypes.c_void_p, ctypes.py_object, ctypes.c_uint64)
+def _alloc_ids(buf, total):
+    import torch
+    try:
+        buf.ids = torch.empty(total, dtype=buf.dtype, device=buf.device)
+        return buf.ids.data_ptr()
+    except BaseException as e:  # raised again by done(), outside the library
+        buf.error = e
+        return None
 
 
 class Tree:
@@ -441,13 +474,12 @@ class Tree:
         offsets = torch.empty(n, dtype=torch.uint64, device=lo.device)
         total = ctypes.c_uint64(0)
         if ids_capacity is None:
-            # count first, then size the ID buffer exactly
-            st = L.bt_range_search(self._h, m, _P(lo.data_ptr()), _P(hi.data_ptr()), n,
-                                   _P(counts.data_ptr()), _P(offsets.data_ptr()), None, 0,
-                                   ctypes.byref(total), _stream_ptr(stream))
-            if st not in (0, 5):
-                _check(st, "bt_range_search")
-            ids_capacity = total.value
+            # the ID buffer is sized exactly, once the hits are counted
+            buf = _IdBuffer(self.value_bytes, lo.device)
+            st = L.bt_range_search_alloc(self._h, m, _P(lo.data_ptr()), _P(hi.data_ptr()), n,
+                                         _P(counts.data_ptr()), _P(offsets.data_ptr()), _alloc_ids,
+                                         buf, ctypes.byref(total), _stream_ptr(stream))
+            return counts, offsets, buf.done(st, "bt_range_search_alloc")
         ids = torch.empty(max(1, ids_capacity), dtype=_torch_dtype(self.value_bytes),
                           device=lo.device)
         _check(L.bt_range_search(self._h, m, _P(lo.data_ptr()), _P(hi.data_ptr()), n,
@@ -628,15 +660,12 @@ def rect_search(tree, x0, y0, x1, y1, stream=None, mode="basic"):
     counts = torch.empty(n, dtype=torch.uint64, device=x0.device)
     offsets = torch.empty(n, dtype=torch.uint64, device=x0.device)
     total = ctypes.c_uint64(0)
-    args = (tree.handle, m, _P(x0.data_ptr()), _P(y0.data_ptr()), _P(x1.data_ptr()),
-            _P(y1.data_ptr()), n, _P(counts.data_ptr()), _P(offsets.data_ptr()))
-    st = L.bt_rect_search_mode(*args, None, 0, ctypes.byref(total), _stream_ptr(stream))
-    if st not in (0, 5):
-        _check(st, "bt_rect_search_mode")
-    ids = torch.empty(max(1, total.value), dtype=_torch_dtype(tree.value_bytes), device=x0.device)
-    _check(L.bt_rect_search_mode(*args, _P(ids.data_ptr()), total.value, ctypes.byref(total),
-                                 _stream_ptr(stream)), "bt_rect_search_mode")
-    return counts, offsets, ids[: total.value]
+    buf = _IdBuffer(tree.value_bytes, x0.device)
+    st = L.bt_rect_search_alloc(tree.handle, m, _P(x0.data_ptr()), _P(y0.data_ptr()),
+                                _P(x1.data_ptr()), _P(y1.data_ptr()), n, _P(counts.data_ptr()),
+                                _P(offsets.data_ptr()), _alloc_ids, buf, ctypes.byref(total),
+                                _stream_ptr(stream))
+    return counts, offsets, buf.done(st, "bt_rect_search_alloc")
 
 
 def version():

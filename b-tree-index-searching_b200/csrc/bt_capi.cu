@@ -274,9 +274,15 @@ bt_status bt_range_count(const bt_tree *t, int mode, const void *d_lo, const voi
     return count_device(t, mode, d_lo, d_hi, nq, d_counts, nullptr, (cudaStream_t)stream);
 }
 
-bt_status bt_range_search(const bt_tree *t, int mode, const void *d_lo, const void *d_hi,
-                          uint64_t nq, uint64_t *d_counts, uint64_t *d_offsets, void *d_ids,
-                          uint64_t ids_capacity, uint64_t *h_total, void *stream) {
+}  // extern "C"
+
+namespace {
+// Counts, offsets and total, then the IDs into what ids_for(total) returns
+// (null: the call ends with the status it left in *st).
+template <typename IdsFor>
+bt_status range_search(const bt_tree *t, int mode, const void *d_lo, const void *d_hi, uint64_t nq,
+                       uint64_t *d_counts, uint64_t *d_offsets, uint64_t *h_total, void *stream,
+                       IdsFor ids_for) {
     using namespace bt;
     bt_status st = check_tree(t);
     if (st != BT_OK) return st;
@@ -289,29 +295,43 @@ bt_status bt_range_search(const bt_tree *t, int mode, const void *d_lo, const vo
     if (nq >= (1ull << 32)) return fail(BT_ERR_INVALID_ARGUMENT, "nq must be below 2^32");
     DeviceGuard g(t->device);
     cudaStream_t s = (cudaStream_t)stream;
-    uint64_t *lb = nullptr, *d_total = nullptr;
-    st = ws_alloc((void **)&lb, nq * sizeof(uint64_t), s);
-    if (st == BT_OK) st = ws_alloc((void **)&d_total, sizeof(uint64_t), s);
+    WsGuard g_lb(s), g_total(s);
+    st = g_lb.alloc(nq * sizeof(uint64_t));
+    if (st == BT_OK) st = g_total.alloc(2 * sizeof(uint64_t));
+    uint64_t *lb = g_lb.as<uint64_t>(), *d_total = g_total.as<uint64_t>();
     if (st == BT_OK) st = count_device(t, mode, d_lo, d_hi, nq, d_counts, lb, s);
     if (st == BT_OK) st = launch_scan_u64(d_counts, d_offsets, nq, d_total, s);
-    uint64_t total = 0;
-    if (st == BT_OK) {
-        cudaError_t e = cudaMemcpyAsync(&total, d_total, sizeof(total), cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess) st = cuda_fail(e, "total hits read-back");
-    }
-    if (st == BT_OK) {
-        *h_total = total;
-        if (total > ids_capacity) {
-            st = fail(BT_ERR_CAPACITY, "ids_capacity is below the total hit count");
-        } else if (total > 0) {
-            if (!d_ids) st = fail(BT_ERR_INVALID_ARGUMENT, "ids is NULL");
-            else st = launch_range_fill(t, lb, d_counts, d_offsets, nq, d_ids, s);
-        }
-    }
-    ws_free(lb, s);
-    ws_free(d_total, s);
-    return st;
+    if (st != BT_OK) return st;
+    uint64_t total[2] = {0, 0};  // hits, and the most of one range
+    BT_CUDA(cudaMemcpyAsync(total, d_total, sizeof(total), cudaMemcpyDeviceToHost, s));
+    BT_CUDA(cudaStreamSynchronize(s));
+    *h_total = total[0];
+    if (total[0] == 0) return BT_OK;
+    void *ids = ids_for(total[0], &st);
+    if (!ids) return st;
+    return launch_range_fill(t, lb, d_counts, d_offsets, nq, total[1], ids, s);
+}
+}  // namespace
+
+extern "C" {
+
+bt_status bt_range_search(const bt_tree *t, int mode, const void *d_lo, const void *d_hi,
+                          uint64_t nq, uint64_t *d_counts, uint64_t *d_offsets, void *d_ids,
+                          uint64_t ids_capacity, uint64_t *h_total, void *stream) {
+    return range_search(t, mode, d_lo, d_hi, nq, d_counts, d_offsets, h_total, stream,
+                        [&](uint64_t total, bt_status *st) {
+                            return bt::ids_buffer(d_ids, ids_capacity, total, st);
+                        });
+}
+
+bt_status bt_range_search_alloc(const bt_tree *t, int mode, const void *d_lo, const void *d_hi,
+                                uint64_t nq, uint64_t *d_counts, uint64_t *d_offsets,
+                                bt_ids_alloc alloc, void *ctx, uint64_t *h_total, void *stream) {
+    if (!alloc) return bt::fail(BT_ERR_INVALID_ARGUMENT, "alloc is NULL");
+    return range_search(t, mode, d_lo, d_hi, nq, d_counts, d_offsets, h_total, stream,
+                        [&](uint64_t total, bt_status *st) {
+                            return bt::ids_from(alloc, ctx, total, st);
+                        });
 }
 
 bt_status bt_range_count_host(const bt_tree *t, int mode, const void *h_lo, const void *h_hi,

@@ -841,10 +841,12 @@ __global__ void __launch_bounds__(kST) scan_reduce_kernel(const T *__restrict__ 
     if (threadIdx.x == 0) sums[blockIdx.x] = total;
 }
 
+// total_max (optional): [0] = sum of the inputs, [1] (zeroed before) = the
+// largest.
 template <typename T>
 __global__ void __launch_bounds__(kST)
 scan_down_kernel(const T *__restrict__ in, uint64_t n, const T *__restrict__ offs,
-                 T *__restrict__ out, T *__restrict__ grand_total) {
+                 T *__restrict__ out, T *__restrict__ total_max) {
     __shared__ T s_warp[kST / 32];
     __shared__ T total;
     const uint64_t t0 = (uint64_t)blockIdx.x * kSTile + (uint64_t)threadIdx.x * kSIPT;
@@ -861,8 +863,20 @@ scan_down_kernel(const T *__restrict__ in, uint64_t n, const T *__restrict__ off
         if (t0 + j < n) out[t0 + j] = run;
         run += v[j];
     }
-    if (grand_total && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0)
-        *grand_total = total + (offs ? offs[blockIdx.x] : (T)0);
+    if (total_max) {
+        T m = 0;
+#pragma unroll
+        for (int j = 0; j < kSIPT; j++) m = v[j] > m ? v[j] : m;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const T y = __shfl_xor_sync(0xffffffffu, m, o);
+            m = y > m ? y : m;
+        }
+        if ((threadIdx.x & 31) == 0 && m)
+            atomicMax(reinterpret_cast<unsigned long long *>(total_max) + 1, (unsigned long long)m);
+        if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0)
+            *total_max = total + (offs ? offs[blockIdx.x] : (T)0);
+    }
 }
 
 // Scratch elements scan_run needs for n inputs (block sums and offsets of
@@ -877,11 +891,12 @@ uint64_t scan_ws_elems(uint64_t n) {
 }
 
 // Exclusive scan d_out = scan(d_in) with caller-provided scratch (ws of
-// scan_ws_elems(n) elements); *d_total (optional) receives the sum.
+// scan_ws_elems(n) elements); d_total (optional, two words) receives the sum
+// and the largest input.
 template <typename T>
 bt_status scan_run(const T *d_in, T *d_out, uint64_t n, T *d_total, T *ws, cudaStream_t s) {
     if (n == 0) {
-        if (d_total) BT_CUDA(cudaMemsetAsync(d_total, 0, sizeof(T), s));
+        if (d_total) BT_CUDA(cudaMemsetAsync(d_total, 0, 2 * sizeof(T), s));
         return BT_OK;
     }
     const uint64_t nb = (n + kSTile - 1) / kSTile;
@@ -904,6 +919,7 @@ bt_status scan_run(const T *d_in, T *d_out, uint64_t n, T *d_total, T *ws, cudaS
 
 template <typename T>
 bt_status scan_impl(const T *d_in, T *d_out, uint64_t n, T *d_total, cudaStream_t s) {
+    if (d_total) BT_CUDA(cudaMemsetAsync(d_total, 0, 2 * sizeof(T), s));
     const uint64_t we = scan_ws_elems(n);
     T *ws = nullptr;
     if (we) {
@@ -1066,8 +1082,12 @@ bt_status partition_point_prealloc(const bt_tree *t, const K *d_q, uint64_t nq, 
 // --------------------------------------------------------- range fill ----
 
 // One warp per query: ids[off .. off+cnt) = values of positions lb .. lb+cnt
-// (read from the leaf blocks, S values per block).
-template <typename K, typename V>
+// (read from the leaf blocks, S values per block).  SORT: up to kWarpSortCap
+// values are put in ascending order on the way (in registers; a fill and a
+// sort of its own read and wrote every ID once more: 2^20 ranges, 34 M IDs,
+// 0.169 + 0.220 ms, fused 0.263).  A warp takes 32 consecutive queries at a
+// time, so that their counts, bounds and offsets arrive in three loads.
+template <typename K, typename V, bool SORT>
 __global__ void __launch_bounds__(256)
 range_fill_kernel(const unsigned char *__restrict__ leaves, const uint64_t *__restrict__ lb,
                   const uint64_t *__restrict__ cnt, const uint64_t *__restrict__ off, uint64_t nq,
@@ -1076,68 +1096,93 @@ range_fill_kernel(const unsigned char *__restrict__ leaves, const uint64_t *__re
     const int lane = threadIdx.x & 31;
     const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
     const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t i = warp; i < nq; i += nw) {
-        const uint64_t c = cnt[i], l = lb[i], o = off[i];
-        for (uint64_t k = lane; k < c; k += 32) {
-            const uint64_t p = l + k;
-            ids[o + k] = reinterpret_cast<const V *>(leaves + (p / LG::S) * LG::BS +
-                                                     kSectorBytes)[p % LG::S];
+    auto value = [&](uint64_t p) {
+        return __ldg(reinterpret_cast<const V *>(leaves + (p / LG::S) * LG::BS + kSectorBytes) + p % LG::S);
+    };
+    for (uint64_t i0 = warp * 32; i0 < nq; i0 += nw * 32) {
+        const uint64_t i = i0 + lane;
+        const uint64_t mc = i < nq ? cnt[i] : 0, ml = i < nq ? lb[i] : 0, mo = i < nq ? off[i] : 0;
+        unsigned todo = __ballot_sync(0xffffffffu, mc != 0);
+        while (todo) {
+            const int j = __ffs((int)todo) - 1;
+            todo &= todo - 1;
+            const uint64_t c = __shfl_sync(0xffffffffu, mc, j), l = __shfl_sync(0xffffffffu, ml, j);
+            V *dst = ids + __shfl_sync(0xffffffffu, mo, j);
+            if (SORT && c > 1 && c <= (uint64_t)kWarpSortCap) {
+                auto at = [&](uint32_t e) { return value(l + e); };
+                warp_sort_small<V>(at, dst, (uint32_t)c, lane);
+            } else {
+                for (uint64_t k = lane; k < c; k += 32) dst[k] = value(l + k);
+            }
         }
     }
 }
 
-// Sorts each query's ID segment when values do not ascend with keys, in
-// three tiers by length.  Up to kWarpSortCap values: one warp sorts the
-// segment in registers (warp_sort_small, a bitonic network) and writes it
-// back.  Up to kSortCap: one CTA per segment, bitonic network in shared
-// memory; the warp pass lists these segments.  Longer: listed afterwards and
-// sorted one CTA each by a bitonic network over a padded copy in global
-// memory.
+// Sorts each query's ID segment when values do not ascend with keys.  Up to
+// kWarpSortCap values: sorted by the pass that wrote them, one warp in
+// registers (warp_sort_small, a bitonic network).  Up to kWarpLongCap: the
+// same, by a pass of its own over the listed segments.  Up to kSortCap: one
+// CTA per segment, bitonic network in shared memory.  Longer: one CTA each by
+// a bitonic network over a padded copy in global memory.
+constexpr int kWarpLongCap = 1024;
 constexpr int kSortCap = 4096;
 constexpr unsigned int kMedListCap = 1u << 16;
-constexpr int kWSortThreads = 256;
 
-// stat[0]: segments of kWarpSortCap < c <= kSortCap (listed in med_list up
-// to kMedListCap); stat[1]: set if a segment is longer than kSortCap.  With
-// skip_small, segments of up to kWarpSortCap values are already sorted.
-template <typename V>
-__global__ void __launch_bounds__(kWSortThreads)
-warp_segment_sort_kernel(const uint64_t *__restrict__ cnt, const uint64_t *__restrict__ off,
-                         uint64_t nq, V *__restrict__ ids, unsigned int *__restrict__ stat,
-                         uint64_t *__restrict__ med_list, bool skip_small) {
-    const int lane = threadIdx.x & 31;
-    const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t i = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; i < nq; i += nw) {
+// Lists the segments of kWarpSortCap < c <= kSortCap (*n_med of them, the
+// first kMedListCap in med_list).
+__global__ void __launch_bounds__(256)
+list_med_segments(const uint64_t *__restrict__ cnt, uint64_t nq, unsigned int *__restrict__ n_med,
+                  uint64_t *__restrict__ med_list) {
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < nq;
+         i += (uint64_t)gridDim.x * blockDim.x) {
         const uint64_t c = cnt[i];
-        if (c < 2) continue;
-        if (c > (uint64_t)kWarpSortCap) {
-            if (lane == 0) {
-                if (c > (uint64_t)kSortCap) {
-                    atomicOr(&stat[1], 1u);
-                } else {
-                    const unsigned int k = atomicAdd(&stat[0], 1u);
-                    if (k < kMedListCap) med_list[k] = i;
-                }
-            }
-            continue;
+        if (c > (uint64_t)kWarpSortCap && c <= (uint64_t)kSortCap) {
+            const unsigned int k = atomicAdd(n_med, 1u);
+            if (k < kMedListCap) med_list[k] = i;
         }
-        if (skip_small) continue;
-        V *seg = ids + off[i];
-        warp_sort_small<V>(seg, seg, (uint32_t)c, lane);
     }
 }
 
-// One CTA per medium segment: the listed ones (list != null, n entries), or
-// every segment with kWarpSortCap < c <= kSortCap (list == null, n = nq).
+// One warp per listed segment of up to kWarpLongCap values (every segment
+// when the list overflowed).  A CTA per segment, its network in shared memory
+// with a barrier per step, took 0.43 ms for some
+// 14,000 segments of 257 to 400 values; this takes 0.058.
+template <typename V>
+__global__ void __launch_bounds__(128)
+warp_long_sort_kernel(const uint64_t *__restrict__ cnt, const uint64_t *__restrict__ off, uint64_t nq,
+                      const unsigned int *__restrict__ n_med, const uint64_t *__restrict__ med_list,
+                      V *__restrict__ ids) {
+    const int lane = threadIdx.x & 31;
+    const unsigned int nm = *n_med;
+    const bool listed = nm <= kMedListCap;
+    const uint64_t n = listed ? nm : nq;
+    const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    for (uint64_t k = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; k < n; k += nw) {
+        const uint64_t i = listed ? med_list[k] : k;
+        const uint64_t c = cnt[i];
+        if (c <= (uint64_t)kWarpSortCap || c > (uint64_t)kWarpLongCap) continue;
+        V *seg = ids + off[i];
+        auto at = [&](uint32_t e) { return seg[e]; };
+        if (c <= 512) warp_sort_copy<V, 16>(at, seg, (uint32_t)c, lane);
+        else warp_sort_copy<V, 32>(at, seg, (uint32_t)c, lane);
+    }
+}
+
+// One CTA per segment of kWarpLongCap < c <= kSortCap: the listed ones, or
+// every one when the list overflowed.
 template <typename V>
 __global__ void __launch_bounds__(512)
-segment_sort_kernel(const uint64_t *__restrict__ cnt, const uint64_t *__restrict__ off,
-                    const uint64_t *__restrict__ list, uint64_t n, V *__restrict__ ids) {
+segment_sort_kernel(const uint64_t *__restrict__ cnt, const uint64_t *__restrict__ off, uint64_t nq,
+                    const unsigned int *__restrict__ n_med, const uint64_t *__restrict__ list,
+                    V *__restrict__ ids) {
     __shared__ V buf[kSortCap];
+    const unsigned int nm = *n_med;
+    const bool listed = nm <= kMedListCap;
+    const uint64_t n = listed ? nm : nq;
     for (uint64_t li = blockIdx.x; li < n; li += gridDim.x) {
-        const uint64_t i = list ? list[li] : li;
+        const uint64_t i = listed ? list[li] : li;
         const uint64_t c = cnt[i];
-        if (c <= (uint64_t)kWarpSortCap || c > (uint64_t)kSortCap) continue;
+        if (c <= (uint64_t)kWarpLongCap || c > (uint64_t)kSortCap) continue;
         uint32_t p2 = 1;
         while (p2 < c) p2 <<= 1;
         V *seg = ids + off[i];
@@ -1361,68 +1406,70 @@ bt_status launch_bucket_gather(int val_bytes, const void *res, const uint8_t *rf
     return BT_OK;
 }
 
-bt_status launch_range_fill(const bt_tree *t, const uint64_t *d_lb, const uint64_t *d_counts,
-                            const uint64_t *d_offsets, uint64_t nq, void *d_ids, cudaStream_t s) {
-    if (nq == 0 || t->n == 0) return BT_OK;
-    const unsigned grid = (unsigned)std::min<uint64_t>((nq + 7) / 8, (uint64_t)sm_count() * 8);
-    count_launch();
+namespace {
+template <typename K, typename V>
+void range_fill(const bt_tree *t, const uint64_t *d_lb, const uint64_t *d_counts,
+                const uint64_t *d_offsets, uint64_t nq, V *ids, cudaStream_t s) {
+    const unsigned grid = (unsigned)std::min<uint64_t>((nq + 255) / 256, (uint64_t)sm_count() * 8);
     const unsigned char *lv = (const unsigned char *)t->d_leaves;
-    if (t->key_bytes == 4 && t->val_bytes == 4)
-        range_fill_kernel<uint32_t, uint32_t><<<grid, 256, 0, s>>>(lv, d_lb, d_counts, d_offsets,
-                                                                   nq, (uint32_t *)d_ids);
-    else if (t->key_bytes == 4)
-        range_fill_kernel<uint32_t, uint64_t><<<grid, 256, 0, s>>>(lv, d_lb, d_counts, d_offsets,
-                                                                   nq, (uint64_t *)d_ids);
-    else if (t->val_bytes == 4)
-        range_fill_kernel<uint64_t, uint32_t><<<grid, 256, 0, s>>>(lv, d_lb, d_counts, d_offsets,
-                                                                   nq, (uint32_t *)d_ids);
+    if (t->values_sorted)
+        range_fill_kernel<K, V, false><<<grid, 256, 0, s>>>(lv, d_lb, d_counts, d_offsets, nq, ids);
     else
-        range_fill_kernel<uint64_t, uint64_t><<<grid, 256, 0, s>>>(lv, d_lb, d_counts, d_offsets,
-                                                                   nq, (uint64_t *)d_ids);
+        range_fill_kernel<K, V, true><<<grid, 256, 0, s>>>(lv, d_lb, d_counts, d_offsets, nq, ids);
+}
+}  // namespace
+
+bt_status launch_range_fill(const bt_tree *t, const uint64_t *d_lb, const uint64_t *d_counts,
+                            const uint64_t *d_offsets, uint64_t nq, uint64_t max_count, void *d_ids,
+                            cudaStream_t s) {
+    if (nq == 0 || t->n == 0) return BT_OK;
+    count_launch();
+    if (t->key_bytes == 4 && t->val_bytes == 4)
+        range_fill<uint32_t, uint32_t>(t, d_lb, d_counts, d_offsets, nq, (uint32_t *)d_ids, s);
+    else if (t->key_bytes == 4)
+        range_fill<uint32_t, uint64_t>(t, d_lb, d_counts, d_offsets, nq, (uint64_t *)d_ids, s);
+    else if (t->val_bytes == 4)
+        range_fill<uint64_t, uint32_t>(t, d_lb, d_counts, d_offsets, nq, (uint32_t *)d_ids, s);
+    else
+        range_fill<uint64_t, uint64_t>(t, d_lb, d_counts, d_offsets, nq, (uint64_t *)d_ids, s);
     BT_CUDA(cudaGetLastError());
     if (t->values_sorted) return BT_OK;
-    return launch_segment_sort(t, d_counts, d_offsets, nq, d_ids, s);
+    return launch_segment_sort(t, d_counts, d_offsets, nq, max_count, d_ids, s);
 }
 
 bt_status launch_segment_sort(const bt_tree *t, const uint64_t *d_counts, const uint64_t *d_offsets,
-                              uint64_t nq, void *d_ids, cudaStream_t s, bool small_sorted) {
-    if (nq == 0) return BT_OK;
+                              uint64_t nq, uint64_t max_count, void *d_ids, cudaStream_t s) {
+    if (nq == 0 || max_count <= (uint64_t)kWarpSortCap) return BT_OK;
     WsGuard g_stat(s), g_med(s);
-    bt_status st = g_stat.alloc(2 * sizeof(unsigned int));
+    bt_status st = g_stat.alloc(sizeof(unsigned int));
     if (st == BT_OK) st = g_med.alloc(kMedListCap * sizeof(uint64_t));
     if (st != BT_OK) return st;
     unsigned int *stat = g_stat.as<unsigned int>();
     uint64_t *med = g_med.as<uint64_t>();
-    BT_CUDA(cudaMemsetAsync(stat, 0, 2 * sizeof(unsigned int), s));
-    const unsigned gw = (unsigned)std::min<uint64_t>((nq + kWSortThreads / 32 - 1) / (kWSortThreads / 32),
-                                                     (uint64_t)sm_count() * 8);
+    BT_CUDA(cudaMemsetAsync(stat, 0, sizeof(unsigned int), s));
+    const unsigned sms = (unsigned)sm_count();
+    count_launch();
+    list_med_segments<<<(unsigned)std::min<uint64_t>((nq + 255) / 256, sms * 8), 256, 0, s>>>(
+        d_counts, nq, stat, med);
     count_launch();
     if (t->val_bytes == 4)
-        warp_segment_sort_kernel<uint32_t><<<gw, kWSortThreads, 0, s>>>(d_counts, d_offsets, nq,
-                                                                        (uint32_t *)d_ids, stat, med,
-                                                                        small_sorted);
+        warp_long_sort_kernel<uint32_t><<<sms * 4, 128, 0, s>>>(d_counts, d_offsets, nq, stat, med,
+                                                                (uint32_t *)d_ids);
     else
-        warp_segment_sort_kernel<uint64_t><<<gw, kWSortThreads, 0, s>>>(d_counts, d_offsets, nq,
-                                                                        (uint64_t *)d_ids, stat, med,
-                                                                        small_sorted);
-    unsigned int h[2] = {0, 0};
-    BT_CUDA(cudaMemcpyAsync(h, stat, sizeof(h), cudaMemcpyDeviceToHost, s));
-    BT_CUDA(cudaStreamSynchronize(s));
-    if (h[0] > 0) {
-        // medium segments: the list, or (if it overflowed) every segment
-        const bool listed = h[0] <= kMedListCap;
-        const uint64_t n = listed ? h[0] : nq;
-        const unsigned g2 = (unsigned)std::min<uint64_t>(n, (uint64_t)sm_count() * 4);
+        warp_long_sort_kernel<uint64_t><<<sms * 4, 128, 0, s>>>(d_counts, d_offsets, nq, stat, med,
+                                                                (uint64_t *)d_ids);
+    BT_CUDA(cudaGetLastError());
+    if (max_count > (uint64_t)kWarpLongCap) {
         count_launch();
         if (t->val_bytes == 4)
-            segment_sort_kernel<uint32_t><<<g2, 512, 0, s>>>(d_counts, d_offsets, listed ? med : nullptr,
-                                                             n, (uint32_t *)d_ids);
+            segment_sort_kernel<uint32_t><<<sms * 4, 512, 0, s>>>(d_counts, d_offsets, nq, stat, med,
+                                                                  (uint32_t *)d_ids);
         else
-            segment_sort_kernel<uint64_t><<<g2, 512, 0, s>>>(d_counts, d_offsets, listed ? med : nullptr,
-                                                             n, (uint64_t *)d_ids);
+            segment_sort_kernel<uint64_t><<<sms * 4, 512, 0, s>>>(d_counts, d_offsets, nq, stat, med,
+                                                                  (uint64_t *)d_ids);
         BT_CUDA(cudaGetLastError());
     }
-    if (!h[1]) return BT_OK;
+    if (max_count <= (uint64_t)kSortCap) return BT_OK;
     // some segments exceed the shared-memory sort: list and sort them one CTA each
     const unsigned int max_list = 1u << 16;
     WsGuard g_list(s);

@@ -211,6 +211,7 @@ bt_status launch_bounds(const bt_tree *t, const void *d_lo, const void *d_hi,
 bt_status launch_partition(const bt_tree *t, int kind, const void *d_a, const void *d_b,
                            uint64_t nq, void *d_out_a, void *d_out_b, uint32_t *d_perm,
                            cudaStream_t s);
+// d_total: two words, the sum and the largest input.
 bt_status launch_scan_u64(const uint64_t *d_in, uint64_t *d_out, uint64_t n, uint64_t *d_total,
                           cudaStream_t s);
 // Point-query partition into caller memory: ws must hold
@@ -219,8 +220,10 @@ size_t partition_point_ws_bytes(uint64_t nq);
 bt_status launch_partition_point_prealloc(const bt_tree *t, const void *d_q, uint64_t nq,
                                           void *out_q, uint32_t *out_perm, void *ws,
                                           cudaStream_t s);
+// IDs of every range, sorted ascending; max_count = the largest count.
 bt_status launch_range_fill(const bt_tree *t, const uint64_t *d_lb, const uint64_t *d_counts,
-                            const uint64_t *d_offsets, uint64_t nq, void *d_ids, cudaStream_t s);
+                            const uint64_t *d_offsets, uint64_t nq, uint64_t max_count, void *d_ids,
+                            cudaStream_t s);
 // Stable sort of n (key, value) pairs by key on the device: LSD radix sort
 // with 8-bit digits (key_bytes passes of the partition kernels, carrying the
 // input index), then one gather of the values.  Equal keys keep their input
@@ -230,10 +233,10 @@ bt_status launch_sort_pairs(int key_bytes, int value_bytes, const void *d_keys, 
 // Stable order of n 16-bit keys (the low halves of d_keys): d_perm[g] = the
 // index of the item in position g (two 8-bit passes of the partition).
 bt_status launch_order_u16(const uint32_t *d_keys, uint64_t n, uint32_t *d_perm, cudaStream_t s);
-// Sorts each segment ids[offsets[i] .. + counts[i]) ascending (value width
-// of t).  small_sorted: segments of up to 256 values are sorted already.
+// Sorts the segments ids[offsets[i] .. + counts[i]) longer than 256 values
+// (shorter ones are sorted as they are written); max_count = the largest.
 bt_status launch_segment_sort(const bt_tree *t, const uint64_t *d_counts, const uint64_t *d_offsets,
-                              uint64_t nseg, void *d_ids, cudaStream_t s, bool small_sorted = false);
+                              uint64_t nseg, uint64_t max_count, void *d_ids, cudaStream_t s);
 
 // (lanes per query, rounds) -> index of the search configuration table in
 // bt_search.cu, or -1.
@@ -241,6 +244,20 @@ int search_cfg_index(int lanes, int rounds);
 int default_search_cfg(int key_bytes);
 int search_cfg_lanes(int cfg);
 int search_cfg_rounds(int cfg);
+
+// Where a search writes its `total` > 0 IDs: the caller's buffer if it is
+// large enough, or what the caller's function returns.  Null: *st says why.
+inline void *ids_buffer(void *ids, uint64_t capacity, uint64_t total, bt_status *st) {
+    if (total > capacity) *st = fail(BT_ERR_CAPACITY, "ids_capacity is below the total hit count");
+    else if (!ids) *st = fail(BT_ERR_INVALID_ARGUMENT, "ids is NULL");
+    else return ids;
+    return nullptr;
+}
+inline void *ids_from(bt_ids_alloc alloc, void *ctx, uint64_t total, bt_status *st) {
+    void *ids = alloc(ctx, total);
+    if (!ids) *st = fail(BT_ERR_OUT_OF_MEMORY, "the ID allocation function returned NULL");
+    return ids;
+}
 
 void free_learned(bt::LearnedState *s);
 // Learned point search of d_q into d_out on s (the tree has a learned index;

@@ -1218,7 +1218,7 @@ bt_status train_impl(bt_tree *t, const bt_learned_config &cfg, cudaStream_t s,
     DevBuf bcnt, boff, btot;
     BT_CUDA(cudaMalloc(&bcnt.p, nchunks * sizeof(uint64_t)));
     BT_CUDA(cudaMalloc(&boff.p, nchunks * sizeof(uint64_t)));
-    BT_CUDA(cudaMalloc(&btot.p, sizeof(uint64_t)));
+    BT_CUDA(cudaMalloc(&btot.p, 2 * sizeof(uint64_t)));
     uint64_t *cnt = (uint64_t *)bcnt.p, *off = (uint64_t *)boff.p, *tot = (uint64_t *)btot.p;
     const unsigned pg = (unsigned)((nchunks * 32 + kPlaThreads - 1) / kPlaThreads);
     auto count_at = [&](uint32_t eps, uint64_t *total) -> bt_status {

@@ -344,7 +344,7 @@ rect_fill_kernel(const __grid_constant__ DevTree t, const uint16_t *__restrict__
         }
         if (buffered) {
             __syncwarp();
-            warp_sort_small<V>(buf, ids + offsets[i], (uint32_t)cnt, lane);
+            warp_sort_small<V>([&](uint32_t e) { return buf[e]; }, ids + offsets[i], (uint32_t)cnt, lane);
             __syncwarp();
         }
     }
@@ -364,10 +364,10 @@ __global__ void rect_group_key_kernel(const uint16_t *__restrict__ x0s,
     }
 }
 
-template <typename V>
+template <typename V, typename IdsFor>
 bt_status rect_impl(const bt_tree *t, int mode, const uint16_t *x0, const uint16_t *y0,
                     const uint16_t *x1, const uint16_t *y1, uint64_t nr, uint64_t *counts,
-                    uint64_t *offsets, void *ids, uint64_t cap, uint64_t *h_total, cudaStream_t s) {
+                    uint64_t *offsets, IdsFor ids_for, uint64_t *h_total, cudaStream_t s) {
     const size_t smem = ((size_t)t->dev.smem_bytes + 15) / 16 * 16 + (size_t)kRWarps * 32 * sizeof(uint32_t);
     auto kc = rect_count_kernel<V>;
     auto kf = rect_fill_kernel<V>;
@@ -379,7 +379,7 @@ bt_status rect_impl(const bt_tree *t, int mode, const uint16_t *x0, const uint16
         1, std::min<uint64_t>((nr + kRWarps - 1) / kRWarps, (uint64_t)sm_count() * std::max(per_sm, 1)));
     WsGuard g_runs(s), g_total(s), g_order(s), g_key(s);
     bt_status st = g_runs.alloc(nr * kMaxCells * sizeof(uint2));
-    if (st == BT_OK) st = g_total.alloc(sizeof(uint64_t));
+    if (st == BT_OK) st = g_total.alloc(2 * sizeof(uint64_t));
     if (st != BT_OK) return st;
     uint2 *runs = g_runs.as<uint2>();
     uint64_t *d_total = g_total.as<uint64_t>();
@@ -401,49 +401,30 @@ bt_status rect_impl(const bt_tree *t, int mode, const uint16_t *x0, const uint16
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) st = cuda_fail(e, "rectangle count pass");
     if (st == BT_OK) st = launch_scan_u64(counts, offsets, nr, d_total, s);
-    uint64_t total = 0;
-    if (st == BT_OK) {
-        e = cudaMemcpyAsync(&total, d_total, sizeof(total), cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess) st = cuda_fail(e, "rectangle total read-back");
-    }
-    if (st == BT_OK) {
-        *h_total = total;
-        if (total > cap) {
-            st = fail(BT_ERR_CAPACITY, "ids_capacity is below the total hit count");
-        } else if (total > 0 && !ids) {
-            st = fail(BT_ERR_INVALID_ARGUMENT, "ids is NULL");
-        } else if (total > 0) {
-            const unsigned fgrid = (unsigned)std::max<uint64_t>(
-                1, std::min<uint64_t>((nr + kRWarps - 1) / kRWarps, (uint64_t)sm_count() * 4));
-            count_launch();
-            kf<<<fgrid, kRThreads, 0, s>>>(t->dev, x0, y0, x1, y1, order, nr, runs, counts, offsets,
-                                           (V *)ids);
-            e = cudaGetLastError();
-            if (e != cudaSuccess) st = cuda_fail(e, "rectangle fill pass");
-            if (st == BT_OK) st = launch_segment_sort(t, counts, offsets, nr, ids, s, true);
-        }
-    }
-    return st;
+    if (st != BT_OK) return st;
+    uint64_t total[2] = {0, 0};  // hits, and the most of one box
+    BT_CUDA(cudaMemcpyAsync(total, d_total, sizeof(total), cudaMemcpyDeviceToHost, s));
+    BT_CUDA(cudaStreamSynchronize(s));
+    *h_total = total[0];
+    if (total[0] == 0) return BT_OK;
+    void *ids = ids_for(total[0], &st);
+    if (!ids) return st;
+    const unsigned fgrid = (unsigned)std::max<uint64_t>(
+        1, std::min<uint64_t>((nr + kRWarps - 1) / kRWarps, (uint64_t)sm_count() * 4));
+    count_launch();
+    kf<<<fgrid, kRThreads, 0, s>>>(t->dev, x0, y0, x1, y1, order, nr, runs, counts, offsets, (V *)ids);
+    BT_CUDA(cudaGetLastError());
+    return launch_segment_sort(t, counts, offsets, nr, total[1], ids, s);
 }
 
 }  // namespace
 }  // namespace bt
 
-extern "C" {
-
-bt_status bt_rect_search(const bt_tree *t, const uint16_t *x0, const uint16_t *y0,
-                         const uint16_t *x1, const uint16_t *y1, uint64_t nr, uint64_t *counts,
-                         uint64_t *offsets, void *ids, uint64_t cap, uint64_t *h_total,
-                         void *stream) {
-    return bt_rect_search_mode(t, BT_RANGE_BASIC, x0, y0, x1, y1, nr, counts, offsets, ids, cap,
-                               h_total, stream);
-}
-
-bt_status bt_rect_search_mode(const bt_tree *t, int mode, const uint16_t *x0, const uint16_t *y0,
-                              const uint16_t *x1, const uint16_t *y1, uint64_t nr,
-                              uint64_t *counts, uint64_t *offsets, void *ids, uint64_t cap,
-                              uint64_t *h_total, void *stream) {
+namespace {
+template <typename IdsFor>
+bt_status rect_search(const bt_tree *t, int mode, const uint16_t *x0, const uint16_t *y0,
+                      const uint16_t *x1, const uint16_t *y1, uint64_t nr, uint64_t *counts,
+                      uint64_t *offsets, uint64_t *h_total, void *stream, IdsFor ids_for) {
     using namespace bt;
     if (!t) return fail(BT_ERR_INVALID_ARGUMENT, "tree is NULL");
     if (mode != BT_RANGE_BASIC && mode != BT_RANGE_GROUPED_2D && mode != BT_RANGE_ZORDER)
@@ -470,10 +451,38 @@ bt_status bt_rect_search_mode(const bt_tree *t, int mode, const uint16_t *x0, co
     }
     const bt_status st =
         t->val_bytes == 4
-            ? rect_impl<uint32_t>(t, mode, x0, y0, x1, y1, nr, counts, offsets, ids, cap, h_total, s)
-            : rect_impl<uint64_t>(t, mode, x0, y0, x1, y1, nr, counts, offsets, ids, cap, h_total, s);
+            ? rect_impl<uint32_t>(t, mode, x0, y0, x1, y1, nr, counts, offsets, ids_for, h_total, s)
+            : rect_impl<uint64_t>(t, mode, x0, y0, x1, y1, nr, counts, offsets, ids_for, h_total, s);
     if (prev != t->device) cudaSetDevice(prev);
     return st;
+}
+}  // namespace
+
+extern "C" {
+
+bt_status bt_rect_search(const bt_tree *t, const uint16_t *x0, const uint16_t *y0,
+                         const uint16_t *x1, const uint16_t *y1, uint64_t nr, uint64_t *counts,
+                         uint64_t *offsets, void *ids, uint64_t cap, uint64_t *h_total,
+                         void *stream) {
+    return bt_rect_search_mode(t, BT_RANGE_BASIC, x0, y0, x1, y1, nr, counts, offsets, ids, cap,
+                               h_total, stream);
+}
+
+bt_status bt_rect_search_mode(const bt_tree *t, int mode, const uint16_t *x0, const uint16_t *y0,
+                              const uint16_t *x1, const uint16_t *y1, uint64_t nr,
+                              uint64_t *counts, uint64_t *offsets, void *ids, uint64_t cap,
+                              uint64_t *h_total, void *stream) {
+    return rect_search(t, mode, x0, y0, x1, y1, nr, counts, offsets, h_total, stream,
+                       [&](uint64_t total, bt_status *st) { return bt::ids_buffer(ids, cap, total, st); });
+}
+
+bt_status bt_rect_search_alloc(const bt_tree *t, int mode, const uint16_t *x0, const uint16_t *y0,
+                               const uint16_t *x1, const uint16_t *y1, uint64_t nr,
+                               uint64_t *counts, uint64_t *offsets, bt_ids_alloc alloc, void *ctx,
+                               uint64_t *h_total, void *stream) {
+    if (!alloc) return bt::fail(BT_ERR_INVALID_ARGUMENT, "alloc is NULL");
+    return rect_search(t, mode, x0, y0, x1, y1, nr, counts, offsets, h_total, stream,
+                       [&](uint64_t total, bt_status *st) { return bt::ids_from(alloc, ctx, total, st); });
 }
 
 }  // extern "C"

@@ -1,4 +1,4 @@
-// Warp-level sort of short value lists (up to 256 values), shared by the
+// Warp-level sort of short value lists (up to 1,024 values), shared by the
 // segment sort of range/rectangle results and the rectangle fill pass.
 //
 // The values sit in registers in striped order -- value e = m * 32 + lane in
@@ -47,15 +47,15 @@ __device__ __forceinline__ void warp_bitonic_sort(V (&v)[E], int lane) {
     }
 }
 
-// dst[0..c) = src[0..c) sorted ascending, c <= 32 * E; src may equal dst.
-// Every lane of the warp must call it.
-template <typename V, int E>
-__device__ __forceinline__ void warp_sort_copy(const V *src, V *dst, uint32_t c, int lane) {
+// dst[0..c) = src(0) .. src(c - 1) sorted ascending, c <= 32 * E; src may read
+// dst.  Every lane of the warp must call it.
+template <typename V, int E, typename Src>
+__device__ __forceinline__ void warp_sort_copy(Src src, V *dst, uint32_t c, int lane) {
     V v[E];
 #pragma unroll
     for (int m = 0; m < E; m++) {
         const uint32_t e = m * 32u + lane;
-        v[m] = e < c ? src[e] : key_max<V>();
+        v[m] = e < c ? src(e) : key_max<V>();
     }
     __syncwarp();  // every load is done before any store (in-place use)
     warp_bitonic_sort<V, E>(v, lane);
@@ -69,8 +69,8 @@ __device__ __forceinline__ void warp_sort_copy(const V *src, V *dst, uint32_t c,
 constexpr int kWarpSortCap = 256;
 
 // As warp_sort_copy, choosing the register count from c (<= kWarpSortCap).
-template <typename V>
-__device__ __forceinline__ void warp_sort_small(const V *src, V *dst, uint32_t c, int lane) {
+template <typename V, typename Src>
+__device__ __forceinline__ void warp_sort_small(Src src, V *dst, uint32_t c, int lane) {
     if (c <= 32) warp_sort_copy<V, 1>(src, dst, c, lane);
     else if (c <= 64) warp_sort_copy<V, 2>(src, dst, c, lane);
     else if (c <= 128) warp_sort_copy<V, 4>(src, dst, c, lane);

@@ -245,6 +245,20 @@ BT_API bt_status bt_range_search(const bt_tree *tree, int mode, const void *d_lo
                           uint64_t ids_capacity, uint64_t *h_total, void *stream);
 
 /*
+ * bt_range_search for callers that do not know the number of hits: once the
+ * total is known (and not 0), alloc(ctx, total) is called on this thread, with
+ * the tree's device current, and returns device memory for `total` values, or
+ * NULL (the call then ends with BT_ERR_OUT_OF_MEMORY, counts, offsets and
+ * *h_total filled).  Against a first bt_range_search for the total and a
+ * second one for the IDs, the ranges are counted once.
+ */
+typedef void *(*bt_ids_alloc)(void *ctx, uint64_t total);
+BT_API bt_status bt_range_search_alloc(const bt_tree *tree, int mode, const void *d_lo,
+                                       const void *d_hi, uint64_t nq, uint64_t *d_counts,
+                                       uint64_t *d_offsets, bt_ids_alloc alloc, void *ctx,
+                                       uint64_t *h_total, void *stream);
+
+/*
  * Rectangle search over 2-D points (an extension beyond the reference's path; the reference only
  * reorders 1-D range queries by a Z-order of (start, end), zOrder2d.cu:27-54).
  * The tree's keys are 32-bit Morton codes of (x, y) in u16 (x in the even
@@ -275,6 +289,14 @@ BT_API bt_status bt_rect_search_mode(const bt_tree *tree, int mode, const uint16
                                      const uint16_t *d_y1, uint64_t nr, uint64_t *d_counts,
                                      uint64_t *d_offsets, void *d_ids, uint64_t ids_capacity,
                                      uint64_t *h_total, void *stream);
+
+/* bt_rect_search_mode with the IDs' memory from alloc (see
+ * bt_range_search_alloc). */
+BT_API bt_status bt_rect_search_alloc(const bt_tree *tree, int mode, const uint16_t *d_x0,
+                                      const uint16_t *d_y0, const uint16_t *d_x1,
+                                      const uint16_t *d_y1, uint64_t nr, uint64_t *d_counts,
+                                      uint64_t *d_offsets, bt_ids_alloc alloc, void *ctx,
+                                      uint64_t *h_total, void *stream);
 
 /* Range count with host buffers (pipelined like bt_point_search_host). */
 BT_API bt_status bt_range_count_host(const bt_tree *tree, int mode, const void *h_lo,
