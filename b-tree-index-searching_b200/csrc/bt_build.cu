@@ -74,19 +74,6 @@ __global__ void pad_kernel(K *__restrict__ dst, uint64_t from, uint64_t to) {
         dst[j] = key_max<K>();
 }
 
-// How evenly the keys fill the buckets of a large point batch.
-bt_status measure_buckets(bt_tree *t, cudaStream_t s) {
-    WsGuard g(s);
-    bt_status st = g.alloc(sizeof(uint32_t));
-    if (st != BT_OK) return st;
-    BT_CUDA(cudaMemsetAsync(g.p, 0, sizeof(uint32_t), s));
-    st = launch_bucket_blocks(t, g.as<uint32_t>(), s);
-    if (st != BT_OK) return st;
-    BT_CUDA(cudaMemcpyAsync(&t->bucket_blocks, g.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-    BT_CUDA(cudaStreamSynchronize(s));
-    return BT_OK;
-}
-
 unsigned grid_for(uint64_t n, int block) {
     uint64_t g = (n + block - 1) / block;
     uint64_t cap = (uint64_t)sm_count() * 16;
@@ -130,10 +117,10 @@ bt_status build_impl(bt_tree *t, const void *d_keys, const void *d_vals, cudaStr
     BT_CUDA(cudaMalloc(&t->d_leaves, leaf_bytes));
     BT_CUDA(cudaMalloc(&t->d_seps, t->seps_elems * sizeof(K)));
     WsGuard g_flags(s);
-    bt_status st = g_flags.alloc(sizeof(unsigned int));
+    bt_status st = g_flags.alloc(2 * sizeof(unsigned int));  // order flags, fullest bucket
     if (st != BT_OK) return st;
     unsigned int *d_flags = g_flags.as<unsigned int>();
-    BT_CUDA(cudaMemsetAsync(d_flags, 0, sizeof(unsigned int), s));
+    BT_CUDA(cudaMemsetAsync(d_flags, 0, 2 * sizeof(unsigned int), s));
 
     K *seps = (K *)t->d_seps;
     K *bottom = seps + dt.lvl_off[L - 1];
@@ -155,25 +142,28 @@ bt_status build_impl(bt_tree *t, const void *d_keys, const void *d_vals, cudaStr
     }
     BT_CUDA(cudaGetLastError());
 
-    unsigned int flags = 0;
+    dt.leaves = t->d_leaves;
+    dt.seps = t->d_seps;
+    dt.n = n;
+    dt.n_sectors = t->n_sectors;
+    st = launch_bucket_blocks(t, d_flags, d_flags + 1, s);
+    if (st != BT_OK) return st;
+    unsigned int flags[2] = {0, 0};
     K kmin = 0, kmax = 0;
-    BT_CUDA(cudaMemcpyAsync(&flags, d_flags, sizeof(flags), cudaMemcpyDeviceToHost, s));
+    BT_CUDA(cudaMemcpyAsync(flags, d_flags, sizeof(flags), cudaMemcpyDeviceToHost, s));
     const unsigned char *lv = (const unsigned char *)t->d_leaves;
     BT_CUDA(cudaMemcpyAsync(&kmin, lv, sizeof(K), cudaMemcpyDeviceToHost, s));
     BT_CUDA(cudaMemcpyAsync(&kmax,
                             lv + ((n - 1) / S) * LeafGeom<K, V>::BS + ((n - 1) % S) * sizeof(K),
                             sizeof(K), cudaMemcpyDeviceToHost, s));
     BT_CUDA(cudaStreamSynchronize(s));
-    if (flags & 1u) return fail(BT_ERR_UNSORTED, "build keys are not sorted ascending");
-    t->values_sorted = (flags & 2u) ? 0 : 1;
+    if (flags[0] & 1u) return fail(BT_ERR_UNSORTED, "build keys are not sorted ascending");
+    t->values_sorted = (flags[0] & 2u) ? 0 : 1;
+    t->bucket_blocks = flags[1];
     t->min_key = (uint64_t)kmin;
     t->max_key = (uint64_t)kmax;
 
-    dt.leaves = t->d_leaves;
-    dt.seps = t->d_seps;
-    dt.n = n;
     dt.max_key = t->max_key;
-    dt.n_sectors = t->n_sectors;
     // The deepest separator level whose real entries fit the shared-memory
     // budget; a binary search over it resolves every level above it at once.
     int sl = 0;
@@ -182,7 +172,7 @@ bt_status build_impl(bt_tree *t, const void *d_keys, const void *d_vals, cudaStr
     dt.smem_entries = (uint32_t)t->lvl_entries[sl];
     // whole 128-byte bank rows, so the swizzle stays inside the staged region
     dt.smem_bytes = (uint32_t)(((t->lvl_entries[sl] * sizeof(K)) + 127) / 128 * 128);
-    return measure_buckets(t, s);
+    return BT_OK;
 }
 
 template <typename K>
@@ -228,7 +218,7 @@ bt_status bt_build(const void *d_sorted_keys, const void *d_values, uint64_t n, 
     t->val_bytes = value_bytes;
     t->n = n;
     t->values_sorted = 1;
-    t->search_cfg = default_search_cfg(key_bytes);
+    t->search_cfg = default_search_cfg();
     if (n > 0) {
         cudaStream_t s = (cudaStream_t)stream;
         st = key_bytes == 4 ? build_k<uint32_t>(t, d_sorted_keys, d_values, s)
@@ -452,7 +442,7 @@ bt_status bt_load(const char *path, void *stream, bt_tree **out) {
     t->seps_elems = h.seps_elems;
     t->min_key = h.min_key;
     t->max_key = h.max_key;
-    t->search_cfg = default_search_cfg(h.key_bytes);
+    t->search_cfg = default_search_cfg();
     for (int l = 0; l < kMaxLevels; l++) {
         t->lvl_nodes[l] = h.lvl_nodes[l];
         t->lvl_entries[l] = h.lvl_entries[l];
@@ -480,7 +470,17 @@ bt_status bt_load(const char *path, void *stream, bt_tree **out) {
     dt.smem_entries = h.smem_entries;
     dt.smem_bytes = h.smem_bytes;
     if (t->n) {
-        st = measure_buckets(t, (cudaStream_t)stream);
+        cudaStream_t s = (cudaStream_t)stream;
+        WsGuard g(s);
+        st = g.alloc(sizeof(uint32_t));
+        if (st == BT_OK) {
+            e = cudaMemsetAsync(g.p, 0, sizeof(uint32_t), s);
+            if (e == cudaSuccess) st = launch_bucket_blocks(t, nullptr, g.as<uint32_t>(), s);
+            if (e == cudaSuccess && st == BT_OK)
+                e = cudaMemcpyAsync(&t->bucket_blocks, g.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
+            if (e == cudaSuccess && st == BT_OK) e = cudaStreamSynchronize(s);
+            if (e != cudaSuccess) st = cuda_fail(e, "tree image: bucket measurement");
+        }
         if (st != BT_OK) {
             free_tree(t);
             return st;
@@ -503,6 +503,7 @@ bt_status bt_set_search_config(bt_tree *t, int lanes_per_query, int rounds) {
     const int k = search_cfg_index(lanes_per_query, rounds);
     if (k < 0) return fail(BT_ERR_INVALID_ARGUMENT, "unsupported (lanes, rounds) search configuration");
     t->search_cfg = k;
+    t->search_cfg_set = 1;
     return BT_OK;
 }
 

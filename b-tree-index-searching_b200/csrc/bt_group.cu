@@ -629,16 +629,22 @@ bucket_start_kernel(const __grid_constant__ DevTree t, const __grid_constant__ B
 }
 
 // *blocks = the most leaf blocks a bucket's keys touch (eight lanes per
-// bucket).
+// bucket).  Takes the key range from the first and last key itself, so that a
+// build need not wait for them first; leaves at once when *unsorted has bit 0
+// set (the walk needs ascending separators).
 template <typename K>
 __global__ void __launch_bounds__(256)
-bucket_blocks_kernel(const __grid_constant__ DevTree t, const __grid_constant__ BucketMap map,
+bucket_blocks_kernel(const __grid_constant__ DevTree t, const K *__restrict__ first_key,
+                     const K *__restrict__ last_key, const unsigned int *__restrict__ unsorted,
                      uint32_t *__restrict__ blocks) {
+    if (unsorted && (*unsorted & 1u)) return;
+    const K tmax = *last_key;
+    const BucketMap map = bucket_map((uint64_t)*first_key, (uint64_t)tmax);
     const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;
     const int lane = threadIdx.x & 31;
     const uint32_t b = i <= map.last ? i : map.last;
-    const uint64_t a = map.first_key(b), z = b == map.last ? t.max_key : map.first_key(b + 1);
-    const K qe[2] = {a < t.max_key ? (K)a : (K)t.max_key, z < t.max_key ? (K)z : (K)t.max_key};
+    const uint64_t a = map.first_key(b), z = b == map.last ? (uint64_t)tmax : map.first_key(b + 1);
+    const K qe[2] = {a < (uint64_t)tmax ? (K)a : tmax, z < (uint64_t)tmax ? (K)z : tmax};
     const bool up[2] = {false, false};
     uint32_t node[2] = {0, 0};
     walk_from<K, 8, 2>(t, 0, qe, up, node, lane >> 3, lane & 7);
@@ -1379,14 +1385,20 @@ bt_status launch_range_gather(const bt_tree *t, const uint32_t *rank, const uint
     return BT_OK;
 }
 
-bt_status launch_bucket_blocks(const bt_tree *t, uint32_t *d_blocks, cudaStream_t s) {
-    const BucketMap map = bucket_map(t->min_key, t->max_key);
-    const unsigned grid = ((map.last + 1) * 8 + 255) / 256;
+bt_status launch_bucket_blocks(const bt_tree *t, const unsigned int *d_unsorted, uint32_t *d_blocks,
+                               cudaStream_t s) {
+    const unsigned grid = kMaxBuckets * 8 / 256;
+    const unsigned char *lv = (const unsigned char *)t->d_leaves;
+    const uint64_t S = kSectorBytes / t->key_bytes;
+    const unsigned char *last = lv + (t->n - 1) / S * leaf_stride(t->key_bytes, t->val_bytes) +
+                                (t->n - 1) % S * t->key_bytes;
     count_launch();
     if (t->key_bytes == 4)
-        bucket_blocks_kernel<uint32_t><<<grid, 256, 0, s>>>(t->dev, map, d_blocks);
+        bucket_blocks_kernel<uint32_t><<<grid, 256, 0, s>>>(t->dev, (const uint32_t *)lv,
+                                                            (const uint32_t *)last, d_unsorted, d_blocks);
     else
-        bucket_blocks_kernel<uint64_t><<<grid, 256, 0, s>>>(t->dev, map, d_blocks);
+        bucket_blocks_kernel<uint64_t><<<grid, 256, 0, s>>>(t->dev, (const uint64_t *)lv,
+                                                            (const uint64_t *)last, d_unsorted, d_blocks);
     BT_CUDA(cudaGetLastError());
     return BT_OK;
 }

@@ -142,6 +142,7 @@ struct bt_tree {
     int values_sorted;
     uint32_t bucket_blocks;  // leaf blocks of the fullest bucket (0: not measured)
     int search_cfg;  // index into the search kernels' (lanes, rounds) table
+    int search_cfg_set;  // set by bt_set_search_config (else each kernel takes its own)
     bt::DevTree dev;
     bt::LearnedState *learned;  // trained learned index, or null
 };
@@ -192,7 +193,7 @@ __host__ __device__ constexpr K key_max() {
     return (K)~(K)0;
 }
 
-inline int bitlen64(uint64_t v) {
+__host__ __device__ inline int bitlen64(uint64_t v) {
     int b = 0;
     while (v) {
         v >>= 1;
@@ -241,7 +242,7 @@ bt_status launch_segment_sort(const bt_tree *t, const uint64_t *d_counts, const 
 // (lanes per query, rounds) -> index of the search configuration table in
 // bt_search.cu, or -1.
 int search_cfg_index(int lanes, int rounds);
-int default_search_cfg(int key_bytes);
+int default_search_cfg();
 int search_cfg_lanes(int cfg);
 int search_cfg_rounds(int cfg);
 
@@ -308,7 +309,7 @@ bt_status launch_bucket_gather(int val_bytes, const void *res, const uint8_t *rf
                                const uint32_t *pos, uint64_t nq, void *d_out, uint8_t *d_found,
                                cudaStream_t s);
 // The tree's map: as many buckets as kMaxBuckets allows.
-inline BucketMap bucket_map(uint64_t min_key, uint64_t max_key) {
+__host__ __device__ inline BucketMap bucket_map(uint64_t min_key, uint64_t max_key) {
     const int span = bitlen64(max_key - min_key);
     BucketMap m;
     m.min = min_key;
@@ -318,8 +319,10 @@ inline BucketMap bucket_map(uint64_t min_key, uint64_t max_key) {
 }
 static_assert(kMaxBuckets == 1 << 11, "bucket_map takes 11 bits");
 // Measures t->bucket_blocks into *d_blocks (zeroed by the caller); the
-// tree's arrays, sizes and key ends are set.
-bt_status launch_bucket_blocks(const bt_tree *t, uint32_t *d_blocks, cudaStream_t s);
+// tree's arrays, sizes and level offsets are set.
+// Does nothing when d_unsorted (optional) has bit 0 set by then.
+bt_status launch_bucket_blocks(const bt_tree *t, const unsigned int *d_unsorted, uint32_t *d_blocks,
+                               cudaStream_t s);
 // Least batches that are put into any order before the search; below them
 // the order costs more than it gives, whatever the mode asks for (2^20 point
 // queries, u32 keys, 2^20 / 2^26: 36 / 47 us directly, 65 / 77 grouped first;

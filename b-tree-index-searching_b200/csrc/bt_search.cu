@@ -13,9 +13,11 @@
 // Both kernels are persistent (grid = SMs x resident CTAs), stage one
 // separator level into shared memory once per CTA, then loop over warp tiles
 // of 32 queries (see bt_search.cuh for the two-phase descent).
-// The leaf stage loads the whole leaf block of the query -- key sector and
-// value sector side by side, one 64-byte DRAM access -- with its chunks
-// spread over the group's lanes, so a hit costs one HBM round trip.
+// A point query's leaf block -- key sector and value sector side by side, one
+// 64-byte DRAM access -- is read by one thread or a lane pair (leaf_answers),
+// so a hit costs one HBM round trip.  2^20 u32 keys, 2^20 queries (in L2):
+// 36 -> 25.8 us against four lanes per query; what is left is the instruction
+// issue of the shared-memory search and of the one separator line below it.
 #include <map>
 #include <mutex>
 #include <type_traits>
@@ -42,9 +44,19 @@ int search_cfg_index(int g, int r) {
 int search_cfg_lanes(int cfg) { return kSearchCfgs[cfg].g; }
 int search_cfg_rounds(int cfg) { return kSearchCfgs[cfg].r; }
 
-int default_search_cfg(int key_bytes) {
-    (void)key_bytes;
-    return search_cfg_index(4, 1);
+int default_search_cfg() { return search_cfg_index(4, 1); }
+
+// The shape of a tree nobody has set one for (us; 2^19 queries or ranges):
+//                          (2,1)  (4,1)  (4,2)  (8,1)  (8,2)
+//   point u32, 2^20 keys                 (4,1) fastest throughout
+//   point u64, 2^20 keys    46.0   31.3   30.8   27.3   25.2
+//   point u64, 2^28         82.7   52.1   54.0   46.5   47.7
+//   range u32, 2^20 / 2^26  32/46  48/64  36/49  98/139 63/85
+//   range u64, 2^20 / 2^26  74/105 73/104 59/82  144/189 93/124
+static int shape_of(const bt_tree *t, bool range) {
+    if (t->search_cfg_set) return t->search_cfg;
+    if (range) return t->key_bytes == 4 ? search_cfg_index(2, 1) : search_cfg_index(4, 2);
+    return t->key_bytes == 4 ? search_cfg_index(4, 1) : search_cfg_index(8, 2);
 }
 
 namespace {
@@ -56,27 +68,161 @@ constexpr int kWarps = kThreads / 32;
 // 8-byte results per warp.
 __host__ __device__ inline size_t scratch_offset(const DevTree &t) { return ((size_t)t.smem_bytes + 15) / 16 * 16; }
 
-template <typename K, typename V, int G, int R, bool PERM>
+// Staged window slot of sorted element p: a padding word after every 32 and
+// every 1,024 elements keeps a binary search's probes in different banks
+// (two instructions, where swz takes four; the window is not a power of two).
+__device__ __forceinline__ uint32_t win_slot(uint32_t p) { return p + (p >> 5) + (p >> 10); }
+constexpr size_t win_words(size_t n) { return n + n / 32 + n / 1024 + 2; }
+
+// First element of the n staged ones at or above q, n if none, for U queries
+// in step.
+template <typename W, int U>
+__device__ __forceinline__ void win_bound(const W *__restrict__ s, uint32_t n, const W (&q)[U],
+                                          uint32_t (&pos)[U]) {
+#pragma unroll
+    for (int u = 0; u < U; u++) pos[u] = 0;
+    while (n > 1) {
+        const uint32_t half = n >> 1;
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const uint32_t p = pos[u] + half;
+            pos[u] = s[win_slot(p)] < q[u] ? p : pos[u];
+        }
+        n -= half;
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) pos[u] += s[win_slot(pos[u])] < q[u] ? 1u : 0u;
+}
+
+// The separator levels from `from` down for the warp's 32 queries, one per
+// lane (q at most the largest key): the leaf block of each, given its node on
+// level `from`.  G lanes read a query's line; R rounds.
+template <typename K, int G, int R>
+__device__ __forceinline__ uint32_t walk_lanes(const DevTree &t, int from, K q, uint32_t node, int lane) {
+    constexpr int NG = 32 / G, I = G / R;
+    const int grp = lane / G, gl = lane % G;
+    uint32_t mine = node;
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        K qe[I];
+        bool up[I];
+        uint32_t nd[I];
+#pragma unroll
+        for (int s = 0; s < I; s++) {
+            const int k = r * (NG * I) + s * NG + grp;
+            qe[s] = __shfl_sync(0xffffffffu, q, k);
+            nd[s] = __shfl_sync(0xffffffffu, node, k);
+            up[s] = false;
+        }
+        walk_from<K, G, I>(t, from, qe, up, nd, grp, gl);
+#pragma unroll
+        for (int s = 0; s < I; s++) {
+            const uint32_t y = __shfl_sync(0xffffffffu, nd[s], (lane % NG) * G);
+            mine = lane / NG == r * I + s ? y : mine;
+        }
+    }
+    return mine;
+}
+
+// 32 bytes of a leaf block by one thread.  Not evict-first: a block's value
+// sector, which comes with its key sector, is read a moment later (evicted
+// before that, 2^24 u64 queries took 1.19 ms instead of 0.84).
+__device__ __forceinline__ void load_sector(const void *p, uint32_t (&w)[8]) {
+    asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]),
+                   "=r"(w[7])
+                 : "l"(p));
+}
+
+// The first of a key sector's S keys equal to q, -1 if none (unused slots
+// hold all-ones keys, which a query above the largest key may equal).
+template <typename K, int S>
+__device__ __forceinline__ int first_match(const uint32_t (&w)[8], K q, K tmax) {
+    int at = -1;
+#pragma unroll
+    for (int k = S - 1; k >= 0; k--)
+        if (key_at<K>(w, k) == q) at = k;
+    return q <= tmax ? at : -1;
+}
+
+// Answers U queries per lane from their leaf blocks: put(u, l, value, hit) is
+// called once for query u of every lane l.
+//   4-byte keys: each thread loads its block's keys (32 bytes), then the
+//     matching value;
+//   8-byte keys: a lane pair per query, one lane the key sector, one the value
+//     sector, as one request.
+// A quarter of the instructions of the form it replaces (four lanes per
+// query, 16 bytes each, combined by shuffles and ballots).
+template <typename K, typename V, int U, bool PAIR, typename Put>
+__device__ __forceinline__ void leaf_answers(const unsigned char *__restrict__ leaves,
+                                             const uint32_t (&node)[U], const K (&qv)[U], K tmax, Put put) {
+    using LG = LeafGeom<K, V>;
+    const int lane = threadIdx.x & 31;
+    if constexpr (PAIR) {
+        static_assert(LG::BS == 2 * kSectorBytes, "values in the second sector");
+        uint32_t w[U][2][8];
+        K qk[U][2];
+#pragma unroll
+        for (int u = 0; u < U; u++)
+#pragma unroll
+            for (int h = 0; h < 2; h++) {  // lanes 2k, 2k + 1: the query of lane 16 h + k
+                const int k = h * 16 + (lane >> 1);
+                const uint32_t nd = __shfl_sync(0xffffffffu, node[u], k);
+                qk[u][h] = __shfl_sync(0xffffffffu, qv[u], k);
+                load_sector(leaves + (size_t)nd * LG::BS + (lane & 1) * kSectorBytes, w[u][h]);
+            }
+#pragma unroll
+        for (int u = 0; u < U; u++)
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                int at = first_match<K, LG::S>(w[u][h], qk[u][h], tmax);
+                at = __shfl_sync(0xffffffffu, at, lane & ~1);  // the key lane's
+                V v = key_max<V>();
+#pragma unroll
+                for (int k = 0; k < LG::S; k++)
+                    if (at == k) v = key_at<V>(w[u][h], k);
+                if (lane & 1) put(u, h * 16 + (lane >> 1), v, at >= 0);
+            }
+    } else {
+        uint32_t w[U][8];
+#pragma unroll
+        for (int u = 0; u < U; u++) load_sector(leaves + (size_t)node[u] * LG::BS, w[u]);
+        int at[U];
+        V v[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            at[u] = first_match<K, LG::S>(w[u], qv[u], tmax);
+            v[u] = at[u] >= 0 ? __ldg(reinterpret_cast<const V *>(leaves + (size_t)node[u] * LG::BS +
+                                                                 kSectorBytes) + at[u])
+                              : key_max<V>();
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) put(u, lane, v[u], at[u] >= 0);
+    }
+}
+
+template <typename K, typename V, int G, int R, bool PERM, bool PAIR>
 __global__ void __launch_bounds__(kThreads, 2)
 point_kernel(const __grid_constant__ DevTree t, const K *__restrict__ q,
              const uint32_t *__restrict__ perm, uint64_t nq, V *__restrict__ out,
              uint8_t *__restrict__ found) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     K *s_lvl = reinterpret_cast<K *>(smem_raw);
-    stage_level<K>(s_lvl, t);
+    {
+        const K *src = static_cast<const K *>(t.seps) + t.lvl_off[t.smem_level];
+#pragma unroll 4
+        for (uint32_t i = threadIdx.x; i < t.smem_entries; i += kThreads) s_lvl[win_slot(i)] = src[i];
+    }
     __syncthreads();
 
-    constexpr int NG = 32 / G;  // lane groups per warp
-    constexpr int I = G / R;    // queries in flight per group and round
+    constexpr int U = 1;  // queries per lane at a time (2: no faster, 1.05x slower on small batches)
     const int lane = threadIdx.x & 31;
-    const int grp = lane / G;
-    const int gl = lane % G;
     const K tmax = (K)t.max_key;
     const unsigned char *leaves = static_cast<const unsigned char *>(t.leaves);
     // Grouped input (PERM): each CTA takes one contiguous run of warp tiles,
     // so a CTA works one key range and its warps share node lines in L1.
     // Ungrouped input: warp tiles are strided over the whole grid.
-    const uint64_t ntiles = (nq + 31) / 32;
+    const uint64_t ntiles = (nq + 32 * U - 1) / (32 * U);
     const uint64_t per_cta = PERM ? (ntiles + gridDim.x - 1) / gridDim.x : 0;
     const uint64_t t_begin = PERM ? blockIdx.x * per_cta + (threadIdx.x >> 5)
                                   : (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
@@ -84,41 +230,25 @@ point_kernel(const __grid_constant__ DevTree t, const K *__restrict__ q,
     const uint64_t t_step = PERM ? (blockDim.x >> 5) : ((uint64_t)gridDim.x * blockDim.x) >> 5;
 
     for (uint64_t tile = t_begin; tile < t_end; tile += t_step) {
-        const uint64_t base = tile * 32;
-        // phase 1: one lane per query, binary search of the staged level
-        const uint64_t my = base + lane;
-        const K myq = my < nq ? q[my] : (K)0;
-        const uint32_t myperm = PERM && my < nq ? perm[my] : 0u;  // loaded early
-        const uint32_t mynode = smem_bound<K>(s_lvl, t.smem_entries, myq < tmax ? myq : tmax, false);
-
-        // phase 2: G lanes per query through the global levels and the leaf
+        const uint64_t base = tile * (32 * U);
+        K qv[U], qe[U];
+        uint32_t node[U];
 #pragma unroll
-        for (int r = 0; r < R; r++) {
-            K qv[I], qe[I];
-            bool up[I];
-            uint32_t node[I], pv[I];
-#pragma unroll
-            for (int s = 0; s < I; s++) {
-                const int k = r * (NG * I) + s * NG + grp;  // query of the tile
-                qv[s] = __shfl_sync(0xffffffffu, myq, k);
-                node[s] = __shfl_sync(0xffffffffu, mynode, k);
-                pv[s] = PERM ? __shfl_sync(0xffffffffu, myperm, k) : 0u;
-                qe[s] = qv[s] < tmax ? qv[s] : tmax;
-                up[s] = false;
-            }
-            walk_global<K, G, I>(t, qe, up, node, grp, gl);
-            leaf_point<K, V, G, I>(
-                leaves, node, qv, qe, tmax, grp, gl,
-                [&](int s) -> V * {
-                    const uint64_t qi = base + (uint64_t)(r * (NG * I) + s * NG + grp);
-                    if (qi >= nq) return nullptr;
-                    return out + (PERM ? (uint64_t)pv[s] : qi);
-                },
-                [&](int s) -> uint8_t * {
-                    const uint64_t qi = base + (uint64_t)(r * (NG * I) + s * NG + grp);
-                    return found ? found + (PERM ? (uint64_t)pv[s] : qi) : nullptr;
-                });
+        for (int u = 0; u < U; u++) {
+            const uint64_t i = base + u * 32 + lane;
+            qv[u] = i < nq ? q[i] : (K)0;
+            qe[u] = qv[u] < tmax ? qv[u] : tmax;
         }
+        win_bound<K, U>(s_lvl, t.smem_entries, qe, node);
+#pragma unroll
+        for (int u = 0; u < U; u++) node[u] = walk_lanes<K, G, R>(t, t.smem_level + 1, qe[u], node[u], lane);
+        leaf_answers<K, V, U, PAIR>(leaves, node, qv, tmax, [&](int u, int l, V v, bool hit) {
+            const uint64_t i = base + u * 32 + l;
+            if (i >= nq) return;
+            const uint64_t d = PERM ? (uint64_t)perm[i] : i;
+            out[d] = v;
+            if (found) found[d] = hit ? 1 : 0;
+        });
     }
 }
 
@@ -269,54 +399,8 @@ point_window_kernel(const __grid_constant__ DevTree t, const K *__restrict__ q,
 // 0.56 ms, thread per query 0.60.
 
 
-// Staged window slot of sorted element p: a padding word after every 32 and
-// every 1,024 elements keeps a binary search's probes in different banks
-// (two instructions, where swz takes four; the window is not a power of two).
-__device__ __forceinline__ uint32_t win_slot(uint32_t p) { return p + (p >> 5) + (p >> 10); }
 constexpr size_t kBktWinBytes = 200 * 1024;
 constexpr size_t kBktWinMin = 16 * 1024;  // room for some level of any tree
-constexpr size_t win_words(size_t n) { return n + n / 32 + n / 1024 + 2; }
-
-// First element of the n staged ones at or above q, n if none, for U queries
-// in step.
-template <typename W, int U>
-__device__ __forceinline__ void win_bound(const W *__restrict__ s, uint32_t n, const W (&q)[U],
-                                          uint32_t (&pos)[U]) {
-#pragma unroll
-    for (int u = 0; u < U; u++) pos[u] = 0;
-    while (n > 1) {
-        const uint32_t half = n >> 1;
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-            const uint32_t p = pos[u] + half;
-            pos[u] = s[win_slot(p)] < q[u] ? p : pos[u];
-        }
-        n -= half;
-    }
-#pragma unroll
-    for (int u = 0; u < U; u++) pos[u] += s[win_slot(pos[u])] < q[u] ? 1u : 0u;
-}
-
-// 32 bytes of a leaf block by one thread.  Not evict-first: a block's value
-// sector, which comes with its key sector, is read a moment later (evicted
-// before that, 2^24 u64 queries took 1.19 ms instead of 0.84).
-__device__ __forceinline__ void load_sector(const void *p, uint32_t (&w)[8]) {
-    asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]),
-                   "=r"(w[7])
-                 : "l"(p));
-}
-
-// The first of a key sector's S keys equal to q, -1 if none (unused slots
-// hold all-ones keys, which a query above the largest key may equal).
-template <typename K, int S>
-__device__ __forceinline__ int first_match(const uint32_t (&w)[8], K q, K tmax) {
-    int at = -1;
-#pragma unroll
-    for (int k = S - 1; k >= 0; k--)
-        if (key_at<K>(w, k) == q) at = k;
-    return q <= tmax ? at : -1;
-}
 
 // What a bucket search writes: values, or (BOUND) ranks of lower bounds.
 template <typename V, bool BOUND>
@@ -331,8 +415,7 @@ __device__ __forceinline__ void bucket_item(const DevTree &t, const W *s_win, ui
                                             BktOut<V, BOUND> *__restrict__ out,
                                             uint8_t *__restrict__ found) {
     using LG = LeafGeom<K, V>;
-    constexpr bool PAIR = sizeof(K) == 8 && !BOUND;
-    constexpr int U = PAIR ? 2 : 4;  // queries per thread at a time
+    constexpr int U = sizeof(K) == 8 && !BOUND ? 2 : 4;  // queries per thread at a time
     const int lane = threadIdx.x & 31;
     const K tmax = (K)t.max_key;
     const unsigned char *leaves = static_cast<const unsigned char *>(t.leaves);
@@ -356,37 +439,19 @@ __device__ __forceinline__ void bucket_item(const DevTree &t, const W *s_win, ui
 #pragma unroll
         for (int u = 0; u < U; u++) node[u] = w0 + (node[u] < wm ? node[u] : wm - 1u);
         if (wlvl + 1 < t.nlevels) {  // uniform: the window is not the bottom level
-            constexpr int G = 4, NG = 32 / G;
-            const int grp = lane / G, gl = lane % G;
 #pragma unroll 1
             for (int u = 0; u < U; u++) {
-                K qe[G];
-                bool up[G];
-                uint32_t nd[G];
+                K x = 0;
+                uint32_t y = 0;
 #pragma unroll
-                for (int s = 0; s < G; s++) {
-                    K x = 0;
-                    uint32_t y = 0;
+                for (int z = 0; z < U; z++)
+                    if (z == u) {
+                        x = qv[z];
+                        y = node[z];
+                    }
+                y = walk_lanes<K, 4, 1>(t, wlvl + 1, x < tmax ? x : tmax, y, lane);
 #pragma unroll
-                    for (int z = 0; z < U; z++)
-                        if (z == u) {
-                            x = qv[z];
-                            y = node[z];
-                        }
-                    qe[s] = __shfl_sync(0xffffffffu, x, s * NG + grp);
-                    nd[s] = __shfl_sync(0xffffffffu, y, s * NG + grp);
-                    qe[s] = qe[s] < tmax ? qe[s] : tmax;
-                    up[s] = false;
-                }
-                walk_from<K, G, G>(t, wlvl + 1, qe, up, nd, grp, gl);
-                uint32_t r = 0;
-#pragma unroll
-                for (int s = 0; s < G; s++) {
-                    const uint32_t y = __shfl_sync(0xffffffffu, nd[s], (lane % NG) * G);
-                    r = lane / NG == s ? y : r;
-                }
-#pragma unroll
-                for (int z = 0; z < U; z++) node[z] = z == u ? r : node[z];
+                for (int z = 0; z < U; z++) node[z] = z == u ? y : node[z];
             }
         }
         if constexpr (BOUND) {  // position of the first key at or above the query
@@ -399,56 +464,14 @@ __device__ __forceinline__ void bucket_item(const DevTree &t, const W *s_win, ui
                 const uint32_t i = i0 + u * T + lane;
                 if (i < qn) out[i] = node[u] * (uint32_t)LG::S + count_below<K, LG::S>(w[u], c, false);
             }
-        } else if constexpr (PAIR) {
-            static_assert(sizeof(K) == 4 || LG::BS == 2 * kSectorBytes, "values in the second sector");
-            uint32_t w[U][2][8];
-            K qk[U][2];
-#pragma unroll
-            for (int u = 0; u < U; u++)
-#pragma unroll
-                for (int h = 0; h < 2; h++) {  // lanes 2k, 2k + 1: query 16 h + k of the 32
-                    const int k = h * 16 + (lane >> 1);
-                    const uint32_t nd = __shfl_sync(0xffffffffu, node[u], k);
-                    qk[u][h] = __shfl_sync(0xffffffffu, qv[u], k);
-                    load_sector(leaves + (size_t)nd * LG::BS + (lane & 1) * kSectorBytes, w[u][h]);
-                }
-#pragma unroll
-            for (int u = 0; u < U; u++)
-#pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    int at = first_match<K, LG::S>(w[u][h], qk[u][h], tmax);
-                    at = __shfl_sync(0xffffffffu, at, lane & ~1);  // the key lane's
-                    V v = key_max<V>();
-#pragma unroll
-                    for (int k = 0; k < LG::S; k++)
-                        if (at == k) v = key_at<V>(w[u][h], k);
-                    const uint32_t i = i0 + u * T + h * 16 + (lane >> 1);
-                    if ((lane & 1) && i < qn) {
-                        out[i] = v;
-                        if (found) found[i] = at >= 0 ? 1 : 0;
-                    }
-                }
         } else {
-            uint32_t w[U][8];
-#pragma unroll
-            for (int u = 0; u < U; u++) load_sector(leaves + (size_t)node[u] * LG::BS, w[u]);
-            int at[U];
-            V v[U];
-#pragma unroll
-            for (int u = 0; u < U; u++) {
-                at[u] = first_match<K, LG::S>(w[u], qv[u], tmax);
-                v[u] = at[u] >= 0 ? __ldg(reinterpret_cast<const V *>(leaves + (size_t)node[u] * LG::BS +
-                                                                     kSectorBytes) + at[u])
-                                  : key_max<V>();
-            }
-#pragma unroll
-            for (int u = 0; u < U; u++) {
-                const uint32_t i = i0 + u * T + lane;
+            leaf_answers<K, V, U, sizeof(K) == 8>(leaves, node, qv, tmax, [&](int u, int l, V v, bool hit) {
+                const uint32_t i = i0 + u * T + l;
                 if (i < qn) {
-                    out[i] = v[u];
-                    if (found) found[i] = at[u] >= 0 ? 1 : 0;
+                    out[i] = v;
+                    if (found) found[i] = hit ? 1 : 0;
                 }
-            }
+            });
         }
     }
 }
@@ -706,11 +729,11 @@ bt_status set_smem(Fn fn, size_t smem) {
     return BT_OK;
 }
 
-template <typename K, typename V, int G, int R, bool PERM>
-bt_status point_launch(const bt_tree *t, const void *d_q, const uint32_t *d_perm, uint64_t nq,
-                       void *d_out, uint8_t *d_found, cudaStream_t s) {
-    auto fn = point_kernel<K, V, G, R, PERM>;
-    const size_t smem = scratch_offset(t->dev);
+template <typename K, typename V, int G, int R, bool PERM, bool PAIR>
+bt_status point_launch_t(const bt_tree *t, const void *d_q, const uint32_t *d_perm, uint64_t nq,
+                         void *d_out, uint8_t *d_found, cudaStream_t s) {
+    auto fn = point_kernel<K, V, G, R, PERM, PAIR>;
+    const size_t smem = win_words(t->dev.smem_entries) * sizeof(K);
     bt_status st = set_smem(fn, smem);
     if (st != BT_OK) return st;
     const unsigned grid = persistent_grid((const void *)fn, smem, nq, kThreads);
@@ -718,6 +741,25 @@ bt_status point_launch(const bt_tree *t, const void *d_q, const uint32_t *d_perm
     fn<<<grid, kThreads, smem, s>>>(t->dev, (const K *)d_q, d_perm, nq, (V *)d_out, d_found);
     BT_CUDA(cudaGetLastError());
     return BT_OK;
+}
+
+// Leaf arrays above this are read by lane pairs also with 4-byte keys: a block
+// that comes from DRAM is then one request for both sectors (2^26 keys, 2^21
+// queries: 80 us; a thread per query 110; four lanes per query 84), where one
+// from L2 is faster by a thread (2^20 keys, 2^20 queries: 25.8 us; pairs 28.0;
+// four lanes 36).  The lines cross between 2^23 and 2^24 keys (64 / 128 MiB).
+constexpr size_t kPairLeafBytes = 64ull << 20;
+
+template <typename K, typename V, int G, int R, bool PERM>
+bt_status point_launch(const bt_tree *t, const void *d_q, const uint32_t *d_perm, uint64_t nq,
+                       void *d_out, uint8_t *d_found, cudaStream_t s) {
+    using LG = LeafGeom<K, V>;
+    if constexpr (sizeof(K) == 8)
+        return point_launch_t<K, V, G, R, PERM, true>(t, d_q, d_perm, nq, d_out, d_found, s);
+    if constexpr (LG::BS == 2 * kSectorBytes)
+        if (t->n_sectors * LG::BS > kPairLeafBytes)
+            return point_launch_t<K, V, G, R, PERM, LG::BS == 2 * kSectorBytes>(t, d_q, d_perm, nq, d_out, d_found, s);
+    return point_launch_t<K, V, G, R, PERM, false>(t, d_q, d_perm, nq, d_out, d_found, s);
 }
 
 template <typename K, typename V, int G, int R>
@@ -767,7 +809,7 @@ template <typename K, typename V, bool PERM>
 bt_status point_cfg(const bt_tree *t, const void *d_q, const uint32_t *d_perm, uint64_t nq,
                     void *d_out, uint8_t *d_found, cudaStream_t s) {
     if (PERM && nq >= kWinMinQueries) {
-        switch (t->search_cfg) {
+        switch (shape_of(t, false)) {
             case 0: return window_launch<K, V, 8, 1>(t, d_q, d_perm, nq, d_out, d_found, s);
             case 1: return window_launch<K, V, 8, 2>(t, d_q, d_perm, nq, d_out, d_found, s);
             case 2: return window_launch<K, V, 4, 1>(t, d_q, d_perm, nq, d_out, d_found, s);
@@ -775,7 +817,7 @@ bt_status point_cfg(const bt_tree *t, const void *d_q, const uint32_t *d_perm, u
             default: return window_launch<K, V, 2, 1>(t, d_q, d_perm, nq, d_out, d_found, s);
         }
     }
-    switch (t->search_cfg) {
+    switch (shape_of(t, false)) {
         case 0: return point_launch<K, V, 8, 1, PERM>(t, d_q, d_perm, nq, d_out, d_found, s);
         case 1: return point_launch<K, V, 8, 2, PERM>(t, d_q, d_perm, nq, d_out, d_found, s);
         case 2: return point_launch<K, V, 4, 1, PERM>(t, d_q, d_perm, nq, d_out, d_found, s);
@@ -803,7 +845,7 @@ bt_status bounds_launch(const bt_tree *t, const void *d_lo, const void *d_hi,
 template <typename K, typename V, bool PERM>
 bt_status bounds_cfg(const bt_tree *t, const void *d_lo, const void *d_hi, const uint32_t *d_perm,
                      uint64_t nq, uint64_t *d_counts, uint64_t *d_lb, cudaStream_t s) {
-    switch (t->search_cfg) {
+    switch (shape_of(t, true)) {
         case 0: return bounds_launch<K, V, 8, 1, PERM>(t, d_lo, d_hi, d_perm, nq, d_counts, d_lb, s);
         case 1: return bounds_launch<K, V, 8, 2, PERM>(t, d_lo, d_hi, d_perm, nq, d_counts, d_lb, s);
         case 2: return bounds_launch<K, V, 4, 1, PERM>(t, d_lo, d_hi, d_perm, nq, d_counts, d_lb, s);
