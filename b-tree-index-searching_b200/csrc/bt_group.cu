@@ -1127,22 +1127,22 @@ range_fill_kernel(const unsigned char *__restrict__ leaves, const uint64_t *__re
 // Sorts each query's ID segment when values do not ascend with keys.  Up to
 // kWarpSortCap values: sorted by the pass that wrote them, one warp in
 // registers (warp_sort_small, a bitonic network).  Up to kWarpLongCap: the
-// same, by a pass of its own over the listed segments.  Up to kSortCap: one
-// CTA per segment, bitonic network in shared memory.  Longer: one CTA each by
-// a bitonic network over a padded copy in global memory.
+// same, by a pass of its own over the listed segments.  Up to kSortBytes of
+// values: one CTA per segment, bitonic network in shared memory.  Longer: one
+// CTA each by a bitonic network over a padded copy in global memory.
 constexpr int kWarpLongCap = 1024;
-constexpr int kSortCap = 4096;
+constexpr size_t kSortBytes = 128 * 1024;
 constexpr unsigned int kMedListCap = 1u << 16;
 
-// Lists the segments of kWarpSortCap < c <= kSortCap (*n_med of them, the
-// first kMedListCap in med_list).
+// Lists the segments of kWarpSortCap < c <= cap (*n_med of them, the first
+// kMedListCap in med_list).
 __global__ void __launch_bounds__(256)
-list_med_segments(const uint64_t *__restrict__ cnt, uint64_t nq, unsigned int *__restrict__ n_med,
-                  uint64_t *__restrict__ med_list) {
+list_med_segments(const uint64_t *__restrict__ cnt, uint64_t nq, uint64_t cap,
+                  unsigned int *__restrict__ n_med, uint64_t *__restrict__ med_list) {
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < nq;
          i += (uint64_t)gridDim.x * blockDim.x) {
         const uint64_t c = cnt[i];
-        if (c > (uint64_t)kWarpSortCap && c <= (uint64_t)kSortCap) {
+        if (c > (uint64_t)kWarpSortCap && c <= cap) {
             const unsigned int k = atomicAdd(n_med, 1u);
             if (k < kMedListCap) med_list[k] = i;
         }
@@ -1174,21 +1174,23 @@ warp_long_sort_kernel(const uint64_t *__restrict__ cnt, const uint64_t *__restri
     }
 }
 
-// One CTA per segment of kWarpLongCap < c <= kSortCap: the listed ones, or
-// every one when the list overflowed.
+// One CTA per segment of kWarpLongCap < c <= cap: the listed ones, or every
+// one when the list overflowed.  Shared memory for the next power of two of
+// the largest.
 template <typename V>
 __global__ void __launch_bounds__(512)
 segment_sort_kernel(const uint64_t *__restrict__ cnt, const uint64_t *__restrict__ off, uint64_t nq,
-                    const unsigned int *__restrict__ n_med, const uint64_t *__restrict__ list,
-                    V *__restrict__ ids) {
-    __shared__ V buf[kSortCap];
+                    uint64_t cap, const unsigned int *__restrict__ n_med,
+                    const uint64_t *__restrict__ list, V *__restrict__ ids) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    V *buf = reinterpret_cast<V *>(smem_raw);
     const unsigned int nm = *n_med;
     const bool listed = nm <= kMedListCap;
     const uint64_t n = listed ? nm : nq;
     for (uint64_t li = blockIdx.x; li < n; li += gridDim.x) {
         const uint64_t i = listed ? list[li] : li;
         const uint64_t c = cnt[i];
-        if (c <= (uint64_t)kWarpLongCap || c > (uint64_t)kSortCap) continue;
+        if (c <= (uint64_t)kWarpLongCap || c > cap) continue;
         uint32_t p2 = 1;
         while (p2 < c) p2 <<= 1;
         V *seg = ids + off[i];
@@ -1196,15 +1198,13 @@ segment_sort_kernel(const uint64_t *__restrict__ cnt, const uint64_t *__restrict
         __syncthreads();
         for (uint32_t size = 2; size <= p2; size <<= 1) {
             for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
-                for (uint32_t k = threadIdx.x; k < p2; k += blockDim.x) {
-                    const uint32_t partner = k ^ stride;
-                    if (partner > k) {
-                        const bool asc = (k & size) == 0;
-                        const V x = buf[k], y = buf[partner];
-                        if ((x > y) == asc) {
-                            buf[k] = y;
-                            buf[partner] = x;
-                        }
+                // pair z: slots k and k + stride
+                for (uint32_t z = threadIdx.x; z < p2 / 2; z += blockDim.x) {
+                    const uint32_t k = ((z & ~(stride - 1)) << 1) | (z & (stride - 1));
+                    const V x = buf[k], y = buf[k + stride];
+                    if ((x > y) == ((k & size) == 0)) {
+                        buf[k] = y;
+                        buf[k + stride] = x;
                     }
                 }
                 __syncthreads();
@@ -1215,13 +1215,13 @@ segment_sort_kernel(const uint64_t *__restrict__ cnt, const uint64_t *__restrict
     }
 }
 
-// Segments longer than kSortCap: list them (index, offset, count).
+// Segments longer than cap: list them (offset, count).
 __global__ void list_long_segments(const uint64_t *__restrict__ cnt, const uint64_t *__restrict__ off,
-                                   uint64_t nq, unsigned int *__restrict__ n_long,
+                                   uint64_t nq, uint64_t cap, unsigned int *__restrict__ n_long,
                                    uint64_t *__restrict__ list, unsigned int max_list) {
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < nq;
          i += (uint64_t)gridDim.x * blockDim.x) {
-        if (cnt[i] > (uint64_t)kSortCap) {
+        if (cnt[i] > cap) {
             const unsigned int k = atomicAdd(n_long, 1u);
             if (k < max_list) {
                 list[2 * k] = off[i];
@@ -1460,9 +1460,10 @@ bt_status launch_segment_sort(const bt_tree *t, const uint64_t *d_counts, const 
     uint64_t *med = g_med.as<uint64_t>();
     BT_CUDA(cudaMemsetAsync(stat, 0, sizeof(unsigned int), s));
     const unsigned sms = (unsigned)sm_count();
+    const uint64_t cap = kSortBytes / (uint64_t)t->val_bytes;
     count_launch();
     list_med_segments<<<(unsigned)std::min<uint64_t>((nq + 255) / 256, sms * 8), 256, 0, s>>>(
-        d_counts, nq, stat, med);
+        d_counts, nq, cap, stat, med);
     count_launch();
     if (t->val_bytes == 4)
         warp_long_sort_kernel<uint32_t><<<sms * 4, 128, 0, s>>>(d_counts, d_offsets, nq, stat, med,
@@ -1472,16 +1473,25 @@ bt_status launch_segment_sort(const bt_tree *t, const uint64_t *d_counts, const 
                                                                 (uint64_t *)d_ids);
     BT_CUDA(cudaGetLastError());
     if (max_count > (uint64_t)kWarpLongCap) {
+        uint64_t p2 = 2 * kWarpLongCap;
+        while (p2 < std::min(max_count, cap)) p2 <<= 1;
+        const size_t smem = p2 * (size_t)t->val_bytes;
+        const unsigned grid = sms * (unsigned)std::min<size_t>(4, 200 * 1024 / smem);
         count_launch();
-        if (t->val_bytes == 4)
-            segment_sort_kernel<uint32_t><<<sms * 4, 512, 0, s>>>(d_counts, d_offsets, nq, stat, med,
+        if (t->val_bytes == 4) {
+            BT_CUDA(cudaFuncSetAttribute(segment_sort_kernel<uint32_t>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSortBytes));
+            segment_sort_kernel<uint32_t><<<grid, 512, smem, s>>>(d_counts, d_offsets, nq, cap, stat, med,
                                                                   (uint32_t *)d_ids);
-        else
-            segment_sort_kernel<uint64_t><<<sms * 4, 512, 0, s>>>(d_counts, d_offsets, nq, stat, med,
+        } else {
+            BT_CUDA(cudaFuncSetAttribute(segment_sort_kernel<uint64_t>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSortBytes));
+            segment_sort_kernel<uint64_t><<<grid, 512, smem, s>>>(d_counts, d_offsets, nq, cap, stat, med,
                                                                   (uint64_t *)d_ids);
+        }
         BT_CUDA(cudaGetLastError());
     }
-    if (max_count <= (uint64_t)kSortCap) return BT_OK;
+    if (max_count <= cap) return BT_OK;
     // some segments exceed the shared-memory sort: list and sort them one CTA each
     const unsigned int max_list = 1u << 16;
     WsGuard g_list(s);
@@ -1492,12 +1502,12 @@ bt_status launch_segment_sort(const bt_tree *t, const uint64_t *d_counts, const 
     BT_CUDA(cudaMemsetAsync(flag, 0, sizeof(unsigned int), s));
     count_launch();
     list_long_segments<<<(unsigned)std::min<uint64_t>((nq + 255) / 256, 4096), 256, 0, s>>>(
-        d_counts, d_offsets, nq, flag, d_list, max_list);
+        d_counts, d_offsets, nq, cap, flag, d_list, max_list);
     unsigned int n_long = 0;
     BT_CUDA(cudaMemcpyAsync(&n_long, flag, sizeof(n_long), cudaMemcpyDeviceToHost, s));
     BT_CUDA(cudaStreamSynchronize(s));
     if (n_long > max_list)
-        return fail(BT_ERR_NOT_SUPPORTED, "more than 65536 result sets exceed 4096 unsorted values");
+        return fail(BT_ERR_NOT_SUPPORTED, "more than 65536 result sets exceed 128 KiB of unsorted values");
     std::vector<uint64_t> list(2 * (size_t)n_long);
     BT_CUDA(cudaMemcpyAsync(list.data(), d_list, list.size() * sizeof(uint64_t),
                             cudaMemcpyDeviceToHost, s));

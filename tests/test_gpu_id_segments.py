@@ -10,7 +10,7 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 EDGES = [0, 1, 2, 31, 32, 33, 64, 65, 128, 129, 255, 256, 257, 511, 512, 513, 1023, 1024, 1025,
-         4095, 4096, 4097, 9000]
+         4095, 4096, 4097, 9000, 16384, 16385, 32768, 32769]
 
 
 def _tree(bt, cuda, kt, vt, n, g):
@@ -38,10 +38,10 @@ def _check(t, keys, vals, first, width, cuda):
 
 @pytest.mark.parametrize("kt,vt", [(np.uint32, np.uint32), (np.uint32, np.uint64),
                                    (np.uint64, np.uint32), (np.uint64, np.uint64)])
-@pytest.mark.parametrize("top", [32, 256, 1024, 4096, 9000])
+@pytest.mark.parametrize("top", [32, 256, 1024, 4096, 9000, 32769])
 def test_segments_at_the_tiers_edges(bt, cuda, kt, vt, top):
     g = np.random.default_rng(top)
-    keys, vals, t = _tree(bt, cuda, kt, vt, 50021, g)
+    keys, vals, t = _tree(bt, cuda, kt, vt, 80021, g)
     with t:
         width = g.permutation(np.repeat([w for w in EDGES if w <= top], 7)).astype(np.int64)
         _check(t, keys, vals, g.integers(1, 40000, size=len(width)), width, cuda)
