@@ -337,4 +337,158 @@ __device__ __forceinline__ void leaf_bound(const unsigned char *__restrict__ lea
     }
 }
 
+// Staged window slot of sorted element p: a padding word after every 32 and
+// every 1,024 elements keeps a binary search's probes in different banks
+// (two instructions, where swz takes four; the window is not a power of two).
+__device__ __forceinline__ uint32_t win_slot(uint32_t p) { return p + (p >> 5) + (p >> 10); }
+constexpr size_t win_words(size_t n) { return n + n / 32 + n / 1024 + 2; }
+
+// First element of the n staged ones at or above q, n if none, for U queries
+// in step.
+template <typename W, int U>
+__device__ __forceinline__ void win_bound(const W *__restrict__ s, uint32_t n, const W (&q)[U],
+                                          uint32_t (&pos)[U]) {
+#pragma unroll
+    for (int u = 0; u < U; u++) pos[u] = 0;
+    while (n > 1) {
+        const uint32_t half = n >> 1;
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const uint32_t p = pos[u] + half;
+            pos[u] = s[win_slot(p)] < q[u] ? p : pos[u];
+        }
+        n -= half;
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) pos[u] += s[win_slot(pos[u])] < q[u] ? 1u : 0u;
+}
+
+// The same for one query, the first element above q when `upper`.
+template <typename W>
+__device__ __forceinline__ uint32_t win_upper(const W *__restrict__ s, uint32_t n, W q, bool upper) {
+    uint32_t pos = 0;
+    while (n > 1) {
+        const uint32_t half = n >> 1;
+        const W v = s[win_slot(pos + half)];
+        pos = (upper ? v <= q : v < q) ? pos + half : pos;
+        n -= half;
+    }
+    const W v = s[win_slot(pos)];
+    return pos + ((upper ? v <= q : v < q) ? 1u : 0u);
+}
+
+// The separator levels [from, nl) for the warp's 32 queries, one per lane (q
+// at most the largest key): the leaf block of each, given its node on level
+// `from`.  seps and lvl_off are the tree's; G lanes read a query's line; R
+// rounds.
+template <typename K, int G, int R>
+__device__ __forceinline__ uint32_t walk_tree(const K *__restrict__ seps, const uint64_t *lvl_off,
+                                              int from, int nl, K q, uint32_t node, int lane) {
+    constexpr int NG = 32 / G, I = G / R;
+    const int grp = lane / G, gl = lane % G;
+    uint32_t mine = node;
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        K qe[I];
+        bool up[I];
+        uint32_t nd[I];
+#pragma unroll
+        for (int s = 0; s < I; s++) {
+            const int k = r * (NG * I) + s * NG + grp;
+            qe[s] = __shfl_sync(0xffffffffu, q, k);
+            nd[s] = __shfl_sync(0xffffffffu, node, k);
+            up[s] = false;
+        }
+        for (int lvl = from; lvl < nl; lvl++) level_step<K, G, I>(seps + lvl_off[lvl], qe, up, nd, grp, gl);
+#pragma unroll
+        for (int s = 0; s < I; s++) {
+            const uint32_t y = __shfl_sync(0xffffffffu, nd[s], (lane % NG) * G);
+            mine = lane / NG == r * I + s ? y : mine;
+        }
+    }
+    return mine;
+}
+
+template <typename K, int G, int R>
+__device__ __forceinline__ uint32_t walk_lanes(const DevTree &t, int from, K q, uint32_t node, int lane) {
+    return walk_tree<K, G, R>(static_cast<const K *>(t.seps), t.lvl_off, from, t.nlevels, q, node, lane);
+}
+
+// 32 bytes of a leaf block by one thread.  Not evict-first: a block's value
+// sector, which comes with its key sector, is read a moment later (evicted
+// before that, 2^24 u64 queries took 1.19 ms instead of 0.84).
+__device__ __forceinline__ void load_sector(const void *p, uint32_t (&w)[8]) {
+    asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]),
+                   "=r"(w[7])
+                 : "l"(p));
+}
+
+// The first of a key sector's S keys equal to q, -1 if none (unused slots
+// hold all-ones keys, which a query above the largest key may equal).
+template <typename K, int S>
+__device__ __forceinline__ int first_match(const uint32_t (&w)[8], K q, K tmax) {
+    int at = -1;
+#pragma unroll
+    for (int k = S - 1; k >= 0; k--)
+        if (key_at<K>(w, k) == q) at = k;
+    return q <= tmax ? at : -1;
+}
+
+// Answers U queries per lane from their leaf blocks: put(u, l, value, hit) is
+// called once for query u of every lane l.
+//   4-byte keys: each thread loads its block's keys (32 bytes), then the
+//     matching value;
+//   8-byte keys: a lane pair per query, one lane the key sector, one the value
+//     sector, as one request.
+// A quarter of the instructions of the form it replaces (four lanes per
+// query, 16 bytes each, combined by shuffles and ballots).
+template <typename K, typename V, int U, bool PAIR, typename Put>
+__device__ __forceinline__ void leaf_answers(const unsigned char *__restrict__ leaves,
+                                             const uint32_t (&node)[U], const K (&qv)[U], K tmax, Put put) {
+    using LG = LeafGeom<K, V>;
+    const int lane = threadIdx.x & 31;
+    if constexpr (PAIR) {
+        static_assert(LG::BS == 2 * kSectorBytes, "values in the second sector");
+        uint32_t w[U][2][8];
+        K qk[U][2];
+#pragma unroll
+        for (int u = 0; u < U; u++)
+#pragma unroll
+            for (int h = 0; h < 2; h++) {  // lanes 2k, 2k + 1: the query of lane 16 h + k
+                const int k = h * 16 + (lane >> 1);
+                const uint32_t nd = __shfl_sync(0xffffffffu, node[u], k);
+                qk[u][h] = __shfl_sync(0xffffffffu, qv[u], k);
+                load_sector(leaves + (size_t)nd * LG::BS + (lane & 1) * kSectorBytes, w[u][h]);
+            }
+#pragma unroll
+        for (int u = 0; u < U; u++)
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                int at = first_match<K, LG::S>(w[u][h], qk[u][h], tmax);
+                at = __shfl_sync(0xffffffffu, at, lane & ~1);  // the key lane's
+                V v = key_max<V>();
+#pragma unroll
+                for (int k = 0; k < LG::S; k++)
+                    if (at == k) v = key_at<V>(w[u][h], k);
+                if (lane & 1) put(u, h * 16 + (lane >> 1), v, at >= 0);
+            }
+    } else {
+        uint32_t w[U][8];
+#pragma unroll
+        for (int u = 0; u < U; u++) load_sector(leaves + (size_t)node[u] * LG::BS, w[u]);
+        int at[U];
+        V v[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            at[u] = first_match<K, LG::S>(w[u], qv[u], tmax);
+            v[u] = at[u] >= 0 ? __ldg(reinterpret_cast<const V *>(leaves + (size_t)node[u] * LG::BS +
+                                                                 kSectorBytes) + at[u])
+                              : key_max<V>();
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) put(u, lane, v[u], at[u] >= 0);
+    }
+}
+
 }  // namespace bt
