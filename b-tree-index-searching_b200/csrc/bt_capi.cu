@@ -55,8 +55,10 @@ bt_status pipe_streams(int dev, cudaStream_t (&out)[kPipeSlots]) {
 
 bt_status point_device(const bt_tree *t, int mode, const void *d_q, uint64_t nq, void *d_out,
                        cudaStream_t s, uint8_t *d_found = nullptr) {
-    if (mode != BT_POINT_LEARNED && bucket_search_pays(t, nq, s)) {
-        const bt_status st = launch_bucket_search(t, d_q, nq, d_out, s, d_found);
+    if (mode == BT_POINT_LEARNED ? learned_buckets_pay(t, nq, s) : bucket_search_pays(t, nq, s)) {
+        const bt_status st = mode == BT_POINT_LEARNED
+                                 ? launch_learned_buckets(t, d_q, nq, d_out, d_found, s)
+                                 : launch_bucket_search(t, d_q, nq, d_out, s, d_found);
         if (st != BT_ERR_OUT_OF_MEMORY) return st;
         cudaGetLastError();  // no room for the ordered copy: the direct search
     }

@@ -120,6 +120,7 @@ struct LearnedDev {
     uint32_t root_err;       // |root's line prediction - line| <= root_err at every staged key
     uint32_t kpu;            // keys per leaf unit
     uint64_t units;          // leaf units
+    const uint32_t *seg_first;  // first segment that a query of bucket b can route to, b = 0 .. last + 1
     uint32_t stage_bytes;    // shared-memory bytes of the staged keys (whole bank rows)
 };
 
@@ -265,6 +266,10 @@ void free_learned(bt::LearnedState *s);
 // the counters of bt_learned_last_stats accumulate).
 bt_status launch_learned_search(const bt_tree *t, const void *d_q, uint64_t nq, void *d_out,
                                 uint8_t *d_found, cudaStream_t s);
+// The same for a batch that learned_buckets_pay for, ordered by bucket
+// (BT_ERR_OUT_OF_MEMORY when the workspace cannot be had).
+bt_status launch_learned_buckets(const bt_tree *t, const void *d_q, uint64_t nq, void *d_out,
+                                 uint8_t *d_found, cudaStream_t s);
 // Zeroes those counters (stream-ordered).
 bt_status reset_learned_stats(const bt_tree *t, cudaStream_t s);
 
@@ -308,6 +313,36 @@ bt_status launch_range_gather(const bt_tree *t, const uint32_t *rank, const uint
 bt_status launch_bucket_gather(int val_bytes, const void *res, const uint8_t *rfound,
                                const uint32_t *pos, uint64_t nq, void *d_out, uint8_t *d_found,
                                cudaStream_t s);
+// Workspace of a bucket search: the ordered queries, every query's slot, the
+// results by slot (and their found flags), the plan.
+struct BucketWs {
+    WsGuard ws;
+    unsigned char *q = nullptr, *res = nullptr;
+    uint32_t *pos = nullptr;
+    uint8_t *found = nullptr;
+    uint64_t max_items = 0;
+    BucketPlan bp;
+    explicit BucketWs(cudaStream_t s) : ws(s) {}
+    bt_status alloc(uint64_t nq, uint32_t buckets, size_t key_bytes, size_t res_bytes, bool flags) {
+        auto up256 = [](size_t x) { return (x + 255) / 256 * 256; };
+        const size_t kb = up256(nq * key_bytes), pb = up256(nq * sizeof(uint32_t));
+        const size_t rb = up256(nq * res_bytes), fb = flags ? up256(nq) : 0;
+        max_items = buckets + nq / kBucketSlice;
+        const bt_status st = ws.alloc(kb + pb + rb + fb + max_items * sizeof(uint4) +
+                                      (3 * kMaxBuckets + 64) * sizeof(uint32_t));
+        if (st != BT_OK) return st;
+        q = ws.as<unsigned char>();
+        pos = reinterpret_cast<uint32_t *>(q + kb);
+        res = q + kb + pb;
+        found = flags ? res + rb : nullptr;
+        bp.items = reinterpret_cast<uint4 *>(res + rb + fb);
+        bp.scratch = reinterpret_cast<uint32_t *>(bp.items + max_items);
+        bp.first = bp.scratch + 2 * kMaxBuckets;
+        bp.n_items = bp.first + kMaxBuckets + 1;
+        return BT_OK;
+    }
+};
+
 // The tree's map: as many buckets as kMaxBuckets allows.
 __host__ __device__ inline BucketMap bucket_map(uint64_t min_key, uint64_t max_key) {
     const int span = bitlen64(max_key - min_key);
@@ -329,9 +364,11 @@ bt_status launch_bucket_blocks(const bt_tree *t, const unsigned int *d_unsorted,
 // 2^19 ranges 50 / 66 us directly, 108 / 127 grouped first).
 constexpr uint64_t kBktMinQueries = 1ull << 22;
 constexpr uint64_t kOrderMinRanges = 1ull << 20;
+constexpr uint64_t kLearnedMinQueries = 1ull << 18;
 // Whether a point batch is searched by buckets, and that search (workspace
 // from the pool; BT_ERR_OUT_OF_MEMORY when it cannot be had).
 bool bucket_search_pays(const bt_tree *t, uint64_t nq, cudaStream_t s);
+bool learned_buckets_pay(const bt_tree *t, uint64_t nq, cudaStream_t s);
 bool bucket_bounds_pay(const bt_tree *t, uint64_t nr, cudaStream_t s);
 bt_status launch_bucket_bounds(const bt_tree *t, const void *d_lo, const void *d_hi, uint64_t nr,
                                uint64_t *d_counts, uint64_t *d_lb, cudaStream_t s);

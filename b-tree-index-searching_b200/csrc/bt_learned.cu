@@ -47,6 +47,7 @@ struct LearnedState {
     SegLine *d_seg = nullptr;
     CodeLine *d_codes = nullptr;
     void *d_stage = nullptr;
+    uint32_t *d_seg_first = nullptr;
     unsigned long long *d_stats = nullptr;
     uint64_t bytes = 0;
     int shape = 1;  // search kernel shape (bt_learned_set_shape)
@@ -59,6 +60,7 @@ void free_learned(LearnedState *s) {
     cudaFree(s->d_seg);
     cudaFree(s->d_codes);
     cudaFree(s->d_stage);
+    cudaFree(s->d_seg_first);
     cudaFree(s->d_stats);
     delete s;
 }
@@ -1060,6 +1062,232 @@ learned_kernel(const __grid_constant__ DevTree t, const __grid_constant__ Learne
     }
 }
 
+// ---- learned search of a batch ordered by bucket (launch_buckets) ----------
+//
+// A CTA takes the queries of one bucket and stages what the index says about
+// the bucket's keys in shared memory: its segments (32 bytes each, some 40 at
+// 2^28 keys and 2^16 segments) and its code lines (45 KB), where the plain
+// bucket search stages 330 KB of separators.  A query finds its segment by a
+// binary search of the bucket's, the segment's line and error give its window
+// of leaf units, a binary search of the window's code lines the line and one of
+// the line's codes the unit.  A key just past its unit's threshold bucket lands
+// a unit early and walks right, as in learned_kernel.  One thread per query up
+// to there (0.23 ms of the kernel at 2^28 keys and 2^24 queries), a lane pair
+// per query for the unit's one or two 64-byte blocks: 0.61 ms in all, against
+// 0.85 with the whole 128-byte unit read by lane quads (700 instructions of
+// the leaf step per 32 queries).
+
+// Shared memory of a bucket's ns segments and nl code lines.
+__host__ __device__ constexpr size_t bucket_index_bytes(size_t ns, size_t nl) {
+    return ns * 28 + nl * 33 * 4;
+}
+
+template <typename K, typename V, int T>
+__global__ void __launch_bounds__(T, 1024 / T)
+learned_bucket_kernel(const __grid_constant__ DevTree t, const __grid_constant__ LearnedDev m,
+                      const uint32_t *__restrict__ first, const uint4 *__restrict__ items,
+                      const uint32_t *__restrict__ n_items, uint32_t smem_bytes,
+                      const K *__restrict__ q, V *__restrict__ out, uint8_t *__restrict__ found) {
+    using LG = LeafGeom<K, V>;
+    constexpr uint32_t KPU = unit_keys<K, V>();
+    constexpr uint32_t BPU = kUnitBytes / LG::BS;
+    extern __shared__ uint4 smem_b[];
+    if (blockIdx.x >= *n_items) return;
+    const uint4 it = items[blockIdx.x];
+    const uint32_t U = (uint32_t)m.units;
+    // the bucket's units, segments and code lines
+    const uint32_t ulo = first[it.x] / BPU, uhi = min(first[it.x + 1] / BPU, U - 1);
+    const uint32_t l0 = ulo / kCodesPerLine;
+    const uint32_t nl = uhi > ulo ? (uhi - 1) / kCodesPerLine - l0 + 1 : 0u;
+    const uint32_t s0 = m.seg_first[it.x], ns = m.seg_first[it.x + 1] - s0 + 1;
+    const K *iq = q + it.y;
+    uint32_t n_extra = 0, n_fallback = 0;
+    // staged: the segments field by field, then the code lines a word apart
+    // from a whole number of bank rows (both are read at random)
+    if (bucket_index_bytes(ns, nl) > smem_bytes) {  // too many segments: the tree's full descent
+        for (uint32_t i = threadIdx.x; i < it.z; i += T) {
+            tree_point<K, V>(t, iq[i], out + it.y + i, found ? found + it.y + i : nullptr);
+            n_fallback++;
+        }
+        if (n_fallback) atomicAdd(&m.stats[1], (unsigned long long)n_fallback);
+        return;
+    }
+    uint64_t *s_key = reinterpret_cast<uint64_t *>(smem_b);
+    uint32_t *s_rlo = reinterpret_cast<uint32_t *>(s_key + ns), *s_cnt = s_rlo + ns, *s_eps = s_cnt + ns;
+    float *s_slope = reinterpret_cast<float *>(s_eps + ns), *s_icpt = s_slope + ns;
+    uint32_t *s_code = reinterpret_cast<uint32_t *>(s_icpt + ns);
+    {
+        const SegRec *gs = reinterpret_cast<const SegRec *>(m.seg) + s0;
+        for (uint32_t i = threadIdx.x; i < ns; i += T) {
+            const SegRec r = gs[i];
+            s_key[i] = r.key;
+            s_rlo[i] = r.r_lo;
+            s_cnt[i] = r.cnt;
+            s_eps[i] = r.eps;
+            s_slope[i] = r.slope;
+            s_icpt[i] = r.icpt;
+        }
+        const uint32_t *gl = reinterpret_cast<const uint32_t *>(m.codes + l0);
+#pragma unroll 8
+        for (uint32_t i = threadIdx.x; i < nl * 32; i += T) s_code[i + (i >> 5)] = gl[i];
+        __syncthreads();
+    }
+    auto line_base = [&](uint32_t l) {  // 64-bit base of staged line l
+        const uint32_t *w = s_code + l * 33;
+        return ((uint64_t)w[1] << 32) | w[0];
+    };
+    const int lane = threadIdx.x & 31;
+    const K tmax = (K)t.max_key;
+    const uint32_t blocks = (uint32_t)t.n_sectors;
+    const unsigned char *leaves = static_cast<const unsigned char *>(t.leaves);
+    for (uint32_t i0 = threadIdx.x & ~31u; i0 < it.z; i0 += T) {
+        const bool live = i0 + lane < it.z;
+        const K qv = live ? iq[i0 + lane] : (K)0;
+        const uint64_t key = (uint64_t)qv;
+        // the last segment that starts below the key (the first one if none does)
+        uint32_t sg = 0;
+        for (uint32_t len = ns; len > 1;) {
+            const uint32_t h = len >> 1;
+            sg = s_key[sg + h] < key ? sg + h : sg;
+            len -= h;
+        }
+        const uint32_t r_lo = s_rlo[sg], eps = s_eps[sg];
+        const float p = seg_pred(s_slope[sg], s_icpt[sg], s_cnt[sg], s_key[sg], key);
+        const uint32_t lo_r = r_lo + (uint32_t)floorf(p), hi_r = r_lo + (uint32_t)ceilf(p);
+        const uint32_t ra = eps >= lo_r ? 0u : lo_r - eps - 1u;
+        const uint32_t rb = hi_r + eps + 1u < hi_r ? 0xFFFFFFFFu : hi_r + eps + 1u;
+        uint32_t un = max(min(ra / KPU, U - 1), ulo);
+        const uint32_t ub = max(un, min(min(rb / KPU, U - 1), uhi));
+        if (ub > un) {
+            // the last of the window's lines that starts below the key: every
+            // unit of the lines before it ends at or before that start
+            uint32_t l = un / kCodesPerLine;
+            for (uint32_t len = (ub - 1) / kCodesPerLine - l + 1; len > 1;) {
+                const uint32_t h = len >> 1;
+                l = line_base(l + h - l0) < key ? l + h : l;
+                len -= h;
+            }
+            const uint64_t base = line_base(l - l0);
+            // a line: base (8 bytes), shift (2), codes (2 each)
+            const uint16_t *cw = reinterpret_cast<const uint16_t *>(s_code + (l - l0) * 33) + 4;
+            const uint64_t d = key > base ? (key - base) >> cw[0] : 0ull;
+            const uint32_t qd = d < kCodeMax ? (uint32_t)d : kCodeMax;
+            const uint32_t j0 = l * kCodesPerLine;
+            un = max(un, j0);
+            for (uint32_t z = min(ub, j0 + kCodesPerLine); un < z;) {  // its thresholds un .. z - 1
+                const uint32_t j = (un + z) >> 1;
+                if (cw[1 + j - j0] <= qd) un = j + 1;
+                else z = j;
+            }
+        }
+        // From the unit's first block on: a key above a block's last one goes to
+        // the next block, in the next unit (an extra unit read) up to the
+        // window's end, then to the tree's full descent.
+        constexpr bool PAIR = LG::BS == 2 * kSectorBytes;
+        constexpr int NH = PAIR ? 2 : 1;
+        uint32_t w[NH][8], blk[NH];
+        K qk[NH];
+#pragma unroll
+        for (int h = 0; h < NH; h++) {  // a lane pair (key sector, value sector) or one lane per query
+            const int k = PAIR ? 16 * h + (lane >> 1) : lane;
+            blk[h] = __shfl_sync(0xffffffffu, un, k) * BPU;
+            qk[h] = __shfl_sync(0xffffffffu, qv, k);
+            load_sector(leaves + (uint64_t)blk[h] * LG::BS + (PAIR ? (lane & 1) * kSectorBytes : 0), w[h]);
+        }
+#pragma unroll
+        for (int h = 0; h < NH; h++) {
+            const int k = PAIR ? 16 * h + (lane >> 1) : lane;
+            const uint32_t slot = it.y + i0 + k;
+            bool pend = i0 + k < it.z;
+            int walked = 0;
+            for (;;) {
+                const int m0 = first_match<K, LG::S>(w[h], qk[h], tmax);
+                int at = m0 >= 0 ? m0 : qk[h] > key_at<K>(w[h], LG::S - 1) ? -2 : -1;  // -2: above the block
+                if (PAIR) at = __shfl_sync(0xffffffffu, at, lane & ~1);  // the key lane's
+                if (pend && (at != -2 || blk[h] + 1 >= blocks)) {
+                    if (!PAIR || (lane & 1)) {
+                        V v = key_max<V>();
+                        if constexpr (PAIR) {
+#pragma unroll
+                            for (int z = 0; z < LG::S; z++)
+                                if (at == z) v = key_at<V>(w[h], z);
+                        } else if (at >= 0) {
+                            v = __ldg(reinterpret_cast<const V *>(leaves + (uint64_t)blk[h] * LG::BS + kSectorBytes) + at);
+                        }
+                        out[slot] = v;
+                        if (found) found[slot] = at >= 0 ? 1 : 0;
+                    }
+                    pend = false;
+                }
+                if (!__any_sync(0xffffffffu, pend)) break;
+                const uint32_t last = __shfl_sync(0xffffffffu, ub, k);
+                if (pend) {
+                    blk[h]++;
+                    if (blk[h] % BPU == 0) {  // a unit further
+                        const bool lost = blk[h] / BPU > last || ++walked > kMaxWalk;
+                        if (!PAIR || !(lane & 1)) {
+                            if (lost) {
+                                tree_point<K, V>(t, qk[h], out + slot, found ? found + slot : nullptr);
+                                n_fallback++;
+                            } else {
+                                n_extra++;
+                            }
+                        }
+                        pend = !lost;
+                    }
+                    if (pend)
+                        load_sector(leaves + (uint64_t)blk[h] * LG::BS + (PAIR ? (lane & 1) * kSectorBytes : 0), w[h]);
+                }
+                if (!__any_sync(0xffffffffu, pend)) break;
+            }
+        }
+    }
+    if (n_extra) atomicAdd(&m.stats[0], (unsigned long long)n_extra);
+    if (n_fallback) atomicAdd(&m.stats[1], (unsigned long long)n_fallback);
+}
+
+// seg_first[b]: the last segment that starts below bucket b's first key (0 if
+// none), b = 0 .. last + 1.
+__global__ void seg_first_kernel(const SegLine *__restrict__ seg, uint32_t nseg,
+                                 const __grid_constant__ BucketMap map, uint32_t *__restrict__ seg_first) {
+    const SegRec *segs = reinterpret_cast<const SegRec *>(seg);
+    const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
+    if (b > map.last + 1) return;
+    if (b == map.last + 1) {
+        seg_first[b] = nseg - 1;
+        return;
+    }
+    const uint64_t key = map.first_key(b);
+    uint32_t sg = 0;
+    for (uint32_t len = nseg; len > 1;) {
+        const uint32_t h = len >> 1;
+        sg = segs[sg + h].key < key ? sg + h : sg;
+        len -= h;
+    }
+    seg_first[b] = sg;
+}
+
+template <typename K, typename V, int T>
+bt_status learned_bucket_launch(const bt_tree *t, const BucketWs &w, size_t smem, cudaStream_t s) {
+    auto fn = learned_bucket_kernel<K, V, T>;
+    BT_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    count_launch();
+    fn<<<(unsigned)w.max_items, T, smem, s>>>(t->dev, t->learned->dev, w.bp.first, w.bp.items, w.bp.n_items,
+                                              (uint32_t)smem, (const K *)w.q, (V *)w.res, w.found);
+    BT_CUDA(cudaGetLastError());
+    return BT_OK;
+}
+
+template <typename K, typename V>
+bt_status learned_buckets(const bt_tree *t, const BucketWs &w, cudaStream_t s) {
+    // the fullest bucket's code lines, and four times the segments of an average one
+    const uint64_t lines = t->bucket_blocks * (uint64_t)LeafGeom<K, V>::BS / kUnitBytes / kCodesPerLine + 3;
+    const uint64_t segs = 4 * (t->learned->dev.nseg / (bucket_map(t->min_key, t->max_key).last + 1) + 16);
+    const size_t need = bucket_index_bytes(segs, lines);
+    if (need <= 100 * 1024) return learned_bucket_launch<K, V, 512>(t, w, need, s);
+    return learned_bucket_launch<K, V, 1024>(t, w, std::min<size_t>(need, 200 * 1024), s);
+}
+
 template <typename K, typename V, int T>
 bt_status learned_launch_t(const bt_tree *t, const void *d_q, uint64_t nq, void *d_out,
                            uint8_t *d_found, cudaStream_t s) {
@@ -1369,6 +1597,15 @@ bt_status train_impl(bt_tree *t, const bt_learned_config &cfg, cudaStream_t s,
     count_launch();
     root_err_kernel<<<grid_of(nls, 256, 4), 256, 0, s>>>(st->d_mlp, H, x, nls, err);
 
+    // ---- where each bucket's segments start
+    {
+        const BucketMap map = bucket_map(t->min_key, t->max_key);
+        BT_CUDA(cudaMalloc((void **)&st->d_seg_first, (map.last + 2) * sizeof(uint32_t)));
+        count_launch();
+        seg_first_kernel<<<(map.last + 2 + 255) / 256, 256, 0, s>>>(st->d_seg, (uint32_t)nseg, map,
+                                                                    st->d_seg_first);
+    }
+
     // ---- unit thresholds
     const uint64_t ncl = units > 1 ? (units - 1 + kCodesPerLine - 1) / kCodesPerLine : 0;
     BT_CUDA(cudaMalloc((void **)&st->d_codes, std::max<uint64_t>(1, ncl) * sizeof(CodeLine)));
@@ -1400,6 +1637,7 @@ bt_status train_impl(bt_tree *t, const bt_learned_config &cfg, cudaStream_t s,
     d.root_err = herr[0];
     d.kpu = kpu;
     d.units = units;
+    d.seg_first = st->d_seg_first;
     d.stage_bytes = (uint32_t)stage_bytes;
     st->bytes = (uint64_t)nls * sizeof(SegLine) + ncl * sizeof(CodeLine) + stage_bytes +
                 np * sizeof(float);
@@ -1447,6 +1685,23 @@ bt_status launch_learned_search(const bt_tree *t, const void *d_q, uint64_t nq, 
                                  : learned_launch<uint32_t, uint64_t>(t, d_q, nq, d_out, d_found, s);
     return t->val_bytes == 4 ? learned_launch<uint64_t, uint32_t>(t, d_q, nq, d_out, d_found, s)
                              : learned_launch<uint64_t, uint64_t>(t, d_q, nq, d_out, d_found, s);
+}
+
+bt_status launch_learned_buckets(const bt_tree *t, const void *d_q, uint64_t nq, void *d_out,
+                                 uint8_t *d_found, cudaStream_t s) {
+    const BucketMap map = bucket_map(t->min_key, t->max_key);
+    BucketWs w(s);
+    bt_status st = w.alloc(nq, map.last + 1, t->key_bytes, t->val_bytes, d_found != nullptr);
+    if (st == BT_OK) st = launch_buckets(t, map, d_q, nullptr, nq, w.q, w.pos, w.bp, s);
+    if (st != BT_OK) return st;
+    if (t->key_bytes == 4)
+        st = t->val_bytes == 4 ? learned_buckets<uint32_t, uint32_t>(t, w, s)
+                               : learned_buckets<uint32_t, uint64_t>(t, w, s);
+    else
+        st = t->val_bytes == 4 ? learned_buckets<uint64_t, uint32_t>(t, w, s)
+                               : learned_buckets<uint64_t, uint64_t>(t, w, s);
+    if (st != BT_OK) return st;
+    return launch_bucket_gather(t->val_bytes, w.res, w.found, w.pos, nq, d_out, d_found, s);
 }
 
 bt_status reset_learned_stats(const bt_tree *t, cudaStream_t s) {

@@ -777,8 +777,8 @@ bt_status launch_point_search(const bt_tree *t, const void *d_q, const uint32_t 
 // into few of the equal stretches (a bucket of over four times the average)
 // keep the direct search: their windows lie levels above the leaves.  So does
 // a stream under capture, whose graph then holds no allocation.
-static bool buckets_suit(const bt_tree *t, uint64_t nq, cudaStream_t s) {
-    if (t->n == 0 || nq >= (1ull << 32) || nq < t->n_sectors / 8) return false;
+static bool buckets_suit(const bt_tree *t, uint64_t nq, uint64_t blocks_per_query, cudaStream_t s) {
+    if (t->n == 0 || nq >= (1ull << 32) || nq < t->n_sectors / blocks_per_query) return false;
     const uint64_t buckets = bucket_map(t->min_key, t->max_key).last + 1;
     if (t->bucket_blocks == 0 || t->bucket_blocks > 4 * (t->n_sectors / buckets) + 64) return false;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -788,7 +788,17 @@ static bool buckets_suit(const bt_tree *t, uint64_t nq, cudaStream_t s) {
 }
 
 bool bucket_search_pays(const bt_tree *t, uint64_t nq, cudaStream_t s) {
-    return nq >= kBktMinQueries && buckets_suit(t, nq, s);
+    return nq >= kBktMinQueries && buckets_suit(t, nq, 8, s);
+}
+
+// Learned searches, one query at a time / by buckets (us; u64 keys):
+//                 2^17 queries   2^18         2^20          2^24
+//   2^20 keys       57 / 57      97 / 59     209 / 87
+//   2^24            57 / 59     100 / 62     213 / 112
+//   2^28            61 / 91     106 / 100    230 / 143    1211 / 848
+// (the staged index is a seventh of the separators: no rule on keys per query)
+bool learned_buckets_pay(const bt_tree *t, uint64_t nq, cudaStream_t s) {
+    return nq >= kLearnedMinQueries && buckets_suit(t, nq, ~0ull, s);
 }
 
 // Range bounds, direct / by buckets (us; the buckets take both bounds of a
@@ -800,40 +810,10 @@ bool bucket_search_pays(const bt_tree *t, uint64_t nq, cudaStream_t s) {
 //                           76 / 90     133 / 110    477 / 229
 //   u64, 2^26              105 / 109    176 / 142    654 / 331
 bool bucket_bounds_pay(const bt_tree *t, uint64_t nr, cudaStream_t s) {
-    return nr >= kOrderMinRanges && nr < (1ull << 31) && t->n < (1ull << 32) && buckets_suit(t, 2 * nr, s);
+    return nr >= kOrderMinRanges && nr < (1ull << 31) && t->n < (1ull << 32) && buckets_suit(t, 2 * nr, 8, s);
 }
 
 namespace {
-// Workspace of a bucket search: the ordered queries, every query's slot, the
-// results by slot (and their found flags), the plan.
-struct BucketWs {
-    WsGuard ws;
-    unsigned char *q = nullptr, *res = nullptr;
-    uint32_t *pos = nullptr;
-    uint8_t *found = nullptr;
-    uint64_t max_items = 0;
-    BucketPlan bp;
-    explicit BucketWs(cudaStream_t s) : ws(s) {}
-    bt_status alloc(uint64_t nq, uint32_t buckets, size_t key_bytes, size_t res_bytes, bool flags) {
-        auto up256 = [](size_t x) { return (x + 255) / 256 * 256; };
-        const size_t kb = up256(nq * key_bytes), pb = up256(nq * sizeof(uint32_t));
-        const size_t rb = up256(nq * res_bytes), fb = flags ? up256(nq) : 0;
-        max_items = buckets + nq / kBucketSlice;
-        const bt_status st = ws.alloc(kb + pb + rb + fb + max_items * sizeof(uint4) +
-                                      (3 * kMaxBuckets + 64) * sizeof(uint32_t));
-        if (st != BT_OK) return st;
-        q = ws.as<unsigned char>();
-        pos = reinterpret_cast<uint32_t *>(q + kb);
-        res = q + kb + pb;
-        found = flags ? res + rb : nullptr;
-        bp.items = reinterpret_cast<uint4 *>(res + rb + fb);
-        bp.scratch = reinterpret_cast<uint32_t *>(bp.items + max_items);
-        bp.first = bp.scratch + 2 * kMaxBuckets;
-        bp.n_items = bp.first + kMaxBuckets + 1;
-        return BT_OK;
-    }
-};
-
 template <bool BOUND>
 bt_status bucket_types(const bt_tree *t, const BucketWs &w, cudaStream_t s) {
     if (t->key_bytes == 4)
