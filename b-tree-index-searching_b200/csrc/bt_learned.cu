@@ -208,8 +208,8 @@ __device__ __forceinline__ typename T::W pla_cross(typename T::X ax, typename T:
 // lines of largest (M = Ma-Mb) and smallest (N = Na-Nb) slope; a point is
 // feasible iff its lower point is not above M and its upper point not below
 // N.  A segment also closes when a hull would exceed kHullCap points.
-// COUNT: counts[c] = segments of chunk c.  Otherwise writes segment k of
-// chunk c at offsets[c] + k: first rank and the mean of M and N as
+// Returns the chunk's segments; without COUNT also writes segment k of chunk c
+// at offsets[c] + k: first rank and the mean of M and N as
 // rank - first = icpt + slope * (key - first key).
 //
 // The fit is a chain of 2^14 dependent points per chunk, bound by its
@@ -239,12 +239,11 @@ __device__ __forceinline__ typename T::W pla_cross(typename T::X ax, typename T:
 // loops); a warp per chunk with a lane per point of both hulls and batches
 // of 32 points tested ahead 12.6 ms; this form 9.6 ms.
 template <typename K, typename V, bool COUNT, typename T>
-__device__ __forceinline__ void pla_chunk(const unsigned char *__restrict__ leaves, uint64_t base,
-                                          uint32_t m, uint64_t key0, uint32_t eps, uint64_t c,
-                                          uint64_t *__restrict__ counts,
-                                          const uint64_t *__restrict__ offsets,
-                                          uint32_t *__restrict__ starts,
-                                          double *__restrict__ slopes, double *__restrict__ icpts) {
+__device__ __forceinline__ uint32_t pla_chunk(const unsigned char *__restrict__ leaves, uint64_t base,
+                                              uint32_t m, uint64_t key0, uint32_t eps, uint64_t c,
+                                              const uint64_t *__restrict__ offsets,
+                                              uint32_t *__restrict__ starts,
+                                              double *__restrict__ slopes, double *__restrict__ icpts) {
     using X = typename T::X;
     using Y = typename T::Y;
     using W = typename T::W;
@@ -395,26 +394,40 @@ __device__ __forceinline__ void pla_chunk(const unsigned char *__restrict__ leav
         }
     }
     close(m);
-    if (COUNT && lane == 0) counts[c] = nseg;
+    return nseg;
 }
 
-// The chunks of one kind (WIDE or narrow); the other kind's warps return, so
-// that each kernel keeps only its own registers.
+// Bounds evaluated by one launch (grid row y takes eps[y]).
+constexpr int kPlaBounds = 8;
+struct PlaBounds {
+    uint32_t eps[kPlaBounds];
+};
+
+// Every stride-th chunk of one kind (WIDE or narrow); the other kind's warps
+// return, so that each kernel keeps only its own registers.  COUNT: totals[y]
+// += the chunk's segments, and counts[y * nchunks + chunk] when counts is not
+// null.
 template <typename K, typename V, bool COUNT, bool WIDE>
 __global__ void __launch_bounds__(kPlaThreads)
-pla_kernel(const unsigned char *__restrict__ leaves, uint64_t n, uint32_t eps, uint64_t nchunks,
-           uint64_t *__restrict__ counts, const uint64_t *__restrict__ offsets,
+pla_kernel(const unsigned char *__restrict__ leaves, uint64_t n, const __grid_constant__ PlaBounds bounds,
+           uint64_t nchunks, uint32_t stride, uint64_t *__restrict__ counts,
+           unsigned long long *__restrict__ totals, const uint64_t *__restrict__ offsets,
            uint32_t *__restrict__ starts, double *__restrict__ slopes, double *__restrict__ icpts) {
-    const uint64_t c = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+    const uint64_t c = ((blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5) * stride;
     if (c >= nchunks) return;
+    const uint32_t eps = bounds.eps[blockIdx.y];
     const uint64_t base = c * kPlaChunk;
     const uint32_t m = (uint32_t)min(kPlaChunk, n - base);
     const uint64_t key0 = (uint64_t)leaf_key<K, V>(leaves, base);
     const uint64_t span = (uint64_t)leaf_key<K, V>(leaves, base + m - 1) - key0;
     const bool wide = span >= (1ull << 31) || eps > kPlaNarrowEps;
     if (wide != WIDE) return;
-    pla_chunk<K, V, COUNT, std::conditional_t<WIDE, PlaWide, PlaNarrow>>(
-        leaves, base, m, key0, eps, c, counts, offsets, starts, slopes, icpts);
+    const uint32_t nseg = pla_chunk<K, V, COUNT, std::conditional_t<WIDE, PlaWide, PlaNarrow>>(
+        leaves, base, m, key0, eps, c, offsets, starts, slopes, icpts);
+    if (COUNT && (threadIdx.x & 31) == 0) {
+        if (counts) counts[blockIdx.y * nchunks + c] = nseg;
+        atomicAdd(&totals[blockIdx.y], (unsigned long long)nseg);
+    }
 }
 
 // Segment lines from the segmentation (one thread per line): first keys,
@@ -1443,50 +1456,123 @@ bt_status train_impl(bt_tree *t, const bt_learned_config &cfg, cudaStream_t s,
 
     // ---- segmentation: the bound, then the segments
     const uint64_t nchunks = (n + kPlaChunk - 1) / kPlaChunk;
+    constexpr int kSlots = 4;  // per-chunk counts: two of the bounds counted last, two with hi's
     DevBuf bcnt, boff, btot;
-    BT_CUDA(cudaMalloc(&bcnt.p, nchunks * sizeof(uint64_t)));
+    BT_CUDA(cudaMalloc(&bcnt.p, kSlots * nchunks * sizeof(uint64_t)));
     BT_CUDA(cudaMalloc(&boff.p, nchunks * sizeof(uint64_t)));
-    BT_CUDA(cudaMalloc(&btot.p, 2 * sizeof(uint64_t)));
+    BT_CUDA(cudaMalloc(&btot.p, kPlaBounds * sizeof(uint64_t)));
     uint64_t *cnt = (uint64_t *)bcnt.p, *off = (uint64_t *)boff.p, *tot = (uint64_t *)btot.p;
-    const unsigned pg = (unsigned)((nchunks * 32 + kPlaThreads - 1) / kPlaThreads);
-    auto count_at = [&](uint32_t eps, uint64_t *total) -> bt_status {
+    // Segments of k bounds over every stride-th chunk; with slot >= 0 the
+    // per-chunk counts of bound y go to slot + y.
+    auto count_at = [&](const PlaBounds &e, int k, uint32_t stride, int slot, uint64_t *total) -> bt_status {
+        const uint64_t warps = (nchunks + stride - 1) / stride;
+        const dim3 grid((unsigned)((warps * 32 + kPlaThreads - 1) / kPlaThreads), (unsigned)k);
+        uint64_t *c = slot < 0 ? nullptr : cnt + (uint64_t)slot * nchunks;
+        BT_CUDA(cudaMemsetAsync(tot, 0, (size_t)k * sizeof(uint64_t), s));
         count_launch();
-        pla_kernel<K, V, true, false><<<pg, kPlaThreads, 0, s>>>(leaves, n, eps, nchunks, cnt, nullptr,
-                                                                 nullptr, nullptr, nullptr);
+        pla_kernel<K, V, true, false><<<grid, kPlaThreads, 0, s>>>(
+            leaves, n, e, nchunks, stride, c, (unsigned long long *)tot, nullptr, nullptr, nullptr, nullptr);
         count_launch();
-        pla_kernel<K, V, true, true><<<pg, kPlaThreads, 0, s>>>(leaves, n, eps, nchunks, cnt, nullptr,
-                                                                nullptr, nullptr, nullptr);
+        pla_kernel<K, V, true, true><<<grid, kPlaThreads, 0, s>>>(
+            leaves, n, e, nchunks, stride, c, (unsigned long long *)tot, nullptr, nullptr, nullptr, nullptr);
         BT_CUDA(cudaGetLastError());
-        bt_status r = launch_scan_u64(cnt, off, nchunks, tot, s);
-        if (r != BT_OK) return r;
-        BT_CUDA(cudaMemcpyAsync(total, tot, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
+        BT_CUDA(cudaMemcpyAsync(total, tot, (size_t)k * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
         BT_CUDA(cudaStreamSynchronize(s));
         return BT_OK;
     };
     uint32_t eps = cfg.max_error;
     uint64_t nseg = 0;
     bt_status r;
-    uint32_t counted = 0;  // the bound of the last count (its per-chunk offsets are in off)
+    int at = 0;  // slot of eps's counts
     if (eps == 0) {
         // The least bound whose segmentation has at most num_segments
-        // segments (the count does not grow with the bound).  The bracket
-        // (lo, hi] -- count(lo) above the target, count(hi) at or below --
-        // grows by 4x from 8, then narrows by interpolating log(count)
-        // against log(bound), with a bisection step whenever an
-        // interpolated step fails to halve it.
+        // segments (the count does not grow with the bound): count(lo) is
+        // above the target, count(hi) at or below it, every count a full one.
         const double tgt = (double)cfg.num_segments;
-        uint32_t lo = 0, hi = 8;
+        uint32_t lo = 0, hi = 0;  // hi = 0: none yet
         uint64_t c_lo = 0, c_hi = 0;
-        for (;;) {
-            if ((r = count_at(hi, &c_hi)) != BT_OK) return r;
-            counted = hi;
-            if (c_hi <= cfg.num_segments || hi >= (1u << 30)) break;
-            lo = hi;
-            c_lo = c_hi;
-            hi = std::min<uint32_t>(hi * 4, 1u << 30);
+        int hi_slot = -1;
+        auto full = [&](uint32_t a, uint32_t b) -> bt_status {  // counts a and (b > a) b
+            const int slot = hi_slot >= 0 && hi_slot < 2 ? 2 : 0;  // not over those of hi
+            PlaBounds e = {{a, b}};
+            uint64_t c[2] = {0, 0};
+            const int k = b > a ? 2 : 1;
+            const bt_status st = count_at(e, k, 1, slot, c);
+            if (st != BT_OK) return st;
+            for (int y = 0; y < k; y++) {
+                if (c[y] > cfg.num_segments) {
+                    if (e.eps[y] > lo) {
+                        lo = e.eps[y];
+                        c_lo = c[y];
+                    }
+                } else if (hi == 0 || e.eps[y] < hi) {
+                    hi = e.eps[y];
+                    c_hi = c[y];
+                    hi_slot = slot + y;
+                }
+            }
+            return BT_OK;
+        };
+        // First guess, from the counts of a few chunks at eight bounds at once,
+        // powers of four and then in equal ratios inside the bracket found (a
+        // launch of few chunks takes as long as one warp's chain, so the eight
+        // come for the price of one).
+        uint32_t guess = 0;
+        if (nchunks >= 256) {
+            const uint32_t stride = (uint32_t)(nchunks / std::max<uint64_t>(128, nchunks / 16));
+            const double scale = (double)nchunks / (double)((nchunks + stride - 1) / stride);
+            PlaBounds e;
+            uint64_t c[kPlaBounds];
+            double x0 = 1.0, x1 = 0.0, y0 = 0.0, y1 = 0.0;
+            for (int y = 0; y < kPlaBounds; y++) e.eps[y] = 1u << (2 * y + 2);
+            for (int pass = 0; pass < 2; pass++) {
+                if ((r = count_at(e, kPlaBounds, stride, -1, c)) != BT_OK) return r;
+                int y = 0;
+                while (y < kPlaBounds && (double)c[y] * scale > tgt) y++;
+                if (y == kPlaBounds) break;  // above the widest bound tried: no guess
+                x1 = e.eps[y];
+                y1 = (double)c[y] * scale;
+                if (y > 0) {
+                    x0 = e.eps[y - 1];
+                    y0 = (double)c[y - 1] * scale;
+                }
+                if (y0 > y1 && y1 > 0) {
+                    const double f = (std::log(y0) - std::log(tgt)) / (std::log(y0) - std::log(y1));
+                    guess = (uint32_t)std::ceil(std::exp(std::log(x0) + f * (std::log(x1) - std::log(x0))));
+                } else {
+                    guess = (uint32_t)x1;
+                }
+                for (int z = 0; z < kPlaBounds; z++)
+                    e.eps[z] = (uint32_t)std::ceil(x0 * std::pow(x1 / x0, (z + 1) / (double)kPlaBounds));
+            }
         }
+        if (guess > 1) {
+            // widen from the guess until it is bracketed
+            uint32_t d = 1;
+            if ((r = full(guess - 1, guess)) != BT_OK) return r;
+            while (hi == 0 && lo < (1u << 30)) {
+                d = std::min<uint32_t>(2 * d, (1u << 30) - lo);
+                if ((r = full(lo + (d + 1) / 2, lo + d)) != BT_OK) return r;
+            }
+            d = 1;
+            while (lo == 0 && hi > 1) {
+                d = std::min<uint32_t>(2 * d, hi - 1);
+                if ((r = full(hi - d, hi - d / 2 > hi - d ? hi - d / 2 : 0)) != BT_OK) return r;
+            }
+        } else {
+            for (uint32_t e = 8;; e = std::min<uint32_t>(e * 4, 1u << 30)) {  // a bracket by factors of 4
+                if ((r = full(e, 0)) != BT_OK) return r;
+                if (hi != 0 || e >= (1u << 30)) break;
+            }
+        }
+        if (hi == 0) {  // more segments than asked for even at the widest bound
+            hi = 1u << 30;
+            if (lo != hi && (r = full(hi, 0)) != BT_OK) return r;
+        }
+        // narrow it by interpolating log(count) against log(bound), with a
+        // bisection step whenever an interpolated step fails to halve it
         bool bisect = false;
-        while (hi - lo > 1) {
+        while (hi - lo > 1 && hi > lo) {
             uint32_t m = lo + (hi - lo) / 2;
             if (!bisect && lo > 0 && c_hi > 0 && c_lo > c_hi) {
                 const double f = (std::log((double)c_lo) - std::log(tgt)) /
@@ -1495,23 +1581,19 @@ bt_status train_impl(bt_tree *t, const bt_learned_config &cfg, cudaStream_t s,
                 const double g = std::ceil(std::exp(lm));
                 m = g <= (double)lo ? lo + 1 : g >= (double)hi ? hi - 1 : (uint32_t)g;
             }
-            uint64_t c = 0;
-            if ((r = count_at(m, &c)) != BT_OK) return r;
-            counted = m;
             const uint32_t w = hi - lo;
-            if (c <= cfg.num_segments) {
-                hi = m;
-                c_hi = c;
-            } else {
-                lo = m;
-                c_lo = c;
-            }
+            if ((r = full(m, 0)) != BT_OK) return r;
             bisect = !bisect && (hi - lo) * 2 > w;
         }
         eps = hi;
+        at = hi_slot;
+        nseg = c_hi;
     }
-    if (counted != eps && (r = count_at(eps, &nseg)) != BT_OK) return r;
-    if (counted == eps) BT_CUDA(cudaMemcpy(&nseg, tot, sizeof(uint64_t), cudaMemcpyDeviceToHost));
+    if (cfg.max_error != 0 || at < 0) {
+        at = 0;
+        if ((r = count_at(PlaBounds{{eps}}, 1, 1, 0, &nseg)) != BT_OK) return r;
+    }
+    if ((r = launch_scan_u64(cnt + (uint64_t)at * nchunks, off, nchunks, nullptr, s)) != BT_OK) return r;
     const uint32_t nls = (uint32_t)((nseg + kSegPerLine - 1) / kSegPerLine);
     const uint32_t row = 128;  // stage in whole bank rows (the swizzle permutes within rows)
     const uint64_t stage_bytes = ((uint64_t)nls * sizeof(K) + row - 1) / row * row;
@@ -1524,12 +1606,15 @@ bt_status train_impl(bt_tree *t, const bt_learned_config &cfg, cudaStream_t s,
     BT_CUDA(cudaMalloc(&bst.p, nseg * sizeof(uint32_t)));
     BT_CUDA(cudaMalloc(&bsl.p, nseg * sizeof(double)));
     BT_CUDA(cudaMalloc(&bic.p, nseg * sizeof(double)));
+    const unsigned pg = (unsigned)((nchunks * 32 + kPlaThreads - 1) / kPlaThreads);
     count_launch();
     pla_kernel<K, V, false, false><<<pg, kPlaThreads, 0, s>>>(
-        leaves, n, eps, nchunks, nullptr, off, (uint32_t *)bst.p, (double *)bsl.p, (double *)bic.p);
+        leaves, n, PlaBounds{{eps}}, nchunks, 1, nullptr, nullptr, off, (uint32_t *)bst.p, (double *)bsl.p,
+        (double *)bic.p);
     count_launch();
     pla_kernel<K, V, false, true><<<pg, kPlaThreads, 0, s>>>(
-        leaves, n, eps, nchunks, nullptr, off, (uint32_t *)bst.p, (double *)bsl.p, (double *)bic.p);
+        leaves, n, PlaBounds{{eps}}, nchunks, 1, nullptr, nullptr, off, (uint32_t *)bst.p, (double *)bsl.p,
+        (double *)bic.p);
     BT_CUDA(cudaGetLastError());
 
     // ---- segment lines and their exact bounds

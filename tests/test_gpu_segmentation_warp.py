@@ -43,3 +43,24 @@ def test_segment_count_equals_the_oracles(bt, orc, cuda, kind, n, eps):
         got = t.point_search_learned(q)
         assert torch.equal(got.view(torch.int64), t.point_search(q).view(torch.int64))
         assert t.learned_last_stats()[1] == 0
+
+
+@pytest.mark.parametrize("kind,segments", [("narrow", 300), ("narrow", 5000), ("narrow", 70000),
+                                           ("bent", 20000), ("equal", 60000), ("wide", 3000)])
+def test_target_gives_the_least_bound_of_a_large_tree(bt, orc, cuda, kind, segments):
+    """256 chunks and more: the bound is guessed from a sample of them, then
+    counted in full on both sides."""
+    import torch
+    n = 257 * CHUNK + 5
+    keys = _keys(kind, n)
+    with bt.Tree.build(torch.from_numpy(keys).to(cuda), torch.arange(n, device=cuda)) as t:
+        if kind == "bent":  # the hull cap alone cuts more segments, whatever the bound
+            with pytest.raises(bt.BTreeError) as e:
+                t.learned_train(num_segments=segments, iterations=1)
+            assert e.value.name == "BT_ERR_NOT_SUPPORTED"
+            return
+        rep = t.learned_train(num_segments=segments, iterations=1)
+    eps = rep["max_error"]
+    count = lambda e: orc.pla_segments(keys, e, chunk=CHUNK, hull_cap=HULL_CAP, lines=False)  # noqa: E731
+    assert rep["num_segments"] == count(eps) <= segments
+    assert eps == 1 or count(eps - 1) > segments
