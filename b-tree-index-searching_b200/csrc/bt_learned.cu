@@ -1092,6 +1092,7 @@ learned_kernel(const __grid_constant__ DevTree t, const __grid_constant__ Learne
 // 0.85 with the whole 128-byte unit read by lane quads (700 instructions of
 // the leaf step per 32 queries).
 
+constexpr size_t kBucketIndexMax = 200 * 1024;
 // Shared memory of a bucket's ns segments and nl code lines.
 __host__ __device__ constexpr size_t bucket_index_bytes(size_t ns, size_t nl) {
     return ns * 28 + nl * 33 * 4;
@@ -1285,7 +1286,8 @@ __global__ void seg_first_kernel(const SegLine *__restrict__ seg, uint32_t nseg,
 template <typename K, typename V, int T>
 bt_status learned_bucket_launch(const bt_tree *t, const BucketWs &w, size_t smem, cudaStream_t s) {
     auto fn = learned_bucket_kernel<K, V, T>;
-    BT_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // one limit for every tree: threads with different trees may set it at once
+    BT_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBucketIndexMax));
     count_launch();
     fn<<<(unsigned)w.max_items, T, smem, s>>>(t->dev, t->learned->dev, w.bp.first, w.bp.items, w.bp.n_items,
                                               (uint32_t)smem, (const K *)w.q, (V *)w.res, w.found);
@@ -1299,8 +1301,8 @@ bt_status learned_buckets(const bt_tree *t, const BucketWs &w, cudaStream_t s) {
     const uint64_t lines = t->bucket_blocks * (uint64_t)LeafGeom<K, V>::BS / kUnitBytes / kCodesPerLine + 3;
     const uint64_t segs = 4 * (t->learned->dev.nseg / (bucket_map(t->min_key, t->max_key).last + 1) + 16);
     const size_t need = bucket_index_bytes(segs, lines);
-    if (need <= 100 * 1024) return learned_bucket_launch<K, V, 512>(t, w, need, s);
-    return learned_bucket_launch<K, V, 1024>(t, w, std::min<size_t>(need, 200 * 1024), s);
+    if (need <= kBucketIndexMax / 2) return learned_bucket_launch<K, V, 512>(t, w, need, s);  // two CTAs per SM
+    return learned_bucket_launch<K, V, 1024>(t, w, std::min(need, kBucketIndexMax), s);
 }
 
 template <typename K, typename V, int T>
