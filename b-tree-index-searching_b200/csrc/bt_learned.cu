@@ -1088,9 +1088,12 @@ learned_kernel(const __grid_constant__ DevTree t, const __grid_constant__ Learne
 // the line's codes the unit.  A key just past its unit's threshold bucket lands
 // a unit early and walks right, as in learned_kernel.  One thread per query up
 // to there (0.23 ms of the kernel at 2^28 keys and 2^24 queries), a lane pair
-// per query for the unit's one or two 64-byte blocks: 0.61 ms in all, against
-// 0.85 with the whole 128-byte unit read by lane quads (700 instructions of
-// the leaf step per 32 queries).
+// per query for the unit's one or two 64-byte blocks, both loaded at once: the
+// whole call takes 0.797 ms, 0.847 with the second block read only after the
+// first one's answer (a chain of two random reads for half the queries), and the
+// kernel alone took 0.85 with the unit read by lane quads (700 instructions of
+// the leaf step per 32 queries).  512 threads twice per SM at 64 registers: with
+// 448 and 384 threads (72 and 80 registers) the call takes 0.891 and 0.927 ms.
 
 constexpr size_t kBucketIndexMax = 200 * 1024;
 // Shared memory of a bucket's ns segments and nl code lines.
@@ -1196,39 +1199,50 @@ learned_bucket_kernel(const __grid_constant__ DevTree t, const __grid_constant__
                 else z = j;
             }
         }
-        // From the unit's first block on: a key above a block's last one goes to
-        // the next block, in the next unit (an extra unit read) up to the
-        // window's end, then to the tree's full descent.
+        // The unit's blocks, those of all the warp's queries in flight at once; a
+        // key above the last one's keys goes to the next unit (an extra unit
+        // read) up to the window's end, then to the tree's full descent.
         constexpr bool PAIR = LG::BS == 2 * kSectorBytes;
         constexpr int NH = PAIR ? 2 : 1;
-        uint32_t w[NH][8], blk[NH];
+        uint32_t w[NH][BPU][8], u2[NH];
         K qk[NH];
+        auto load = [&](int h) {  // a lane pair (key sectors, value sectors) or one lane per query
 #pragma unroll
-        for (int h = 0; h < NH; h++) {  // a lane pair (key sector, value sector) or one lane per query
+            for (uint32_t z = 0; z < BPU; z++) {
+                // the last unit may lack its second block: its first one again
+                const uint32_t blk = min(u2[h] * BPU + z, blocks - 1);
+                load_sector(leaves + (uint64_t)blk * LG::BS + (PAIR ? (lane & 1) * kSectorBytes : 0), w[h][z]);
+            }
+        };
+#pragma unroll
+        for (int h = 0; h < NH; h++) {
             const int k = PAIR ? 16 * h + (lane >> 1) : lane;
-            blk[h] = __shfl_sync(0xffffffffu, un, k) * BPU;
+            u2[h] = __shfl_sync(0xffffffffu, un, k);
             qk[h] = __shfl_sync(0xffffffffu, qv, k);
-            load_sector(leaves + (uint64_t)blk[h] * LG::BS + (PAIR ? (lane & 1) * kSectorBytes : 0), w[h]);
+            load(h);
         }
 #pragma unroll
         for (int h = 0; h < NH; h++) {
             const int k = PAIR ? 16 * h + (lane >> 1) : lane;
             const uint32_t slot = it.y + i0 + k;
             bool pend = i0 + k < it.z;
-            int walked = 0;
-            for (;;) {
-                const int m0 = first_match<K, LG::S>(w[h], qk[h], tmax);
-                int at = m0 >= 0 ? m0 : qk[h] > key_at<K>(w[h], LG::S - 1) ? -2 : -1;  // -2: above the block
+            for (int walked = 0;; walked++) {
+                int at = qk[h] > key_at<K>(w[h][BPU - 1], LG::S - 1) && u2[h] + 1 < U ? -2 : -1;  // -2: above the unit
+#pragma unroll
+                for (int z = (int)BPU - 1; z >= 0; z--) {
+                    const int m0 = first_match<K, LG::S>(w[h][z], qk[h], tmax);
+                    if (m0 >= 0) at = m0 + z * LG::S;
+                }
                 if (PAIR) at = __shfl_sync(0xffffffffu, at, lane & ~1);  // the key lane's
-                if (pend && (at != -2 || blk[h] + 1 >= blocks)) {
+                if (pend && at != -2) {
                     if (!PAIR || (lane & 1)) {
                         V v = key_max<V>();
                         if constexpr (PAIR) {
 #pragma unroll
-                            for (int z = 0; z < LG::S; z++)
-                                if (at == z) v = key_at<V>(w[h], z);
+                            for (int z = 0; z < (int)BPU * LG::S; z++)
+                                if (at == z) v = key_at<V>(w[h][z / LG::S], z % LG::S);
                         } else if (at >= 0) {
-                            v = __ldg(reinterpret_cast<const V *>(leaves + (uint64_t)blk[h] * LG::BS + kSectorBytes) + at);
+                            v = __ldg(reinterpret_cast<const V *>(leaves + (uint64_t)u2[h] * LG::BS + kSectorBytes) + at);
                         }
                         out[slot] = v;
                         if (found) found[slot] = at >= 0 ? 1 : 0;
@@ -1238,21 +1252,18 @@ learned_bucket_kernel(const __grid_constant__ DevTree t, const __grid_constant__
                 if (!__any_sync(0xffffffffu, pend)) break;
                 const uint32_t last = __shfl_sync(0xffffffffu, ub, k);
                 if (pend) {
-                    blk[h]++;
-                    if (blk[h] % BPU == 0) {  // a unit further
-                        const bool lost = blk[h] / BPU > last || ++walked > kMaxWalk;
-                        if (!PAIR || !(lane & 1)) {
-                            if (lost) {
-                                tree_point<K, V>(t, qk[h], out + slot, found ? found + slot : nullptr);
-                                n_fallback++;
-                            } else {
-                                n_extra++;
-                            }
+                    u2[h]++;
+                    const bool lost = u2[h] > last || walked >= kMaxWalk;
+                    if (!PAIR || !(lane & 1)) {
+                        if (lost) {
+                            tree_point<K, V>(t, qk[h], out + slot, found ? found + slot : nullptr);
+                            n_fallback++;
+                        } else {
+                            n_extra++;
                         }
-                        pend = !lost;
                     }
-                    if (pend)
-                        load_sector(leaves + (uint64_t)blk[h] * LG::BS + (PAIR ? (lane & 1) * kSectorBytes : 0), w[h]);
+                    pend = !lost;
+                    if (pend) load(h);
                 }
                 if (!__any_sync(0xffffffffu, pend)) break;
             }
