@@ -24,6 +24,22 @@ SEARCH_CONFIGS = ((8, 1), (8, 2), (4, 1), (4, 2), (2, 1))
 LEARNED_SHAPES = ((2, 1), (2, 2), (2, 3), (2, 4))
 
 
+# A tree's own shape (point, range) per key width, the measured best of the
+# direct kernels.  Large batches go through kernels with one shape: their times
+# differ by noise only, and a shape picked from noise would slow the tree's
+# smaller batches (up to 2x).
+DEFAULT_CONFIGS = {4: ((4, 1), (2, 1)), 8: ((8, 2), (4, 2))}
+TIE = 0.02
+
+
+def _pick(ms, default):
+    """The fastest configuration's name; `default` if it is within TIE of it."""
+    best = min(ms, key=ms.get)
+    if default in ms and ms[default] <= ms[best] * (1 + TIE):
+        return default
+    return best
+
+
 def _key(tree, mode, nq):
     cls = max(0, int(nq).bit_length() - 1)
     return f"n{tree.info.num_keys}_k{tree.key_bytes}_v{tree.value_bytes}_{mode}_q2^{cls}"
@@ -84,8 +100,8 @@ def tune(tree, queries, mode="basic", hi=None, repeats=5, cache_path=None, confi
     for g, i in configs:
         set_cfg(g, i)
         ms[f"{g}x{i}"] = _time(fn, stream, repeats)
-    best = min(ms, key=ms.get)
-    g, i = (int(x) for x in best.split("x"))
+    default = (2, 1) if mode == "learned" else DEFAULT_CONFIGS[tree.key_bytes][mode == "range"]
+    g, i = (int(x) for x in _pick(ms, "%dx%d" % default).split("x"))
     set_cfg(g, i)
     if cache_path:
         data = {}

@@ -629,10 +629,14 @@ bt_status point_launch(const bt_tree *t, const void *d_q, const uint32_t *d_perm
     return point_launch_t<K, V, G, R, PERM, false>(t, d_q, d_perm, nq, d_out, d_found, s);
 }
 
-template <typename K, typename V, int G, int R>
+// One shape per key width, whatever the tree's is set to: that is chosen on
+// point_kernel, whose best differs (2^24 grouped queries, us: u32 2^26 keys (4,1)
+// 560 (4,2) 591 (8,2) 753 (2,1) 847 (8,1) 1080; u64 2^28 keys (4,2) 1317 (4,1)
+// 1335 (2,1) 1389 (8,2) 1501 (8,1) 1834; the same order at 2^22 queries).
+template <typename K, typename V>
 bt_status window_launch(const bt_tree *t, const void *d_q, const uint32_t *d_perm, uint64_t nq,
                         void *d_out, uint8_t *d_found, cudaStream_t s) {
-    auto fn = point_window_kernel<K, V, G, R>;
+    auto fn = point_window_kernel<K, V, 4, sizeof(K) == 4 ? 1 : 2>;
     bt_status st = set_smem(fn, kWinBytes);
     if (st != BT_OK) return st;
     const uint64_t ntiles = (nq + 31) / 32;
@@ -675,15 +679,7 @@ bt_status bucket_cfg(const bt_tree *t, const BucketPlan &bp, uint64_t max_items,
 template <typename K, typename V, bool PERM>
 bt_status point_cfg(const bt_tree *t, const void *d_q, const uint32_t *d_perm, uint64_t nq,
                     void *d_out, uint8_t *d_found, cudaStream_t s) {
-    if (PERM && nq >= kWinMinQueries) {
-        switch (shape_of(t, false)) {
-            case 0: return window_launch<K, V, 8, 1>(t, d_q, d_perm, nq, d_out, d_found, s);
-            case 1: return window_launch<K, V, 8, 2>(t, d_q, d_perm, nq, d_out, d_found, s);
-            case 2: return window_launch<K, V, 4, 1>(t, d_q, d_perm, nq, d_out, d_found, s);
-            case 3: return window_launch<K, V, 4, 2>(t, d_q, d_perm, nq, d_out, d_found, s);
-            default: return window_launch<K, V, 2, 1>(t, d_q, d_perm, nq, d_out, d_found, s);
-        }
-    }
+    if (PERM && nq >= kWinMinQueries) return window_launch<K, V>(t, d_q, d_perm, nq, d_out, d_found, s);
     switch (shape_of(t, false)) {
         case 0: return point_launch<K, V, 8, 1, PERM>(t, d_q, d_perm, nq, d_out, d_found, s);
         case 1: return point_launch<K, V, 8, 2, PERM>(t, d_q, d_perm, nq, d_out, d_found, s);
