@@ -496,7 +496,7 @@ def range_section(args, device, bt, flush, tree, keys):
         "autotune": {"lanes_per_query": r_lanes, "rounds": r_rounds, "ms": r_ms},
         "ids": {"ranges_per_s": nr / (ms_ids / 1e3), "ms": ms_ids, "hits": hits,
                 "api": "Tree.range_search (counts, scan, offsets, ID fill)"},
-        "roofline": {"bound": "hbm", "kernel": "bounds_line_kernel (basic counts)",
+        "roofline": {"bound": "hbm", "kernel": "bucket order and search of both bounds (basic counts)",
                      "achieved": alg / (base_ms / 1e3) / 1e9, "peak": peak, "unit": "GB/s",
                      "frac": alg / (base_ms / 1e3) / 1e9 / peak},
     }
@@ -898,7 +898,7 @@ def run_ours(args):
     leaf_bytes = -(-len(keys) // 4) * 64
     chain = {f"{l}_line": bt.measure_chain(max(rep["index_bytes"], 1 << 20), leaf_bytes, 1 << 24,
                                            128, l, 2) for l in (1, 2)}
-    tq = profiled_traffic("learned_kernel_lognormal_k28_q24")
+    tq = profiled_traffic("learned_buckets_lognormal_k28_q24")
 
     sections = {}
     if world == 1:
@@ -949,8 +949,8 @@ def run_ours(args):
                       "api": "bt_point_search(BT_POINT_BASIC)"},
             "plain_grouped": {"value": world * nq / (grouped_ms / 1e3), "unit": "queries/s",
                               "ms_per_step": grouped_ms, "equals_plain": grouped_same,
-                              "api": "bt_point_search(BT_POINT_GROUPED): radix grouping + grouped "
-                                     "search, the grouping timed"},
+                              "api": "bt_point_search(BT_POINT_GROUPED): bucket order, search and "
+                                     "gather, the ordering timed"},
             "learned_over_plain": plain_ms / ms,
             "learned_over_plain_grouped": grouped_ms / ms,
             "learned_equals_plain": bool(np.array_equal(learned_res, plain_res)),
@@ -958,9 +958,9 @@ def run_ours(args):
                          "frac": achieved / peak, "peak_source": peak_kind,
                          "traffic": None if tq is None else tq * nq,
                          "traffic_source": "not measured in this run: ncu DRAM bytes per query "
-                                           "of learned_kernel from a 2^24-key capture "
+                                           "of the learned call's kernels from a 2^24-key capture "
                                            "(profiles/traffic.json, command there) x queries",
-                         "kernel": "learned_kernel",
+                         "kernel": "learned_bucket_kernel with the bucket order and gather",
                          "algorithmic_bytes_per_launch": alg_bytes,
                          "kernel_ms": statistics.mean(step_ms),
                          "chain_ceiling": {
