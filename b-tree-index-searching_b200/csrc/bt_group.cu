@@ -1,4 +1,4 @@
-// Query grouping, exclusive scan and range-ID fill.
+// Query grouping, device sort, bucket order, exclusive scan and range-ID fill.
 //
 // Grouping reorders a query batch so that queries that walk the same part of
 // the tree run next to each other (in the same CTAs, at the same time), which
@@ -9,9 +9,10 @@
 // radixGroupGPU :776; radixGroupSingleKernelGPU :1288), and one CTA per group.
 //
 // Here a group key of D bits is computed per query and the batch is sorted by
-// it with D/8 stable LSD counting passes (histogram -> scan -> scatter), all
+// it with D/8 stable LSD counting passes (count -> prefix -> scatter), all
 // on the device with no host round trip.  Each scatter carries the caller's
-// index, so results are written straight back in the caller's order.
+// index, so results are written straight back in the caller's order.  (Large
+// batches take the unstable one-pass bucket order below instead.)
 //   point : the top D bits of the key (relative to the tree's key width);
 //   2D    : (top D/2 bits of start, top D/2 bits of end), row-major -- a true
 //           2-D cell, where the reference buckets by the product of two

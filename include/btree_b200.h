@@ -59,6 +59,11 @@ typedef enum bt_point_mode {
     BT_POINT_LEARNED = 2  /* through the tree's learned index (bt_learned_train); no
                              counterpart in the reference */
 } bt_point_mode;
+/* Results do not depend on the mode.  Large batches (2^22 queries; 2^18 learned
+ * ones; 2^20 ranges) are ordered by key range inside the library whatever the
+ * mode, in scratch from its memory pool (about two key widths, a value width
+ * and 4 bytes per query; without room for it, and on a stream under capture,
+ * they are searched in their own order). */
 
 typedef enum bt_range_mode {
     BT_RANGE_BASIC = 0,      /* SearchingBTreeGPURange, BtreeRangeSearch.cu:786 */
@@ -154,7 +159,8 @@ BT_API bt_status bt_get_info(const bt_tree *tree, bt_info *info);
  * on the levels below shared memory (2, 4 or 8) and the number of rounds in
  * which a warp's 32 queries pass through those levels (1 or 2; each lane
  * group keeps lanes/rounds queries in flight).  Supported pairs: (8,1) (8,2)
- * (4,1) (4,2) (2,1).  Results do not depend on it; speed does.  The
+ * (4,1) (4,2) (2,1).  Results do not depend on it; the speed of point batches
+ * and ranges below the large-batch sizes (see bt_point_mode) does.  The
  * reference has no such knob (one thread per query, BPTreeExactSearch.cu:31);
  * the autotuner sets it.
  */
@@ -516,10 +522,8 @@ BT_API uint64_t bt_kernel_launches(void);
  * call allocated nothing. */
 BT_API uint64_t bt_workspace_allocations(void);
 
-/* Number of times a grouping or sorting pass on the current device gave up
- * waiting for the digit counts of an earlier tile (its look-back is bounded;
- * a correct launch never gives up, and a pass that did has wrong output).
- * Synchronous; all-ones if it cannot be read. */
+/* Number of times a grouping or sorting pass gave up waiting for another tile.
+ * No pass waits on another CTA: always 0. */
 BT_API uint64_t bt_partition_lookback_timeouts(void);
 
 #ifdef __cplusplus
