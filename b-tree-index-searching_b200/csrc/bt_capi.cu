@@ -54,8 +54,11 @@ bt_status pipe_streams(int dev, cudaStream_t (&out)[kPipeSlots]) {
 }
 
 bt_status point_device(const bt_tree *t, int mode, const void *d_q, uint64_t nq, void *d_out,
-                       cudaStream_t s, uint8_t *d_found = nullptr) {
-    if (mode == BT_POINT_LEARNED ? learned_buckets_pay(t, nq, s) : bucket_search_pays(t, nq, s)) {
+                       cudaStream_t s, uint8_t *d_found = nullptr, bool piped = false) {
+    // A learned chunk of the host pipeline goes direct: the copies bound it, and the
+    // bucket passes beside them cost more than the search gains (2^24 queries in 8
+    // chunks over 2^28 u64 keys: 4.86-4.96 G queries/s direct, 4.70 by buckets).
+    if (mode == BT_POINT_LEARNED ? !piped && learned_buckets_pay(t, nq, s) : bucket_search_pays(t, nq, s)) {
         const bt_status st = mode == BT_POINT_LEARNED
                                  ? launch_learned_buckets(t, d_q, nq, d_out, d_found, s)
                                  : launch_bucket_search(t, d_q, nq, d_out, s, d_found);
@@ -231,7 +234,7 @@ bt_status bt_point_search_host(const bt_tree *t, int mode, const void *h_queries
     return host_pipeline(t, (cudaStream_t)stream, nq, pipeline_chunk(nq), 1, ins, w, h_out,
                          (size_t)t->val_bytes,
                          [&](void *const *din, uint64_t m, void *dout, cudaStream_t s) {
-                             return point_device(t, mode, din[0], m, dout, s);
+                             return point_device(t, mode, din[0], m, dout, s, nullptr, true);
                          });
 }
 
