@@ -27,6 +27,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "bt_part_cut.h"
 #include "bt_search.cuh"
 #include "bt_sort.cuh"
 
@@ -84,10 +85,6 @@ __device__ __forceinline__ uint32_t group_key(K a, K b, const GroupKeyParams &p)
 // with three CTAs per SM: 0.47 ms; 256-thread CTAs: 0.51 and more.
 constexpr int kPT = 512;             // partition threads per CTA
 constexpr int kPWarps = kPT / 32;
-constexpr int kPartCtas = 2;         // CTAs per SM
-constexpr int kPartMaxChunks = 512;
-constexpr uint64_t kPartMinTile = 1024;  // items a CTA takes at least
-constexpr int kPartDirect = 64;      // tables of up to so many rows are summed by the scatter
 
 // Items per thread of a tile, as many as two CTAs per SM have registers (64 a
 // thread) and shared memory for: a tile's stretch of a digit gets longer.
@@ -150,13 +147,6 @@ __device__ __forceinline__ uint32_t pass_digit(K a, K b, const GroupKeyParams &g
     if (gp.kind == kPartRadix) return (uint32_t)(a >> (8 * p)) & 0xFFu;
     return (group_key<K>(a, b, gp) >> (8 * p)) & 0xFFu;
 }
-
-// How a batch is cut: tiles of `tile` items, `per` consecutive tiles to a
-// chunk.
-struct PartCut {
-    uint64_t n;
-    uint32_t tile, per, ntiles, nchunks;
-};
 
 // Row c of chunk_tab: the digits of chunk c.  Row t of tile_tab (when a chunk
 // has several tiles): those of the chunk's tiles before tile t.  Counters per
@@ -347,13 +337,13 @@ part_scatter_kernel(const __grid_constant__ IO io_in, const __grid_constant__ Pa
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint32_t rows = cut.nchunks;
 
-    // where the batch's items of digit `threadIdx.x` start (for a small table
+    // where the batch's items of digit `threadIdx.x` start (for a direct cut
     // also where this CTA's one tile puts its own)
     uint32_t first = 0;
     {
         uint32_t tot = 0, pre = 0;
         if (threadIdx.x < 256) {
-            if (rows > kPartDirect) {
+            if (!cut.direct) {
                 tot = chunk_tab[rows * 256u + threadIdx.x];
             } else {
 #pragma unroll 8
@@ -418,7 +408,7 @@ part_scatter_kernel(const __grid_constant__ IO io_in, const __grid_constant__ Pa
         }
         uint32_t run = first;  // where the tile's first item of digit `threadIdx.x` goes
         if (threadIdx.x < 256) {
-            if (rows > kPartDirect) run += chunk_tab[(t / cut.per) * 256u + threadIdx.x];
+            if (!cut.direct) run += chunk_tab[(t / cut.per) * 256u + threadIdx.x];
             if (tile_tab) run += tile_tab[t * 256u + threadIdx.x];
         }
         __syncthreads();
@@ -968,27 +958,18 @@ bt_status part_pass(const IO &io, uint64_t n, GroupKeyParams gp, int pass, uint3
                     cudaStream_t s) {
     bt_status st = scatter_smem_attr<K, P, HAS_B, SORT, IO>();
     if (st != BT_OK) return st;
-    // two CTAs per SM; a batch that does not fill them with whole tiles gets
-    // smaller ones, in whole rows of a warp
-    const uint64_t ctas = std::min<uint64_t>(kPartMaxChunks, (uint64_t)kPartCtas * (uint64_t)sm_count());
-    constexpr uint64_t T = PartSmem<K, P, HAS_B>::T;
-    PartCut cut;
-    cut.n = n;
-    cut.tile = (uint32_t)std::min<uint64_t>(
-        T, std::max<uint64_t>(kPartMinTile, ((n + ctas - 1) / ctas + 31) / 32 * 32));
-    cut.ntiles = (uint32_t)((n + cut.tile - 1) / cut.tile);
-    cut.per = (uint32_t)((cut.ntiles + ctas - 1) / ctas);
-    cut.nchunks = (cut.ntiles + cut.per - 1) / cut.per;
+    const uint64_t sms = (uint64_t)sm_count();
+    const PartCut cut = part_cut(n, PartSmem<K, P, HAS_B>::T, sms);
     uint32_t *tile_tab = cut.per > 1 ? table + (kPartMaxChunks + 1) * 256 : nullptr;
     count_launch();
     part_count_kernel<K, P, HAS_B, SORT, IO><<<cut.nchunks, kPT, 0, s>>>(io, cut, gp, pass, table, tile_tab);
-    if (cut.nchunks > kPartDirect) {
+    if (!cut.direct) {
         count_launch();
         part_prefix_kernel<<<32, 256, 0, s>>>(table, (int)cut.nchunks);
     }
     count_launch();
     part_scatter_kernel<K, P, HAS_B, SORT, IO>
-        <<<(unsigned)std::min<uint64_t>(cut.ntiles, ctas), kPT, PartSmem<K, P, HAS_B>::bytes, s>>>(
+        <<<(unsigned)std::min<uint64_t>(cut.ntiles, kPartCtas * sms), kPT, PartSmem<K, P, HAS_B>::bytes, s>>>(
             io, cut, gp, pass, table, tile_tab);
     BT_CUDA(cudaGetLastError());
     return BT_OK;
