@@ -556,8 +556,9 @@ bucket_count_kernel(const __grid_constant__ B q, uint64_t n, const __grid_consta
 // Block 0: start = cursor = exclusive scan of total (start[nb] = n), and the
 // search's work items: every bucket's queries in equal slices of at most
 // kBucketSlice (item = bucket, first query, queries).  The others: first[b] =
-// leaf block of the first key at or above bucket b's first key (b = nb: the
-// last block), so bucket b's keys lie in blocks first[b] .. first[b + 1].
+// leaf block of the first key at or above bucket b's first key (b = nb: of the
+// first key equal to the largest), so the first key at or above a query of
+// bucket b lies in blocks first[b] .. first[b + 1], at most bucket_blocks ones.
 template <typename K>
 __global__ void __launch_bounds__(1024)
 bucket_start_kernel(const __grid_constant__ DevTree t, const __grid_constant__ BucketMap map,
@@ -567,13 +568,13 @@ bucket_start_kernel(const __grid_constant__ DevTree t, const __grid_constant__ B
     const uint32_t nb = map.last + 1;
     if (blockIdx.x > 0) {  // eight lanes per bucket
         const uint32_t i = ((blockIdx.x - 1) * blockDim.x + threadIdx.x) >> 3;
-        const uint64_t k = map.first_key(i < nb ? i : 0u);
+        const uint64_t k = i < nb ? map.first_key(i) : t.max_key;
         const K qe[1] = {k < t.max_key ? (K)k : (K)t.max_key};
         const bool up[1] = {false};
         uint32_t node[1] = {0};
         const int lane = threadIdx.x & 31;
         walk_from<K, 8, 1>(t, 0, qe, up, node, lane >> 3, lane & 7);
-        if ((lane & 7) == 0 && i <= nb) first[i] = i == nb ? (uint32_t)(t.n_sectors - 1) : node[0];
+        if ((lane & 7) == 0 && i <= nb) first[i] = node[0];
         return;
     }
     constexpr int PER = kMaxBuckets / 1024;  // buckets per thread

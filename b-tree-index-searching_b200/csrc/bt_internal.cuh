@@ -266,6 +266,9 @@ void free_learned(bt::LearnedState *s);
 // the counters of bt_learned_last_stats accumulate).
 bt_status launch_learned_search(const bt_tree *t, const void *d_q, uint64_t nq, void *d_out,
                                 uint8_t *d_found, cudaStream_t s);
+// Whether the bucket search's shared memory holds every bucket's part of the
+// tree's learned index.
+bool learned_index_fits(const bt_tree *t);
 // The same for a batch that learned_buckets_pay for, ordered by bucket
 // (BT_ERR_OUT_OF_MEMORY when the workspace cannot be had).
 bt_status launch_learned_buckets(const bt_tree *t, const void *d_q, uint64_t nq, void *d_out,
@@ -296,7 +299,7 @@ constexpr uint32_t kBucketSlice = 16384;
 // What the passes of the bucket order leave for the search.
 struct BucketPlan {
     uint32_t *scratch;  // 2 * kMaxBuckets words
-    uint32_t *first;    // leaf block where bucket b's keys start, b = 0 .. last + 1
+    uint32_t *first;    // leaf block where bucket b's keys start, b = 0 .. last; last + 1: of the largest key
     uint4 *items;       // work items: bucket, first slot, slots
     uint32_t *n_items;  // at most kMaxBuckets + nq / kBucketSlice
 };

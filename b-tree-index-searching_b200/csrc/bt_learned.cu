@@ -52,6 +52,7 @@ struct LearnedState {
     uint32_t *d_seg_first = nullptr;
     unsigned long long *d_stats = nullptr;
     uint64_t bytes = 0;
+    uint32_t bucket_segs = 0;  // most segments that the queries of one bucket can route to
     int shape = 1;  // search kernel shape (bt_learned_set_shape)
     LearnedDev dev;
 };
@@ -1105,8 +1106,8 @@ template <typename K, typename V, int T>
 __global__ void __launch_bounds__(T, 1024 / T)
 learned_bucket_kernel(const __grid_constant__ DevTree t, const __grid_constant__ LearnedDev m,
                       const uint32_t *__restrict__ first, const uint4 *__restrict__ items,
-                      const uint32_t *__restrict__ n_items, uint32_t smem_bytes,
-                      const K *__restrict__ q, V *__restrict__ out, uint8_t *__restrict__ found) {
+                      const uint32_t *__restrict__ n_items, const K *__restrict__ q,
+                      V *__restrict__ out, uint8_t *__restrict__ found) {
     using LG = LeafGeom<K, V>;
     constexpr uint32_t KPU = unit_keys<K, V>();
     constexpr uint32_t BPU = kUnitBytes / LG::BS;
@@ -1123,14 +1124,6 @@ learned_bucket_kernel(const __grid_constant__ DevTree t, const __grid_constant__
     uint32_t n_extra = 0, n_fallback = 0;
     // staged: the segments field by field, then the code lines a word apart
     // from a whole number of bank rows (both are read at random)
-    if (bucket_index_bytes(ns, nl) > smem_bytes) {  // too many segments: the tree's full descent
-        for (uint32_t i = threadIdx.x; i < it.z; i += T) {
-            tree_point<K, V>(t, iq[i], out + it.y + i, found ? found + it.y + i : nullptr);
-            n_fallback++;
-        }
-        if (n_fallback) atomicAdd(&m.stats[1], (unsigned long long)n_fallback);
-        return;
-    }
     uint64_t *s_key = reinterpret_cast<uint64_t *>(smem_b);
     uint32_t *s_rlo = reinterpret_cast<uint32_t *>(s_key + ns), *s_cnt = s_rlo + ns, *s_eps = s_cnt + ns;
     float *s_slope = reinterpret_cast<float *>(s_eps + ns), *s_icpt = s_slope + ns;
@@ -1227,7 +1220,8 @@ learned_bucket_kernel(const __grid_constant__ DevTree t, const __grid_constant__
             const uint32_t slot = it.y + i0 + k;
             bool pend = i0 + k < it.z;
             for (int walked = 0;; walked++) {
-                int at = qk[h] > key_at<K>(w[h][BPU - 1], LG::S - 1) && u2[h] + 1 < U ? -2 : -1;  // -2: above the unit
+                // -2: above the unit's keys (and not above the tree's)
+                int at = qk[h] > key_at<K>(w[h][BPU - 1], LG::S - 1) && qk[h] <= tmax && u2[h] + 1 < U ? -2 : -1;
 #pragma unroll
                 for (int z = (int)BPU - 1; z >= 0; z--) {
                     const int m0 = first_match<K, LG::S>(w[h][z], qk[h], tmax);
@@ -1301,19 +1295,24 @@ bt_status learned_bucket_launch(const bt_tree *t, const BucketWs &w, size_t smem
     BT_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBucketIndexMax));
     count_launch();
     fn<<<(unsigned)w.max_items, T, smem, s>>>(t->dev, t->learned->dev, w.bp.first, w.bp.items, w.bp.n_items,
-                                              (uint32_t)smem, (const K *)w.q, (V *)w.res, w.found);
+                                              (const K *)w.q, (V *)w.res, w.found);
     BT_CUDA(cudaGetLastError());
     return BT_OK;
 }
 
+// Shared memory of the fullest bucket's index: its segments as counted by the
+// training, and the code lines of bucket_blocks blocks -- their units, rounded
+// up, less one, and a part of a line at either end.
+size_t bucket_index_need(const bt_tree *t) {
+    const uint64_t bytes = t->bucket_blocks * (uint64_t)leaf_stride(t->key_bytes, t->val_bytes);
+    return bucket_index_bytes(t->learned->bucket_segs, bytes / kUnitBytes / kCodesPerLine + 3);
+}
+
 template <typename K, typename V>
 bt_status learned_buckets(const bt_tree *t, const BucketWs &w, cudaStream_t s) {
-    // the fullest bucket's code lines, and four times the segments of an average one
-    const uint64_t lines = t->bucket_blocks * (uint64_t)LeafGeom<K, V>::BS / kUnitBytes / kCodesPerLine + 3;
-    const uint64_t segs = 4 * (t->learned->dev.nseg / (bucket_map(t->min_key, t->max_key).last + 1) + 16);
-    const size_t need = bucket_index_bytes(segs, lines);
+    const size_t need = bucket_index_need(t);
     if (need <= kBucketIndexMax / 2) return learned_bucket_launch<K, V, 512>(t, w, need, s);  // two CTAs per SM
-    return learned_bucket_launch<K, V, 1024>(t, w, std::min(need, kBucketIndexMax), s);
+    return learned_bucket_launch<K, V, 1024>(t, w, need, s);
 }
 
 template <typename K, typename V, int T>
@@ -1772,13 +1771,14 @@ bt_status train_impl(bt_tree *t, const bt_learned_config &cfg, cudaStream_t s,
     root_err_kernel<<<grid_of(nls, 256, 4), 256, 0, s>>>(st->d_mlp, H, x, nls, err);
 
     // ---- where each bucket's segments start
-    {
-        const BucketMap map = bucket_map(t->min_key, t->max_key);
-        BT_CUDA(cudaMalloc((void **)&st->d_seg_first, (map.last + 2) * sizeof(uint32_t)));
-        count_launch();
-        seg_first_kernel<<<(map.last + 2 + 255) / 256, 256, 0, s>>>(st->d_seg, (uint32_t)nseg, map,
-                                                                    st->d_seg_first);
-    }
+    const BucketMap map = bucket_map(t->min_key, t->max_key);
+    std::vector<uint32_t> seg_first(map.last + 2);
+    BT_CUDA(cudaMalloc((void **)&st->d_seg_first, seg_first.size() * sizeof(uint32_t)));
+    count_launch();
+    seg_first_kernel<<<(map.last + 2 + 255) / 256, 256, 0, s>>>(st->d_seg, (uint32_t)nseg, map,
+                                                                st->d_seg_first);
+    BT_CUDA(cudaMemcpyAsync(seg_first.data(), st->d_seg_first, seg_first.size() * sizeof(uint32_t),
+                            cudaMemcpyDeviceToHost, s));
 
     // ---- unit thresholds
     const uint64_t ncl = units > 1 ? (units - 1 + kCodesPerLine - 1) / kCodesPerLine : 0;
@@ -1813,6 +1813,8 @@ bt_status train_impl(bt_tree *t, const bt_learned_config &cfg, cudaStream_t s,
     d.units = units;
     d.seg_first = st->d_seg_first;
     d.stage_bytes = (uint32_t)stage_bytes;
+    for (uint32_t b = 0; b <= map.last; b++)
+        st->bucket_segs = std::max(st->bucket_segs, seg_first[b + 1] - seg_first[b] + 1);
     st->bytes = (uint64_t)nls * sizeof(SegLine) + ncl * sizeof(CodeLine) + stage_bytes +
                 np * sizeof(float);
     (void)LG::S;
@@ -1860,6 +1862,8 @@ bt_status launch_learned_search(const bt_tree *t, const void *d_q, uint64_t nq, 
     return t->val_bytes == 4 ? learned_launch<uint64_t, uint32_t>(t, d_q, nq, d_out, d_found, s)
                              : learned_launch<uint64_t, uint64_t>(t, d_q, nq, d_out, d_found, s);
 }
+
+bool learned_index_fits(const bt_tree *t) { return bucket_index_need(t) <= kBucketIndexMax; }
 
 bt_status launch_learned_buckets(const bt_tree *t, const void *d_q, uint64_t nq, void *d_out,
                                  uint8_t *d_found, cudaStream_t s) {

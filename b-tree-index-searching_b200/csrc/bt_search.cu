@@ -792,9 +792,10 @@ bool bucket_search_pays(const bt_tree *t, uint64_t nq, cudaStream_t s) {
 //   2^20 keys       57 / 57      97 / 59     209 / 87
 //   2^24            57 / 59     100 / 62     213 / 112
 //   2^28            61 / 91     106 / 100    230 / 143    1211 / 848
-// (the staged index is a seventh of the separators: no rule on keys per query)
+// (the staged index is a seventh of the separators: no rule on keys per query).
+// Not where some bucket's part of the index exceeds the shared memory.
 bool learned_buckets_pay(const bt_tree *t, uint64_t nq, cudaStream_t s) {
-    return nq >= kLearnedMinQueries && buckets_suit(t, nq, ~0ull, s);
+    return nq >= kLearnedMinQueries && buckets_suit(t, nq, ~0ull, s) && learned_index_fits(t);
 }
 
 // Range bounds, direct / by buckets (us; the buckets take both bounds of a
