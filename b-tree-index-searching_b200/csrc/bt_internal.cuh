@@ -23,6 +23,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <string>
 
 #include "../../include/btree_b200.h"
@@ -316,6 +317,18 @@ bt_status launch_range_gather(const bt_tree *t, const uint32_t *rank, const uint
 bt_status launch_bucket_gather(int val_bytes, const void *res, const uint8_t *rfound,
                                const uint32_t *pos, uint64_t nq, void *d_out, uint8_t *d_found,
                                cudaStream_t s);
+// Queries that a bucket search orders at a time.  A larger batch goes in equal
+// parts of this many to twice this many, so that its scratch is bounded (20 bytes
+// a query for 8-byte keys and values).  Larger parts gain nothing, their scattered
+// passes having left the L2; smaller ones stage the tree's separators more often,
+// so a tree of over 2^26 leaf blocks takes half as many queries as it has blocks.
+// In one part / in parts of 2^25 (ms): 2^27 queries, 2^24 u32 keys 3.39 / 2.59;
+// in parts of 2^25 / 2^24: 2^25 bounds, 2^27 u64 keys 1.01 / 1.30.
+constexpr uint64_t kBucketBatch = 1ull << 25;
+inline uint64_t bucket_batch(const bt_tree *t, uint64_t nq) {
+    const uint64_t parts = std::max<uint64_t>(1, nq / std::max<uint64_t>(kBucketBatch, t->n_sectors / 2));
+    return (nq + parts - 1) / parts;
+}
 // Workspace of a bucket search: the ordered queries, every query's slot, the
 // results by slot (and their found flags), the plan.
 struct BucketWs {

@@ -1868,18 +1868,24 @@ bool learned_index_fits(const bt_tree *t) { return bucket_index_need(t) <= kBuck
 bt_status launch_learned_buckets(const bt_tree *t, const void *d_q, uint64_t nq, void *d_out,
                                  uint8_t *d_found, cudaStream_t s) {
     const BucketMap map = bucket_map(t->min_key, t->max_key);
+    const uint64_t per = bucket_batch(t, nq);
     BucketWs w(s);
-    bt_status st = w.alloc(nq, map.last + 1, t->key_bytes, t->val_bytes, d_found != nullptr);
-    if (st == BT_OK) st = launch_buckets(t, map, d_q, nullptr, nq, w.q, w.pos, w.bp, s);
-    if (st != BT_OK) return st;
-    if (t->key_bytes == 4)
-        st = t->val_bytes == 4 ? learned_buckets<uint32_t, uint32_t>(t, w, s)
-                               : learned_buckets<uint32_t, uint64_t>(t, w, s);
-    else
-        st = t->val_bytes == 4 ? learned_buckets<uint64_t, uint32_t>(t, w, s)
-                               : learned_buckets<uint64_t, uint64_t>(t, w, s);
-    if (st != BT_OK) return st;
-    return launch_bucket_gather(t->val_bytes, w.res, w.found, w.pos, nq, d_out, d_found, s);
+    bt_status st = w.alloc(per, map.last + 1, t->key_bytes, t->val_bytes, d_found != nullptr);
+    for (uint64_t i = 0; i < nq && st == BT_OK; i += per) {
+        const uint64_t m = std::min(per, nq - i);
+        st = launch_buckets(t, map, (const char *)d_q + i * t->key_bytes, nullptr, m, w.q, w.pos, w.bp, s);
+        if (st != BT_OK) break;
+        if (t->key_bytes == 4)
+            st = t->val_bytes == 4 ? learned_buckets<uint32_t, uint32_t>(t, w, s)
+                                   : learned_buckets<uint32_t, uint64_t>(t, w, s);
+        else
+            st = t->val_bytes == 4 ? learned_buckets<uint64_t, uint32_t>(t, w, s)
+                                   : learned_buckets<uint64_t, uint64_t>(t, w, s);
+        if (st == BT_OK)
+            st = launch_bucket_gather(t->val_bytes, w.res, w.found, w.pos, m, (char *)d_out + i * t->val_bytes,
+                                      d_found ? d_found + i : nullptr, s);
+    }
+    return st;
 }
 
 bt_status reset_learned_stats(const bt_tree *t, cudaStream_t s) {

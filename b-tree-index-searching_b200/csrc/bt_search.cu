@@ -826,24 +826,36 @@ bt_status bucket_types(const bt_tree *t, const BucketWs &w, cudaStream_t s) {
 bt_status launch_bucket_search(const bt_tree *t, const void *d_q, uint64_t nq, void *d_out,
                                cudaStream_t s, uint8_t *d_found) {
     const BucketMap map = bucket_map(t->min_key, t->max_key);
+    const uint64_t per = bucket_batch(t, nq);
     BucketWs w(s);
-    bt_status st = w.alloc(nq, map.last + 1, t->key_bytes, t->val_bytes, d_found != nullptr);
-    if (st == BT_OK) st = launch_buckets(t, map, d_q, nullptr, nq, w.q, w.pos, w.bp, s);
-    if (st == BT_OK) st = bucket_types<false>(t, w, s);
-    if (st != BT_OK) return st;
-    return launch_bucket_gather(t->val_bytes, w.res, w.found, w.pos, nq, d_out, d_found, s);
+    bt_status st = w.alloc(per, map.last + 1, t->key_bytes, t->val_bytes, d_found != nullptr);
+    for (uint64_t i = 0; i < nq && st == BT_OK; i += per) {
+        const uint64_t m = std::min(per, nq - i);
+        st = launch_buckets(t, map, (const char *)d_q + i * t->key_bytes, nullptr, m, w.q, w.pos, w.bp, s);
+        if (st == BT_OK) st = bucket_types<false>(t, w, s);
+        if (st == BT_OK)
+            st = launch_bucket_gather(t->val_bytes, w.res, w.found, w.pos, m, (char *)d_out + i * t->val_bytes,
+                                      d_found ? d_found + i : nullptr, s);
+    }
+    return st;
 }
 
 bt_status launch_bucket_bounds(const bt_tree *t, const void *d_lo, const void *d_hi, uint64_t nr,
                                uint64_t *d_counts, uint64_t *d_lb, cudaStream_t s) {
     const BucketMap map = bucket_map(t->min_key, t->max_key);
+    const uint64_t per = (bucket_batch(t, 2 * nr) + 1) / 2;
     BucketWs w(s);
-    bt_status st = w.alloc(2 * nr, map.last + 1, t->key_bytes, sizeof(uint32_t), false);
-    if (st == BT_OK) st = launch_buckets(t, map, d_lo, d_hi, nr, w.q, w.pos, w.bp, s);
-    if (st == BT_OK) st = bucket_types<true>(t, w, s);
-    if (st != BT_OK) return st;
-    return launch_range_gather(t, reinterpret_cast<const uint32_t *>(w.res), w.pos, d_lo, d_hi, nr,
-                               d_counts, d_lb, s);
+    bt_status st = w.alloc(2 * per, map.last + 1, t->key_bytes, sizeof(uint32_t), false);
+    for (uint64_t i = 0; i < nr && st == BT_OK; i += per) {
+        const uint64_t m = std::min(per, nr - i);
+        const char *lo = (const char *)d_lo + i * t->key_bytes, *hi = (const char *)d_hi + i * t->key_bytes;
+        st = launch_buckets(t, map, lo, hi, m, w.q, w.pos, w.bp, s);
+        if (st == BT_OK) st = bucket_types<true>(t, w, s);
+        if (st == BT_OK)
+            st = launch_range_gather(t, reinterpret_cast<const uint32_t *>(w.res), w.pos, lo, hi, m,
+                                     d_counts + i, d_lb ? d_lb + i : nullptr, s);
+    }
+    return st;
 }
 
 bt_status launch_bounds(const bt_tree *t, const void *d_lo, const void *d_hi,

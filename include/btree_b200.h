@@ -61,9 +61,11 @@ typedef enum bt_point_mode {
 } bt_point_mode;
 /* Results do not depend on the mode.  Large batches (2^22 queries; 2^18 learned
  * ones; 2^20 ranges) are ordered by key range inside the library whatever the
- * mode, in scratch from its memory pool (about two key widths, a value width
- * and 4 bytes per query; without room for it, and on a stream under capture,
- * they are searched in their own order). */
+ * mode, in scratch from its memory pool (a key width, a value width, 4 bytes and,
+ * with found flags, one more byte per query, for at most 2^26 queries, or as many
+ * as the tree has leaf blocks, at a time; two key widths and 16 bytes per range,
+ * for at most half as many ranges).  Without room for it, and on a stream under
+ * capture, they are searched in their own order. */
 
 typedef enum bt_range_mode {
     BT_RANGE_BASIC = 0,      /* SearchingBTreeGPURange, BtreeRangeSearch.cu:786 */
