@@ -6,6 +6,30 @@
 #include "bt_internal.cuh"
 
 namespace bt {
+
+bt_status point_device(const bt_tree *t, int mode, const void *d_q, uint64_t nq, void *d_out,
+                       cudaStream_t s, uint8_t *d_found, bool scratch) {
+    const bool learned = mode == BT_POINT_LEARNED;
+    if (scratch && (learned ? learned_buckets_pay(t, nq, s) : bucket_search_pays(t, nq, s))) {
+        const bt_status st = learned ? launch_learned_buckets(t, d_q, nq, d_out, d_found, s)
+                                     : launch_bucket_search(t, d_q, nq, d_out, s, d_found);
+        if (st != BT_ERR_OUT_OF_MEMORY) return st;
+        cudaGetLastError();  // no room for the ordered copy: the direct search
+    }
+    if (mode == BT_POINT_BASIC || t->n == 0 || (mode == BT_POINT_GROUPED && nq < kBktMinQueries))
+        return launch_point_search(t, d_q, nullptr, nq, d_out, s, d_found);
+    if (learned) return launch_learned_search(t, d_q, nq, d_out, d_found, s);
+    void *gq = nullptr;
+    uint32_t *perm = nullptr;
+    bt_status st = ws_alloc(&gq, nq * t->key_bytes, s);
+    if (st == BT_OK) st = ws_alloc((void **)&perm, nq * sizeof(uint32_t), s);
+    if (st == BT_OK) st = launch_partition(t, kPartPoint, d_q, nullptr, nq, gq, nullptr, perm, s);
+    if (st == BT_OK) st = launch_point_search(t, gq, perm, nq, d_out, s, d_found);
+    ws_free(gq, s);
+    ws_free(perm, s);
+    return st;
+}
+
 namespace {
 
 struct DeviceGuard {
@@ -51,32 +75,6 @@ bt_status pipe_streams(int dev, cudaStream_t (&out)[kPipeSlots]) {
     }
     for (int i = 0; i < kPipeSlots; i++) out[i] = p.s[i];
     return BT_OK;
-}
-
-bt_status point_device(const bt_tree *t, int mode, const void *d_q, uint64_t nq, void *d_out,
-                       cudaStream_t s, uint8_t *d_found = nullptr, bool piped = false) {
-    // A learned chunk of the host pipeline goes direct: the copies bound it, and the
-    // bucket passes beside them cost more than the search gains (2^24 queries in 8
-    // chunks over 2^28 u64 keys: 4.86-4.96 G queries/s direct, 4.70 by buckets).
-    if (mode == BT_POINT_LEARNED ? !piped && learned_buckets_pay(t, nq, s) : bucket_search_pays(t, nq, s)) {
-        const bt_status st = mode == BT_POINT_LEARNED
-                                 ? launch_learned_buckets(t, d_q, nq, d_out, d_found, s)
-                                 : launch_bucket_search(t, d_q, nq, d_out, s, d_found);
-        if (st != BT_ERR_OUT_OF_MEMORY) return st;
-        cudaGetLastError();  // no room for the ordered copy: the direct search
-    }
-    if (mode == BT_POINT_BASIC || t->n == 0 || (mode == BT_POINT_GROUPED && nq < kBktMinQueries))
-        return launch_point_search(t, d_q, nullptr, nq, d_out, s, d_found);
-    if (mode == BT_POINT_LEARNED) return launch_learned_search(t, d_q, nq, d_out, d_found, s);
-    void *gq = nullptr;
-    uint32_t *perm = nullptr;
-    bt_status st = ws_alloc(&gq, nq * t->key_bytes, s);
-    if (st == BT_OK) st = ws_alloc((void **)&perm, nq * sizeof(uint32_t), s);
-    if (st == BT_OK) st = launch_partition(t, kPartPoint, d_q, nullptr, nq, gq, nullptr, perm, s);
-    if (st == BT_OK) st = launch_point_search(t, gq, perm, nq, d_out, s, d_found);
-    ws_free(gq, s);
-    ws_free(perm, s);
-    return st;
 }
 
 bt_status count_device(const bt_tree *t, int mode, const void *d_lo, const void *d_hi, uint64_t nq,
@@ -190,7 +188,7 @@ bt_status bt_point_search(const bt_tree *t, int mode, const void *d_queries, uin
         st = reset_learned_stats(t, (cudaStream_t)stream);
         if (st != BT_OK) return st;
     }
-    return point_device(t, mode, d_queries, nq, d_out, (cudaStream_t)stream);
+    return point_device(t, mode, d_queries, nq, d_out, (cudaStream_t)stream, nullptr, true);
 }
 
 bt_status bt_point_search_found(const bt_tree *t, int mode, const void *d_queries, uint64_t nq,
@@ -210,7 +208,7 @@ bt_status bt_point_search_found(const bt_tree *t, int mode, const void *d_querie
         st = reset_learned_stats(t, (cudaStream_t)stream);
         if (st != BT_OK) return st;
     }
-    return point_device(t, mode, d_queries, nq, d_out, (cudaStream_t)stream, d_found);
+    return point_device(t, mode, d_queries, nq, d_out, (cudaStream_t)stream, d_found, true);
 }
 
 bt_status bt_point_search_host(const bt_tree *t, int mode, const void *h_queries, uint64_t nq,
@@ -234,7 +232,12 @@ bt_status bt_point_search_host(const bt_tree *t, int mode, const void *h_queries
     return host_pipeline(t, (cudaStream_t)stream, nq, pipeline_chunk(nq), 1, ins, w, h_out,
                          (size_t)t->val_bytes,
                          [&](void *const *din, uint64_t m, void *dout, cudaStream_t s) {
-                             return point_device(t, mode, din[0], m, dout, s, nullptr, true);
+                             // A learned chunk goes direct: the copies bound it, and the
+                             // bucket passes beside them cost more than the search gains
+                             // (2^24 queries in 8 chunks over 2^28 u64 keys: 4.86-4.96 G
+                             // queries/s direct, 4.70 by buckets).
+                             return point_device(t, mode, din[0], m, dout, s, nullptr,
+                                                 mode != BT_POINT_LEARNED);
                          });
 }
 

@@ -204,6 +204,11 @@ __host__ __device__ inline int bitlen64(uint64_t v) {
     return b;
 }
 
+// The point search behind bt_point_search (arguments checked, the tree's device
+// current, the learned counters reset).  `scratch`: whether it may order a large
+// batch by bucket.
+bt_status point_device(const bt_tree *t, int mode, const void *d_q, uint64_t nq, void *d_out,
+                       cudaStream_t s, uint8_t *d_found, bool scratch);
 // Host launchers implemented in the .cu files.
 bt_status launch_point_search(const bt_tree *t, const void *d_q, const uint32_t *d_perm,
                               uint64_t nq, void *d_out, cudaStream_t s,
@@ -325,8 +330,11 @@ bt_status launch_bucket_gather(int val_bytes, const void *res, const uint8_t *rf
 // In one part / in parts of 2^25 (ms): 2^27 queries, 2^24 u32 keys 3.39 / 2.59;
 // in parts of 2^25 / 2^24: 2^25 bounds, 2^27 u64 keys 1.01 / 1.30.
 constexpr uint64_t kBucketBatch = 1ull << 25;
+inline uint64_t bucket_least(const bt_tree *t) {
+    return std::max<uint64_t>(kBucketBatch, t->n_sectors / 2);
+}
 inline uint64_t bucket_batch(const bt_tree *t, uint64_t nq) {
-    const uint64_t parts = std::max<uint64_t>(1, nq / std::max<uint64_t>(kBucketBatch, t->n_sectors / 2));
+    const uint64_t parts = std::max<uint64_t>(1, nq / bucket_least(t));
     return (nq + parts - 1) / parts;
 }
 // Workspace of a bucket search: the ordered queries, every query's slot, the
@@ -339,13 +347,17 @@ struct BucketWs {
     uint64_t max_items = 0;
     BucketPlan bp;
     explicit BucketWs(cudaStream_t s) : ws(s) {}
+    static size_t up256(size_t x) { return (x + 255) / 256 * 256; }
+    static size_t bytes(uint64_t nq, uint32_t buckets, size_t key_bytes, size_t res_bytes, bool flags) {
+        return up256(nq * key_bytes) + up256(nq * sizeof(uint32_t)) + up256(nq * res_bytes) +
+               (flags ? up256(nq) : 0) + (buckets + nq / kBucketSlice) * sizeof(uint4) +
+               (3 * kMaxBuckets + 64) * sizeof(uint32_t);
+    }
     bt_status alloc(uint64_t nq, uint32_t buckets, size_t key_bytes, size_t res_bytes, bool flags) {
-        auto up256 = [](size_t x) { return (x + 255) / 256 * 256; };
         const size_t kb = up256(nq * key_bytes), pb = up256(nq * sizeof(uint32_t));
         const size_t rb = up256(nq * res_bytes), fb = flags ? up256(nq) : 0;
         max_items = buckets + nq / kBucketSlice;
-        const bt_status st = ws.alloc(kb + pb + rb + fb + max_items * sizeof(uint4) +
-                                      (3 * kMaxBuckets + 64) * sizeof(uint32_t));
+        const bt_status st = ws.alloc(bytes(nq, buckets, key_bytes, res_bytes, flags));
         if (st != BT_OK) return st;
         q = ws.as<unsigned char>();
         pos = reinterpret_cast<uint32_t *>(q + kb);

@@ -55,6 +55,7 @@ struct Slot {
 struct bt_server {
     const bt_tree *tree;
     int mode;
+    bool scratch;  // the budget holds the bucket order's scratch in every slot too
     uint64_t max_batch;
     std::vector<Slot> slots;
     std::mutex mu;
@@ -74,14 +75,14 @@ namespace {
 
 bt_status run_job(bt_server *s, Slot &sl, const void *dq, uint64_t m) {
     const bt_tree *t = s->tree;
-    switch (s->mode) {
-        case BT_SERVE_LEARNED:
-            return bt_point_search_learned(t, dq, m, sl.dout, sl.stream);
-        case BT_SERVE_GROUPED:
-            return bt_point_search(t, BT_POINT_GROUPED, dq, m, sl.dout, sl.stream);
-        default:
-            return bt_point_search(t, BT_POINT_BASIC, dq, m, sl.dout, sl.stream);
+    if (s->mode == BT_SERVE_LEARNED) {
+        const bt_status st = bt::reset_learned_stats(t, sl.stream);
+        if (st != BT_OK) return st;
     }
+    const int mode = s->mode == BT_SERVE_LEARNED   ? BT_POINT_LEARNED
+                     : s->mode == BT_SERVE_GROUPED ? BT_POINT_GROUPED
+                                                   : BT_POINT_BASIC;
+    return bt::point_device(t, mode, dq, m, sl.dout, sl.stream, nullptr, s->scratch);
 }
 
 void worker_loop(bt_server *s) {
@@ -174,6 +175,11 @@ bt_status bt_server_create(const bt_tree *t, const bt_server_config *cfg_in, bt_
     s->tree = t;
     s->mode = cfg.mode;
     s->max_batch = cfg.max_batch;
+    // Jobs large enough for the bucket order take its scratch only out of what
+    // the slots leave of the budget; else they are searched in their own order.
+    const uint64_t part = std::min<uint64_t>(cfg.max_batch, 2 * bucket_least(t));
+    s->scratch = (cfg.memory_budget_bytes - nslots * per_slot) / nslots >=
+                 BucketWs::bytes(part, kMaxBuckets, t->key_bytes, t->val_bytes, false);
     s->slots.resize(nslots);
     bt_status st = BT_OK;
     for (Slot &sl : s->slots) {

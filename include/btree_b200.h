@@ -474,7 +474,9 @@ typedef enum bt_serve_mode {
 
 typedef struct bt_server_config {
     uint32_t slots;               /* concurrent device jobs wanted (default 8) */
-    uint64_t memory_budget_bytes; /* device memory for job buffers (default 256 MiB) */
+    uint64_t memory_budget_bytes; /* device memory for job buffers (default 256 MiB), and for the
+                                     scratch of jobs above the large-batch sizes (see
+                                     bt_point_mode) where it holds every slot's */
     uint32_t max_batch;           /* queries per job; larger requests are split (default 65536) */
     int32_t mode;                 /* bt_serve_mode */
 } bt_server_config;
