@@ -320,7 +320,9 @@ struct ImageHeader {
 
 // Copies `bytes` between a device buffer and a file through a host bounce
 // buffer of at most 64 MiB.
-bt_status stream_file(FILE *f, void *dptr, uint64_t bytes, bool write) {
+// Uploads are ordered on `s` (a pageable one has left the buffer when the call
+// returns, but need not have reached the device).
+bt_status stream_file(FILE *f, void *dptr, uint64_t bytes, bool write, cudaStream_t s) {
     using namespace bt;
     const uint64_t chunk = std::min<uint64_t>(bytes, 64ull << 20);
     std::vector<unsigned char> buf(chunk ? chunk : 1);
@@ -331,7 +333,7 @@ bt_status stream_file(FILE *f, void *dptr, uint64_t bytes, bool write) {
             if (fwrite(buf.data(), 1, m, f) != m) return fail(BT_ERR_INVALID_ARGUMENT, "tree image: write failed");
         } else {
             if (fread(buf.data(), 1, m, f) != m) return fail(BT_ERR_INVALID_ARGUMENT, "tree image: file is truncated");
-            BT_CUDA(cudaMemcpy((unsigned char *)dptr + o, buf.data(), m, cudaMemcpyHostToDevice));
+            BT_CUDA(cudaMemcpyAsync((unsigned char *)dptr + o, buf.data(), m, cudaMemcpyHostToDevice, s));
         }
     }
     return BT_OK;
@@ -405,8 +407,8 @@ bt_status bt_save(const bt_tree *t, const char *path) {
     cudaSetDevice(t->device);
     bt_status st = fwrite(&h, sizeof(h), 1, f) == 1 ? BT_OK
                                                     : fail(BT_ERR_INVALID_ARGUMENT, "tree image: write failed");
-    if (st == BT_OK && h.leaf_bytes) st = stream_file(f, t->d_leaves, h.leaf_bytes, true);
-    if (st == BT_OK && h.sep_bytes) st = stream_file(f, t->d_seps, h.sep_bytes, true);
+    if (st == BT_OK && h.leaf_bytes) st = stream_file(f, t->d_leaves, h.leaf_bytes, true, nullptr);
+    if (st == BT_OK && h.sep_bytes) st = stream_file(f, t->d_seps, h.sep_bytes, true, nullptr);
     cudaSetDevice(prev);
     if (fclose(f) != 0 && st == BT_OK) st = fail(BT_ERR_INVALID_ARGUMENT, "tree image: close failed");
     return st;
@@ -452,8 +454,10 @@ bt_status bt_load(const char *path, void *stream, bt_tree **out) {
     if (h.leaf_bytes) e = cudaMalloc(&t->d_leaves, h.leaf_bytes);
     if (e == cudaSuccess && h.sep_bytes) e = cudaMalloc(&t->d_seps, h.sep_bytes);
     st = e == cudaSuccess ? BT_OK : cuda_fail(e, "tree image: device allocation");
-    if (st == BT_OK && h.leaf_bytes) st = stream_file(f, t->d_leaves, h.leaf_bytes, false);
-    if (st == BT_OK && h.sep_bytes) st = stream_file(f, t->d_seps, h.sep_bytes, false);
+    // on the stream of the measurement below, which reads them
+    const cudaStream_t s = (cudaStream_t)stream;
+    if (st == BT_OK && h.leaf_bytes) st = stream_file(f, t->d_leaves, h.leaf_bytes, false, s);
+    if (st == BT_OK && h.sep_bytes) st = stream_file(f, t->d_seps, h.sep_bytes, false, s);
     fclose(f);
     if (st != BT_OK) {
         free_tree(t);
@@ -470,7 +474,6 @@ bt_status bt_load(const char *path, void *stream, bt_tree **out) {
     dt.smem_entries = h.smem_entries;
     dt.smem_bytes = h.smem_bytes;
     if (t->n) {
-        cudaStream_t s = (cudaStream_t)stream;
         WsGuard g(s);
         st = g.alloc(sizeof(uint32_t));
         if (st == BT_OK) {
