@@ -25,6 +25,7 @@ LIB_PATH = os.path.join(PKG_DIR, "lib", "libbtree_b200.so")
 
 POINT_MODES = {"basic": 0, "grouped": 1, "learned": 2}
 RANGE_MODES = {"basic": 0, "2d": 1, "zorder": 2}
+SEARCH_OPS = {"point": 0, "range": 1}
 
 STATUS = {
     0: "BT_OK", 1: "BT_ERR_INVALID_ARGUMENT", 2: "BT_ERR_UNSORTED",
@@ -123,6 +124,8 @@ _PROTOS = {
     "bt_build_from_files": (_I, [ctypes.c_char_p, ctypes.c_char_p, _U64, _P, ctypes.POINTER(_P)]),
     "bt_load": (_I, [ctypes.c_char_p, _P, ctypes.POINTER(_P)]),
     "bt_set_search_config": (_I, [_P, _I, _I]),
+    "bt_set_op_config": (_I, [_P, _I, _I, _I]),
+    "bt_own_op_config": (_I, [_I, _I, _U64, ctypes.POINTER(_I), ctypes.POINTER(_I)]),
     "bt_point_search_grouped_noalloc": (_I, [_P, _P, _U64, _P, _P]),
     "bt_learned_train": (_I, [_P, ctypes.POINTER(bt_learned_config), _P,
                               ctypes.POINTER(bt_learned_report)]),
@@ -222,6 +225,15 @@ def _alloc_ids(buf, total):
     except BaseException as e:  # raised again by done(), outside the library
         buf.error = e
         return None
+
+
+def own_op_config(key_bytes, op, nq):
+    """(lanes, rounds) of a tree's own shape for nq "point" queries or "range"
+    counts (bt_own_op_config)."""
+    g, r = _I(), _I()
+    _check(lib().bt_own_op_config(key_bytes, SEARCH_OPS[op], nq, ctypes.byref(g), ctypes.byref(r)),
+           "bt_own_op_config")
+    return g.value, r.value
 
 
 class Tree:
@@ -328,6 +340,13 @@ class Tree:
         L = lib()
         _check(L.bt_set_search_config(self._h, lanes_per_query, rounds), "bt_set_search_config")
         _check(L.bt_get_info(self._h, ctypes.byref(self.info)), "bt_get_info")
+
+    def set_op_config(self, op, lanes_per_query=0, rounds=0):
+        """Shape of "point" searches or "range" counts alone; 0, 0: the tree's
+        own again (bt_set_op_config)."""
+        _check(lib().bt_set_op_config(self._h, SEARCH_OPS[op], lanes_per_query, rounds),
+               "bt_set_op_config")
+        _check(lib().bt_get_info(self._h, ctypes.byref(self.info)), "bt_get_info")
 
     SEARCH_CONFIGS = ((8, 1), (8, 2), (4, 1), (4, 2), (2, 1))
 

@@ -14,6 +14,7 @@ what is tuned is how many lanes share a query below the shared-memory level
 and in how many rounds a warp's 32 queries pass through those levels (that
 is, how many queries each lane group keeps in flight).
 """
+import importlib
 import json
 import os
 import statistics
@@ -24,12 +25,17 @@ SEARCH_CONFIGS = ((8, 1), (8, 2), (4, 1), (4, 2), (2, 1))
 LEARNED_SHAPES = ((2, 1), (2, 2), (2, 3), (2, 4))
 
 
-# A tree's own shape (point, range) per key width, the measured best of the
-# direct kernels.  Large batches go through kernels with one shape: their times
-# differ by noise only, and a shape picked from noise would slow the tree's
-# smaller batches (up to 2x).
-DEFAULT_CONFIGS = {4: ((4, 1), (2, 1)), 8: ((8, 2), (4, 2))}
+# Large batches go through kernels with one shape: their times differ by noise
+# only, and a shape picked from noise would slow the tree's smaller batches (up
+# to 2x).  Within TIE of the best the tree keeps its own shape.
 TIE = 0.02
+
+
+def __getattr__(name):
+    if name == "DEFAULT_CONFIGS":  # a tree's own shapes (point, range) per key width
+        own = importlib.import_module(__package__).own_op_config
+        return {kb: tuple(own(kb, op, 1 << 19) for op in ("point", "range")) for kb in (4, 8)}
+    raise AttributeError(name)
 
 
 def _pick(ms, default):
@@ -62,7 +68,8 @@ def _time(fn, stream, repeats):
 
 
 def tune(tree, queries, mode="basic", hi=None, repeats=5, cache_path=None, configs=SEARCH_CONFIGS):
-    """Pick and set the fastest search configuration for `tree` on this batch.
+    """Pick and set the fastest search configuration of `tree` for point searches
+    or for range counts, whichever this batch is.
 
     mode: "basic" / "grouped" / "learned" (point search; `queries` a CUDA
     tensor), or "range" (`queries` = lo, `hi` = hi).  Returns (lanes, slots,
@@ -70,15 +77,24 @@ def tune(tree, queries, mode="basic", hi=None, repeats=5, cache_path=None, confi
     (LEARNED_SHAPES).
     """
     import torch
-    set_cfg = tree.set_search_config
+    op = "range" if mode == "range" else "point"
     if mode == "learned":
+        default = (2, 1)
         set_cfg = lambda g, i: tree.learned_set_shape(i)  # noqa: E731
+    else:
+        default = importlib.import_module(__package__).own_op_config(tree.key_bytes, op,
+                                                                     len(queries))
+        set_cfg = lambda g, i: tree.set_op_config(op, g, i)  # noqa: E731
+
+    def choose(g, i):  # the tree's own shape is left to the tree
+        set_cfg(*((0, 0) if mode != "learned" and (g, i) == default else (g, i)))
+
     key = _key(tree, mode, len(queries))
     if cache_path and os.path.exists(cache_path):
         with open(cache_path) as f:
             cached = json.load(f).get(key)
         if cached:
-            set_cfg(*cached["best"])
+            choose(*cached["best"])
             return cached["best"][0], cached["best"][1], cached["ms"]
     stream = torch.cuda.current_stream(queries.device)
     out = None
@@ -100,9 +116,8 @@ def tune(tree, queries, mode="basic", hi=None, repeats=5, cache_path=None, confi
     for g, i in configs:
         set_cfg(g, i)
         ms[f"{g}x{i}"] = _time(fn, stream, repeats)
-    default = (2, 1) if mode == "learned" else DEFAULT_CONFIGS[tree.key_bytes][mode == "range"]
     g, i = (int(x) for x in _pick(ms, "%dx%d" % default).split("x"))
-    set_cfg(g, i)
+    choose(g, i)
     if cache_path:
         data = {}
         if os.path.exists(cache_path):

@@ -218,7 +218,7 @@ bt_status bt_build(const void *d_sorted_keys, const void *d_values, uint64_t n, 
     t->val_bytes = value_bytes;
     t->n = n;
     t->values_sorted = 1;
-    t->search_cfg = default_search_cfg();
+    t->search_cfg[BT_OP_POINT] = t->search_cfg[BT_OP_RANGE] = -1;
     if (n > 0) {
         cudaStream_t s = (cudaStream_t)stream;
         st = key_bytes == 4 ? build_k<uint32_t>(t, d_sorted_keys, d_values, s)
@@ -444,7 +444,7 @@ bt_status bt_load(const char *path, void *stream, bt_tree **out) {
     t->seps_elems = h.seps_elems;
     t->min_key = h.min_key;
     t->max_key = h.max_key;
-    t->search_cfg = default_search_cfg();
+    t->search_cfg[BT_OP_POINT] = t->search_cfg[BT_OP_RANGE] = -1;
     for (int l = 0; l < kMaxLevels; l++) {
         t->lvl_nodes[l] = h.lvl_nodes[l];
         t->lvl_entries[l] = h.lvl_entries[l];
@@ -505,8 +505,29 @@ bt_status bt_set_search_config(bt_tree *t, int lanes_per_query, int rounds) {
     if (!t) return fail(BT_ERR_INVALID_ARGUMENT, "tree is NULL");
     const int k = search_cfg_index(lanes_per_query, rounds);
     if (k < 0) return fail(BT_ERR_INVALID_ARGUMENT, "unsupported (lanes, rounds) search configuration");
-    t->search_cfg = k;
-    t->search_cfg_set = 1;
+    t->search_cfg[BT_OP_POINT] = t->search_cfg[BT_OP_RANGE] = k;
+    return BT_OK;
+}
+
+bt_status bt_set_op_config(bt_tree *t, int op, int lanes_per_query, int rounds) {
+    using namespace bt;
+    if (!t) return fail(BT_ERR_INVALID_ARGUMENT, "tree is NULL");
+    if (op != BT_OP_POINT && op != BT_OP_RANGE) return fail(BT_ERR_INVALID_ARGUMENT, "unknown search operation");
+    const bool own = lanes_per_query == 0 && rounds == 0;
+    const int k = own ? -1 : search_cfg_index(lanes_per_query, rounds);
+    if (k < 0 && !own) return fail(BT_ERR_INVALID_ARGUMENT, "unsupported (lanes, rounds) search configuration");
+    t->search_cfg[op] = k;
+    return BT_OK;
+}
+
+bt_status bt_own_op_config(int key_bytes, int op, uint64_t nq, int *lanes_per_query, int *rounds) {
+    using namespace bt;
+    if ((key_bytes != 4 && key_bytes != 8) || (op != BT_OP_POINT && op != BT_OP_RANGE) ||
+        !lanes_per_query || !rounds)
+        return fail(BT_ERR_INVALID_ARGUMENT, "key width, operation or output is invalid");
+    const int k = own_search_cfg(key_bytes, op, nq);
+    *lanes_per_query = search_cfg_lanes(k);
+    *rounds = search_cfg_rounds(k);
     return BT_OK;
 }
 
@@ -527,8 +548,10 @@ bt_status bt_get_info(const bt_tree *t, bt_info *info) {
     info->max_key = t->max_key;
     info->device = t->device;
     info->values_sorted = t->values_sorted;
-    info->lanes_per_query = (uint32_t)search_cfg_lanes(t->search_cfg);
-    info->rounds = (uint32_t)search_cfg_rounds(t->search_cfg);
+    const int cfg = t->search_cfg[BT_OP_POINT] >= 0 ? t->search_cfg[BT_OP_POINT]
+                                                    : own_search_cfg(t->key_bytes, BT_OP_POINT, 1ull << 19);
+    info->lanes_per_query = (uint32_t)search_cfg_lanes(cfg);
+    info->rounds = (uint32_t)search_cfg_rounds(cfg);
     return BT_OK;
 }
 

@@ -143,8 +143,7 @@ struct bt_tree {
     uint64_t min_key, max_key;
     int values_sorted;
     uint32_t bucket_blocks;  // leaf blocks of the fullest bucket (0: not measured)
-    int search_cfg;  // index into the search kernels' (lanes, rounds) table
-    int search_cfg_set;  // set by bt_set_search_config (else each kernel takes its own)
+    int search_cfg[2];  // per bt_search_op: index into the (lanes, rounds) table, -1: own_search_cfg
     bt::DevTree dev;
     bt::LearnedState *learned;  // trained learned index, or null
 };
@@ -249,7 +248,9 @@ bt_status launch_segment_sort(const bt_tree *t, const uint64_t *d_counts, const 
 // (lanes per query, rounds) -> index of the search configuration table in
 // bt_search.cu, or -1.
 int search_cfg_index(int lanes, int rounds);
-int default_search_cfg();
+// The shape in which nq queries or ranges are searched on a tree whose own is
+// not set.
+int own_search_cfg(int key_bytes, int op, uint64_t nq);
 int search_cfg_lanes(int cfg);
 int search_cfg_rounds(int cfg);
 

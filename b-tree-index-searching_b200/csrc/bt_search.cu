@@ -44,19 +44,21 @@ int search_cfg_index(int g, int r) {
 int search_cfg_lanes(int cfg) { return kSearchCfgs[cfg].g; }
 int search_cfg_rounds(int cfg) { return kSearchCfgs[cfg].r; }
 
-int default_search_cfg() { return search_cfg_index(4, 1); }
-
-// The shape of a tree nobody has set one for (us; 2^19 queries or ranges):
+// The shapes of a tree nobody has set one for (us; 2^19 queries or ranges):
 //                          (2,1)  (4,1)  (4,2)  (8,1)  (8,2)
 //   point u32, 2^20 keys                 (4,1) fastest throughout
 //   point u64, 2^20 keys    46.0   31.3   30.8   27.3   25.2
 //   point u64, 2^28         82.7   52.1   54.0   46.5   47.7
 //   range u32, 2^20 / 2^26  32/46  48/64  36/49  98/139 63/85
 //   range u64, 2^20 / 2^26  74/105 73/104 59/82  144/189 93/124
-static int shape_of(const bt_tree *t, bool range) {
-    if (t->search_cfg_set) return t->search_cfg;
-    if (range) return t->key_bytes == 4 ? search_cfg_index(2, 1) : search_cfg_index(4, 2);
-    return t->key_bytes == 4 ? search_cfg_index(4, 1) : search_cfg_index(8, 2);
+int own_search_cfg(int key_bytes, int op, uint64_t nq) {
+    (void)nq;
+    if (op == BT_OP_RANGE) return key_bytes == 4 ? search_cfg_index(2, 1) : search_cfg_index(4, 2);
+    return key_bytes == 4 ? search_cfg_index(4, 1) : search_cfg_index(8, 2);
+}
+
+static int shape_of(const bt_tree *t, int op, uint64_t nq) {
+    return t->search_cfg[op] >= 0 ? t->search_cfg[op] : own_search_cfg(t->key_bytes, op, nq);
 }
 
 namespace {
@@ -680,7 +682,7 @@ template <typename K, typename V, bool PERM>
 bt_status point_cfg(const bt_tree *t, const void *d_q, const uint32_t *d_perm, uint64_t nq,
                     void *d_out, uint8_t *d_found, cudaStream_t s) {
     if (PERM && nq >= kWinMinQueries) return window_launch<K, V>(t, d_q, d_perm, nq, d_out, d_found, s);
-    switch (shape_of(t, false)) {
+    switch (shape_of(t, BT_OP_POINT, nq)) {
         case 0: return point_launch<K, V, 8, 1, PERM>(t, d_q, d_perm, nq, d_out, d_found, s);
         case 1: return point_launch<K, V, 8, 2, PERM>(t, d_q, d_perm, nq, d_out, d_found, s);
         case 2: return point_launch<K, V, 4, 1, PERM>(t, d_q, d_perm, nq, d_out, d_found, s);
@@ -708,7 +710,7 @@ bt_status bounds_launch(const bt_tree *t, const void *d_lo, const void *d_hi,
 template <typename K, typename V, bool PERM>
 bt_status bounds_cfg(const bt_tree *t, const void *d_lo, const void *d_hi, const uint32_t *d_perm,
                      uint64_t nq, uint64_t *d_counts, uint64_t *d_lb, cudaStream_t s) {
-    switch (shape_of(t, true)) {
+    switch (shape_of(t, BT_OP_RANGE, nq)) {
         case 0: return bounds_launch<K, V, 8, 1, PERM>(t, d_lo, d_hi, d_perm, nq, d_counts, d_lb, s);
         case 1: return bounds_launch<K, V, 8, 2, PERM>(t, d_lo, d_hi, d_perm, nq, d_counts, d_lb, s);
         case 2: return bounds_launch<K, V, 4, 1, PERM>(t, d_lo, d_hi, d_perm, nq, d_counts, d_lb, s);

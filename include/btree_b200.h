@@ -88,7 +88,8 @@ typedef struct bt_info {
     uint64_t max_key;
     int32_t device;
     int32_t values_sorted;      /* values ascend with keys (range IDs need no sort) */
-    uint32_t lanes_per_query;   /* search kernel configuration (see bt_set_search_config) */
+    uint32_t lanes_per_query;   /* shape of point searches (see bt_set_search_config; the tree's
+                                   own is that of 2^19 queries) */
     uint32_t rounds;
 } bt_info;
 
@@ -167,6 +168,17 @@ BT_API bt_status bt_get_info(const bt_tree *tree, bt_info *info);
  * the autotuner sets it.
  */
 BT_API bt_status bt_set_search_config(bt_tree *tree, int lanes_per_query, int rounds);
+
+/*
+ * The same for point searches or for range counts alone; lanes_per_query = 0
+ * and rounds = 0 give the operation the tree's own shape again, which is what
+ * it has until one is set.  bt_own_op_config tells that shape for nq queries
+ * or ranges.
+ */
+typedef enum bt_search_op { BT_OP_POINT = 0, BT_OP_RANGE = 1 } bt_search_op;
+BT_API bt_status bt_set_op_config(bt_tree *tree, int op, int lanes_per_query, int rounds);
+BT_API bt_status bt_own_op_config(int key_bytes, int op, uint64_t nq, int *lanes_per_query,
+                                  int *rounds);
 
 /*
  * Point search: d_out[i] = value of key d_queries[i], or all-ones on a miss.
