@@ -51,10 +51,13 @@ int search_cfg_rounds(int cfg) { return kSearchCfgs[cfg].r; }
 //   point u64, 2^28         82.7   52.1   54.0   46.5   47.7
 //   range u32, 2^20 / 2^26  32/46  48/64  36/49  98/139 63/85
 //   range u64, 2^20 / 2^26  74/105 73/104 59/82  144/189 93/124
+// A batch of a few warps waits for one chain of reads, which two rounds make
+// longer: u64 keys, 2^26, 64 queries: (4,1) 19.1 (8,2) 21.1; 64 ranges: (2,1) 24.2
+// (4,2) 28.7, 2^16 ranges 30.9 / 34.5, 2^17 42.8 / 40.8.
 int own_search_cfg(int key_bytes, int op, uint64_t nq) {
-    (void)nq;
-    if (op == BT_OP_RANGE) return key_bytes == 4 ? search_cfg_index(2, 1) : search_cfg_index(4, 2);
-    return key_bytes == 4 ? search_cfg_index(4, 1) : search_cfg_index(8, 2);
+    if (op == BT_OP_RANGE)
+        return key_bytes == 4 || nq < (1ull << 17) ? search_cfg_index(2, 1) : search_cfg_index(4, 2);
+    return key_bytes == 4 || nq < 512 ? search_cfg_index(4, 1) : search_cfg_index(8, 2);
 }
 
 static int shape_of(const bt_tree *t, int op, uint64_t nq) {
