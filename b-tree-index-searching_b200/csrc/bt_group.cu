@@ -1074,36 +1074,76 @@ bt_status partition_point_prealloc(const bt_tree *t, const K *d_q, uint64_t nq, 
 // (read from the leaf blocks, S values per block).  SORT: up to kWarpSortCap
 // values are put in ascending order on the way (in registers; a fill and a
 // sort of its own read and wrote every ID once more: 2^20 ranges, 34 M IDs,
-// 0.169 + 0.220 ms, fused 0.263).  A warp takes 32 consecutive queries at a
-// time, so that their counts, bounds and offsets arrive in three loads.
+// 0.169 + 0.220 ms, fused 0.263).  A warp takes `per` consecutive queries at a
+// time, so that their counts, bounds and offsets arrive in three loads: 32 in
+// large batches, fewer in those that would leave warps idle.  Queries of more
+// than kFillLong values are left to the whole CTA, which reads eight values per
+// thread at a time.  Whole searches over 2^24 keys with 32 queries to every warp
+// and one warp to a query / now: 64 ranges of up to 20,000 values 1.47 / 0.10 ms,
+// 16 of up to 10^6 25.3 / 1.25 ms, 4,096 of up to 1,000 0.165 / 0.078 ms.
+constexpr int kFillThreads = 256;
+constexpr int kFillWarps = kFillThreads / 32;
+constexpr uint64_t kFillLong = 2048;
+
 template <typename K, typename V, bool SORT>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kFillThreads)
 range_fill_kernel(const unsigned char *__restrict__ leaves, const uint64_t *__restrict__ lb,
                   const uint64_t *__restrict__ cnt, const uint64_t *__restrict__ off, uint64_t nq,
-                  V *__restrict__ ids) {
+                  uint32_t per, V *__restrict__ ids) {
     using LG = LeafGeom<K, V>;
-    const int lane = threadIdx.x & 31;
-    const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-    const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    __shared__ unsigned s_long[kFillWarps];
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const uint64_t step = (uint64_t)kFillWarps * per;  // the CTA's queries of one round
+    bool more = false;
     auto value = [&](uint64_t p) {
         return __ldg(reinterpret_cast<const V *>(leaves + (p / LG::S) * LG::BS + kSectorBytes) + p % LG::S);
     };
-    for (uint64_t i0 = warp * 32; i0 < nq; i0 += nw * 32) {
-        const uint64_t i = i0 + lane;
-        const uint64_t mc = i < nq ? cnt[i] : 0, ml = i < nq ? lb[i] : 0, mo = i < nq ? off[i] : 0;
-        unsigned todo = __ballot_sync(0xffffffffu, mc != 0);
+    for (uint64_t b0 = blockIdx.x * step; b0 < nq; b0 += gridDim.x * step) {
+        const uint64_t i = b0 + w * per + lane;
+        const bool mine = lane < per && i < nq;
+        const uint64_t mc = mine ? cnt[i] : 0, ml = mine ? lb[i] : 0, mo = mine ? off[i] : 0;
+        more |= mc > kFillLong;
+        unsigned todo = __ballot_sync(0xffffffffu, mc != 0 && mc <= kFillLong);
         while (todo) {
             const int j = __ffs((int)todo) - 1;
             todo &= todo - 1;
-            const uint64_t c = __shfl_sync(0xffffffffu, mc, j), l = __shfl_sync(0xffffffffu, ml, j);
+            const uint32_t c = __shfl_sync(0xffffffffu, (uint32_t)mc, j);
+            const uint64_t l = __shfl_sync(0xffffffffu, ml, j);
             V *dst = ids + __shfl_sync(0xffffffffu, mo, j);
-            if (SORT && c > 1 && c <= (uint64_t)kWarpSortCap) {
+            if (SORT && c > 1 && c <= (uint32_t)kWarpSortCap) {
                 auto at = [&](uint32_t e) { return value(l + e); };
-                warp_sort_small<V>(at, dst, (uint32_t)c, lane);
+                warp_sort_small<V>(at, dst, c, (int)lane);
             } else {
-                for (uint64_t k = lane; k < c; k += 32) dst[k] = value(l + k);
+#pragma unroll 4
+                for (uint32_t k = lane; k < c; k += 32) dst[k] = value(l + k);
             }
         }
+    }
+    if (!__syncthreads_or(more)) return;
+    for (uint64_t b0 = blockIdx.x * step; b0 < nq; b0 += gridDim.x * step) {
+        const uint64_t i = b0 + threadIdx.x;  // step <= kFillThreads
+        const bool big = threadIdx.x < step && i < nq && cnt[i] > kFillLong;
+        const unsigned m = __ballot_sync(0xffffffffu, big);
+        if (lane == 0) s_long[w] = m;
+        __syncthreads();
+        for (int z = 0; z < kFillWarps; z++) {
+            for (unsigned todo = s_long[z]; todo; todo &= todo - 1) {
+                const uint64_t j = b0 + z * 32 + __ffs((int)todo) - 1;
+                const uint64_t c = cnt[j], l = lb[j];
+                V *dst = ids + off[j];
+                constexpr int U = 8;
+                uint64_t k = threadIdx.x;
+                for (; k + (U - 1) * kFillThreads < c; k += U * kFillThreads) {
+                    V v[U];
+#pragma unroll
+                    for (int u = 0; u < U; u++) v[u] = value(l + k + u * kFillThreads);
+#pragma unroll
+                    for (int u = 0; u < U; u++) dst[k + u * kFillThreads] = v[u];
+                }
+                for (; k < c; k += kFillThreads) dst[k] = value(l + k);
+            }
+        }
+        __syncthreads();
     }
 }
 
@@ -1405,12 +1445,15 @@ namespace {
 template <typename K, typename V>
 void range_fill(const bt_tree *t, const uint64_t *d_lb, const uint64_t *d_counts,
                 const uint64_t *d_offsets, uint64_t nq, V *ids, cudaStream_t s) {
-    const unsigned grid = (unsigned)std::min<uint64_t>((nq + 255) / 256, (uint64_t)sm_count() * 8);
+    const uint64_t ctas = (uint64_t)sm_count() * 8;
+    const uint32_t per = (uint32_t)std::min<uint64_t>(32, std::max<uint64_t>(1, nq / (ctas * kFillWarps)));
+    const uint64_t step = (uint64_t)kFillWarps * per;
+    const unsigned grid = (unsigned)std::min<uint64_t>((nq + step - 1) / step, ctas);
     const unsigned char *lv = (const unsigned char *)t->d_leaves;
     if (t->values_sorted)
-        range_fill_kernel<K, V, false><<<grid, 256, 0, s>>>(lv, d_lb, d_counts, d_offsets, nq, ids);
+        range_fill_kernel<K, V, false><<<grid, kFillThreads, 0, s>>>(lv, d_lb, d_counts, d_offsets, nq, per, ids);
     else
-        range_fill_kernel<K, V, true><<<grid, 256, 0, s>>>(lv, d_lb, d_counts, d_offsets, nq, ids);
+        range_fill_kernel<K, V, true><<<grid, kFillThreads, 0, s>>>(lv, d_lb, d_counts, d_offsets, nq, per, ids);
 }
 }  // namespace
 
