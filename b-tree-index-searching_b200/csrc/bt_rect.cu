@@ -301,9 +301,33 @@ rect_count_kernel(const __grid_constant__ DevTree t, const uint16_t *__restrict_
 // 719, 2^20 boxes 3066 / 2296; 2^20 points: 2^14 boxes 90 / 83).
 constexpr uint64_t kDirPointsPerBox = 128;
 
+// Stretches of entries without a key longer than this are listed, in pieces of
+// this many entries, for a launch of their own (code_dir_fill_kernel): points
+// crowded into a part of the plane leave most of the directory to a few warps.
+// 2^24 points, 2^17 boxes, whole searches with one launch / with both (descents):
+// points in a quarter of the plane 766 / 270 us (578), in 1/256 of it 946 / 286
+// (529).  The second launch costs 4 us, so directories of up to kDirOneLaunch
+// entries do without it (2^20 points in 1/4,096 of the plane: 127 / 94, 177).
+constexpr uint32_t kDirPiece = 4096;
+constexpr uint32_t kDirOneLaunch = 1u << 18;
+// Most pieces of a directory of nh + 1 entries: a stretch has one more than its
+// length gives, and is longer than a piece.
+constexpr uint32_t dir_pieces(uint32_t nh) { return 2 * (nh / kDirPiece + 1); }
+
+__global__ void __launch_bounds__(256)
+code_dir_fill_kernel(const uint32_t *__restrict__ n_pieces, const uint4 *__restrict__ pieces,
+                     uint32_t *__restrict__ dir) {
+    const uint32_t np = *n_pieces;
+    for (uint32_t p = blockIdx.x; p < np; p += gridDim.x) {
+        const uint4 f = pieces[p];  // first entry, entries, value
+        for (uint32_t k = threadIdx.x; k < f.y; k += 256) dir[f.x + k] = f.z;
+    }
+}
+
+// n_pieces null: nothing is listed.
 __global__ void __launch_bounds__(256)
 code_dir_kernel(const unsigned char *__restrict__ leaves, int stride, uint32_t n, int shift, uint32_t nh,
-                uint32_t *__restrict__ dir) {
+                uint32_t *__restrict__ dir, uint32_t *__restrict__ n_pieces, uint4 *__restrict__ pieces) {
     const int lane = threadIdx.x & 31;
     const uint32_t step = gridDim.x * blockDim.x;
     auto slot_of = [&](uint32_t i) -> uint32_t {  // entries up to this one start at or before key i
@@ -323,7 +347,16 @@ code_dir_kernel(const unsigned char *__restrict__ leaves, int stride, uint32_t n
             const int j = __ffs((int)wide) - 1;
             wide &= wide - 1;
             const uint32_t f = __shfl_sync(0xffffffffu, from, j), l = __shfl_sync(0xffffffffu, len, j);
-            for (uint32_t k = lane; k < l; k += 32) dir[f + k] = i0 + (uint32_t)j;
+            if (n_pieces && l > kDirPiece) {
+                const uint32_t np = (l + kDirPiece - 1) / kDirPiece;
+                uint32_t at = lane == 0 ? atomicAdd(n_pieces, np) : 0u;
+                at = __shfl_sync(0xffffffffu, at, 0);
+                for (uint32_t p = lane; p < np; p += 32)
+                    pieces[at + p] = make_uint4(f + p * kDirPiece, min(kDirPiece, l - p * kDirPiece),
+                                                i0 + (uint32_t)j, 0u);
+            } else {
+                for (uint32_t k = lane; k < l; k += 32) dir[f + k] = i0 + (uint32_t)j;
+            }
         }
     }
 }
@@ -550,14 +583,26 @@ bt_status rect_impl(const bt_tree *t, int mode, const uint16_t *x0, const uint16
     WsGuard g_dir(s);
     const int bits = std::min(22, std::max(8, bitlen64(t->n) - 3));  // four points or more to an entry
     bool by_dir = nr >= t->n / kDirPointsPerBox;
-    if (by_dir) by_dir = g_dir.alloc(((1ull << bits) + 1) * sizeof(uint32_t)) == BT_OK;
+    const uint32_t nh = 1u << bits;
+    const bool listed = nh > kDirOneLaunch;
+    const size_t db = ((size_t)(nh + 1) * sizeof(uint32_t) + 15) / 16 * 16;  // then the pieces and their number
+    const size_t fb = listed ? dir_pieces(nh) * sizeof(uint4) : 0;
+    if (by_dir) by_dir = g_dir.alloc(db + fb + sizeof(uint32_t)) == BT_OK;
     cudaError_t e = cudaSuccess;
     if (by_dir) {
         uint32_t *dir = g_dir.as<uint32_t>();
+        uint4 *pieces = listed ? reinterpret_cast<uint4 *>(g_dir.as<unsigned char>() + db) : nullptr;
+        uint32_t *n_pieces = listed ? reinterpret_cast<uint32_t *>(g_dir.as<unsigned char>() + db + fb) : nullptr;
+        if (listed) BT_CUDA(cudaMemsetAsync(n_pieces, 0, sizeof(uint32_t), s));
         const unsigned char *lv = (const unsigned char *)t->d_leaves;
         count_launch();
         code_dir_kernel<<<(unsigned)std::min<uint64_t>((t->n + 256) / 256, (uint64_t)sm_count() * 16), 256, 0, s>>>(
-            lv, LeafGeom<uint32_t, V>::BS, (uint32_t)t->n, 32 - bits, 1u << bits, dir);
+            lv, LeafGeom<uint32_t, V>::BS, (uint32_t)t->n, 32 - bits, nh, dir, n_pieces, pieces);
+        if (listed) {
+            count_launch();
+            code_dir_fill_kernel<<<std::min<unsigned>(dir_pieces(nh), (unsigned)sm_count() * 8), 256, 0, s>>>(
+                n_pieces, pieces, dir);
+        }
         count_launch();
         rect_dir_count_kernel<V>
             <<<(unsigned)std::min<uint64_t>((nr + 15) / 16, (uint64_t)sm_count() * 8), 256, 0, s>>>(
