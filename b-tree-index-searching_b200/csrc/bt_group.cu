@@ -554,14 +554,14 @@ bucket_count_kernel(const __grid_constant__ B q, uint64_t n, const __grid_consta
 }
 
 // Block 0: start = cursor = exclusive scan of total (start[nb] = n), and the
-// search's work items: every bucket's queries in equal slices of at most
-// kBucketSlice (item = bucket, first query, queries).  The others: first[b] =
+// search's work items: every bucket's queries in equal slices of at most `slice`
+// (item = bucket, first query, queries).  The others: first[b] =
 // leaf block of the first key at or above bucket b's first key (b = nb: of the
 // first key equal to the largest), so the first key at or above a query of
 // bucket b lies in blocks first[b] .. first[b + 1], at most bucket_blocks ones.
 template <typename K>
 __global__ void __launch_bounds__(1024)
-bucket_start_kernel(const __grid_constant__ DevTree t, const __grid_constant__ BucketMap map,
+bucket_start_kernel(const __grid_constant__ DevTree t, const __grid_constant__ BucketMap map, uint32_t slice,
                     const uint32_t *__restrict__ total, uint32_t *__restrict__ cursor,
                     uint32_t *__restrict__ first, uint4 *__restrict__ items,
                     uint32_t *__restrict__ n_items) {
@@ -585,7 +585,7 @@ bucket_start_kernel(const __grid_constant__ DevTree t, const __grid_constant__ B
 #pragma unroll
     for (int k = 0; k < PER; k++) {
         c[k] = i + k < nb ? total[i + k] : 0u;
-        sl[k] = (c[k] + kBucketSlice - 1) / kBucketSlice;
+        sl[k] = (c[k] + slice - 1) / slice;
         cs += c[k];
         ss += sl[k];
     }
@@ -1365,7 +1365,7 @@ bt_status bucket_impl(const bt_tree *t, const BucketMap &map, const B &q, uint64
         q, nq, map, total);
     count_launch();
     bucket_start_kernel<K><<<1 + ((map.last + 2) * 8 + 1023) / 1024, 1024, 0, s>>>(
-        t->dev, map, total, cursor, bp.first, bp.items, bp.n_items);
+        t->dev, map, bucket_slice(nq), total, cursor, bp.first, bp.items, bp.n_items);
     count_launch();
     constexpr uint64_t T = BucketSmem<K>::T;
     bucket_scatter_kernel<K, B><<<(unsigned)std::min<uint64_t>((nq + T - 1) / T, sms * 2), kBT,

@@ -301,14 +301,20 @@ struct BucketMap {
         return b == 0 ? 0ull : min + ((uint64_t)b << shift);
     }
 };
-// Most queries of one work item of the bucket search.
+// Most queries of one work item of the bucket search; fewer in a batch that falls
+// on few buckets, so that its items still fill the GPU's 296 CTAs (2^20 u64 keys,
+// 2^18 learned queries for 64 of them: 111 -> 67 us).
 constexpr uint32_t kBucketSlice = 16384;
+constexpr uint32_t kBucketMinSlice = 1024;
+inline uint32_t bucket_slice(uint64_t nq) {
+    return (uint32_t)std::min<uint64_t>(kBucketSlice, std::max<uint64_t>(kBucketMinSlice, nq / 512));
+}
 // What the passes of the bucket order leave for the search.
 struct BucketPlan {
     uint32_t *scratch;  // 2 * kMaxBuckets words
     uint32_t *first;    // leaf block where bucket b's keys start, b = 0 .. last; last + 1: of the largest key
     uint4 *items;       // work items: bucket, first slot, slots
-    uint32_t *n_items;  // at most kMaxBuckets + nq / kBucketSlice
+    uint32_t *n_items;  // at most kMaxBuckets + nq / bucket_slice(nq)
 };
 // d_q ordered by bucket into out_q (query i in slot pos[i]).  With d_hi, the
 // 2 nq bounds of the ranges [d_q[i], d_hi[i]]: d_q[i], then d_hi[i] + 1.
@@ -351,13 +357,13 @@ struct BucketWs {
     static size_t up256(size_t x) { return (x + 255) / 256 * 256; }
     static size_t bytes(uint64_t nq, uint32_t buckets, size_t key_bytes, size_t res_bytes, bool flags) {
         return up256(nq * key_bytes) + up256(nq * sizeof(uint32_t)) + up256(nq * res_bytes) +
-               (flags ? up256(nq) : 0) + (buckets + nq / kBucketSlice) * sizeof(uint4) +
+               (flags ? up256(nq) : 0) + (buckets + nq / bucket_slice(nq)) * sizeof(uint4) +
                (3 * kMaxBuckets + 64) * sizeof(uint32_t);
     }
     bt_status alloc(uint64_t nq, uint32_t buckets, size_t key_bytes, size_t res_bytes, bool flags) {
         const size_t kb = up256(nq * key_bytes), pb = up256(nq * sizeof(uint32_t));
         const size_t rb = up256(nq * res_bytes), fb = flags ? up256(nq) : 0;
-        max_items = buckets + nq / kBucketSlice;
+        max_items = buckets + nq / bucket_slice(nq);
         const bt_status st = ws.alloc(bytes(nq, buckets, key_bytes, res_bytes, flags));
         if (st != BT_OK) return st;
         q = ws.as<unsigned char>();

@@ -254,7 +254,7 @@ point_window_kernel(const __grid_constant__ DevTree t, const K *__restrict__ q,
 
 // ---- point search of a batch ordered by bucket (launch_buckets) ------------
 //
-// A CTA takes one work item: up to kBucketSlice queries of one bucket, whose
+// A CTA takes one work item: up to bucket_slice queries of one bucket, whose
 // leaf blocks lie between first[bucket] and first[bucket + 1].  It stages that
 // window of the deepest separator level that fits in its shared memory, 64-bit
 // separators as 32-bit offsets where their span allows it, so that one binary
@@ -281,7 +281,7 @@ using BktOut = std::conditional_t<BOUND, uint32_t, V>;
 // The qn queries of an item by their staged window: node = w0 + position in
 // the window of level wlvl, then the levels below it (lane quads, one line
 // per query and level), then the leaf block.
-template <typename K, typename V, typename W, int T, bool BOUND>
+template <typename K, typename V, typename W, int T, bool BOUND, bool KEEP>
 __device__ __forceinline__ void bucket_item(const DevTree &t, const W *s_win, uint32_t w0, uint32_t wm,
                                             int wlvl, K base, const K *__restrict__ q, uint32_t qn,
                                             BktOut<V, BOUND> *__restrict__ out,
@@ -329,7 +329,7 @@ __device__ __forceinline__ void bucket_item(const DevTree &t, const W *s_win, ui
         if constexpr (BOUND) {  // position of the first key at or above the query
             uint32_t w[U][8];
 #pragma unroll
-            for (int u = 0; u < U; u++) load_sector(leaves + (size_t)node[u] * LG::BS, w[u]);
+            for (int u = 0; u < U; u++) load_sector_as<KEEP>(leaves + (size_t)node[u] * LG::BS, w[u]);
 #pragma unroll
             for (int u = 0; u < U; u++) {
                 const K c = qv[u] < tmax ? qv[u] : tmax;
@@ -337,7 +337,7 @@ __device__ __forceinline__ void bucket_item(const DevTree &t, const W *s_win, ui
                 if (i < qn) out[i] = node[u] * (uint32_t)LG::S + count_below<K, LG::S>(w[u], c, false);
             }
         } else {
-            leaf_answers<K, V, U, sizeof(K) == 8>(leaves, node, qv, tmax, [&](int u, int l, V v, bool hit) {
+            leaf_answers<K, V, U, sizeof(K) == 8, KEEP>(leaves, node, qv, tmax, [&](int u, int l, V v, bool hit) {
                 const uint32_t i = i0 + u * T + l;
                 if (i < qn) {
                     out[i] = v;
@@ -348,7 +348,7 @@ __device__ __forceinline__ void bucket_item(const DevTree &t, const W *s_win, ui
     }
 }
 
-template <typename K, typename V, int T, bool BOUND>
+template <typename K, typename V, int T, bool BOUND, bool KEEP>
 __global__ void __launch_bounds__(T, 1024 / T)
 bucket_search_kernel(const __grid_constant__ DevTree t, const uint32_t *__restrict__ first,
                      const uint4 *__restrict__ items, const uint32_t *__restrict__ n_items,
@@ -382,14 +382,14 @@ bucket_search_kernel(const __grid_constant__ DevTree t, const uint32_t *__restri
 #pragma unroll 8
         for (uint32_t i = threadIdx.x; i < wm; i += T) s_win[win_slot(i)] = (uint32_t)(src[i] - base);
         __syncthreads();
-        bucket_item<K, V, uint32_t, T, BOUND>(t, s_win, w0, wm, wlvl, base, q + it.y, it.z, out + it.y,
+        bucket_item<K, V, uint32_t, T, BOUND, KEEP>(t, s_win, w0, wm, wlvl, base, q + it.y, it.z, out + it.y,
                                        found ? found + it.y : nullptr);
     } else if constexpr (sizeof(K) == 8) {
         uint64_t *s_win = reinterpret_cast<uint64_t *>(smem_raw);
 #pragma unroll 8
         for (uint32_t i = threadIdx.x; i < wm; i += T) s_win[win_slot(i)] = (uint64_t)src[i];
         __syncthreads();
-        bucket_item<K, V, uint64_t, T, BOUND>(t, s_win, w0, wm, wlvl, base, q + it.y, it.z, out + it.y,
+        bucket_item<K, V, uint64_t, T, BOUND, KEEP>(t, s_win, w0, wm, wlvl, base, q + it.y, it.z, out + it.y,
                                        found ? found + it.y : nullptr);
     }
 }
@@ -654,10 +654,10 @@ bt_status window_launch(const bt_tree *t, const void *d_q, const uint32_t *d_per
     return BT_OK;
 }
 
-template <typename K, typename V, int T, bool BOUND>
+template <typename K, typename V, int T, bool BOUND, bool KEEP = false>
 bt_status bucket_launch(const bt_tree *t, const BucketPlan &bp, uint64_t max_items, size_t smem,
                         const void *d_q, void *d_out, uint8_t *d_found, cudaStream_t s) {
-    auto fn = bucket_search_kernel<K, V, T, BOUND>;
+    auto fn = bucket_search_kernel<K, V, T, BOUND, KEEP>;
     bt_status st = set_smem(fn, smem);
     if (st != BT_OK) return st;
     count_launch();
@@ -676,6 +676,8 @@ bt_status bucket_cfg(const bt_tree *t, const BucketPlan &bp, uint64_t max_items,
     size_t m = t->bucket_blocks;
     while (win_words(m) * sizeof(uint32_t) > kBktWinBytes) m = (m >> LOGF) + 2;
     const size_t smem = std::max<size_t>(win_words(m) * sizeof(uint32_t), kBktWinMin);
+    if (t->bucket_blocks <= kKeepBlocks)
+        return bucket_launch<K, V, 512, BOUND, true>(t, bp, max_items, smem, d_q, d_out, d_found, s);
     // two CTAs per SM where two windows fit
     if (smem <= kBktWinBytes / 2) return bucket_launch<K, V, 512, BOUND>(t, bp, max_items, smem, d_q, d_out, d_found, s);
     return bucket_launch<K, V, 1024, BOUND>(t, bp, max_items, smem, d_q, d_out, d_found, s);

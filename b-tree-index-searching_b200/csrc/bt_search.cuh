@@ -424,6 +424,26 @@ __device__ __forceinline__ void load_sector(const void *p, uint32_t (&w)[8]) {
                  : "l"(p));
 }
 
+// The same, kept in L1 when KEEP.
+template <bool KEEP>
+__device__ __forceinline__ void load_sector_as(const void *p, uint32_t (&w)[8]) {
+    if constexpr (KEEP)
+        asm volatile("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                     : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]),
+                       "=r"(w[7])
+                     : "l"(p));
+    else
+        load_sector(p, w);
+}
+
+// Trees whose fullest bucket has up to so many leaf blocks (32 KB) are searched
+// by buckets through L1: a batch that falls on a few hundred keys reads the same
+// // lines from every SM, and the L2 slices that hold them bound it.  2^18 u64 keys,
+// 2^24 queries for 64 of them: point search 1.52 -> 0.38 ms, learned 2.19 -> 0.56.
+// Larger trees (2^27 u64 keys) are 2-4% slower that way, and 5-7% with both loads
+// in one kernel (registers).
+constexpr uint32_t kKeepBlocks = 512;
+
 // The first of a key sector's S keys equal to q, -1 if none (unused slots
 // hold all-ones keys, which a query above the largest key may equal).
 template <typename K, int S>
@@ -443,7 +463,7 @@ __device__ __forceinline__ int first_match(const uint32_t (&w)[8], K q, K tmax) 
 //     sector, as one request.
 // A quarter of the instructions of the form it replaces (four lanes per
 // query, 16 bytes each, combined by shuffles and ballots).
-template <typename K, typename V, int U, bool PAIR, typename Put>
+template <typename K, typename V, int U, bool PAIR, bool KEEP = false, typename Put>
 __device__ __forceinline__ void leaf_answers(const unsigned char *__restrict__ leaves,
                                              const uint32_t (&node)[U], const K (&qv)[U], K tmax, Put put) {
     using LG = LeafGeom<K, V>;
@@ -459,7 +479,7 @@ __device__ __forceinline__ void leaf_answers(const unsigned char *__restrict__ l
                 const int k = h * 16 + (lane >> 1);
                 const uint32_t nd = __shfl_sync(0xffffffffu, node[u], k);
                 qk[u][h] = __shfl_sync(0xffffffffu, qv[u], k);
-                load_sector(leaves + (size_t)nd * LG::BS + (lane & 1) * kSectorBytes, w[u][h]);
+                load_sector_as<KEEP>(leaves + (size_t)nd * LG::BS + (lane & 1) * kSectorBytes, w[u][h]);
             }
 #pragma unroll
         for (int u = 0; u < U; u++)
@@ -476,7 +496,7 @@ __device__ __forceinline__ void leaf_answers(const unsigned char *__restrict__ l
     } else {
         uint32_t w[U][8];
 #pragma unroll
-        for (int u = 0; u < U; u++) load_sector(leaves + (size_t)node[u] * LG::BS, w[u]);
+        for (int u = 0; u < U; u++) load_sector_as<KEEP>(leaves + (size_t)node[u] * LG::BS, w[u]);
         int at[U];
         V v[U];
 #pragma unroll
