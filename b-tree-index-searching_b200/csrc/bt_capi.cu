@@ -16,7 +16,7 @@ bt_status point_device(const bt_tree *t, int mode, const void *d_q, uint64_t nq,
         if (st != BT_ERR_OUT_OF_MEMORY) return st;
         cudaGetLastError();  // no room for the ordered copy: the direct search
     }
-    if (mode == BT_POINT_BASIC || t->n == 0 || (mode == BT_POINT_GROUPED && nq < kBktMinQueries))
+    if (mode == BT_POINT_BASIC || t->n == 0 || (mode == BT_POINT_GROUPED && !point_order_pays(t, nq)))
         return launch_point_search(t, d_q, nullptr, nq, d_out, s, d_found);
     if (learned) return launch_learned_search(t, d_q, nq, d_out, d_found, s);
     void *gq = nullptr;
@@ -84,7 +84,7 @@ bt_status count_device(const bt_tree *t, int mode, const void *d_lo, const void 
         if (st != BT_ERR_OUT_OF_MEMORY) return st;
         cudaGetLastError();
     }
-    if (mode == BT_RANGE_BASIC || t->n == 0 || nq < kOrderMinRanges)
+    if (mode == BT_RANGE_BASIC || t->n == 0 || !range_order_pays(t, nq))
         return launch_bounds(t, d_lo, d_hi, nullptr, nq, d_counts, d_lb, s);
     const int kind = mode == BT_RANGE_GROUPED_2D ? kPart2D : kPartZ;
     void *ga = nullptr, *gb = nullptr;

@@ -276,6 +276,8 @@ bt_status launch_learned_search(const bt_tree *t, const void *d_q, uint64_t nq, 
 // Whether the bucket search's shared memory holds every bucket's part of the
 // tree's learned index.
 bool learned_index_fits(const bt_tree *t);
+// The least batch that pays for the bucket order on the tree's learned index.
+uint64_t learned_least(const bt_tree *t);
 // The same for a batch that learned_buckets_pay for, ordered by bucket
 // (BT_ERR_OUT_OF_MEMORY when the workspace cannot be had).
 bt_status launch_learned_buckets(const bt_tree *t, const void *d_q, uint64_t nq, void *d_out,
@@ -393,13 +395,13 @@ static_assert(kMaxBuckets == 1 << 11, "bucket_map takes 11 bits");
 // Does nothing when d_unsorted (optional) has bit 0 set by then.
 bt_status launch_bucket_blocks(const bt_tree *t, const unsigned int *d_unsorted, uint32_t *d_blocks,
                                cudaStream_t s);
-// Least batches that are put into any order before the search; below them
-// the order costs more than it gives, whatever the mode asks for (2^20 point
-// queries, u32 keys, 2^20 / 2^26: 36 / 47 us directly, 65 / 77 grouped first;
-// 2^19 ranges 50 / 66 us directly, 108 / 127 grouped first).
-constexpr uint64_t kBktMinQueries = 1ull << 22;
-constexpr uint64_t kOrderMinRanges = 1ull << 20;
-constexpr uint64_t kLearnedMinQueries = 1ull << 18;
+// Whether a batch is large enough to be put into an order before the search, by
+// buckets or, where those do not serve and the mode asks for it, in groups.  Below
+// that the order costs more than it gives, whatever the mode asks for (2^20 point
+// queries, u32 keys, 2^20 / 2^26: 36 / 47 us directly, 65 / 77 grouped first; 2^19
+// ranges 50 / 66 us directly, 108 / 127 grouped first).
+bool point_order_pays(const bt_tree *t, uint64_t nq);
+bool range_order_pays(const bt_tree *t, uint64_t nr);
 // Whether a point batch is searched by buckets, and that search (workspace
 // from the pool; BT_ERR_OUT_OF_MEMORY when it cannot be had).
 bool bucket_search_pays(const bt_tree *t, uint64_t nq, cudaStream_t s);

@@ -53,6 +53,7 @@ struct LearnedState {
     unsigned long long *d_stats = nullptr;
     uint64_t bytes = 0;
     uint32_t bucket_segs = 0;  // most segments that the queries of one bucket can route to
+    uint64_t bucket_least = 0;  // least batch searched by buckets
     int shape = 1;  // search kernel shape (bt_learned_set_shape)
     LearnedDev dev;
 };
@@ -1525,6 +1526,28 @@ bt_status root_train(float *p, int H, const float *x, const float *y, uint32_t n
     return BT_OK;
 }
 
+// The direct kernel reads a code line for every query whose window spans units,
+// and a second one the further the windows reach; the bucket kernel does not care.
+// Direct / by buckets (us), by how many code lines beyond the first a window
+// spans on average over the keys (u64):
+//                            2^18      2^19      2^20       2^21       2^22
+//   0.0065  const gaps, 2^24  34 / 70   50 / 77   74 / 97   125 / 135  226 / 197
+//   0.023   lognormal, 2^20   41 / 80   60 / 85  102 / 106  176 / 143  316 / 216
+//   0.072   lognormal, 2^20   48 / 72   74 / 79  130 / 98   224 / 137
+//   0.14    lognormal, 2^24   56 / 80   88 / 88  152 / 116  262 / 154
+//   0.27    lognormal, 2^24   66 / 80  114 / 88  194 / 115
+//   0.53    lognormal, 2^26   90 / 95  158 / 101
+//   0.53    lognormal, 2^20   91 / 72  159 / 78
+//   1.8     lognormal, 2^24  165 / 81
+// (Batches for one single key: 33 us / 60 at 2^18, 67 / 97 at 2^20.)
+uint64_t least_batch(double extra_lines) {
+    return extra_lines >= 0.4     ? 1ull << 18
+           : extra_lines >= 0.2   ? 1ull << 19
+           : extra_lines >= 0.05  ? 1ull << 20
+           : extra_lines >= 0.015 ? 1ull << 21
+                                  : 1ull << 22;
+}
+
 template <typename K, typename V>
 bt_status train_impl(bt_tree *t, const bt_learned_config &cfg, cudaStream_t s,
                      bt_learned_report *rep) {
@@ -1818,6 +1841,18 @@ bt_status train_impl(bt_tree *t, const bt_learned_config &cfg, cudaStream_t s,
                 np * sizeof(float);
     (void)LG::S;
 
+    double esum = 0, lsum = 0;
+    uint64_t emax = 0;
+    for (uint64_t g = 0; g < nseg; g++) {
+        const SegRec &r = segs[g / kSegPerLine].s[g % kSegPerLine];
+        esum += r.eps;
+        emax = std::max<uint64_t>(emax, r.eps);
+        // window of 2 eps + 3 ranks: units it spans, then code lines
+        const double win_units = (2.0 * r.eps + 3.0) / kpu + 1.0;
+        lsum += (double)r.cnt * (1.0 + (win_units - 1.0) / kCodesPerLine);
+    }
+    const double code_lines = lsum / (double)n;
+    st->bucket_least = least_batch(code_lines - 1.0);
     if (rep) {
         std::memset(rep, 0, sizeof(*rep));
         rep->root_loss_initial = hl[0];
@@ -1826,20 +1861,9 @@ bt_status train_impl(bt_tree *t, const bt_learned_config &cfg, cudaStream_t s,
         rep->root_error_initial = herr[1];
         rep->num_segments = (uint32_t)nseg;
         rep->max_error = eps;
-        double esum = 0, lsum = 0;
-        uint64_t emax = 0;
-        for (uint64_t g = 0; g < nseg; g++) {
-            const SegLine &sl = segs[g / kSegPerLine];
-            const int k = (int)(g % kSegPerLine);
-            esum += sl.s[k].eps;
-            emax = std::max<uint64_t>(emax, sl.s[k].eps);
-            // window of 2 eps + 3 ranks: units it spans, then code lines
-            const double win_units = (2.0 * sl.s[k].eps + 3.0) / kpu + 1.0;
-            lsum += (double)sl.s[k].cnt * (1.0 + (win_units - 1.0) / kCodesPerLine);
-        }
         rep->eps_mean = nseg ? esum / (double)nseg : 0;
         rep->eps_max = emax;
-        rep->code_lines_mean = n ? lsum / (double)n : 0;
+        rep->code_lines_mean = code_lines;
         rep->index_bytes = st->bytes;
         rep->keys_per_unit = kpu;
         rep->train_ms = ms;
@@ -1861,6 +1885,8 @@ bt_status launch_learned_search(const bt_tree *t, const void *d_q, uint64_t nq, 
     return t->val_bytes == 4 ? learned_launch<uint64_t, uint32_t>(t, d_q, nq, d_out, d_found, s)
                              : learned_launch<uint64_t, uint64_t>(t, d_q, nq, d_out, d_found, s);
 }
+
+uint64_t learned_least(const bt_tree *t) { return t->learned->bucket_least; }
 
 bool learned_index_fits(const bt_tree *t) { return bucket_index_need(t) <= kBucketIndexMax; }
 

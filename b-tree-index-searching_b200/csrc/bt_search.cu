@@ -766,20 +766,11 @@ bt_status launch_point_search(const bt_tree *t, const void *d_q, const uint32_t 
                   : point_types<false>(t, d_q, d_perm, nq, d_out, d_found, s);
 }
 
-// Both ways timed at 2^14 to 2^28 keys, u32 and u64, 2^17 to 2^24 queries (us,
-// direct / by buckets):
-//                 2^21 queries   2^22          2^24
-//   u32, 2^14      52 / 68       97 / 91      381 / 247
-//   u32, 2^26      86 / 108     160 / 152     607 / 374
-//   u64, 2^18      81 / 97      155 / 141     604 / 423
-//   u64, 2^26     148 / 149     275 / 204    1056 / 544
-//   u64, 2^28     187 / 268     352 / 361    1305 / 808
-// The passes of the order cost some 70 us at 2^21 queries, and every query
-// pays for its share of the staged separators: eight per query (2^23 queries
-// at 2^28 u64 keys: 674 / 515) are still worth it.  Trees whose keys crowd
-// into few of the equal stretches (a bucket of over four times the average)
-// keep the direct search: their windows lie levels above the leaves.  So does
-// a stream under capture, whose graph then holds no allocation.
+// Trees whose keys crowd into few of the equal stretches (a bucket of over four
+// times the average) keep the direct search: their windows lie levels above the
+// leaves.  So does a stream under capture, whose graph then holds no allocation.
+// And the passes must pay for the separators staged: every query for eight
+// (2^23 queries at 2^28 u64 keys: 674 us directly, 515 by buckets).
 static bool buckets_suit(const bt_tree *t, uint64_t nq, uint64_t blocks_per_query, cudaStream_t s) {
     if (t->n == 0 || nq >= (1ull << 32) || nq < t->n_sectors / blocks_per_query) return false;
     const uint64_t buckets = bucket_map(t->min_key, t->max_key).last + 1;
@@ -790,31 +781,51 @@ static bool buckets_suit(const bt_tree *t, uint64_t nq, uint64_t blocks_per_quer
     return false;
 }
 
-bool bucket_search_pays(const bt_tree *t, uint64_t nq, cudaStream_t s) {
-    return nq >= kBktMinQueries && buckets_suit(t, nq, 8, s);
+// Point searches, direct / by buckets (us, whole calls on uniform queries):
+//                 2^21 queries   2^22       2^23       2^24
+//   u32, 2^16                    78 / 108   128 / 166  238 / 274
+//   u32, 2^18                    98 / 113   174 / 172  326 / 289
+//   u32, 2^22                   109 / 130   189 / 190  347 / 324
+//   u32, 2^23                   134 / 133   239 / 199  450 / 333
+//   u32, 2^26      98 / 108     166 / 163              607 / 392
+//   u64, 2^14                    93 / 141   164 / 240  308 / 400
+//   u64, 2^18                   132 / 148   240 / 246  458 / 422
+//   u64, 2^20      91 / 97      164 / 155   302 / 253  583 / 441
+//   u64, 2^26     137 / 149     249 / 213             1056 / 544
+// (u64, 2^18: 4 us a million queries one way or the other, but 352 / 132 where
+// they fall on 64 keys.)
+bool point_order_pays(const bt_tree *t, uint64_t nq) {
+    const uint64_t bytes = t->n_sectors * (uint64_t)leaf_stride(t->key_bytes, t->val_bytes);
+    if (bytes <= 1ull << 20) return false;  // in L1 without any order
+    return nq >= (t->key_bytes == 4 && bytes <= kPairLeafBytes ? 1ull << 23 : 1ull << 22);
 }
 
-// Learned searches, one query at a time / by buckets (us; u64 keys):
-//                 2^17 queries   2^18         2^20          2^24
-//   2^20 keys       57 / 57      97 / 59     209 / 87
-//   2^24            57 / 59     100 / 62     213 / 112
-//   2^28            61 / 91     106 / 100    230 / 143    1211 / 848
-// (the staged index is a seventh of the separators: no rule on keys per query).
-// Not where some bucket's part of the index exceeds the shared memory.
+bool bucket_search_pays(const bt_tree *t, uint64_t nq, cudaStream_t s) {
+    return point_order_pays(t, nq) && buckets_suit(t, nq, 8, s);
+}
+
+// Learned searches: how many queries pay for the order depends on how far the
+// direct kernel's rank windows reach (learned_least).
 bool learned_buckets_pay(const bt_tree *t, uint64_t nq, cudaStream_t s) {
-    return nq >= kLearnedMinQueries && buckets_suit(t, nq, ~0ull, s) && learned_index_fits(t);
+    return nq >= learned_least(t) && buckets_suit(t, nq, ~0ull, s) && learned_index_fits(t);
 }
 
 // Range bounds, direct / by buckets (us; the buckets take both bounds of a
-// range as queries of their own, so its width does not matter):
-//                          2^19 ranges   2^20        2^22
-//   u32, 2^20 keys          50 / 65      83 / 77    312 / 184
-//   u32, 2^26              66 / 90     113 / 109    409 / 227
-//   u32, 2^26, 100,000 keys wide
-//                           76 / 90     133 / 110    477 / 229
-//   u64, 2^26              105 / 109    176 / 142    654 / 331
+// range as queries of their own, so its width does not matter), uniform ranges
+// and (sorted ones):
+//                    2^20 ranges          1.5 * 2^20           2^21                 2^22
+//   u32, 2^20 keys   56 / 95 (48 / 87)    72 / 116 (62 / 98)   91 / 126 (76 / 113)  157 / 198 (126 / 178)
+//   u32, 2^24        77 / 110 (63 / 106) 105 / 130 (83 / 118) 132 / 147 (103 / 135) 236 / 217 (176 / 199)
+//   u32, 2^26        92 / 124 (80 / 119) 126 / 147 (108 / 140) 154 / 167 (130 / 158) 276 / 244 (229 / 230)
+//   u64, 2^20       100 / 107 (79 / 100) 144 / 125 (106 / 113) 179 / 158 (138 / 140) 332 / 245 (227 / 232)
+//   u64, 2^26       134 / 154 (114 / 153) 191 / 181 (158 / 176) 238 / 221 (192 / 214) 442 / 336 (343 / 327)
+// On few keys the buckets gain more (2^22 ranges from 256 of 2^20 u32 keys: 415 / 182).
+bool range_order_pays(const bt_tree *t, uint64_t nr) {
+    return nr >= (t->key_bytes == 4 ? 1ull << 22 : 3ull << 19);
+}
+
 bool bucket_bounds_pay(const bt_tree *t, uint64_t nr, cudaStream_t s) {
-    return nr >= kOrderMinRanges && nr < (1ull << 31) && t->n < (1ull << 32) && buckets_suit(t, 2 * nr, 8, s);
+    return range_order_pays(t, nr) && nr < (1ull << 31) && t->n < (1ull << 32) && buckets_suit(t, 2 * nr, 8, s);
 }
 
 namespace {

@@ -59,9 +59,10 @@ typedef enum bt_point_mode {
     BT_POINT_LEARNED = 2  /* through the tree's learned index (bt_learned_train); no
                              counterpart in the reference */
 } bt_point_mode;
-/* Results do not depend on the mode.  Large batches (2^22 queries; 2^18 learned
- * ones; 2^20 ranges) are ordered by key range inside the library whatever the
- * mode, in scratch from its memory pool (a key width, a value width, 4 bytes and,
+/* Results do not depend on the mode.  Large batches (from 2^22 queries, 2^18
+ * learned ones, 1.5 * 2^20 ranges on; more on small trees, with 4-byte keys and
+ * where the learned model is exact) are ordered by key range inside the library
+ * whatever the mode, in scratch from its memory pool (a key width, a value width, 4 bytes and,
  * with found flags, one more byte per query, for at most 2^26 queries, or as many
  * as the tree has leaf blocks, at a time; two key widths and 16 bytes per range,
  * for at most half as many ranges).  Without room for it, and on a stream under

@@ -32,7 +32,7 @@ def test_crowded_segments_take_no_full_descent(bt, orc, cuda, kt, vt, n, crowd, 
     with bt.Tree.build(torch.from_numpy(keys).to(cuda), torch.from_numpy(vals).to(cuda)) as t:
         t.learned_train(iterations=20, **target)
         for span in ((0, n), (at, at + crowd)):
-            q = keys[g.integers(*span, size=(1 << 20) + 77)]
+            q = keys[g.integers(*span, size=(1 << 22) + 77)]
             q[::5] += kt(1)
             q[:2] = [0, np.iinfo(kt).max]
             dq = torch.from_numpy(q).to(cuda)
