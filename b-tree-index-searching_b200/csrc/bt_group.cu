@@ -105,16 +105,17 @@ struct PassIO {
     P *p_out;
 };
 
-// The sort's buffers.  `vary` has a bit set where some key differs from the
-// first one: a pass whose digit has no such bit would change nothing and is
-// skipped (pass 0, which fills vary in, never is), so which buffers a pass
-// uses depends on how many are skipped.
+// The sort's buffers: the passes go back and forth between the output and one
+// copy, so that the last one ends in the output.  `vary` has a bit set where some
+// key differs from the first one: a pass whose digit has no such bit would change
+// nothing and is skipped (pass 0, which fills vary in, never is), so which of the
+// two a pass writes depends on how many run after it.
 template <typename K, typename P>
 struct SortIO {
     const K *in;
     const P *p_in;
-    K *tk[2], *out;
-    P *tp[2], *p_out;
+    K *tk, *out;
+    P *tp, *p_out;
     unsigned long long *vary;
     int passes;
 };
@@ -131,10 +132,11 @@ __device__ __forceinline__ bool sort_pass(const SortIO<K, P> &s, int p, PassIO<K
         before += k < p && runs;
         after += k > p && runs;
     }
-    io.a_in = before == 0 ? s.in : s.tk[(before - 1) & 1];
-    io.p_in = before == 0 ? s.p_in : s.tp[(before - 1) & 1];
-    io.a_out = after == 0 ? s.out : s.tk[before & 1];
-    io.p_out = after == 0 ? s.p_out : s.tp[before & 1];
+    const bool to_out = (after & 1) == 0;  // the pass before it, if any, wrote the other one
+    io.a_in = before == 0 ? s.in : to_out ? s.tk : s.out;
+    io.p_in = before == 0 ? s.p_in : to_out ? s.tp : s.p_out;
+    io.a_out = to_out ? s.out : s.tk;
+    io.p_out = to_out ? s.p_out : s.tp;
     io.b_in = nullptr;
     io.b_out = nullptr;
     return true;
@@ -1024,7 +1026,7 @@ bt_status radix_sort(const K *d_keys, const P *p_in, uint64_t n, int passes, K *
     const size_t kb = align256(n * sizeof(K)), pb = align256(n * sizeof(P));
     const size_t tb = align256(part_table_bytes(n, PartSmem<K, P, false>::T));
     WsGuard ws(s);
-    bt_status st = ws.alloc(256 + tb + 2 * (kb + pb));
+    bt_status st = ws.alloc(256 + tb + kb + pb);
     if (st != BT_OK) return st;
     unsigned char *w = ws.as<unsigned char>();
     using IO = SortIO<K, P>;
@@ -1036,10 +1038,8 @@ bt_status radix_sort(const K *d_keys, const P *p_in, uint64_t n, int passes, K *
     io.vary = reinterpret_cast<unsigned long long *>(w);
     io.passes = passes;
     uint32_t *table = reinterpret_cast<uint32_t *>(w + 256);
-    for (int i = 0; i < 2; i++) {
-        io.tk[i] = reinterpret_cast<K *>(w + 256 + tb + i * (kb + pb));
-        io.tp[i] = reinterpret_cast<P *>(w + 256 + tb + i * (kb + pb) + kb);
-    }
+    io.tk = reinterpret_cast<K *>(w + 256 + tb);
+    io.tp = reinterpret_cast<P *>(w + 256 + tb + kb);
     BT_CUDA(cudaMemsetAsync(io.vary, 0, sizeof(*io.vary), s));
     GroupKeyParams gp{kPartRadix, 0, 8};
     for (int p = 0; p < passes && st == BT_OK; p++)

@@ -232,9 +232,9 @@ bt_status launch_range_fill(const bt_tree *t, const uint64_t *d_lb, const uint64
                             const uint64_t *d_offsets, uint64_t nq, uint64_t max_count, void *d_ids,
                             cudaStream_t s);
 // Stable sort of n (key, value) pairs by key on the device: LSD radix sort
-// with 8-bit digits (key_bytes passes of the partition kernels, carrying the
-// input index), then one gather of the values.  Equal keys keep their input
-// order.  n < 2^32; outputs must not alias inputs.
+// with 8-bit digits (key_bytes passes of the partition kernels, the values
+// carried with their keys).  Equal keys keep their input order.  Scratch: one
+// copy of the pairs and a table.  n < 2^32; outputs must not alias inputs.
 bt_status launch_sort_pairs(int key_bytes, int value_bytes, const void *d_keys, const void *d_vals,
                             uint64_t n, void *out_keys, void *out_vals, cudaStream_t s);
 // Stable order of n 16-bit keys (the low halves of d_keys): d_perm[g] = the
