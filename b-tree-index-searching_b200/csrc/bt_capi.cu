@@ -107,9 +107,9 @@ bool valid_range_mode(int m) {
     return m == BT_RANGE_BASIC || m == BT_RANGE_GROUPED_2D || m == BT_RANGE_ZORDER;
 }
 
-// Host-buffer pipeline: chunks alternate between two streams; each chunk is
+// Host-buffer pipeline: chunks take turns on three streams; each chunk is
 // H2D -> kernels -> D2H on its stream, so copies of one chunk overlap the
-// kernels of the other.  `run` issues the kernels of one chunk.
+// kernels and copies of the others.  `run` issues the kernels of one chunk.
 template <typename Run>
 bt_status host_pipeline(const bt_tree *t, cudaStream_t caller, uint64_t nq, uint64_t chunk,
                         int n_in, const void *const *h_in, const size_t *in_w, void *h_out,
@@ -160,11 +160,17 @@ bt_status host_pipeline(const bt_tree *t, cudaStream_t caller, uint64_t nq, uint
 }
 
 uint64_t pipeline_chunk(uint64_t nq) {
-    // Eight chunks or more for large batches (copy/compute overlap), but not
-    // below 2M queries (per-chunk launch and grouping overheads; the grouped
-    // search's window kernel starts at 2^21 queries).
+    // Eight chunks for large batches (copy/compute overlap), but not below 2^20
+    // queries (a chunk's launches and copies cost some 30 us).  Both sides on one
+    // box, 2^26 u64 keys (us; bare copies both ways at once):
+    //                    8 chunks, 2^21 and up  2^20    16, 2^20  32, 2^19  copies
+    //   2^21 queries      827                   660     664       655        377
+    //   2^22             1187                  1125    1124      1176        710
+    //   2^24             3621                  3693    3924      4315       2707
+    //   2^22 learned     1304                  1197    1200      1487
+    //   2^22 ranges      1930                  1754    1765      1666
     const uint64_t c = (nq + 7) / 8;
-    return std::max<uint64_t>(c, std::min<uint64_t>(nq, 1ull << 21));
+    return std::max<uint64_t>(c, std::min<uint64_t>(nq, 1ull << 20));
 }
 
 }  // namespace
@@ -232,12 +238,13 @@ bt_status bt_point_search_host(const bt_tree *t, int mode, const void *h_queries
     return host_pipeline(t, (cudaStream_t)stream, nq, pipeline_chunk(nq), 1, ins, w, h_out,
                          (size_t)t->val_bytes,
                          [&](void *const *din, uint64_t m, void *dout, cudaStream_t s) {
-                             // A learned chunk goes direct: the copies bound it, and the
-                             // bucket passes beside them cost more than the search gains
-                             // (2^24 queries in 8 chunks over 2^28 u64 keys: 4.86-4.96 G
-                             // queries/s direct, 4.70 by buckets).
+                             // The copies bound a chunk, so the order of the larger ones
+                             // decides little.  2^28 u64 keys, 8 chunks, direct / by
+                             // buckets (ms): learned 2^24 queries 3.63, 3.62 / 3.69, 3.65,
+                             // 2^25 6.94, 6.84 / 6.71, 6.66; basic 2^25 6.80, 6.77 / 6.72,
+                             // 6.74, 2^26 13.2 / 12.9; 2^25 ranges 11.8 / 11.8.
                              return point_device(t, mode, din[0], m, dout, s, nullptr,
-                                                 mode != BT_POINT_LEARNED);
+                                                 mode != BT_POINT_LEARNED || m >= 1ull << 22);
                          });
 }
 
