@@ -78,10 +78,10 @@ __device__ __forceinline__ uint32_t group_key(K a, K b, const GroupKeyParams &p)
 // The keys are read twice, but no tile waits for another: a single pass with
 // decoupled look-back (Merrill & Garland 2016) walked back over most of the
 // hundreds of tiles in flight.  u32 pairs, 2^26: 1.09 ms a pass with the
-// look-back, 0.45 ms here (count 0.065, scatter 0.37; 1.3 GB, 0.2 ms at the
-// copy rate).  What bounds the scatter: 72 warp instructions a row of 32
-// items, 42 of them on the half-rate integer pipe, and 22 shared-memory
-// wavefronts, at 47% issue (32 warps per SM between barriers).  Smaller tiles
+// look-back, 0.46 ms here (count 0.075, scatter 0.38; 1.3 GB, 0.2 ms at the
+// copy rate).  What bounds the scatter: 102 warp instructions a row of 32
+// items, most of them on the half-rate integer pipe, and 22 shared-memory
+// wavefronts (32 warps per SM between barriers).  Smaller tiles
 // with three CTAs per SM: 0.47 ms; 256-thread CTAs: 0.51 and more.
 constexpr int kPT = 512;             // partition threads per CTA
 constexpr int kPWarps = kPT / 32;
@@ -89,7 +89,7 @@ constexpr int kPWarps = kPT / 32;
 // Items per thread of a tile, as many as two CTAs per SM have registers (64 a
 // thread) and shared memory for: a tile's stretch of a digit gets longer.
 // Whole sorts at 2^26, items per thread 8 / 12 / 16: u32 pairs 1.93 / 1.80 /
-// 1.78 ms, u64 pairs 5.8 / 7.2 / 7.3 ms.
+// 1.78 ms, u64 pairs 5.8 / 7.2 / 7.3 ms (with votes 0.07 ms faster than now's).
 template <int ITEM_BYTES>
 __host__ __device__ constexpr int part_ipt() {
     return ITEM_BYTES <= 8 ? 16 : ITEM_BYTES <= 12 ? 12 : 8;
@@ -287,24 +287,19 @@ struct PartSmem {
 };
 
 // The lanes whose 8-bit digit equals this lane's, among those with `valid`
-// (0 for the others): one vote per bit, four instructions each (the compiler's
-// own form of the same took six).  The whole sort of 2^26 u32 pairs: 3.05 ms
-// with __match_any_sync, whose time grows with the number of distinct digits,
-// 2.0 with the votes left to the compiler, 1.95 with a shared-memory word per
-// digit that lanes set their bit in (conflicts), 1.82 with these.
+// (0 for the others): a vote per bit, from which every lane whose bit is another
+// is dropped (vote xor this lane's bit in all places).  The whole sort of 2^26 u32
+// pairs: 3.05 ms with __match_any_sync, whose time grows with the number of
+// distinct digits, 1.95 with a shared-memory word per digit that lanes set their
+// bit in (conflicts), 1.93 with the bit made a mask by a subtraction, 2.03 with a
+// branch on it, 1.85 like this.
 template <bool ALL>
 __device__ __forceinline__ unsigned same_digit(uint32_t d, bool valid) {
     unsigned m = ALL ? 0xffffffffu : __ballot_sync(0xffffffffu, valid);
 #pragma unroll
     for (int b = 0; b < 8; b++) {
-        asm("{\n\t.reg .pred p;\n\t.reg .b32 t, v;\n\t"
-            "and.b32 t, %1, %2;\n\t"
-            "setp.ne.u32 p, t, 0;\n\t"
-            "vote.sync.ballot.b32 v, p, 0xffffffff;\n\t"
-            "@!p not.b32 v, v;\n\t"
-            "and.b32 %0, %0, v;\n\t}"
-            : "+r"(m)
-            : "r"(d), "r"(1u << b));
+        const int mine = (int)(d << (31 - b)) >> 31;  // this lane's bit in all 32 places
+        m &= ~(__ballot_sync(0xffffffffu, mine < 0) ^ (unsigned)mine);
     }
     return m;
 }
