@@ -16,7 +16,8 @@
 // A point query's leaf block -- key sector and value sector side by side, one
 // 64-byte DRAM access -- is read by one thread or a lane pair (leaf_answers),
 // so a hit costs one HBM round trip.  2^20 u32 keys, 2^20 queries (in L2):
-// 36 -> 25.8 us against four lanes per query; what is left is the instruction
+// 36 -> 25.8 us a call against four lanes per query, 34.9 -> 23.5 with the padded
+// window and two CTAs per SM; what is left is the instruction
 // issue of the shared-memory search and of the one separator line below it.
 #include <map>
 #include <mutex>
@@ -767,8 +768,14 @@ bt_status launch_point_search(const bt_tree *t, const void *d_q, const uint32_t 
 }
 
 // Trees whose keys crowd into few of the equal stretches (a bucket of over four
-// times the average) keep the direct search: their windows lie levels above the
-// leaves.  So does a stream under capture, whose graph then holds no allocation.
+// times the average) keep the direct search: the windows of the full ones lie
+// levels above the leaves.  Half the keys in 1 / 2R of the range, so that the
+// fullest bucket is R times the average one, direct / by buckets (us):
+//   u64, 2^26, 2^22 queries   R 1.5 250 / 240   2.5 250 / 243   3.5 248 / 287   6.5 250 / 282
+//              2^24 queries         898 / 707       898 / 689       898 / 730       899 / 857
+//              2^22 ranges          392 / 405       390 / 399       391 / 442       390 / 487
+//   u64, 2^24, 2^22 queries         223 / 218       222 / 213       224 / 217  16.6 225 / 256
+// (learned batches gain up to R 16, where their index fits: 1079 / 768.)  So does a stream under capture, whose graph then holds no allocation.
 // And the passes must pay for the separators staged: every query for eight
 // (2^23 queries at 2^28 u64 keys: 674 us directly, 515 by buckets).
 static bool buckets_suit(const bt_tree *t, uint64_t nq, uint64_t blocks_per_query, cudaStream_t s) {

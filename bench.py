@@ -813,7 +813,6 @@ def run_ours(args):
     clocks.start()
     at = importlib.import_module(PKG + ".autotune")
     p_lanes, p_rounds, _ = at.tune(tree, dq, mode="basic", repeats=3)
-    _, l_shape, l_tune_ms = at.tune(tree, dq, mode="learned", repeats=3)
     for _ in range(max(args.warmup, 3)):
         search_learned()
     torch.cuda.synchronize(device)
@@ -838,7 +837,6 @@ def run_ours(args):
     ms = max_over_ranks(statistics.mean(step_ms), dist, device)
     value = world * nq / (ms / 1000.0)
     extra, fallback = tree.learned_last_stats()
-    extra_lines = tree.learned_last_lines()
 
     # ---- the plain tree search of the same batch ----------------------------
     for _ in range(2):
@@ -974,9 +972,7 @@ def run_ours(args):
                                                   "root_loss_initial", "root_loss_final",
                                                   "code_lines_mean", "index_bytes",
                                                   "keys_per_unit", "train_ms")},
-            "learned_stats": {"extra_unit_reads": extra, "full_descents": fallback,
-                              "extra_code_lines": extra_lines},
-            "learned_shape": {"shape": l_shape, "autotune_ms": l_tune_ms},
+            "learned_stats": {"extra_unit_reads": extra, "full_descents": fallback},
             "cpu_baseline": cpu,
             "cpu_sample_matches_gpu": checked,
             "clocks": clk,
@@ -1020,8 +1016,7 @@ def learned_kernel_section(args, device, bt, flush, stream):
         extra, fallback = tree.learned_last_stats()
         return {"keys": len(keys), "queries": len(q), "segments": rep["num_segments"],
                 "eps_max": rep["eps_max"], "ms": ms, "equals_plain": bool(torch.equal(out, ref)),
-                "extra_unit_reads": extra, "full_descents": fallback,
-                "extra_code_lines": tree.learned_last_lines()}
+                "extra_unit_reads": extra, "full_descents": fallback}
     finally:
         tree.close()
 

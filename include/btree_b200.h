@@ -270,7 +270,7 @@ BT_API bt_status bt_range_search(const bt_tree *tree, int mode, const void *d_lo
  * total is known (and not 0), alloc(ctx, total) is called on this thread, with
  * the tree's device current, and returns device memory for `total` values, or
  * NULL (the call then ends with BT_ERR_OUT_OF_MEMORY, counts, offsets and
- * *h_total filled).  Against a first bt_range_search for the total and a
+ * *h_total filled).  alloc must not throw and leaves the device current.  Against a first bt_range_search for the total and a
  * second one for the IDs, the ranges are counted once.
  */
 typedef void *(*bt_ids_alloc)(void *ctx, uint64_t total);
@@ -378,7 +378,8 @@ typedef struct bt_learned_report {
     uint64_t eps_max;         /* largest measured segment bound (FP32 search arithmetic) */
     double eps_mean;          /* mean measured segment bound */
     double code_lines_mean;   /* mean code lines a query's window spans (over the keys) */
-    uint64_t index_bytes;     /* device bytes of the model, segment lines and codes */
+    uint64_t index_bytes;     /* device bytes of the model, segment lines and codes (beside them
+                                 the large batches' bucket table: 8 KB at most) */
     uint32_t keys_per_unit;   /* keys in one 128-byte leaf unit */
     uint32_t pad;
     double train_ms;          /* device time of the whole build */
@@ -397,10 +398,11 @@ BT_API bt_status bt_learned_train(bt_tree *tree, const bt_learned_config *cfg, v
 BT_API bt_status bt_point_search_learned(const bt_tree *tree, const void *d_queries, uint64_t nq,
                                          void *d_out, void *stream);
 
-/* Shape of the learned search kernel (one CTA per SM): 1 = 1024-thread CTAs
- * (the default), 2 = 768, 3 = 640, 4 = 512.  Fewer threads leave more
+/* Shape of the direct learned search kernel (one CTA per SM): 1 = 1024-thread
+ * CTAs (the default), 2 = 768, 3 = 640, 4 = 512.  Fewer threads leave more
  * registers to each.  Results do not depend on it; the autotuner picks the
- * fastest. */
+ * fastest.  Large batches (see bt_point_mode) run in another kernel, which has
+ * one shape. */
 BT_API bt_status bt_learned_set_shape(bt_tree *tree, uint32_t shape);
 
 /* Counters of the last learned search on this tree: leaf units read beyond
@@ -411,7 +413,8 @@ BT_API bt_status bt_learned_last_stats(const bt_tree *tree, uint64_t *extra_unit
 
 /* Code lines the last learned search on this tree counted beyond each
  * query's first (queries whose rank window continues into a neighbouring
- * line and whose count had to go on there). */
+ * line and whose count had to go on there).  Large batches (see bt_point_mode)
+ * search their lines in shared memory and count none. */
 BT_API bt_status bt_learned_last_lines(const bt_tree *tree, uint64_t *extra_code_lines);
 
 /*
