@@ -1799,8 +1799,6 @@ bt_status train_impl(bt_tree *t, const bt_learned_config &cfg, cudaStream_t s,
     count_launch();
     seg_first_kernel<<<(map.last + 2 + 255) / 256, 256, 0, s>>>(st->d_seg, (uint32_t)nseg, map,
                                                                 st->d_seg_first);
-    BT_CUDA(cudaMemcpyAsync(seg_first.data(), st->d_seg_first, seg_first.size() * sizeof(uint32_t),
-                            cudaMemcpyDeviceToHost, s));
 
     // ---- unit thresholds
     const uint64_t ncl = units > 1 ? (units - 1 + kCodesPerLine - 1) / kCodesPerLine : 0;
@@ -1815,6 +1813,8 @@ bt_status train_impl(bt_tree *t, const bt_learned_config &cfg, cudaStream_t s,
     std::vector<SegLine> segs(nls);
     BT_CUDA(cudaMemcpyAsync(herr, err, sizeof(herr), cudaMemcpyDeviceToHost, s));
     BT_CUDA(cudaMemcpyAsync(segs.data(), st->d_seg, nls * sizeof(SegLine), cudaMemcpyDeviceToHost, s));
+    BT_CUDA(cudaMemcpyAsync(seg_first.data(), st->d_seg_first, seg_first.size() * sizeof(uint32_t),
+                            cudaMemcpyDeviceToHost, s));
     BT_CUDA(cudaStreamSynchronize(s));
     float ms = 0.f;
     cudaEventElapsedTime(&ms, e0, e1);

@@ -618,7 +618,7 @@ bt_status point_launch_t(const bt_tree *t, const void *d_q, const uint32_t *d_pe
 
 // Leaf arrays above this are read by lane pairs also with 4-byte keys: a block
 // that comes from DRAM is then one request for both sectors (2^26 keys, 2^21
-// queries: 80 us; a thread per query 110; four lanes per query 84), where one
+// queries: 80 us a call; a thread per query 110; four lanes per query 84), where one
 // from L2 is faster by a thread (2^20 keys, 2^20 queries: 25.8 us; pairs 28.0;
 // four lanes 36).  The lines cross between 2^23 and 2^24 keys (64 / 128 MiB).
 constexpr size_t kPairLeafBytes = 64ull << 20;
