@@ -775,9 +775,10 @@ bt_status launch_point_search(const bt_tree *t, const void *d_q, const uint32_t 
 //              2^24 queries         898 / 707       898 / 689       898 / 730       899 / 857
 //              2^22 ranges          392 / 405       390 / 399       391 / 442       390 / 487
 //   u64, 2^24, 2^22 queries         223 / 218       222 / 213       224 / 217  16.6 225 / 256
-// (learned batches gain up to R 16, where their index fits: 1079 / 768.)  So does a stream under capture, whose graph then holds no allocation.
-// And the passes must pay for the separators staged: every query for eight
-// (2^23 queries at 2^28 u64 keys: 674 us directly, 515 by buckets).
+// (learned batches gain up to R 16, where their index fits: 1079 / 768.)  So does
+// a stream under capture, whose graph then holds no allocation.  And the passes
+// must pay for the separators staged: every query for eight leaf blocks (2^23
+// queries at 2^28 u64 keys: 674 us directly, 515 by buckets).
 static bool buckets_suit(const bt_tree *t, uint64_t nq, uint64_t blocks_per_query, cudaStream_t s) {
     if (t->n == 0 || nq >= (1ull << 32) || nq < t->n_sectors / blocks_per_query) return false;
     const uint64_t buckets = bucket_map(t->min_key, t->max_key).last + 1;

@@ -438,7 +438,7 @@ __device__ __forceinline__ void load_sector_as(const void *p, uint32_t (&w)[8]) 
 
 // Trees whose fullest bucket has up to so many leaf blocks (32 KB) are searched
 // by buckets through L1: a batch that falls on a few hundred keys reads the same
-// // lines from every SM, and the L2 slices that hold them bound it.  2^18 u64 keys,
+// lines from every SM, and the L2 slices that hold them bound it.  2^18 u64 keys,
 // 2^24 queries for 64 of them: point search 1.52 -> 0.38 ms, learned 2.19 -> 0.56.
 // Larger trees (2^27 u64 keys) are 2-4% slower that way, and 5-7% with both loads
 // in one kernel (registers).
