@@ -16,7 +16,8 @@ bt_status point_device(const bt_tree *t, int mode, const void *d_q, uint64_t nq,
         if (st != BT_ERR_OUT_OF_MEMORY) return st;
         cudaGetLastError();  // no room for the ordered copy: the direct search
     }
-    if (mode == BT_POINT_BASIC || t->n == 0 || (mode == BT_POINT_GROUPED && !point_order_pays(t, nq)))
+    if (mode == BT_POINT_BASIC || t->n == 0 ||
+        (mode == BT_POINT_GROUPED && !(scratch && point_order_pays(t, nq))))
         return launch_point_search(t, d_q, nullptr, nq, d_out, s, d_found);
     if (learned) return launch_learned_search(t, d_q, nq, d_out, d_found, s);
     void *gq = nullptr;

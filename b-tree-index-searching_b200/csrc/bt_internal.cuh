@@ -205,7 +205,7 @@ __host__ __device__ inline int bitlen64(uint64_t v) {
 
 // The point search behind bt_point_search (arguments checked, the tree's device
 // current, the learned counters reset).  `scratch`: whether it may order a large
-// batch by bucket.
+// batch, by bucket or in groups.
 bt_status point_device(const bt_tree *t, int mode, const void *d_q, uint64_t nq, void *d_out,
                        cudaStream_t s, uint8_t *d_found, bool scratch);
 // Host launchers implemented in the .cu files.

@@ -7,7 +7,7 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("mode,batch", [("basic", 1 << 22), ("learned", 1 << 22)])
+@pytest.mark.parametrize("mode,batch", [("basic", 1 << 22), ("grouped", 1 << 22), ("learned", 1 << 22)])
 @pytest.mark.parametrize("room", [0, 1])
 def test_scratch_within_the_budget(bt, cuda, mode, batch, room):
     import torch
