@@ -1539,13 +1539,14 @@ bt_status root_train(float *p, int H, const float *x, const float *y, uint32_t n
 //   0.53    lognormal, 2^26   90 / 95  158 / 101
 //   0.53    lognormal, 2^20   91 / 72  159 / 78
 //   1.8     lognormal, 2^24  165 / 81
-// (Batches for one single key: 33 us / 60 at 2^18, 67 / 97 at 2^20.)
+// (Batches for one single key: 33 us / 60 at 2^18, 67 / 97 at 2^20.)  Where one
+// segment holds most keys the direct kernel may take twice its time, all SMs
+// waiting for its line: constant gaps, 2^20 keys, 2^21 queries 227 / 112.
 uint64_t least_batch(double extra_lines) {
     return extra_lines >= 0.4     ? 1ull << 18
            : extra_lines >= 0.2   ? 1ull << 19
            : extra_lines >= 0.05  ? 1ull << 20
-           : extra_lines >= 0.015 ? 1ull << 21
-                                  : 1ull << 22;
+                                  : 1ull << 21;
 }
 
 template <typename K, typename V>

@@ -801,8 +801,15 @@ static bool buckets_suit(const bt_tree *t, uint64_t nq, uint64_t blocks_per_quer
 //   u64, 2^20      91 / 97      164 / 155   302 / 253  583 / 441
 //   u64, 2^26     137 / 149     249 / 213             1056 / 544
 // (u64, 2^18: 4 us a million queries one way or the other, but 352 / 132 where
-// they fall on 64 keys.)
+// they fall on 64 keys.)  The SMs of a direct u64 search of a tree of a few leaf
+// blocks wait for the same L2 lines:
+//   blocks           5          13         25        50        100       200
+//   2^20 queries    37 / 66    96 / 66    70 / 60   51 / 62   33 / 70   25 / 62
+//   2^21            68 / 90   182 / 86   133 / 80   92 / 84   59 / 88   43 / 82
+//   2^22           125 / 133  354 / 125  256 / 119 174 / 121 108 / 131  74 / 123
+// (u32, 13 to 25 blocks: 45 / 88 at 2^22.)
 bool point_order_pays(const bt_tree *t, uint64_t nq) {
+    if (t->key_bytes == 8 && t->n_sectors > 8 && t->n_sectors <= 64) return nq >= 1ull << 21;
     const uint64_t bytes = t->n_sectors * (uint64_t)leaf_stride(t->key_bytes, t->val_bytes);
     if (bytes <= 1ull << 20) return false;  // in L1 without any order
     return nq >= (t->key_bytes == 4 && bytes <= kPairLeafBytes ? 1ull << 23 : 1ull << 22);
@@ -827,8 +834,14 @@ bool learned_buckets_pay(const bt_tree *t, uint64_t nq, cudaStream_t s) {
 //   u32, 2^26        92 / 124 (80 / 119) 126 / 147 (108 / 140) 154 / 167 (130 / 158) 276 / 244 (229 / 230)
 //   u64, 2^20       100 / 107 (79 / 100) 144 / 125 (106 / 113) 179 / 158 (138 / 140) 332 / 245 (227 / 232)
 //   u64, 2^26       134 / 154 (114 / 153) 191 / 181 (158 / 176) 238 / 221 (192 / 214) 442 / 336 (343 / 327)
-// On few keys the buckets gain more (2^22 ranges from 256 of 2^20 u32 keys: 415 / 182).
+// On few keys the buckets gain more (2^22 ranges from 256 of 2^20 u32 keys: 415 / 182),
+// and on few leaf blocks, whose lines all SMs then wait for:
+//   blocks                 7         13        25        50       100       200
+//   2^20 ranges, u32    80 / 58  188 / 58  170 / 58  117 / 62   74 / 62   45 / 64
+//   2^20 ranges, u64   166 / 68  281 / 66  207 / 66  141 / 66   86 / 70   66 / 68
+//   2^19, u32           45 / 52   98 / 49   90 / 49   64 / 49   41 / 53
 bool range_order_pays(const bt_tree *t, uint64_t nr) {
+    if (t->n_sectors <= 128) return nr >= 1ull << 20;
     return nr >= (t->key_bytes == 4 ? 1ull << 22 : 3ull << 19);
 }
 

@@ -60,8 +60,9 @@ typedef enum bt_point_mode {
                              counterpart in the reference */
 } bt_point_mode;
 /* Results do not depend on the mode.  Large batches (from 2^22 queries, 2^18
- * learned ones, 1.5 * 2^20 ranges on; more on small trees, with 4-byte keys and
- * where the learned model is exact) are ordered by key range inside the library
+ * learned ones, 1.5 * 2^20 ranges on; half as many on trees of a few leaf blocks,
+ * more on other small trees, with 4-byte keys and where the learned model is
+ * exact) are ordered by key range inside the library
  * whatever the mode, in scratch from its memory pool (a key width, a value width, 4 bytes and,
  * with found flags, one more byte per query, for at most 2^26 queries, or as many
  * as the tree has leaf blocks, at a time; two key widths and 16 bytes per range,

@@ -9,7 +9,10 @@ pytestmark = pytest.mark.gpu
 
 POINT = [  # key type, keys, first ordered batch (None: never)
     (np.uint32, 1 << 16, None), (np.uint32, 1 << 20, 1 << 23), (np.uint32, 3 << 22, 1 << 22),
-    (np.uint64, 1 << 16, None), (np.uint64, 1 << 18, 1 << 22)]
+    (np.uint64, 1 << 16, None), (np.uint64, 1 << 18, 1 << 22),
+    # a few leaf blocks: 8, 9, 64 and 65 of u64 keys, 16 of u32 keys
+    (np.uint64, 32, None), (np.uint64, 33, 1 << 21), (np.uint64, 256, 1 << 21), (np.uint64, 257, None),
+    (np.uint32, 128, None)]
 
 
 def _tree(bt, torch, cuda, kt, n):
@@ -37,11 +40,13 @@ def test_point_lines(bt, cuda, kt, n, line, mode):
             assert torch.equal(got.view(it), torch.where(q % 3 == 0, q // 3, -1).to(it))
 
 
-@pytest.mark.parametrize("kt,line", [(np.uint32, 1 << 22), (np.uint64, 3 << 19)])
+@pytest.mark.parametrize("kt,n,line", [(np.uint32, 1 << 20, 1 << 22), (np.uint64, 1 << 20, 3 << 19),
+                                       (np.uint32, 3, 1 << 20), (np.uint32, 1024, 1 << 20),
+                                       (np.uint32, 1025, 1 << 22), (np.uint64, 512, 1 << 20),
+                                       (np.uint64, 513, 3 << 19)])
 @pytest.mark.parametrize("mode", ["basic", "2d", "zorder"])
-def test_range_lines(bt, cuda, kt, line, mode):
+def test_range_lines(bt, cuda, kt, n, line, mode):
     import torch
-    n = 1 << 20
     t, it = _tree(bt, torch, cuda, kt, n)
     with t:
         for nr in (line - 1, line):
@@ -52,7 +57,7 @@ def test_range_lines(bt, cuda, kt, line, mode):
             assert torch.equal(got.view(torch.int64), want.to(torch.int64))
 
 
-@pytest.mark.parametrize("gap,max_error,line", [("even", 2, 1 << 22), ("random", 4, 1 << 21),
+@pytest.mark.parametrize("gap,max_error,line", [("even", 2, 1 << 21), ("random", 4, 1 << 21),
                                                 ("random", 20, 1 << 20), ("random", 80, 1 << 19),
                                                 ("random", 400, 1 << 18)])
 def test_learned_lines(bt, cuda, gap, max_error, line):
