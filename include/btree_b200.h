@@ -60,7 +60,7 @@ typedef enum bt_point_mode {
                              counterpart in the reference */
 } bt_point_mode;
 /* Results do not depend on the mode.  Large batches (from 2^22 queries, 2^18
- * learned ones, 1.5 * 2^20 ranges on; half as many on trees of a few leaf blocks,
+ * learned ones, 1.5 * 2^20 ranges on; fewer on trees of a few leaf blocks,
  * more on other small trees, with 4-byte keys and where the learned model is
  * exact) are ordered by key range inside the library
  * whatever the mode, in scratch from its memory pool (a key width, a value width, 4 bytes and,
