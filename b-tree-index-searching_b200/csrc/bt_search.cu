@@ -807,9 +807,12 @@ static bool buckets_suit(const bt_tree *t, uint64_t nq, uint64_t blocks_per_quer
 //   2^20 queries    37 / 66    96 / 66    70 / 60   51 / 62   33 / 70   25 / 62
 //   2^21            68 / 90   182 / 86   133 / 80   92 / 84   59 / 88   43 / 82
 //   2^22           125 / 133  354 / 125  256 / 119 174 / 121 108 / 131  74 / 123
-// (u32, 13 to 25 blocks: 45 / 88 at 2^22.)
+// (u32, 13 to 25 blocks: 45 / 88 at 2^22.)  75 blocks, 2^24 queries: uniform 452 / 350,
+// Zipf 729 / 346; 250: 284 / 344, 279 / 350.  Larger ones up to 1 MiB lose only where a
+// batch falls on neighbouring keys (64 of them, 2^22 queries: 328 / 130).
 bool point_order_pays(const bt_tree *t, uint64_t nq) {
-    if (t->key_bytes == 8 && t->n_sectors > 8 && t->n_sectors <= 64) return nq >= 1ull << 21;
+    if (t->key_bytes == 8 && t->n_sectors > 8 && t->n_sectors <= 128)
+        return nq >= (t->n_sectors <= 64 ? 1ull << 21 : 1ull << 22);
     const uint64_t bytes = t->n_sectors * (uint64_t)leaf_stride(t->key_bytes, t->val_bytes);
     if (bytes <= 1ull << 20) return false;  // in L1 without any order
     return nq >= (t->key_bytes == 4 && bytes <= kPairLeafBytes ? 1ull << 23 : 1ull << 22);

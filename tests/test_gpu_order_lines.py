@@ -10,8 +10,9 @@ pytestmark = pytest.mark.gpu
 POINT = [  # key type, keys, first ordered batch (None: never)
     (np.uint32, 1 << 16, None), (np.uint32, 1 << 20, 1 << 23), (np.uint32, 3 << 22, 1 << 22),
     (np.uint64, 1 << 16, None), (np.uint64, 1 << 18, 1 << 22),
-    # a few leaf blocks: 8, 9, 64 and 65 of u64 keys, 16 of u32 keys
-    (np.uint64, 32, None), (np.uint64, 33, 1 << 21), (np.uint64, 256, 1 << 21), (np.uint64, 257, None),
+    # a few leaf blocks: 8, 9, 64, 65, 128 and 129 of u64 keys, 16 of u32 keys
+    (np.uint64, 32, None), (np.uint64, 33, 1 << 21), (np.uint64, 256, 1 << 21), (np.uint64, 257, 1 << 22),
+    (np.uint64, 512, 1 << 22), (np.uint64, 513, None),
     (np.uint32, 128, None)]
 
 
